@@ -8,111 +8,145 @@
 // 2 PP|QQ, 3 QQ|PP): R_t = rho1^T T_t rho2 with rho1 the symmetric band
 // density of (a,c) in basis A_t and rho2 that of (b,d) in basis B_t.  The
 // direct pair potential Kd_t[(b,d)] (factor.cu; the convol case 1 of T_t
-// with rho2) is the potential rho2 makes for electron 1, so
-//   R_t = sum over the band of rho1 * Kd_t[(b,d)],
-//   dR_t/d f_a = Kd_t[(b,d)]~ f_c,  dR_t/d f_c = Kd_t[(b,d)]~ f_a  (basis A_t)
-// with K~ the symmetric band matrix of the 's' storage.  The tables are
+// with rho2) is the potential rho2 makes for electron 1.  The tables are
 // symmetric under exchanging the electrons with types 2 and 3 swapped, so
-// the potential of rho1 for electron 2 is Kd_swap(t)[(a,c)]:
-//   dR_t/d f_b = Kd_swap(t)[(a,c)]~ f_d,  dR_t/d f_d = ... f_b  (basis B_t).
+// with
+//   V_P[(p,q)] = Kd_0[(p,q)] + Kd_2[(p,q)],  V_Q = Kd_1 + Kd_3,
+// the potential that the whole density of the pair makes for a P or a Q
+// function of the other electron (symmetric band matrices, the same for
+// (q,p)), an entry c R^k(a,b;c,d) adds c V_X[(b,d)] to the potential W_X of
+// the pair {a,c} and c V_X[(a,c)] to that of {b,d}, and
+//   dE/df_u += W_X{u,v} f_v,  dE/df_v += W_X{u,v} f_u  (component X),
+//   E = 1/2 sum over {u,v}, X of f_u W_X{u,v} f_v
+// (without the gradient, only the first of the two and E without the 1/2).
+// So the work is one sum of band potentials per (k, pair), in entry order
+// from a host-built list, and two band products; the terms are summed per
+// (orbital, component) in a fixed order: deterministic, no atomics.
 // The pair potentials are built from the cell moments and diagonal cells,
-// recomputed when the tables were released.  Every gradient term is a
-// vector of ns; the terms are summed per (orbital, component) in entry order
-// from a host-built list, so the result is deterministic without atomics.
+// recomputed when the tables were released.
 #include "internal.cuh"
 
 #include <algorithm>
-#include <numeric>
 
 namespace {
-
-// electron-1 / electron-2 basis of table type t (1 P, 2 Q), and the type with
-// the electrons exchanged
-__host__ __device__ inline int TA(int t) { return (t == 0 || t == 2) ? 1 : 2; }
-__host__ __device__ inline int TB(int t) { return (t == 0 || t == 3) ? 1 : 2; }
-__host__ __device__ inline int SWAP(int t) { return t < 2 ? t : 5 - t; }
 
 struct KdTypes {
   const double *K[4];  // Kd_t[pair][ns*ks], 's' storage
 };
 
-// R_e = sum_t sum_{i,ip} rho1_t(i,ip) Kd_t[(b,d)](i,ip), one warp per entry
-__global__ void k_rk_energy(int n, int ns, int ks, int nb, const int *ent, const int *ia,
-                            const int *ib, const int *ic, const int *id, const int *bmap,
-                            const double *pq, KdTypes kd, double *R) {
-  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 32), lane = threadIdx.x % 32;
-  if (w >= n) return;
-  const int e = ent[w];
-  const int a = ia[e], b = ib[e], c = ic[e], d = id[e];
-  const int pair2 = bmap[b - 1] * nb + bmap[d - 1];
-  const size_t per = (size_t)ns * ks;
-  double acc = 0.0;
-  for (int t = 0; t < 4; t++) {
-    const double *fa = pq + (size_t)2 * ns * (a - 1) + (size_t)ns * (TA(t) - 1);
-    const double *fc = pq + (size_t)2 * ns * (c - 1) + (size_t)ns * (TA(t) - 1);
-    const double *K = kd.K[t] + (size_t)pair2 * per;
-    for (int i = lane; i < ns; i += 32) {
-      const double ai = fa[i], ci = fc[i];
-      double s = K[i] * (ai * ci);
-      for (int ip = 2; ip <= ks && i + ip - 1 < ns; ip++) {
-        const int j = i + ip - 1;
-        s = fma(K[i + (size_t)ns * (ip - 1)], ai * fc[j] + fa[j] * ci, s);
-      }
-      acc += s;
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) R[e] = acc;
+// V[X][up][q] = Kd_t0[pair][q] + Kd_t1[pair][q] over the unordered bound pairs
+// (upair: their ordered index), X = P: t = 0, 2; X = Q: t = 1, 3
+__global__ void k_rk_vsum(size_t per, int nup, const int *upair, KdTypes kd, double *V) {
+  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= per) return;
+  const int up = blockIdx.y, X = blockIdx.z;
+  const size_t o = (size_t)upair[up] * per + q;
+  V[((size_t)X * nup + up) * per + q] = kd.K[X][o] + kd.K[X + 2][o];
 }
 
-// E = sum_e c_e R_e in a fixed order (one block, fixed tree)
-__global__ void k_energy_sum(int n, const double *c, const double *R, double *E) {
+// One item = one (multipole, unordered pair {u,v}) with its list of (pair,
+// coefficient); a block takes MC rows m of one component X of an item.  It
+// forms the rows of W_X that those rows meet (ks - 1 before them as well) in
+// shared memory, one thread per band element, the potentials of UE entries
+// loaded together; then row m of W f_v and of W f_u (128 threads each).
+// Bound by the L2 reads of the potentials: 16 ks bytes per row, entry and
+// component.  ns 300, 30 orbitals, 5e4 entries of k = 0..8: 1e5 list
+// positions.  One thread per (entry, type, role, row) with 17-term sums and a
+// launch per run of entries took 355 ms of the evaluation's 367.7 (44 453
+// launches, and the terms of every entry written and read back); with this
+// kernel the evaluation takes 15.2 ms, 12 of them the pair potentials.
+constexpr int MC = 128;
+constexpr int UE = 4;
+__global__ void __launch_bounds__(2 * MC) k_rk_pot(int ns, int ks, int nup, size_t per,
+                                                   const int *istart, const int2 *iuv,
+                                                   const int *lpair, const double *lcoef,
+                                                   const double *V, const double *pq, int grad,
+                                                   double *T, double *Epart) {
+  extern __shared__ double W[];  // [ks][MC + ks - 1]
+  __shared__ double wsum[MC / 32];
+  const int m0 = blockIdx.x * MC, it = blockIdx.y, X = blockIdx.z;
+  const int nr = MC + ks - 1, r0 = m0 - (ks - 1);
+  const int e0 = istart[it], e1 = istart[it + 1];
+  const double *Vx = V + (size_t)X * nup * per;
+  for (int el = threadIdx.x; el < nr * ks; el += 2 * MC) {
+    const int i = r0 + el % nr, dl = el / nr;
+    double acc = 0.0;
+    if (i >= 0 && i + dl < ns) {
+      const double *v = Vx + (size_t)i + (size_t)ns * dl;
+      int e = e0;
+      for (; e + UE <= e1; e += UE) {
+        double k[UE];
+#pragma unroll
+        for (int u = 0; u < UE; u++) k[u] = v[(size_t)lpair[e + u] * per];
+#pragma unroll
+        for (int u = 0; u < UE; u++) acc = fma(lcoef[e + u], k[u], acc);
+      }
+      for (; e < e1; e++) acc = fma(lcoef[e], v[(size_t)lpair[e] * per], acc);
+    }
+    W[el] = acc;
+  }
+  __syncthreads();
+  const int role = threadIdx.x / MC, ml = threadIdx.x % MC, m = m0 + ml;
+  const int2 uv = iuv[it];
+  const double *fu = pq + (size_t)2 * ns * (uv.x - 1) + (size_t)ns * X;
+  const double *fv = pq + (size_t)2 * ns * (uv.y - 1) + (size_t)ns * X;
+  const double *f = role == 0 ? fv : fu;
+  double acc = 0.0;
+  if (m < ns && (grad || role == 0)) {
+    for (int j = max(0, m - ks + 1); j <= min(ns - 1, m + ks - 1); j++) {
+      const int lo = min(m, j), dl = abs(m - j);
+      acc = fma(W[(lo - r0) + nr * dl], f[j], acc);
+    }
+    if (grad) T[(((size_t)it * 2 + X) * 2 + role) * ns + m] = acc;
+  }
+  if (role == 0) {
+    double s = m < ns ? fu[m] * acc : 0.0;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (ml % 32 == 0) wsum[ml / 32] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < MC / 32; w++) s += wsum[w];
+    Epart[((size_t)it * 2 + X) * gridDim.x + blockIdx.x] = s;
+  }
+}
+
+// E = f sum of n partial energies in a fixed order (one block, fixed tree)
+__global__ void k_energy_sum(int n, double f, const double *R, double *E) {
   __shared__ double sh[256];
   double s = 0.0;
-  for (int e = threadIdx.x; e < n; e += 256) s = fma(c[e], R[e], s);
+  for (int e = threadIdx.x; e < n; e += 256) s += R[e];
   sh[threadIdx.x] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *E = sh[0];
+  if (threadIdx.x == 0) *E = f * sh[0];
 }
 
-// gradient terms: T[(e*4 + t)*4 + role][m] = c_e (K~ f)(m) with
-// role 0: target a, K = Kd_t[(b,d)], f = f_c (basis A_t); 1: target c, f = f_a;
-// role 2: target b, K = Kd_swap(t)[(a,c)], f = f_d (basis B_t); 3: target d, f = f_b
-__global__ void k_rk_grad_terms(int n, int ns, int ks, int nb, const int *ia, const int *ib,
-                                const int *ic, const int *id, const double *coef,
-                                const int *bmap, const double *pq, KdTypes kd, double *T) {
-  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (size_t)n * 16 * ns) return;
-  const int m = (int)(q % ns), r = (int)(q / ns) % 4, t = (int)(q / ns / 4) % 4;
-  const int e = (int)(q / ((size_t)ns * 16));
-  const int a = ia[e], b = ib[e], c = ic[e], d = id[e];
-  const int pr = r < 2 ? bmap[b - 1] * nb + bmap[d - 1] : bmap[a - 1] * nb + bmap[c - 1];
-  const int comp = r < 2 ? TA(t) : TB(t);
-  const int src = r == 0 ? c : r == 1 ? a : r == 2 ? d : b;
-  const double *K = kd.K[r < 2 ? t : SWAP(t)] + (size_t)pr * ns * ks;
-  const double *f = pq + (size_t)2 * ns * (src - 1) + (size_t)ns * (comp - 1);
+// grad[(o, comp, m)] = the terms of orbital o (lidx: 2 item + role) in a fixed
+// order: GS slices of the list summed side by side, then the slices in order
+constexpr int GS = 8;
+__global__ void __launch_bounds__(32 * GS) k_rk_grad_reduce(int ns, const int *lstart,
+                                                            const int *lidx, const double *T,
+                                                            double *grad) {
+  __shared__ double sh[GS][32];
+  const int tx = threadIdx.x % 32, sl = threadIdx.x / 32;
+  const int m = blockIdx.x * 32 + tx, o = blockIdx.y, X = blockIdx.z;
   double acc = 0.0;
-  for (int j = max(0, m - ks + 1); j <= min(ns - 1, m + ks - 1); j++) {
-    const int lo = min(m, j), dl = abs(m - j);
-    acc = fma(K[lo + (size_t)ns * dl], f[j], acc);
+  if (m < ns)
+    for (int l = lstart[o] + sl; l < lstart[o + 1]; l += GS) {
+      const int r = lidx[l];
+      acc += T[(((size_t)(r >> 1) * 2 + X) * 2 + (r & 1)) * ns + m];
+    }
+  sh[sl][tx] = acc;
+  __syncthreads();
+  if (sl == 0 && m < ns) {
+    for (int k = 1; k < GS; k++) acc += sh[k][tx];
+    grad[((size_t)o * 2 + X) * ns + m] = acc;  // pq layout
   }
-  T[q] = coef[e] * acc;
-}
-
-// grad[(o, comp, m)] = sum over the term list of (o, comp), in list order
-__global__ void k_rk_grad_reduce(int ns, int nbf, const int *lstart, const int *lidx,
-                                 const double *T, double *grad) {
-  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= (size_t)ns * 2 * nbf) return;
-  const int m = (int)(q % ns);
-  const int oc = (int)(q / ns);  // o * 2 + comp (pq layout)
-  double acc = 0.0;
-  for (int l = lstart[oc]; l < lstart[oc + 1]; l++) acc += T[(size_t)lidx[l] * ns + m];
-  grad[q] = acc;
 }
 
 }  // namespace
@@ -151,35 +185,83 @@ extern "C" int dbsrg_backward(dbsrg_ctx *c, int n, const int *k, const int *i1, 
   }
   if (nb < 1 || nb > 64)
     return set_err(c, DBSRG_EINVAL, "backward: 1..64 bound orbitals (ipbs = 0)");
-  // device arrays: entries, per-k entry order, R, terms, term lists, E
-  std::vector<int> order(n);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return hk[x] < hk[y]; });
-  // term lists per (orbital, component): (e*4 + t)*4 + role in entry order
-  std::vector<int> cnt((size_t)2 * nbf + 1, 0);
-  auto target = [&](int e, int t, int r) {
-    const int o = r == 0 ? h1[e] : r == 1 ? h3[e] : r == 2 ? h2[e] : h4[e];
-    const int comp = r < 2 ? TA(t) : TB(t);
-    return (o - 1) * 2 + (comp - 1);
-  };
+  // items: (multipole, unordered bound pair), each with the pairs and
+  // coefficients of its list in entry order (counting sort)
   const bool want_grad = grad != nullptr;
-  std::vector<int> lstart((size_t)2 * nbf + 1, 0), lidx;
-  if (want_grad) {
-    for (int e = 0; e < n; e++)
-      for (int t = 0; t < 4; t++)
-        for (int r = 0; r < 4; r++) cnt[target(e, t, r) + 1]++;
-    for (int i = 0; i < 2 * nbf; i++) lstart[i + 1] = lstart[i] + cnt[i + 1];
-    lidx.resize((size_t)16 * n);
-    std::vector<int> fill(lstart.begin(), lstart.end() - 1);
-    for (int e = 0; e < n; e++)
-      for (int t = 0; t < 4; t++)
-        for (int r = 0; r < 4; r++) lidx[fill[target(e, t, r)]++] = (e * 4 + t) * 4 + r;
+  auto upair = [&](int o1, int o2) {
+    const int x = c->h_bmap[o1 - 1], y = c->h_bmap[o2 - 1], lo = std::min(x, y), hi = std::max(x, y);
+    return hi * (hi + 1) / 2 + lo;
+  };
+  const int nup = nb * (nb + 1) / 2;
+  std::vector<int> up(nup), p1(n), p2(n);
+  for (int hi = 0; hi < nb; hi++)
+    for (int lo = 0; lo <= hi; lo++) up[hi * (hi + 1) / 2 + lo] = lo * nb + hi;
+  int kmax = -1;
+  for (int e = 0; e < n; e++) {
+    p1[e] = upair(h1[e], h3[e]);
+    p2[e] = upair(h2[e], h4[e]);
+    kmax = std::max(kmax, hk[e]);
   }
+  std::vector<int> pos((size_t)(kmax + 1) * nup + 1, 0);
+  for (int e = 0; e < n; e++) {
+    pos[(size_t)hk[e] * nup + p1[e] + 1]++;
+    if (want_grad) pos[(size_t)hk[e] * nup + p2[e] + 1]++;
+  }
+  std::vector<int> istart, kitem(kmax + 2, 0);  // list start of each item; first item of each k
+  std::vector<int2> iuv;
+  std::vector<int> b2o(nb);
+  for (int o = 0; o < nbf; o++)
+    if (c->h_bmap[o] >= 0) b2o[c->h_bmap[o]] = o + 1;
+  for (int k1 = 0; k1 <= kmax; k1++) {
+    kitem[k1] = (int)iuv.size();
+    for (int u = 0; u < nup; u++) {
+      const size_t q = (size_t)k1 * nup + u;
+      if (pos[q + 1]) {
+        istart.push_back(pos[q]);
+        iuv.push_back(make_int2(b2o[up[u] / nb], b2o[up[u] % nb]));
+      }
+      pos[q + 1] += pos[q];
+    }
+  }
+  const int nitem = (int)iuv.size(), nl = kmax < 0 ? 0 : pos.back();
+  if (kmax >= 0) kitem[kmax + 1] = nitem;
+  istart.push_back(nl);
+  std::vector<int> lpair(nl);
+  std::vector<double> lcoef(nl);
+  for (int e = 0; e < n; e++) {
+    const size_t q = (size_t)hk[e] * nup;
+    int &x = pos[q + p1[e]];
+    lpair[x] = p2[e];
+    lcoef[x++] = hc[e];
+    if (want_grad) {
+      int &y = pos[q + p2[e]];
+      lpair[y] = p1[e];
+      lcoef[y++] = hc[e];
+    }
+  }
+  // gradient terms of every orbital: 2 item + role (0: target u, 1: target v)
+  std::vector<int> lstart((size_t)nbf + 1, 0), lidx;
+  if (want_grad) {
+    for (const int2 &x : iuv) {
+      lstart[x.x]++;
+      lstart[x.y]++;
+    }
+    for (int o = 0; o < nbf; o++) lstart[o + 1] += lstart[o];
+    lidx.resize((size_t)2 * nitem);
+    std::vector<int> fill(lstart.begin(), lstart.end() - 1);
+    for (int i = 0; i < nitem; i++) {
+      lidx[fill[iuv[i].x - 1]++] = 2 * i;
+      lidx[fill[iuv[i].y - 1]++] = 2 * i + 1;
+    }
+  }
+  const size_t per = (size_t)ns * ks, ng = (size_t)ns * 2 * nbf;
+  const int nmc = (ns + MC - 1) / MC;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t tn = want_grad ? (size_t)n * 16 * ns : 0;
-  const size_t bytes = 6 * al(ib) + 2 * al(sizeof(double) * (size_t)n) + al(sizeof(double) * tn) +
-                       al(sizeof(int) * lstart.size()) + al(sizeof(int) * lidx.size()) +
-                       al(sizeof(double) * (size_t)ns * 2 * nbf) + 256;
+  const size_t tn = want_grad ? (size_t)nitem * 4 * ns : 0, vn = 2 * (size_t)nup * per;
+  const size_t en = (size_t)nitem * 2 * nmc;
+  const size_t bytes = al(4 * (size_t)nup) + al(4 * istart.size()) + al(8 * (size_t)nitem) +
+                       al(4 * (size_t)nl) + al(8 * (size_t)nl) + al(8 * vn) + al(8 * tn) +
+                       al(8 * en) + al(4 * lstart.size()) + al(4 * lidx.size()) + al(8 * ng) + 512;
   if ((rc = ensure_scratch(c, bytes))) return rc;
   char *base = (char *)c->scratch;
   auto take = [&](size_t b) {
@@ -187,60 +269,49 @@ extern "C" int dbsrg_backward(dbsrg_ctx *c, int n, const int *k, const int *i1, 
     base += al(b);
     return (void *)p;
   };
-  int *dk = (int *)take(ib), *d1 = (int *)take(ib), *d2 = (int *)take(ib), *d3 = (int *)take(ib),
-      *d4 = (int *)take(ib), *dord = (int *)take(ib);
-  double *dc = (double *)take(sizeof(double) * n), *dR = (double *)take(sizeof(double) * n);
-  double *dT = (double *)take(sizeof(double) * tn);
-  int *dls = (int *)take(sizeof(int) * lstart.size()), *dli = (int *)take(sizeof(int) * lidx.size());
-  double *dG = (double *)take(sizeof(double) * (size_t)ns * 2 * nbf);
+  int *dup = (int *)take(4 * (size_t)nup), *dis = (int *)take(4 * istart.size());
+  int2 *duv = (int2 *)take(8 * (size_t)nitem);
+  int *dlp = (int *)take(4 * (size_t)nl);
+  double *dlc = (double *)take(8 * (size_t)nl), *dV = (double *)take(8 * vn);
+  double *dT = (double *)take(8 * tn), *dEp = (double *)take(8 * en);
+  int *dls = (int *)take(4 * lstart.size()), *dli = (int *)take(4 * lidx.size());
+  double *dG = (double *)take(8 * ng);
   double *dE = (double *)take(sizeof(double));
-  if ((rc = copy_in(c, dk, hk.data(), ib)) || (rc = copy_in(c, d1, h1.data(), ib)) ||
-      (rc = copy_in(c, d2, h2.data(), ib)) || (rc = copy_in(c, d3, h3.data(), ib)) ||
-      (rc = copy_in(c, d4, h4.data(), ib)) || (rc = copy_in(c, dord, order.data(), ib)) ||
-      (rc = copy_in(c, dc, hc.data(), sizeof(double) * n)))
+  if ((rc = copy_in(c, dup, up.data(), 4 * (size_t)nup)) ||
+      (rc = copy_in(c, dis, istart.data(), 4 * istart.size())) ||
+      (rc = copy_in(c, duv, iuv.data(), 8 * (size_t)nitem)) ||
+      (rc = copy_in(c, dlp, lpair.data(), 4 * (size_t)nl)) ||
+      (rc = copy_in(c, dlc, lcoef.data(), 8 * (size_t)nl)))
     return rc;
-  if (want_grad &&
-      ((rc = copy_in(c, dls, lstart.data(), sizeof(int) * lstart.size())) ||
-       (rc = copy_in(c, dli, lidx.data(), sizeof(int) * lidx.size()))))
+  if (want_grad && ((rc = copy_in(c, dls, lstart.data(), 4 * lstart.size())) ||
+                    (rc = copy_in(c, dli, lidx.data(), 4 * lidx.size()))))
     return rc;
-  // per multipole: the four pair potentials, then energy and gradient terms
-  for (int lo = 0; lo < n;) {
-    int hi = lo;
-    while (hi < n && hk[order[hi]] == hk[order[lo]]) hi++;
-    const int kp = hk[order[lo]];
+  // per multipole: the four pair potentials, their sums, the items
+  const size_t smem = (size_t)(MC + ks - 1) * ks * sizeof(double);
+  for (int kp = 0; kp <= kmax; kp++) {
+    const int i0 = kitem[kp], ni = kitem[kp + 1] - i0;
+    if (ni == 0) continue;
     KdTypes kd{};
-    for (int t = 0; t < 4; t++)
-      if ((rc = get_pairpot_direct(c, 0, t, kp, 1, TB(t), TB(t), &kd.K[t]))) return rc;
-    const int m = hi - lo;
-    DBSRG_RUN(c, "k_rk_energy",
-              k_rk_energy<<<(unsigned)((m * 32 + 255) / 256), 256, 0, st>>>(
-                  m, ns, ks, nb, dord + lo, d1, d2, d3, d4, c->bmap, c->pq, kd, dR));
-    if (want_grad) {
-      // the terms of the entries of this multipole: one launch per entry run
-      // (entries of one k are contiguous in 'order' but not in the arrays)
-      std::vector<int> run(order.begin() + lo, order.begin() + hi);
-      std::sort(run.begin(), run.end());
-      for (size_t s0 = 0; s0 < run.size();) {
-        size_t s1 = s0 + 1;
-        while (s1 < run.size() && run[s1] == run[s1 - 1] + 1) s1++;
-        const int e0 = run[s0], ne = (int)(s1 - s0);
-        const size_t nt = (size_t)ne * 16 * ns;
-        DBSRG_RUN(c, "k_rk_grad_terms",
-                  k_rk_grad_terms<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(
-                      ne, ns, ks, nb, d1 + e0, d2 + e0, d3 + e0, d4 + e0, dc + e0, c->bmap,
-                      c->pq, kd, dT + (size_t)e0 * 16 * ns));
-        s0 = s1;
-      }
+    for (int t = 0; t < 4; t++) {
+      const int comp = (t == 0 || t == 3) ? 1 : 2;  // electron-2 basis of the table
+      if ((rc = get_pairpot_direct(c, 0, t, kp, 1, comp, comp, &kd.K[t]))) return rc;
     }
-    lo = hi;
+    DBSRG_RUN(c, "k_rk_vsum",
+              k_rk_vsum<<<dim3((unsigned)((per + 255) / 256), (unsigned)nup, 2), 256, 0, st>>>(
+                  per, nup, dup, kd, dV));
+    DBSRG_RUN(c, "k_rk_pot",
+              k_rk_pot<<<dim3((unsigned)nmc, (unsigned)ni, 2), 2 * MC, smem, st>>>(
+                  ns, ks, nup, per, dis + i0, duv + i0, dlp, dlc, dV, c->pq, want_grad ? 1 : 0,
+                  dT + (want_grad ? (size_t)i0 * 4 * ns : 0), dEp + (size_t)i0 * 2 * nmc));
   }
-  if (n > 0) DBSRG_RUN(c, "k_energy_sum", k_energy_sum<<<1, 256, 0, st>>>(n, dc, dR, dE));
+  if (n > 0)
+    DBSRG_RUN(c, "k_energy_sum",
+              k_energy_sum<<<1, 256, 0, st>>>((int)en, want_grad ? 0.5 : 1.0, dEp, dE));
   else DBSRG_TRY(c, cudaMemsetAsync(dE, 0, sizeof(double), st));
   if (want_grad) {
-    const size_t ng = (size_t)ns * 2 * nbf;
     DBSRG_RUN(c, "k_rk_grad_reduce",
-              k_rk_grad_reduce<<<(unsigned)((ng + 255) / 256), 256, 0, st>>>(ns, nbf, dls, dli,
-                                                                             dT, dG));
+              k_rk_grad_reduce<<<dim3((unsigned)((ns + 31) / 32), (unsigned)nbf, 2), 32 * GS, 0,
+                                 st>>>(ns, dls, dli, dT, dG));
     if ((rc = copy_out(c, grad, dG, sizeof(double) * ng))) return rc;
   }
   return copy_out(c, energy, dE, sizeof(double));

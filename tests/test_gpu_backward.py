@@ -142,3 +142,22 @@ def test_rk_on_reference_orbitals_pinned_by_configuration_energies(golden):
             assert abs(val - r) <= 2e-11, (rec["log"], key, val, r)
             n += 1
     assert n == 13
+
+
+@pytest.mark.parametrize("ns,norb,n", [(128, 2, 7), (137, 5, 90), (150, 1, 5)])
+def test_backward_row_chunks_and_pair_lists(ns, norb, n):
+    """Row chunks of 128 with and without a remainder, pairs with themselves,
+    lists shorter and longer than a load batch; energy alone and with the
+    gradient.  FP64 sums of at most a few hundred terms: the 1e-12 of the
+    other cases."""
+    w = synth.energy_workload("chunks", 81 + ns, ns, 15.0, 9.0, norb, 3, n)
+    a = assembler(w)
+    E, G = a.backward(w.k, w.i1, w.i2, w.i3, w.i4, w.coef)
+    E0, none = a.backward(w.k, w.i1, w.i2, w.i3, w.i4, w.coef, grad=False)
+    a.close()
+    Er, Gr = O.Grid(w.t, w.ks, w.ksp, w.ksq).rk_energy_grad(w.k, w.i1, w.i2, w.i3, w.i4, w.coef,
+                                                            w.pq)
+    assert none is None
+    for e in (E, E0):
+        assert abs(e - Er) <= 1e-12 * max(abs(Er), 1.0)
+    assert np.abs(G - Gr).max() <= 1e-12 * np.abs(Gr).max()
