@@ -478,17 +478,26 @@ __global__ void k_acf(int nseg_owner, const int *owners, const SegInfo *info, in
 // O_data itype 3 (<i|.><.|j>, O_data.f90:50-61) with UPDATE_HW
 // (updates.f90:183-216).  V_ch is restated as the B-spline overlap vector
 // of the bound orbital: v(1:ns) = fpbs*P, v(ns+1:ms) = fqbs*Q.
-__global__ void k_vch(int ns, int nbf, const double *fpbs, const double *fqbs,
-                      const double *pq, double *vch) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= 2 * ns * nbf) return;
-  int i = q % (2 * ns), b = q / (2 * ns);
-  int comp = i / ns, ii = i % ns;
+// 32 rows of one orbital a block, VSL slices of the sum over j side by side
+// and then added in order (a serial sum over all j per thread took 62 us at
+// ns 180 and 16 orbitals, a chain of ns loads)
+constexpr int VSL = 8;
+__global__ void __launch_bounds__(32 * VSL) k_vch(int ns, const double *fpbs, const double *fqbs,
+                                                  const double *pq, double *vch) {
+  __shared__ double sh[VSL][32];
+  const int tx = threadIdx.x % 32, sl = threadIdx.x / 32;
+  const int i = blockIdx.x * 32 + tx, comp = blockIdx.z, b = blockIdx.y;
   const double *F = comp == 0 ? fpbs : fqbs;
   const double *p = pq + (size_t)2 * ns * b + (size_t)ns * comp;
   double s = 0.0;
-  for (int j = 0; j < ns; j++) s += F[(size_t)ii + (size_t)ns * j] * p[j];
-  vch[q] = s;
+  if (i < ns)
+    for (int j = sl; j < ns; j += VSL) s = fma(F[(size_t)i + (size_t)ns * j], p[j], s);
+  sh[sl][tx] = s;
+  __syncthreads();
+  if (sl == 0 && i < ns) {
+    for (int k = 1; k < VSL; k++) s += sh[k][tx];
+    vch[(size_t)2 * ns * b + (size_t)ns * comp + i] = s;
+  }
 }
 
 // One thread per row r of a touched block and 32 consecutive columns: the
@@ -548,6 +557,24 @@ __global__ void k_update_hx(int ms, int ich, int jch, const double *d, double cc
 }  // namespace
 
 // ---------------------------------------------------------------------------
+int get_vch(dbsrg_ctx *c, const double **out) {
+  if (!c->vch) {
+    const int ns = c->g.ns;
+    double *v = (double *)cache_alloc(c, sizeof(double) * 2 * (size_t)ns * c->nbf);
+    if (!v) return set_err(c, DBSRG_ENOMEM, "overlap vectors allocation failed");
+    c->vch = v;
+    for (int b0 = 0; b0 < c->nbf; b0 += 65535) {  // grid y limit
+      const dim3 gv((unsigned)((ns + 31) / 32), (unsigned)std::min(65535, c->nbf - b0), 2);
+      DBSRG_RUN(c, "k_vch",
+                k_vch<<<gv, 32 * VSL, 0, c->stream>>>(ns, c->g.fpbs, c->g.fqbs,
+                                                      c->pq + (size_t)2 * ns * b0,
+                                                      v + (size_t)2 * ns * b0));
+    }
+  }
+  *out = c->vch;
+  return DBSRG_OK;
+}
+
 int update_hx(dbsrg_ctx *c, int ich, int jch, const double *d, double cc) {
   const int ms = c->g.ms;
   if (!c->hch) return set_err(c, DBSRG_ESTATE, "no matrix allocated");
@@ -604,7 +631,6 @@ struct ListPlan {
   SegInfo *info = nullptr;
   int *work = nullptr;   // chunk members and owner slots | acf owners
   XQuad *dxq = nullptr;  // quadrant records
-  double *vch = nullptr;
   int *bstart = nullptr, *tlist = nullptr, *order = nullptr;  // overlap list
   std::vector<Chunk> chunks;
   std::vector<int> wchunk, wown, wtl;  // per window: [w], [w+1] ranges
@@ -625,8 +651,7 @@ size_t plan_bytes(const dbsrg_ctx *c, int icase, int itype, int n) {
              al256(sizeof(SegInfo) * (size_t)(n + 1)) + al256(sizeof(int) * (size_t)(7 * (n + 1))) +
              al256(sizeof(XQuad) * 4 * (size_t)(n + 1)) + al256(sizeof(float2) * (size_t)n);
   if (icase == 0)
-    t += al256(sizeof(double) * (size_t)c->g.ms * c->nbf) +
-         al256(sizeof(int) * (2 * (size_t)(c->iicc + 2) + n));
+    t += al256(sizeof(int) * (2 * (size_t)(c->iicc + 2) + n));
   return t;
 }
 
@@ -700,7 +725,6 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
   if (icase == 0) {
     if (itype != 3) return set_err(c, DBSRG_EINVAL, "O_data: unknown structure (itype)");
     const int iicc = c->iicc;
-    P.vch = (double *)take(sizeof(double) * (size_t)ms * c->nbf);
     P.bstart = (int *)take(sizeof(int) * (2 * (size_t)(iicc + 2) + n));
     P.tlist = P.bstart + (iicc + 2);  // blocks with entries, ascending
     P.order = P.tlist + (iicc + 2);
@@ -926,11 +950,8 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
     if (prep) return DBSRG_OK;
     const int t0 = P.wtl[w], nt = P.wtl[w + 1] - t0;
     if (nt <= 0) return DBSRG_OK;
-    // the overlap vectors depend on the orbitals only: built by the first
-    // window with blocks of this list, kept by the plan for the later ones
-    if (t0 == P.wtl[0])
-      DBSRG_RUN(c, "k_vch", k_vch<<<(2 * ns * c->nbf + 255) / 256, 256, 0, st>>>(
-                                ns, c->nbf, g.fpbs, g.fqbs, c->pq, P.vch));
+    const double *vch;
+    if ((rc = get_vch(c, &vch))) return rc;
     for (int t = 0; t < nt; t += 65535) {  // grid z limit
       const int nz = std::min(65535, nt - t);
       dim3 grid((unsigned)((ms + 127) / 128), (unsigned)((ms + 31) / 32), (unsigned)nz);
@@ -940,7 +961,7 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
       const double of = t == 0 ? P.wovl[w] : 0.0;
       DBSRG_RUN_W(c, "k_overlap_update", ob, of,
                   k_overlap_update<<<grid, 128, 0, st>>>(ns, P.tlist + t0 + t, P.bstart, P.order,
-                                                         P.lk1, P.lk2, P.lcd, c->ipbs, P.vch,
+                                                         P.lk1, P.lk2, P.lcd, c->ipbs, vch,
                                                          hch_base(c)));
     }
     return DBSRG_OK;
@@ -1096,7 +1117,7 @@ namespace {
 int prepare_list(dbsrg_ctx *c, const ListPlan &P, bool overlap) {
   if (P.icase == 0 && !P.sp) return DBSRG_OK;
   int rc;
-  if (P.factored && !P.sp) {  // shared by the builds of every k
+  if (P.sp ? structure_uses_pairs(*P.sp) : P.factored) {  // shared by the builds of every k
     bool built = false;
     if ((rc = ensure_bound_rows(c, &built))) return rc;
     if (built) overlap = false;

@@ -900,6 +900,10 @@ static int set_smem(dbsrg_ctx *c, const void *fn, size_t smem) {
   return raise_smem_limit(c, fn, smem);
 }
 
+bool pair_potentials_fit(const dbsrg_ctx *c) {
+  return c->g.ks <= FAR && c->nbound >= 1 && c->nbound <= 64;
+}
+
 // direct pair potentials of (family, type, k, case icv) with density
 // components jp1/jp2: Kd[pair][ns*ncol], cached
 int get_pairpot_direct(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1,
@@ -1051,7 +1055,8 @@ static int get_pairpot_band(dbsrg_ctx *c, int family, int type, int k, int cs, i
 
 void free_orbital_products(dbsrg_ctx *c) {
   graph_drop(c);
-  if (!c->rfar.empty() || !c->sfar.empty() || !c->ppot.empty() || c->brows || !c->ffc.empty())
+  if (!c->rfar.empty() || !c->sfar.empty() || !c->ppot.empty() || c->brows || c->vch ||
+      !c->ffc.empty())
     cudaStreamSynchronize(c->stream);
   for (auto *v : {&c->rfar, &c->sfar})
     for (auto &kv : *v) {
@@ -1065,6 +1070,8 @@ void free_orbital_products(dbsrg_ctx *c) {
   c->ppot.clear();
   cache_free(c, c->brows);
   c->brows = nullptr;
+  cache_free(c, c->vch);
+  c->vch = nullptr;
   for (auto &kv : c->ffc) cache_free(c, kv.second);
   c->ffc.clear();
 }

@@ -101,6 +101,10 @@ struct dbsrg_ctx {
   std::map<const void *, float2 *> ffc;
   // bound-orbital rows brows[(comp-1)*nbound*ns + a*ns + x] = pq(x+1, comp, b2o[a])
   double *brows = nullptr;
+  // overlap vectors V_ch of every orbital, vch[2 ns (orbital - 1)] = (fpbs P;
+  // fqbs Q); an orbital product like the others, built on the contraction
+  // stream by the first list of an assembly that reads it
+  double *vch = nullptr;
   // bound-orbital map: bmap[orb-1] = dense bound index or -1; nbound
   int nbound = 0;
   int *bmap = nullptr;  // (nbf)
@@ -349,6 +353,7 @@ int gen_matrix_plain(dbsrg_ctx *c, int icase, int itype, int kpol, int n,
                      const int *ipt, const int *k1, const int *k2,
                      const int *k3, const int *k4, const double *cdata);
 int update_hx(dbsrg_ctx *c, int ich, int jch, const double *d, double cc);
+int get_vch(dbsrg_ctx *c, const double **out);  // call with the contraction stream current
 // convol cases 1/2 (icase) of nsg band densities X[s][ns*kb] with the full
 // table rkb (kb = ks for R, 2ks-1 for S) into Y[s][ns*kb], on the context stream
 int band_contract(dbsrg_ctx *c, int kb, int icase, const double *rkb, int nsg, const double *X,
@@ -385,6 +390,8 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
                     const double *cdata, int blo0, int nwin, int nw, void *dev,
                     cudaStream_t ss, StructPlan **out, const int *wstart = nullptr);
 int exec_structures(dbsrg_ctx *c, const StructPlan &P, int w, bool prep);
+// the list reads direct pair potentials (and so the bound-orbital rows)
+bool structure_uses_pairs(const StructPlan &P);
 void free_structure_plan(StructPlan *P);
 // zeroes hcp, hp, htarg, otarg (with the matrix); frees them (destroy)
 int zero_structures(dbsrg_ctx *c);
@@ -453,6 +460,9 @@ struct SplitExchange {
   long long nent;     // entries of the member segments (executed-work statements)
 };
 int split_exchange(dbsrg_ctx *c, const SplitExchange &x);
+// whether the direct pair potentials of all bound pairs can be built for a
+// list that needs some of them (spline order, number of bound orbitals)
+bool pair_potentials_fit(const dbsrg_ctx *c);
 // Direct pair potentials of table (family, type, k) for convol case icv with
 // density components jp1/jp2: Kd[pair][ns*ncol] over the ordered bound-orbital
 // pairs (pair = a*nbound + b), cached until release_tables/set_orbitals.

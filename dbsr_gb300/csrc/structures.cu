@@ -14,17 +14,29 @@
 // A list is planned once on the host: every entry is classified exactly as
 // the reference routes it (the same bound checks, returned as status codes
 // where the reference stops), and each update becomes a term that names a
-// coefficient slot and one or two vectors.  The terms are grouped, in the
-// reference's order (atype by atype, entries in IPT order), by the block,
-// perturber column or scalar they update.  Execution computes on the device
-// what the terms read -- the potentials of the bound pairs (density and
-// convol on the full tables, FP64), the per-entry integrals (SUM_AmB), the
-// potential-times-orbital vectors (BAV), the one-electron values and
-// vectors, the overlap vectors V_ch and the coefficient slots -- then
-// applies the terms: one thread per row of 32 columns of a block walks that
-// block's terms in order (no atomics), likewise per perturber column and
-// per scalar.  The work is small beside the channel-pair contraction and
-// stays FP64 in every precision form.
+// coefficient slot and one or two vectors.  The four PQ types of an R^k entry
+// update the same place with the same overlap vectors, so their integrals
+// (itype 1) or vectors (itype 2) are summed first and make one term, where
+// the reference makes four.  The terms are grouped, entries in IPT order, by
+// the block, perturber column or scalar they update.  Execution computes on
+// the device what the terms read -- the potentials of the bound pairs, the
+// per-entry integrals (SUM_AmB), the potential-times-orbital vectors (BAV),
+// the one-electron values and vectors, the overlap vectors V_ch and the
+// coefficient slots -- then applies the terms: one thread per row of 32
+// columns of a block walks that block's terms in order (no atomics),
+// likewise per perturber column and per scalar.  Everything here is FP64 in
+// every precision form.
+//
+// The potentials come from one of two places, chosen when the list is
+// planned:
+//   * the factored forms read the direct pair potentials of factor.cu (the
+//     same convolution from cell sums, all bound pairs of a table at once)
+//     where every K1 orbital is bound and they can be built (spline order at
+//     most 9, at most 64 bound orbitals);
+//   * otherwise, and in the plain form, the pair densities are contracted with
+//     the full table (band_contract), 2 (ns kb)^2 FP64 operations per pair:
+//     2.7 ms a table and list at ns 180 with 10 bound orbitals, against
+//     0.085 ms for the pair potentials of all of their 100 ordered pairs.
 //
 // Routines that live only in the unvendored Libraries_03 are restated:
 //   V_ch / KBORT: the B-spline overlap vector (fpbs P; fqbs Q) of the bound
@@ -57,6 +69,21 @@ static_assert(sizeof(StTerm) == 16, "StTerm is 16 bytes");
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// pair potentials of the PQ types of a list and the components its terms read
+struct StPots {
+  int na;
+  const double *Y[4];  // [potential][ns*kb]
+  const int *pix;      // position of each potential in Y, or null (in order)
+  int c1[4], c2[4];    // SUM_AmB: components of the K2 density
+  int ipo[4], ipv[4];  // BAV: orbital component, vector half
+};
+
+// vector a of the overlap vectors (a < nbf) or of the list's pool
+__device__ __forceinline__ const double *st_vec(const double *vch, const double *pool, int nbf,
+                                                int ms, int a) {
+  return a < nbf ? vch + (size_t)ms * a : pool + (size_t)ms * (a - nbf);
+}
+
 // ---------------------------------------------------------------------------
 // densities of bound pairs (density, dbsr_lib_dbs.f90:2834-2891): X[q] of
 // pair (a, b) with components c1, c2, 's' (ns,ks) or 'n' (ns,2ks-1) storage
@@ -84,33 +111,37 @@ __global__ void k_st_density(int ns, int ks, char sym, int kb, int npot, const i
 }
 
 // SUM_AmB (dbsr_lib_dbs.f90:4027-4080) of a pair potential with the density
-// of the entry's K2 pair, one warp per entry: Ce = S * cdata
+// of the entry's K2 pair, summed over the PQ types, one warp per entry:
+// Ce = S * cdata
 __global__ void k_st_sumamb(int ns, int ks, char sym, int kb, int n, const int *epot,
-                            const int *ej1, const int *ej2, int c1, int c2, const double *pq,
-                            const double *Y, const double *cd, double *Ce) {
+                            const int *ej1, const int *ej2, const StPots P, const double *pq,
+                            const double *cd, double *Ce) {
   const int e = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
   if (e >= n || epot[e] < 0) return;
-  const double *y = Y + (size_t)epot[e] * ns * kb;
-  const double *p1 = pq + (size_t)ns * (c1 - 1) + (size_t)2 * ns * (ej1[e] - 1) - 1;
-  const double *p2 = pq + (size_t)ns * (c2 - 1) + (size_t)2 * ns * (ej2[e] - 1) - 1;
+  const size_t off = (size_t)(P.pix ? P.pix[epot[e]] : epot[e]) * ns * kb;
   double acc = 0.0;
-  for (int jp = 1; jp <= kb; jp++) {
-    int i0, i1;
-    if (sym == 's') {
-      i0 = 1;
-      i1 = ns - jp + 1;
-    } else {
-      i0 = max(1, 1 + ks - jp);
-      i1 = min(ns, ns + ks - jp);
-    }
-    for (int i = i0 + lane; i <= i1; i += 32) {
-      double d;
-      if (sym == 's')
-        d = jp == 1 ? p1[i] * p2[i] : p1[i] * p2[i + jp - 1] + p1[i + jp - 1] * p2[i];
-      else
-        d = p1[i] * p2[i + jp - ks];
-      acc = fma(y[(i - 1) + (size_t)ns * (jp - 1)], d, acc);
+  for (int a = 0; a < P.na; a++) {
+    const double *y = P.Y[a] + off;
+    const double *p1 = pq + (size_t)ns * (P.c1[a] - 1) + (size_t)2 * ns * (ej1[e] - 1) - 1;
+    const double *p2 = pq + (size_t)ns * (P.c2[a] - 1) + (size_t)2 * ns * (ej2[e] - 1) - 1;
+    for (int jp = 1; jp <= kb; jp++) {
+      int i0, i1;
+      if (sym == 's') {
+        i0 = 1;
+        i1 = ns - jp + 1;
+      } else {
+        i0 = max(1, 1 + ks - jp);
+        i1 = min(ns, ns + ks - jp);
+      }
+      for (int i = i0 + lane; i <= i1; i += 32) {
+        double d;
+        if (sym == 's')
+          d = jp == 1 ? p1[i] * p2[i] : p1[i] * p2[i + jp - 1] + p1[i + jp - 1] * p2[i];
+        else
+          d = p1[i] * p2[i + jp - ks];
+        acc = fma(y[(i - 1) + (size_t)ns * (jp - 1)], d, acc);
+      }
     }
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -118,50 +149,44 @@ __global__ void k_st_sumamb(int ns, int ks, char sym, int kb, int n, const int *
 }
 
 // BAV: the potential of pair pot times orbital b (component ipo), into half
-// ipv of an ms-vector of the pool (the other half zero); one thread per row
+// ipv of an ms-vector of the pool, summed over the PQ types; one thread per row
 __global__ void k_st_bav(int ns, int ks, char sym, char dir, int kb, int nvj, const int2 *vj,
-                         int ipo, int ipv, const double *pq, const double *Y, double *pool) {
+                         const StPots P, const double *pq, double *pool) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int q = blockIdx.y;
   if (i > ns || q >= nvj) return;
   const int2 job = vj[q];  // (potential, orbital)
-  const double *a = Y + (size_t)job.x * ns * kb;
-  const double *b = pq + (size_t)ns * (ipo - 1) + (size_t)2 * ns * (job.y - 1) - 1;
-  auto A = [&](int r, int c) { return a[(r - 1) + (size_t)ns * (c - 1)]; };
-  double v = 0.0;
-  if (sym == 's') {
-    for (int jp = 1; jp <= ks; jp++)
-      if (i + jp - 1 <= ns) v = fma(A(i, jp), b[i + jp - 1], v);
-    for (int jp = 2; jp <= ks; jp++)
-      if (i - jp + 1 >= 1) v = fma(A(i - jp + 1, jp), b[i - jp + 1], v);
-  } else {
-    for (int jp = 1; jp <= 2 * ks - 1; jp++) {
-      const int i0 = max(1, 1 + ks - jp), i1 = min(ns, ns + ks - jp);
-      if (dir == 'l') {
-        const int r = i - jp + ks;  // row whose band element lands in column i
-        if (r >= i0 && r <= i1) v = fma(A(r, jp), b[r], v);
-      } else if (i >= i0 && i <= i1) {
-        v = fma(A(i, jp), b[i + jp - ks], v);
+  const size_t off = (size_t)(P.pix ? P.pix[job.x] : job.x) * ns * kb;
+  double half[2] = {0.0, 0.0};
+  for (int t = 0; t < P.na; t++) {
+    const double *a = P.Y[t] + off;
+    const double *b = pq + (size_t)ns * (P.ipo[t] - 1) + (size_t)2 * ns * (job.y - 1) - 1;
+    auto A = [&](int r, int c) { return a[(r - 1) + (size_t)ns * (c - 1)]; };
+    double v = 0.0;
+    if (sym == 's') {
+      for (int jp = 1; jp <= ks; jp++)
+        if (i + jp - 1 <= ns) v = fma(A(i, jp), b[i + jp - 1], v);
+      for (int jp = 2; jp <= ks; jp++)
+        if (i - jp + 1 >= 1) v = fma(A(i - jp + 1, jp), b[i - jp + 1], v);
+    } else {
+      for (int jp = 1; jp <= 2 * ks - 1; jp++) {
+        const int i0 = max(1, 1 + ks - jp), i1 = min(ns, ns + ks - jp);
+        if (dir == 'l') {
+          const int r = i - jp + ks;  // row whose band element lands in column i
+          if (r >= i0 && r <= i1) v = fma(A(r, jp), b[r], v);
+        } else if (i >= i0 && i <= i1) {
+          v = fma(A(i, jp), b[i + jp - ks], v);
+        }
       }
     }
+    if (P.ipv[t] == 1)
+      half[0] += v;
+    else
+      half[1] += v;
   }
   double *out = pool + (size_t)q * 2 * ns;
-  out[(size_t)ns * (ipv - 1) + i - 1] = v;
-  out[(size_t)ns * (2 - ipv) + i - 1] = 0.0;
-}
-
-// V_ch restatement: (fpbs P_b; fqbs Q_b) for every orbital b
-__global__ void k_st_vch(int ns, int nbf, const double *fpbs, const double *fqbs,
-                         const double *pq, double *vch) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= 2 * ns * nbf) return;
-  const int i = q % (2 * ns), b = q / (2 * ns);
-  const int comp = i / ns, ii = i % ns;
-  const double *F = comp == 0 ? fpbs : fqbs;
-  const double *p = pq + (size_t)2 * ns * b + (size_t)ns * comp;
-  double s = 0.0;
-  for (int j = 0; j < ns; j++) s += F[(size_t)ii + (size_t)ns * j] * p[j];
-  vch[q] = s;
+  out[i - 1] = half[0];
+  out[(size_t)ns + i - 1] = half[1];
 }
 
 // Gen_Lvec restatement: hd(:,:,k) (P; Q)_orbital for each (orbital, k)
@@ -193,17 +218,21 @@ __global__ void k_st_lval(int ms, int n, const int *ej1, const int *elv, const d
 }
 
 // the coefficient slots of the structures whose factor is the coefficient
-__global__ void k_st_copyc(int n, int na, const double *cd, double *Ce) {
+__global__ void k_st_copyc(int n, const double *cd, double *Ce) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n * na) return;
-  Ce[q] = cd[q % n];
+  if (q < n) Ce[q] = cd[q];
 }
 
 // UPDATE_HW / UPDATE_HX terms of the window's blocks: one thread per row r
-// and 32 consecutive columns of block tlist[z], its terms in list order
-__global__ void k_st_block_terms(int ms, const int *tlist, const int *bstart,
-                                 const StTerm *terms, const double *Ce, const double *pool,
-                                 const double *fppqq, const double *hd, double *hch) {
+// and 32 consecutive columns of block tlist[z], its terms in list order; the
+// row factor of a rank-1 term is formed once, so an element takes one FMA a
+// term (two on diagonal blocks): bound by the FP64 pipe.  200 entries over
+// 21 blocks of 360 x 360: 202 -> 51 us a list against three operations an
+// element and a term per PQ type
+__global__ void k_st_block_terms(int ms, int nbf, const int *tlist, const int *bstart,
+                                 const StTerm *terms, const double *Ce, const double *vch,
+                                 const double *pool, const double *fppqq, const double *hd,
+                                 double *hch) {
   constexpr int NC = 32;
   const int bi = blockIdx.z;
   const int b = tlist[bi];
@@ -219,24 +248,18 @@ __global__ void k_st_block_terms(int ms, const int *tlist, const int *bstart,
     const StTerm T = terms[t];
     const double C = Ce[T.cidx];
     if (T.kind <= 2) {
-      const double *v = pool + (size_t)ms * T.a, *w = pool + (size_t)ms * T.b;
-      if (T.kind == 0) {  // C * (v(r) w(c))
-        const double vr = v[r];
+      const double *v = st_vec(vch, pool, nbf, ms, T.a), *w = st_vec(vch, pool, nbf, ms, T.b);
+      if (T.kind <= 1) {  // C v(r) w(c), or C w(r) v(c)
+        const double *u = T.kind == 0 ? w : v;  // column vector
+        const double f = C * (T.kind == 0 ? v[r] : w[r]);
 #pragma unroll
         for (int j = 0; j < NC; j++)
-          if (j < ncol) val[j] = __dadd_rn(val[j], __dmul_rn(C, __dmul_rn(vr, w[c0 + j])));
-      } else if (T.kind == 1) {  // C * (v(c) w(r))
-        const double wr = w[r];
+          if (j < ncol) val[j] = fma(f, u[c0 + j], val[j]);
+      } else {  // (C/2) (v(r) w(c) + v(c) w(r))
+        const double f1 = 0.5 * C * v[r], f2 = 0.5 * C * w[r];
 #pragma unroll
         for (int j = 0; j < NC; j++)
-          if (j < ncol) val[j] = __dadd_rn(val[j], __dmul_rn(C, __dmul_rn(v[c0 + j], wr)));
-      } else {  // (C/2) * (v(r) w(c) + v(c) w(r))
-        const double h2 = C / 2.0, vr = v[r], wr = w[r];
-#pragma unroll
-        for (int j = 0; j < NC; j++)
-          if (j < ncol)
-            val[j] = __dadd_rn(val[j], __dmul_rn(h2, __dadd_rn(__dmul_rn(vr, w[c0 + j]),
-                                                                __dmul_rn(v[c0 + j], wr))));
+          if (j < ncol) val[j] = fma(f1, w[c0 + j], fma(f2, v[c0 + j], val[j]));
       }
     } else {
       const double *d = T.a == 0 ? fppqq : hd + (size_t)ms * ms * (T.a - 1);
@@ -254,8 +277,9 @@ __global__ void k_st_block_terms(int ms, const int *tlist, const int *bstart,
 }
 
 // UPDATE_HV terms: one thread per row of a perturber column, terms in order
-__global__ void k_st_hv_terms(int ms, const int *cols, const int *cstart, const StTerm *terms,
-                              const double *Ce, const double *pool, double *hcp) {
+__global__ void k_st_hv_terms(int ms, int nbf, const int *cols, const int *cstart,
+                              const StTerm *terms, const double *Ce, const double *vch,
+                              const double *pool, double *hcp) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   const int ci = blockIdx.y;
   if (r >= ms) return;
@@ -263,7 +287,7 @@ __global__ void k_st_hv_terms(int ms, const int *cols, const int *cstart, const 
   double val = *h;
   for (int t = cstart[ci]; t < cstart[ci + 1]; t++) {
     const StTerm T = terms[t];
-    val = __dadd_rn(val, __dmul_rn(Ce[T.cidx], pool[(size_t)ms * T.a + r]));
+    val = __dadd_rn(val, __dmul_rn(Ce[T.cidx], st_vec(vch, pool, nbf, ms, T.a)[r]));
   }
   *h = val;
 }
@@ -324,6 +348,8 @@ struct StructPlan {
   bool sum_amb = false, bav = false, lval = false, lvec = false, copyc = false;
   int npot = 0, npv = 0, nlv = 0, nbf = 0;
   int2 *pots = nullptr, *vjobs = nullptr, *ljobs = nullptr;
+  bool fact = false;    // potentials from the direct pair potentials of factor.cu
+  int *ppix = nullptr;  // their pair index per potential
   int *epot = nullptr, *ej1 = nullptr, *ej2 = nullptr, *elv = nullptr;
   double *Ce = nullptr, *lcd = nullptr;
   StTerm *terms = nullptr;
@@ -353,20 +379,21 @@ bool is_structure_list(int icase, int itype) {
 // device bytes of a structure list's plan (upper bounds by entry count)
 size_t structure_plan_bytes(const dbsrg_ctx *c, int icase, int itype, int n) {
   (void)itype;
-  const size_t na = icase == 2 ? 4 : 1;
+  (void)icase;
   const size_t N = (size_t)n + 1;
   size_t t = 0;
   t += al256(sizeof(double) * N);                      // coefficients in IPT order
-  t += al256(sizeof(double) * N * na);                 // coefficient slots
+  t += al256(sizeof(double) * N);                      // coefficient slots
   t += 3 * al256(sizeof(int2) * N);                    // potentials, BAV and L vector jobs
-  t += 4 * al256(sizeof(int) * N);                     // per-entry jobs
-  t += 3 * al256(sizeof(StTerm) * 2 * N * na);         // block, column and scalar terms
-  t += 2 * al256(sizeof(int) * (2 * N * na + 2));      // block and column groups
-  t += al256(sizeof(int) * (2 * N * na + 2));          // scalar groups
+  t += 5 * al256(sizeof(int) * N);                     // per-entry jobs, pair indices
+  t += 3 * al256(sizeof(StTerm) * 2 * N);              // block, column and scalar terms
+  t += 2 * al256(sizeof(int) * (2 * N + 2));           // block and column groups
+  t += al256(sizeof(int) * (2 * N + 2));               // scalar groups
   (void)c;
   return t;
 }
 
+bool structure_uses_pairs(const StructPlan &P) { return P.fact; }
 void free_structure_plan(StructPlan *P) { delete P; }
 
 namespace {
@@ -623,10 +650,10 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
     }
     P->npot = (int)pots.size();
     P->npv = (int)vjobs.size();
-    // terms, atype by atype (Gen_matrix calls R_data per atype), entries in order
-    for (int a = 0; a < P->na; a++)
+    // terms, one per entry for all its PQ types, entries in order
+    {
       for (int e = 0; e < n; e++) {
-        const int cidx = a * n + e;
+        const int cidx = e;
         if (it == 1) {  // route by ic = -k3, jc = -k4 (R_data.f90:116-158)
           const int ic = -h3[e], jc = -h4[e], io = -ic, jo = -jc;
           int vi, wi;
@@ -650,7 +677,7 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
           }
         } else {  // ich = k3, io = k4 (R_data.f90:189-206)
           const int ich = h3[e], io = h4[e];
-          const int vi = nbf + a * P->npv + vq[e];
+          const int vi = nbf + vq[e];
           int wi;
           if (io > 0) {
             if (!(rc = B.vch(io, &wi))) rc = B.hw(ich, B.chan_of(io), vi, wi, cidx);
@@ -663,6 +690,7 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
         }
         if (rc) return rc;
       }
+    }
     P->copyc = it >= 2;
   } else if (icase == 1) {
     if (c->nkap < 1 || (int)c->h_kbs.size() < nbf)
@@ -808,8 +836,8 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
   P->any_block = !bt.empty();
 
   // ---- device copies (plan memory)
-  const size_t N = (size_t)n + 1, na = P->na;
-  if (bt.size() > 2 * N * na || ht.size() > 2 * N * na || st.size() > 2 * N * na)
+  const size_t N = (size_t)n + 1;
+  if (bt.size() > 2 * N || ht.size() > 2 * N || st.size() > 2 * N)
     return set_err(c, DBSRG_ECUDA, "structure terms overflow");
   char *base = (char *)dev;
   auto take = [&](size_t bytes) {
@@ -818,7 +846,7 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
     return (void *)p;
   };
   P->lcd = (double *)take(sizeof(double) * N);
-  P->Ce = (double *)take(sizeof(double) * N * na);
+  P->Ce = (double *)take(sizeof(double) * N);
   P->pots = (int2 *)take(sizeof(int2) * N);
   P->vjobs = (int2 *)take(sizeof(int2) * N);
   P->ljobs = (int2 *)take(sizeof(int2) * N);
@@ -826,14 +854,24 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
   P->ej1 = (int *)take(sizeof(int) * N);
   P->ej2 = (int *)take(sizeof(int) * N);
   P->elv = (int *)take(sizeof(int) * N);
-  P->terms = (StTerm *)take(sizeof(StTerm) * 2 * N * na);
-  P->hvterms = (StTerm *)take(sizeof(StTerm) * 2 * N * na);
-  P->scterms = (StTerm *)take(sizeof(StTerm) * 2 * N * na);
-  P->blist = (int *)take(sizeof(int) * (2 * N * na + 2));
+  // the factored forms' pair potentials serve the list where every potential
+  // is of two bound orbitals
+  std::vector<int> ppix;
+  P->fact = P->family >= 0 && c->precision != DBSRG_PLAIN_FP64 && pair_potentials_fit(c);
+  for (const int2 &pr : pots) {
+    const int x = c->h_bmap[pr.x - 1], y = c->h_bmap[pr.y - 1];
+    if (x < 0 || y < 0) P->fact = false;
+    ppix.push_back(x * c->nbound + y);
+  }
+  P->ppix = (int *)take(sizeof(int) * N);
+  P->terms = (StTerm *)take(sizeof(StTerm) * 2 * N);
+  P->hvterms = (StTerm *)take(sizeof(StTerm) * 2 * N);
+  P->scterms = (StTerm *)take(sizeof(StTerm) * 2 * N);
+  P->blist = (int *)take(sizeof(int) * (2 * N + 2));
   P->bstart = P->blist + blist.size();
-  P->hvcol = (int *)take(sizeof(int) * (2 * N * na + 2));
+  P->hvcol = (int *)take(sizeof(int) * (2 * N + 2));
   P->hvstart = P->hvcol + hvcol.size();
-  P->scstart = (int *)take(sizeof(int) * (2 * N * na + 2));
+  P->scstart = (int *)take(sizeof(int) * (2 * N + 2));
   if ((size_t)((char *)base - (char *)dev) > structure_plan_bytes(c, icase, itype, n))
     return set_err(c, DBSRG_ECUDA, "structure plan overflow");
   auto up = [&](void *dst, const void *src, size_t bytes) -> int {
@@ -847,6 +885,7 @@ int plan_structures(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const i
       (rc = up(P->ej1, ej1.data(), sizeof(int) * n)) ||
       (rc = up(P->ej2, ej2.data(), sizeof(int) * n)) ||
       (rc = up(P->elv, elv.data(), sizeof(int) * n)) ||
+      (P->fact && (rc = up(P->ppix, ppix.data(), sizeof(int) * ppix.size()))) ||
       (rc = up(P->terms, bt.data(), sizeof(StTerm) * bt.size())) ||
       (rc = up(P->hvterms, ht.data(), sizeof(StTerm) * ht.size())) ||
       (rc = up(P->scterms, st.data(), sizeof(StTerm) * st.size())) ||
@@ -873,31 +912,45 @@ int exec_structures(dbsrg_ctx *c, const StructPlan &P, int w, bool prep) {
   const bool work = prep ? (P.any_block || P.nhv || P.nsc)
                          : (g1 > g0 || (first && (P.nhv > 0 || P.nsc > 0)));
   if (!work) return DBSRG_OK;
-  // the full tables the potentials read (FP64 in every form)
+  // the pair potentials, or the full tables they are contracted from
   const double *tabs[4] = {nullptr, nullptr, nullptr, nullptr};
+  StPots pt{};
+  pt.na = P.na;
   if (P.family >= 0)
     for (int a = 0; a < P.na; a++) {
-      rc = P.family == 0 ? get_rtable(c, P.ttype[a], P.kpol, &tabs[a])
-                         : get_stable(c, P.ttype[a], P.kpol, &tabs[a]);
+      if (P.fact) {
+        // convol case 2 of an R^k table is case 1 of the table with the
+        // electrons exchanged (types 2 and 3 swapped)
+        const bool sw = P.family == 0 && P.icv == 2;
+        const int t = sw && P.ttype[a] >= 2 ? 5 - P.ttype[a] : P.ttype[a];
+        rc = get_pairpot_direct(c, P.family, t, P.kpol, sw ? 1 : P.icv, P.dc1[a], P.dc2[a],
+                                &pt.Y[a]);
+      } else {
+        rc = P.family == 0 ? get_rtable(c, P.ttype[a], P.kpol, &tabs[a])
+                           : get_stable(c, P.ttype[a], P.kpol, &tabs[a]);
+      }
       if (rc) return rc;
     }
   if (prep) return DBSRG_OK;
   if (P.nlv > 0 && !c->hd) return set_err(c, DBSRG_ESTATE, "L_data: no one-electron matrices");
-  // scratch: pair densities and potentials, then the vector pool
+  const double *vch;
+  if ((rc = get_vch(c, &vch))) return rc;
+  // scratch: the vector pool, then (full tables) pair densities and potentials
   const size_t per = (size_t)ns * P.kb;
-  const size_t nvec = (size_t)nbf + (size_t)P.na * P.npv + P.nlv;
-  const size_t xb = al256(sizeof(double) * per * std::max(P.npot, 1));
-  if ((rc = ensure_scratch(c, 2 * xb + sizeof(double) * nvec * ms))) return rc;
-  double *X = (double *)c->scratch;
-  double *Y = (double *)((char *)c->scratch + xb);
-  double *pool = (double *)((char *)c->scratch + 2 * xb);
-  DBSRG_RUN(c, "k_st_vch", k_st_vch<<<(2 * ns * nbf + 255) / 256, 256, 0, st>>>(
-                               ns, nbf, g.fpbs, g.fqbs, c->pq, pool));
+  const size_t pb = al256(sizeof(double) * ((size_t)P.npv + P.nlv) * ms);
+  const size_t xb = P.fact ? 0 : al256(sizeof(double) * per * std::max(P.npot, 1));
+  if ((rc = ensure_scratch(c, pb + (1 + (size_t)P.na) * xb + 256))) return rc;
+  double *pool = (double *)c->scratch;
+  double *X = (double *)((char *)c->scratch + pb);
   if (P.copyc)
-    DBSRG_RUN(c, "k_st_copyc", k_st_copyc<<<(n * P.na + 255) / 256, 256, 0, st>>>(
-                                   n, P.na, P.lcd, P.Ce));
+    DBSRG_RUN(c, "k_st_copyc", k_st_copyc<<<(n + 255) / 256, 256, 0, st>>>(n, P.lcd, P.Ce));
   if (P.family >= 0 && P.npot > 0) {
     for (int a = 0; a < P.na; a++) {
+      pt.c1[a] = P.ec1[a];
+      pt.c2[a] = P.ec2[a];
+      pt.ipo[a] = P.ipo[a];
+      pt.ipv[a] = P.ipv[a];
+      if (P.fact) continue;
       for (int p0 = 0; p0 < P.npot; p0 += 65535) {  // grid y limit
         const int np = std::min(65535, P.npot - p0);
         dim3 gd((unsigned)((per + 255) / 256), (unsigned)np);
@@ -906,24 +959,25 @@ int exec_structures(dbsrg_ctx *c, const StructPlan &P, int w, bool prep) {
                                                    P.dc1[a], P.dc2[a], c->pq, X + per * p0));
       }
       // convol case icv of every pair density with the full table
+      double *Y = (double *)((char *)X + (1 + (size_t)a) * xb);
       if ((rc = band_contract(c, P.kb, P.icv, tabs[a], P.npot, X, Y))) return rc;
-      if (P.sum_amb)
-        DBSRG_RUN(c, "k_st_sumamb",
-                  k_st_sumamb<<<(n + 7) / 8, 256, 0, st>>>(ns, ks, P.sym, P.kb, n, P.epot, P.ej1,
-                                                           P.ej2, P.ec1[a], P.ec2[a], c->pq, Y,
-                                                           P.lcd, P.Ce + (size_t)a * n));
-      for (int q0 = 0; P.bav && q0 < P.npv; q0 += 65535) {
-        const int nq = std::min(65535, P.npv - q0);
-        dim3 gb((unsigned)((ns + 127) / 128), (unsigned)nq);
-        DBSRG_RUN(c, "k_st_bav",
-                  k_st_bav<<<gb, 128, 0, st>>>(
-                      ns, ks, P.sym, P.dir, P.kb, nq, P.vjobs + q0, P.ipo[a], P.ipv[a], c->pq, Y,
-                      pool + (size_t)ms * (nbf + (size_t)a * P.npv + q0)));
-      }
+      pt.Y[a] = Y;
+    }
+    pt.pix = P.fact ? P.ppix : nullptr;
+    if (P.sum_amb)
+      DBSRG_RUN(c, "k_st_sumamb",
+                k_st_sumamb<<<(n + 7) / 8, 256, 0, st>>>(ns, ks, P.sym, P.kb, n, P.epot, P.ej1,
+                                                         P.ej2, pt, c->pq, P.lcd, P.Ce));
+    for (int q0 = 0; P.bav && q0 < P.npv; q0 += 65535) {
+      const int nq = std::min(65535, P.npv - q0);
+      dim3 gb((unsigned)((ns + 127) / 128), (unsigned)nq);
+      DBSRG_RUN(c, "k_st_bav",
+                k_st_bav<<<gb, 128, 0, st>>>(ns, ks, P.sym, P.dir, P.kb, nq, P.vjobs + q0, pt,
+                                             c->pq, pool + (size_t)ms * q0));
     }
   }
   if (P.nlv > 0) {
-    double *lpool = pool + (size_t)ms * (nbf + (size_t)P.na * P.npv);
+    double *lpool = pool + (size_t)ms * P.npv;
     for (int l0 = 0; l0 < P.nlv; l0 += 65535) {
       const int nl = std::min(65535, P.nlv - l0);
       dim3 gl((unsigned)((ms + 127) / 128), (unsigned)nl);
@@ -939,16 +993,17 @@ int exec_structures(dbsrg_ctx *c, const StructPlan &P, int w, bool prep) {
     const int nb = std::min(65535, g1 - t);
     dim3 grid((unsigned)((ms + 127) / 128), (unsigned)((ms + 31) / 32), (unsigned)nb);
     DBSRG_RUN(c, "k_st_block_terms",
-              k_st_block_terms<<<grid, 128, 0, st>>>(ms, P.blist + t, P.bstart + t, P.terms,
-                                                     P.Ce, pool, g.fppqq, c->hd, hch_base(c)));
+              k_st_block_terms<<<grid, 128, 0, st>>>(ms, nbf, P.blist + t, P.bstart + t, P.terms,
+                                                     P.Ce, vch, pool, g.fppqq, c->hd,
+                                                     hch_base(c)));
   }
   if (first && P.nhv > 0) {
     if (!c->hcp) return set_err(c, DBSRG_ESTATE, "no perturbers allocated");
     for (int t = 0; t < P.nhv; t += 65535) {
       dim3 grid((unsigned)((ms + 127) / 128), (unsigned)std::min(65535, P.nhv - t));
       DBSRG_RUN(c, "k_st_hv_terms",
-                k_st_hv_terms<<<grid, 128, 0, st>>>(ms, P.hvcol + t, P.hvstart + t, P.hvterms,
-                                                    P.Ce, pool, c->hcp));
+                k_st_hv_terms<<<grid, 128, 0, st>>>(ms, nbf, P.hvcol + t, P.hvstart + t,
+                                                    P.hvterms, P.Ce, vch, pool, c->hcp));
     }
   }
   if (first && P.nsc > 0)  // one thread per scalar: a 1-D grid of ceil(nsc/128) blocks

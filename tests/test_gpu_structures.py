@@ -325,3 +325,26 @@ def test_core_energy_shift_scales_hch_hcp_hp(wl):
         m.gen_matrix(L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
     compare(a, m, wl, lists)
     a.close()
+
+
+@pytest.mark.parametrize("precision", [FACTOR_FP64, SPLIT_BF16])
+@pytest.mark.parametrize("extra,unbound", [(0, False), (0, True), (62, False)])
+def test_pair_potential_and_full_table_routes(precision, extra, unbound):
+    """The structure lists in the factored forms: from the pair potentials of
+    the bound orbitals, and from the full tables where a K1 orbital is not
+    bound or more than 64 orbitals are (bound orbitals after the channel
+    ones).  The orbitals added and the unbound ones (zero coefficients) leave
+    the oracle's result as it is."""
+    w = synth.structures_case(seed=55)
+    if extra:
+        add = np.concatenate([w.pq[:, :, : w.nbound]] * (extra // w.nbound + 1), axis=2)
+        w.pq = np.asfortranarray(np.concatenate([w.pq, add[:, :, :extra]], axis=2))
+        w.ipbs = np.concatenate([w.ipbs, np.zeros(extra, np.int32)])
+        w.kbs = np.concatenate([w.kbs, np.full(extra, w.kbs[0], np.int32)])
+    for L in w.lists:
+        if unbound and L.icase in (2, 3):
+            L.k1 = L.k1.copy()
+            L.k1[-1] = synth.IBO + w.nbound + 1  # a bound orbital with a channel orbital
+    a, m = run_both(w, w.lists, precision)
+    compare(a, m, w, w.lists)
+    a.close()
