@@ -184,80 +184,109 @@ __global__ void k_density_acc(int ns, int ks, char sym, int ncol, int na, DensSp
 // :2517-2608): for every segment n of the chunk
 //   case 1: a(i,ip) = sum_{j,jp} d(j,jp) rkb(i,j,ip,jp)
 //   case 2: a(j,jp) = sum_{i,ip} d(i,ip) rkb(i,j,ip,jp)
-// as one product over all segments that share the table: rows r=(i,ip),
-// columns n, contraction over (j,jp).  Tiles: 64 rows x 64 segments x 16,
-// 256 threads with 4x4 outputs each.
-constexpr int GBM = 64, GBN = 64, GBK = 16;
+// as one product over all segments that share the table: rows q = (i,ip)
+// flattened over the band, columns n, contraction over (j,jp).  Tiles of 64
+// rows x BN segments x 16, 256 threads with TM x TN outputs each.  The work is
+// bound by the FP64 pipe (about 1.75 FMAs a clock and SM), so what counts is
+// that no output is padding and every SM has blocks: BN follows the number
+// of segments (band_contract), the rows run on across band columns, and the
+// band columns of the contraction are split over blockIdx.z where the tiles
+// alone would leave SMs idle (partial sums in A[z], added by k_sum_parts in
+// order).  ns 101, about 8 segments a list: 1466 us a launch with 64 x 64 tiles
+// of one band column (18 or 34 blocks, seven of eight columns padding), 49 us
+// and 6 us for the sums this way; ns 400, 40 channels (about 40 segments):
+// 9.8 -> 4.5 ms a launch.
+constexpr int GBM = 64, GBK = 16;
 
+template <int BN>
 __global__ void __launch_bounds__(256) k_band_contract(int ns, int kb, int icase,
                                                       const double *__restrict__ rkb,
                                                       int nsg, const double *__restrict__ X,
-                                                      double *__restrict__ A) {
+                                                      double *__restrict__ A, int cper) {
+  constexpr int TM = BN >= 32 ? 4 : BN >= 8 ? 2 : 1;
+  constexpr int TN = GBM * BN / 256 / TM;
+  constexpr int TX = BN / TN;
   __shared__ double Rs[GBK][GBM + 1];
-  __shared__ double Xs[GBK][GBN + 1];
-  const int nrt = (ns + GBM - 1) / GBM;  // row tiles per band column
-  const int rt = blockIdx.x % nrt;
-  const int obp = blockIdx.x / nrt;  // output band column (ip for case 1)
-  const int n0 = blockIdx.y * GBN;
-  const int r0 = rt * GBM;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const size_t per = (size_t)ns * kb;
+  __shared__ double Xs[GBK][BN + 1];
+  const int n0 = blockIdx.y * BN;
+  const int q0 = blockIdx.x * GBM;
+  const int per = ns * kb;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const size_t ns2 = (size_t)ns * ns;
-  double acc[4][4];
+  // the table rows this thread loads: case 1 one row (consecutive threads
+  // read consecutive rows), case 2 four rows of 16 consecutive columns
+  constexpr int NL = GBM * GBK / 256;
+  int lr[NL], lc[NL];
+  size_t lbase[NL];
+  bool lok[NL];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int k = 0; k < NL; k++) {
+    lr[k] = icase == 1 ? threadIdx.x % GBM : threadIdx.x / GBK + k * (256 / GBK);
+    lc[k] = icase == 1 ? threadIdx.x / GBM + k * (256 / GBM) : threadIdx.x % GBK;
+    const int q = q0 + lr[k];
+    const int r = q % ns, ob = q / ns;
+    lok[k] = q < per;
+    lbase[k] = icase == 1 ? (size_t)r + ns2 * ob : (size_t)ns * r + ns2 * (size_t)kb * ob;
+  }
+  double acc[TM][TN];
 #pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-  for (int cbp = 0; cbp < kb; cbp++) {  // contracted band column
+  for (int a = 0; a < TM; a++)
+#pragma unroll
+    for (int b = 0; b < TN; b++) acc[a][b] = 0.0;
+  const int cb1 = min(kb, (int)(blockIdx.z + 1) * cper);
+  for (int cbp = blockIdx.z * cper; cbp < cb1; cbp++) {  // contracted band column
     for (int c0 = 0; c0 < ns; c0 += GBK) {
-      // table tile: rows r0..r0+63 (output index), cols c0..c0+15
-      for (int q = threadIdx.x; q < GBK * GBM; q += 256) {
-        int rr = q % GBM, cc = q / GBM;
-        int r = r0 + rr, cidx = c0 + cc;
-        double v = 0.0;
-        if (r < ns && cidx < ns) {
-          size_t off;
-          if (icase == 1)  // rkb(r, cidx, obp, cbp)
-            off = (size_t)r + (size_t)ns * cidx + ns2 * ((size_t)obp + (size_t)kb * cbp);
-          else  // rkb(cidx, r, cbp, obp)
-            off = (size_t)cidx + (size_t)ns * r + ns2 * ((size_t)cbp + (size_t)kb * obp);
-          v = rkb[off];
-        }
-        Rs[cc][rr] = v;
+      // case 1: rkb(r, cidx, obp, cbp); case 2: rkb(cidx, r, cbp, obp)
+#pragma unroll
+      for (int k = 0; k < NL; k++) {
+        const int cidx = c0 + lc[k];
+        Rs[lc[k]][lr[k]] =
+            lok[k] && cidx < ns
+                ? rkb[icase == 1 ? lbase[k] + (size_t)ns * cidx + ns2 * (size_t)kb * cbp
+                                 : lbase[k] + (size_t)cidx + ns2 * cbp]
+                : 0.0;
       }
-      for (int q = threadIdx.x; q < GBK * GBN; q += 256) {
-        int cc = q % GBK, nn = q / GBK;
-        int cidx = c0 + cc, n = n0 + nn;
-        double v = 0.0;
-        if (cidx < ns && n < nsg) v = X[(size_t)n * per + cidx + (size_t)ns * cbp];
-        Xs[cc][nn] = v;
+      for (int q = threadIdx.x; q < GBK * BN; q += 256) {
+        const int cc = q % GBK, nn = q / GBK;
+        const int cidx = c0 + cc, n = n0 + nn;
+        Xs[cc][nn] = cidx < ns && n < nsg ? X[(size_t)n * per + cidx + (size_t)ns * cbp] : 0.0;
       }
       __syncthreads();
+      const int kc = min(GBK, ns - c0);
+      for (int kk = 0; kk < kc; kk++) {
+        double rv[TM], xv[TN];
 #pragma unroll
-      for (int kk = 0; kk < GBK; kk++) {
-        double rv[4], xv[4];
+        for (int a = 0; a < TM; a++) rv[a] = Rs[kk][ty * TM + a];
 #pragma unroll
-        for (int a = 0; a < 4; a++) rv[a] = Rs[kk][ty * 4 + a];
+        for (int b = 0; b < TN; b++) xv[b] = Xs[kk][tx * TN + b];
 #pragma unroll
-        for (int b = 0; b < 4; b++) xv[b] = Xs[kk][tx * 4 + b];
+        for (int a = 0; a < TM; a++)
 #pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-          for (int b = 0; b < 4; b++) acc[a][b] = fma(rv[a], xv[b], acc[a][b]);
+          for (int b = 0; b < TN; b++) acc[a][b] = fma(rv[a], xv[b], acc[a][b]);
       }
       __syncthreads();
     }
   }
+  double *Az = A + (size_t)blockIdx.z * nsg * per;
 #pragma unroll
-  for (int a = 0; a < 4; a++) {
-    int r = r0 + ty * 4 + a;
-    if (r >= ns) continue;
+  for (int a = 0; a < TM; a++) {
+    const int q = q0 + ty * TM + a;
+    if (q >= per) continue;
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
-      int n = n0 + tx * 4 + b;
-      if (n < nsg) A[(size_t)n * per + r + (size_t)ns * obp] = acc[a][b];
+    for (int b = 0; b < TN; b++) {
+      const int n = n0 + tx * TN + b;
+      if (n < nsg) Az[(size_t)n * per + q] = acc[a][b];
     }
   }
+}
+
+// A[q] = the nz partial sums P[z][q] in order
+__global__ void k_sum_parts(size_t n, int nz, const double *P, double *A) {
+  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  double s = P[q];
+  for (int z = 1; z < nz; z++) s += P[(size_t)z * n + q];
+  A[q] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -1048,10 +1077,7 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
       const double *Xa = X + (size_t)a * nm * per;
       double *Ya = Y + (size_t)a * nm * per;
       if (icv <= 2) {
-        int nrt = (ns + GBM - 1) / GBM;
-        dim3 gg((unsigned)(nrt * P.kb), (unsigned)((nm + GBN - 1) / GBN));
-        DBSRG_RUN(c, "k_band_contract",
-                  k_band_contract<<<gg, 256, 0, st>>>(ns, P.kb, icv, tabs[a], nm, Xa, Ya));
+        if ((rc2 = band_contract(c, P.kb, icv, tabs[a], nm, Xa, Ya))) return rc2;
       } else {
         int mode = P.tabfam == 0 ? 0 : (icv == 3 ? 1 : 2);
         dim3 gx((unsigned)(((size_t)ns * ns + 255) / 256), (unsigned)((nm + XNB - 1) / XNB));
@@ -1087,13 +1113,46 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
 int band_contract(dbsrg_ctx *c, int kb, int icase, const double *rkb, int nsg, const double *X,
                   double *Y) {
   const int ns = c->g.ns;
-  const int nrt = (ns + GBM - 1) / GBM;
-  for (int s0 = 0; s0 < nsg; s0 += 65535 * GBN) {
-    const int nn = std::min(nsg - s0, 65535 * GBN);
-    const size_t off = (size_t)s0 * ns * kb;
-    dim3 gg((unsigned)(nrt * kb), (unsigned)((nn + GBN - 1) / GBN));
-    DBSRG_RUN(c, "k_band_contract",
-              k_band_contract<<<gg, 256, 0, c->stream>>>(ns, kb, icase, rkb, nn, X + off, Y + off));
+  const size_t per = (size_t)ns * kb;
+  const unsigned nrt = (unsigned)((per + GBM - 1) / GBM);
+  for (int s0 = 0; s0 < nsg;) {
+    // segments per tile: the least padding, the wider tile where two pad the
+    // same (it reads the table less often)
+    const int nn = std::min(nsg - s0, 65535 * 4);
+    int bn = 64;
+    auto padded = [&](int b) { return (nn + b - 1) / b * b; };
+    for (int b : {32, 16, 8, 4})
+      if (padded(b) < padded(bn)) bn = b;
+    const unsigned nt = (unsigned)((nn + bn - 1) / bn);
+    // split of the contracted band columns: at least four blocks an SM (one
+    // block holds 8 warps, and the FP64 pipe wants 16 or more)
+    const long long tiles = (long long)nrt * nt;
+    const int want = (int)std::min<long long>(kb, (4LL * c->nsm + tiles - 1) / tiles);
+    const int cper = (kb + want - 1) / want, nz = (kb + cper - 1) / cper;
+    double *out = Y + (size_t)s0 * per;
+    if (nz > 1) {
+      int rc = ensure_fscratch(c, sizeof(double) * nz * nn * per);
+      if (rc) return rc;
+      out = (double *)c->fscratch;
+    }
+    const double *Xs = X + (size_t)s0 * per;
+    const dim3 gg(nrt, nt, (unsigned)nz);
+    auto launch = [&](auto k) -> int {
+      DBSRG_RUN(c, "k_band_contract",
+                k<<<gg, 256, 0, c->stream>>>(ns, kb, icase, rkb, nn, Xs, out, cper));
+      return DBSRG_OK;
+    };
+    const int rc = bn == 64   ? launch(k_band_contract<64>)
+                   : bn == 32 ? launch(k_band_contract<32>)
+                   : bn == 16 ? launch(k_band_contract<16>)
+                   : bn == 8  ? launch(k_band_contract<8>)
+                              : launch(k_band_contract<4>);
+    if (rc) return rc;
+    if (nz > 1)
+      DBSRG_RUN(c, "k_sum_parts",
+                k_sum_parts<<<(unsigned)((nn * per + 255) / 256), 256, 0, c->stream>>>(
+                    nn * per, nz, out, Y + (size_t)s0 * per));
+    s0 += nn;
   }
   return DBSRG_OK;
 }

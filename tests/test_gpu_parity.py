@@ -161,3 +161,14 @@ def test_update_hx_matches_oracle():
         ref[:, :, w.icc[ich - 1, ich - 1] - 1] += fppqq
     ref[:, :, w.icc[0, 1] - 1] += (2.0 * (0.5 * fppqq)).T
     assert relmax(a.get_matrix(), ref) <= TIGHT
+
+
+@pytest.mark.parametrize("ns,nch", [(40, 1), (41, 3), (40, 8), (37, 12)])
+def test_band_contraction_tiles_by_segment_count(ns, nch):
+    """One, six, 36 and 78 segments per list: the segment tiles of the plain
+    band contraction and the splits of its contracted columns, 's' and 'n'
+    storage."""
+    w = synth.small(ns=ns, nch=nch, mk=1, n_entries=40 * nch, breit=True, seed=31)
+    a, m = run_both(w)
+    check_blocks(a, m, w)
+    a.close()
