@@ -190,12 +190,11 @@ __global__ void k_density_acc(int ns, int ks, char sym, int ncol, int na, DensSp
 // bound by the FP64 pipe (about 1.75 FMAs a clock and SM), so what counts is
 // that no output is padding and every SM has blocks: BN follows the number
 // of segments (band_contract), the rows run on across band columns, and the
-// band columns of the contraction are split over blockIdx.z where the tiles
-// alone would leave SMs idle (partial sums in A[z], added by k_sum_parts in
-// order).  ns 101, about 8 segments a list: 1466 us a launch with 64 x 64 tiles
+// band columns of the contraction are split over blockIdx.z (partial sums in
+// A[z], added by k_sum_parts in order).  ns 101, about 8 segments a list: 1466 us a launch with 64 x 64 tiles
 // of one band column (18 or 34 blocks, seven of eight columns padding), 49 us
 // and 6 us for the sums this way; ns 400, 40 channels (about 40 segments):
-// 9.8 -> 4.5 ms a launch.
+// 9.8 -> 4.2 ms a launch.
 constexpr int GBM = 64, GBK = 16;
 
 template <int BN>
@@ -1115,20 +1114,22 @@ int band_contract(dbsrg_ctx *c, int kb, int icase, const double *rkb, int nsg, c
   const int ns = c->g.ns;
   const size_t per = (size_t)ns * kb;
   const unsigned nrt = (unsigned)((per + GBM - 1) / GBM);
+  // split of the contracted band columns: four blocks an SM with one segment
+  // tile (a block holds 8 warps, and the FP64 pipe wants 16 or more).  It
+  // depends on the table's shape only: a segment's sum has the same order
+  // whatever segments share the launch, so windows and chunks of a list give
+  // the same bits.
+  const int want = std::min<int>(kb, (4 * 152 + (int)nrt - 1) / (int)nrt);
+  const int cper = (kb + want - 1) / want, nz = (kb + cper - 1) / cper;
   for (int s0 = 0; s0 < nsg;) {
     // segments per tile: the least padding, the wider tile where two pad the
-    // same (it reads the table less often)
-    const int nn = std::min(nsg - s0, 65535 * 4);
+    // same (it reads the table less often); 512 segments bound the partial sums
+    const int nn = std::min(nsg - s0, nz > 1 ? 512 : 65535 * 4);
     int bn = 64;
     auto padded = [&](int b) { return (nn + b - 1) / b * b; };
     for (int b : {32, 16, 8, 4})
       if (padded(b) < padded(bn)) bn = b;
     const unsigned nt = (unsigned)((nn + bn - 1) / bn);
-    // split of the contracted band columns: at least four blocks an SM (one
-    // block holds 8 warps, and the FP64 pipe wants 16 or more)
-    const long long tiles = (long long)nrt * nt;
-    const int want = (int)std::min<long long>(kb, (4LL * c->nsm + tiles - 1) / tiles);
-    const int cper = (kb + want - 1) / want, nz = (kb + cper - 1) / cper;
     double *out = Y + (size_t)s0 * per;
     if (nz > 1) {
       int rc = ensure_fscratch(c, sizeof(double) * nz * nn * per);
