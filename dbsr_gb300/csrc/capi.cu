@@ -762,6 +762,23 @@ static std::vector<int> host_windows(int iicc, int nwin, int nslot) {
   return ws;
 }
 
+// blocks per window of dbsrg_assemble_to_host when the caller leaves them to
+// the library: at most tune_windows windows, of at least 2 GB each.  A window
+// costs every list a round of launches (5 to 9 ms at 59 lists), what it hides
+// is the copy of the one before (2 GB: 10 ms on this link), so smaller ones
+// cost more than they hide.  24 channels of ns 351 (1.2 GB): 93 ms with 16
+// windows, 36 with one; 6 GB: 102 with 16, 65-70 with two to six; 16.6 GB: 155
+// with 16, 130 with 8; at 37 GB the 16 windows of the tuning stay.  Two
+// windows have to fit the allocation.
+static int default_window(const dbsrg_ctx *c, int iicc) {
+  const int least = std::max(1, (iicc + c->tune_windows - 1) / c->tune_windows);
+  const double bytes = 8.0 * (double)c->g.ms * c->g.ms * iicc;
+  const int nw = (int)std::min(std::max(bytes / 2.0e9, 1.0), (double)c->tune_windows);
+  const int nwin = std::max(least, (iicc + nw - 1) / nw);
+  if (nwin >= iicc && iicc <= c->hcap) return iicc;
+  return std::max(least, std::min(nwin, c->hcap / 2));
+}
+
 int dbsrg_assemble_to_host(dbsrg_ctx *c, int nlists, const dbsrg_list *lists, int nwin,
                            double *hch_host, double *acf_host) {
   if (!c) return DBSRG_EINVAL;
@@ -771,7 +788,7 @@ int dbsrg_assemble_to_host(dbsrg_ctx *c, int nlists, const dbsrg_list *lists, in
   cudaSetDevice(c->device);
   SETTLE(c);
   const int iicc = c->iicc;
-  if (nwin <= 0) nwin = std::max(1, (iicc + c->tune_windows - 1) / c->tune_windows);
+  if (nwin <= 0) nwin = default_window(c, iicc);
   nwin = std::min(nwin, iicc);
   const int nslot = nwin < iicc ? 2 : 1;
   if (nslot * nwin > c->hcap)

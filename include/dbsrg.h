@@ -200,8 +200,9 @@ int dbsrg_assemble_to_host(dbsrg_ctx *ctx, int nlists, const dbsrg_list *lists,
  * runs on the calling thread with the window's blocks blo .. blo+nblocks-1
  * (hch layout) and may read them until it returns, the device meanwhile
  * assembling the next window.  Windows, their sizes (first and last
- * window short), nwin <= 0, the allocation rule, acf_host and the zeroed
- * parts are as for dbsrg_assemble_to_host.  No counterpart in DBSR_MAT3,
+ * window short), the allocation rule, acf_host and the zeroed parts are as
+ * for dbsrg_assemble_to_host; nwin <= 0 means iicc / "windows" blocks,
+ * rounded up.  No counterpart in DBSR_MAT3,
  * which holds the whole matrix (updates.f90:2-76) and writes it with
  * Record_matrix. */
 int dbsrg_assemble_streamed_host(dbsrg_ctx *ctx, int nlists,
@@ -526,7 +527,8 @@ int dbsrg_sync(dbsrg_ctx *ctx);
  *   "xchunk"  segments per pass of the factored exchange (default 256; the
  *             batch of the Z-digit and tensor-core exchange kernels)
  *   "dchunk"  segments per pass of the factored direct contraction (4096)
- *   "windows" windows of dbsrg_assemble_to_host when nwin <= 0 (8)
+ *   "windows" most windows of dbsrg_assemble_to_host when nwin <= 0 (8;
+ *             fewer where a window would hold less than 2 GB)
  * Results do not depend on them (every block sums the same terms in the
  * same order). */
 int dbsrg_set_tuning(dbsrg_ctx *ctx, const char *name, int value);

@@ -237,3 +237,16 @@ def test_host_matrix_destination():
     hm.close()
     x = np.zeros(16)
     assert load().dbsrg_host_free(C.c_void_p(x.ctypes.data)) == -1
+
+
+@pytest.mark.parametrize("hcap", [15, 4, 5])
+def test_default_windows_fit_the_allocation(hcap):
+    """nwin <= 0: one window where the whole matrix is held, otherwise windows
+    two of which fit the blocks allocated; the same bits either way."""
+    w = synth.small(ns=50, nch=5, mk=2, n_entries=600, seed=59)
+    h0, acf0 = full(w, SPLIT_BF16)
+    a = make(w, SPLIT_BF16, window=hcap)
+    out, acf = a.assemble_to_host(items(w))
+    a.close()
+    assert np.array_equal(out, h0)
+    assert np.array_equal(acf, acf0)
