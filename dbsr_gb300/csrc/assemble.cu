@@ -646,7 +646,7 @@ struct Chunk {
 };
 struct ListPlan {
   int icase = 0, itype = 0, kpol = 0, n = 0, nseg = 0;
-  bool factored = false, split_x = false;
+  bool factored = false, split_x = false, dseg = false;
   int na = 0, icv = 0, tabfam = 0, ncol = 0, kb = 0;
   char sym_d = 's';
   size_t per = 0;
@@ -906,6 +906,9 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
       return set_err(c, DBSRG_ECUDA, "inconsistent segment table");
   }
 
+  P.dseg = P.factored && P.icv <= 2 && g.ks <= 9 &&
+           direct_by_segment(c, P.tabfam, P.icv, P.na, P.ttype, nseg, n);
+
   // ---- chunks of owner segments per window, each owner with its partner (a
   // channel pair listed in both orders maps to one block; both lists
   // contribute to that block in list order within every atype, so they stay
@@ -1054,6 +1057,7 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
       job.cd = P.lcd;
       job.cdf = P.lcdf;
       job.Y = Y;
+      job.dseg = P.dseg;
       job.split = c->precision == DBSRG_SPLIT_BF16;
       job.xq = ch.nxq ? P.dxq + ch.xoff : nullptr;
       job.hxq = ch.nxq ? P.hxq.data() + ch.xoff : nullptr;
@@ -1107,6 +1111,25 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
 }
 
 }  // namespace
+
+int scatter_band(dbsrg_ctx *c, int na, const int *ii, const int *jj, char sym, int ncol, int nm,
+                 const int *members, int nown, const int *own, const SegInfo *info,
+                 const double *Y) {
+  const int ns = c->g.ns, ks = c->g.ks;
+  ScatterSpec sp{};
+  sp.na = na;
+  sp.sym = sym;
+  sp.ncol = ncol;
+  for (int a = 0; a < na; a++) {
+    sp.ii[a] = ii[a];
+    sp.jj[a] = jj[a];
+  }
+  dim3 gs((unsigned)(((size_t)4 * ns * (2 * ks - 1) + 255) / 256), (unsigned)nown);
+  DBSRG_RUN(c, "k_scatter",
+            k_scatter<<<gs, 256, 0, c->stream>>>(ns, ks, 1, sp, nm, members, own, info, Y,
+                                                 hch_base(c)));
+  return DBSRG_OK;
+}
 
 // convol cases 1/2 of nsg band densities X with one full table (k_band_contract)
 int band_contract(dbsrg_ctx *c, int kb, int icase, const double *rkb, int nsg, const double *X,

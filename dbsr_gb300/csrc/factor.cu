@@ -37,6 +37,7 @@
 // (exchange_tc.cu).
 #include "internal.cuh"
 #include "ff.cuh"
+#include "pairs.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -49,44 +50,6 @@ constexpr int BAND = FAR - 1;     // near band |y - x| <= 8
 constexpr int NDB = 2 * BAND + 1; // band diagonals
 constexpr int PXC = 4;            // output rows per block of the band pair potentials
 constexpr int PBC = 4;            // second-orbital chunk of the diagonal-cell stage
-
-struct PairSpec {
-  int k1, k2, sym;  // orders of the first / second function; packed symmetric
-};
-
-__device__ __forceinline__ int pidx(PairSpec s, int h1, int h2) {  // 1-based locals
-  if (s.sym) {
-    int a = min(h1, h2), b = max(h1, h2);
-    return (a - 1) * s.k1 - ((a - 1) * (a - 2)) / 2 + (b - a);
-  }
-  return (h1 - 1) * s.k2 + (h2 - 1);
-}
-
-// bases of the four functions of a table: 1 = P, 2 = Q
-struct TableBases {
-  int a1, a2, b1, b2;
-  PairSpec e1, e2;
-};
-
-TableBases table_bases(const DeviceGrid &g, int family, int type) {
-  TableBases t;
-  auto ord = [&](int b) { return b == 1 ? g.ksp : g.ksq; };
-  if (family == 0) {
-    int A = (type == 0 || type == 2) ? 1 : 2, B = (type == 0 || type == 3) ? 1 : 2;
-    t.a1 = t.a2 = A;
-    t.b1 = t.b2 = B;
-    t.e1 = {ord(A), ord(A), 1};
-    t.e2 = {ord(B), ord(B), 1};
-  } else {
-    t.a1 = 1;
-    t.a2 = 2;
-    t.b1 = type == 0 ? 1 : 2;
-    t.b2 = type == 0 ? 2 : 1;
-    t.e1 = {g.ksp, g.ksq, 0};
-    t.e2 = {ord(t.b1), ord(t.b2), 0};
-  }
-  return t;
-}
 
 // target quadrants of the atypes of one list (UPDATE_HS)
 struct QuadSpec {
@@ -1098,6 +1061,11 @@ int ff_of(dbsrg_ctx *c, const double *src, size_t n, const float2 **out) {
   return DBSRG_OK;
 }
 
+int ff_bound_rows(dbsrg_ctx *c, const float2 **out) {
+  const int rc = ensure_brows(c);
+  return rc ? rc : ff_of(c, c->brows, (size_t)2 * c->nbound * c->g.ns, out);
+}
+
 int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
   const DeviceGrid &g = c->g;
   const int ns = g.ns, ks = g.ks, nb = c->nbound;
@@ -1189,7 +1157,8 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
                                               j.family == 0 ? 1 : 0, hch_base(c)));
     return DBSRG_OK;
   }
-  // direct
+  if (j.dseg) return direct_segments(c, j);
+  // direct, from the pair potentials
   KdSet kd{};
   for (int a = 0; a < j.na; a++) {
     if (j.split && j.cdf)

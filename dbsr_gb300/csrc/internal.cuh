@@ -41,6 +41,9 @@ struct DeviceGrid {
 // resident cell moments and diagonal-cell integrals of one table
 struct CellData {
   double *lo1 = nullptr, *hi1 = nullptr, *lo2 = nullptr, *hi2 = nullptr, *rkd = nullptr;
+  // rkd as float-float pairs without padding, rkf[(pair1 + np1 pair2) + cell np1 np2]
+  // (np1, np2 the numbers of pairs of the two electrons)
+  float2 *rkf = nullptr;
 };
 
 // far-field orbital vectors of one exchange table and contraction case:
@@ -338,7 +341,7 @@ int ff_of(dbsrg_ctx *c, const double *src, size_t n, const float2 **out);
 // ---- tables.cu ------------------------------------------------------------
 int build_grid(dbsrg_ctx *c, const double *t_host_or_dev);
 int compute_moments(dbsrg_ctx *c, int which, int k, double *rkm_dev);
-int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd_dev);
+int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd_dev, float2 *rkf_dev = nullptr);
 // returns device pointer of the cached table (building it if needed)
 int get_rtable(dbsrg_ctx *c, int type, int k, const double **out);
 int get_stable(dbsrg_ctx *c, int type, int k, const double **out);
@@ -421,6 +424,7 @@ struct FactorJob {
   const double *cd;
   const float2 *cdf;  // split form: the coefficients as float-float pairs
   double *Y;         // exchange results [a][slot][ns*ns] (FP64 far field)
+  bool dseg;         // direct cases: segment by segment (direct.cu)
   bool split;        // exchange on the tensor cores (split BF16), fused scatter
   int nxq;           // split exchange: (owner block, quadrant) records of the chunk
   const struct XQuad *xq;
@@ -429,6 +433,19 @@ struct FactorJob {
   long long nent;    // entries of the member segments (executed-work statements)
 };
 int factored_contract(dbsrg_ctx *c, const FactorJob &job);
+// float-float copy of the bound-orbital rows (both components)
+int ff_bound_rows(dbsrg_ctx *c, const float2 **out);
+// ---- direct.cu: the direct cases segment by segment
+// whether a list of nseg segments and nent entries takes fewer operations that
+// way than through the pair potentials
+bool direct_by_segment(const dbsrg_ctx *c, int family, int icv, int na, const int *types,
+                       long long nseg, long long nent);
+int direct_segments(dbsrg_ctx *c, const FactorJob &j);
+// UPDATE_HS of band results Y[a][slot][ns*ncol] of na quadrants (ii, jj) into
+// the owners' blocks (assemble.cu), on the context stream
+int scatter_band(dbsrg_ctx *c, int na, const int *ii, const int *jj, char sym, int ncol, int nm,
+                 const int *members, int nown, const int *own, const SegInfo *info,
+                 const double *Y);
 // One quadrant of one owner's block in the split exchange and the terms it
 // receives (UPDATE_HS, updates.f90:110-179), in the order of k_scatter_x
 // (atype-major, owner then partner, direct before transposed).  Term code:

@@ -5,7 +5,9 @@
 // uses explicit round-to-nearest intrinsics where the reference forms a
 // product and then a sum, so the tables reproduce the reference's loop
 // arithmetic instead of a contracted variant.
+#include "ff.cuh"
 #include "internal.cuh"
+#include "pairs.cuh"
 
 #include <cmath>
 
@@ -278,7 +280,7 @@ __global__ void k_triang_points(int nv, int ks, int ksp, int ksq, const double *
 
 __global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, const double *tri,
                          const double *grm, const double *grw, const double *pbsp,
-                         const double *qbsp, double *rkd) {
+                         const double *qbsp, double *rkd, float2 *rkf) {
   extern __shared__ double sm[];
   const int iv = blockIdx.x;  // 0-based interval
   // this block's share of the interval's kk*kk output cells (blockIdx.y of
@@ -391,7 +393,10 @@ __global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, cons
     __syncthreads();
     for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
       int ii = q % kk, jj = q / kk;
-      out[q] = (ii < ik && jj < ik) ? __dadd_rn(A[ii + ik * jj], A[jj + ik * ii]) : 0.0;
+      const bool ok = ii < ik && jj < ik;
+      const double v = ok ? __dadd_rn(A[ii + ik * jj], A[jj + ik * ii]) : 0.0;
+      out[q] = v;
+      if (rkf && ok) rkf[(size_t)iv * ik * ik + ii + (size_t)ik * jj] = ffa::split(v);
     }
   } else if (type == 2 || type == 3) {
     const int ikp = ksp * (ksp + 1) / 2, ikq = ksq * (ksq + 1) / 2;
@@ -408,6 +413,8 @@ __global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, cons
         for (int m = 0; m < ks; m++) s1 = fma(o1[m], INTQ[j + ksq * (jp + ksq * m)], s1);
         for (int m = 0; m < ks; m++) s2 = fma(o2[m], INTP[i + ksp * (ip + ksp * m)], s2);
         v = __dadd_rn(s1, s2);
+        const int n1 = type == 2 ? ikp : ikq;  // pairs of the first electron
+        if (rkf) rkf[(size_t)iv * ikp * ikq + r + (size_t)n1 * cc] = ffa::split(v);
       }
       out[q] = v;
     }
@@ -422,6 +429,7 @@ __global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, cons
         double s = 0.0;
         for (int m = 0; m < ks; m++) s = fma(o[m], INTPQ[j + ksp * (jp + ksq * m)], s);
         v = s;
+        if (rkf) rkf[(size_t)iv * np * np + jj + (size_t)np * ii] = ffa::split(v);
       }
       out[q] = v;
     }
@@ -440,7 +448,7 @@ static int build_triang_points(dbsrg_ctx *c) {
   return DBSRG_OK;
 }
 
-int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd) {
+int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd, float2 *rkf) {
   const DeviceGrid &g = c->g;
   const int ks = g.ks, kk = ks * ks;
   size_t nsm = (size_t)ks * ks + (size_t)ks * ks * g.ksp + (size_t)ks * ks * g.ksq +
@@ -451,7 +459,7 @@ int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd) {
   if (rc) return rc;
   DBSRG_RUN(c, "k_triang",
             k_triang<<<dim3(g.nv, 1), 256, bytes, c->stream>>>(g.nv, ks, g.ksp, g.ksq, type, k, g.tri,
-                                                      g.grm, g.grw, g.pbsp, g.qbsp, rkd));
+                                                      g.grm, g.grw, g.pbsp, g.qbsp, rkd, rkf));
   return DBSRG_OK;
 }
 
@@ -595,8 +603,10 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
   }
   const int nv = g.nv, kk = g.ks * g.ks;
   size_t m = (size_t)kk * nv, d = (size_t)kk * kk * nv;
+  const TableBases tb = table_bases(g, family, type);
+  const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
   double *base = nullptr;
-  if (!(base = (double *)cache_alloc(c, (4 * m + d) * sizeof(double))))
+  if (!(base = (double *)cache_alloc(c, (4 * m + d + f) * sizeof(double))))
     return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
   CellData cd;
   cd.lo1 = base;
@@ -604,18 +614,19 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
   cd.lo2 = base + 2 * m;
   cd.hi2 = base + 3 * m;
   cd.rkd = base + 4 * m;
+  cd.rkf = (float2 *)(cd.rkd + d);
   int rc;
   if (family == 0) {
     int wa = (type == 0 || type == 2) ? 0 : 1, wb = (type == 0 || type == 3) ? 0 : 1;
     const int wh[4] = {wa, wa, wb, wb}, kp[4] = {k, -(k + 1), k, -(k + 1)};
     double *const out[4] = {cd.lo1, cd.hi1, cd.lo2, cd.hi2};
     if ((rc = compute_moment_set(c, 4, wh, kp, out))) return rc;
-    if ((rc = compute_diag_cells(c, type, k, cd.rkd))) return rc;
+    if ((rc = compute_diag_cells(c, type, k, cd.rkd, cd.rkf))) return rc;
   } else {
     const int wh[2] = {2, type == 0 ? 2 : 3}, kp[2] = {k, -(k + 1)};
     double *const out[2] = {cd.lo1, cd.hi2};
     if ((rc = compute_moment_set(c, 2, wh, kp, out))) return rc;
-    if ((rc = compute_diag_cells(c, type == 0 ? 4 : 5, k, cd.rkd))) return rc;
+    if ((rc = compute_diag_cells(c, type == 0 ? 4 : 5, k, cd.rkd, cd.rkf))) return rc;
     cd.hi1 = nullptr;
     cd.lo2 = nullptr;
   }

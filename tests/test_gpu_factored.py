@@ -159,3 +159,33 @@ def test_bound_orbital_limit_of_the_factored_forms():
     h, _ = run(w, PLAIN_FP64, [L])
     ref, _ = oracle(w, [L])
     check(h, ref, 1e-12)
+
+
+@pytest.mark.parametrize("precision,tol", [(FACTOR_FP64, 1e-12), (SPLIT_BF16, 1e-10)])
+@pytest.mark.parametrize("ns,nch,norb,by_segment", [(61, 9, 20, True), (64, 3, 20, True),
+                                                    (60, 13, 4, False)])
+def test_direct_lists_by_segment_and_by_pairs(precision, tol, ns, nch, norb, by_segment):
+    """The direct lists (R^k, S^k structures 6, 7, 16 and 17, channel pairs in
+    both orders) segment by segment -- more segments than the 32 of a warp,
+    fewer, odd and even ns -- and through the pair potentials, whichever the
+    list's counts select; every block against the oracle."""
+    w = synth.small(ns=ns, nch=nch, mk=2, n_entries=60 * nch, breit=True, seed=71, norb=norb)
+    lists = [L for L in w.lists if (L.icase, L.itype) in ((2, 3), (3, 6), (3, 16))]
+    for L in list(lists):
+        if L.icase == 3 and L.kpol % 2:  # the density on the first electron
+            lists.append(synth.CList(3, L.itype + 1, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c))
+    a = Assembler(w.t, w.ks, w.ksp, w.ksq)
+    a.set_orbitals(w.pq, w.ipbs)
+    a.alloc_matrix(w.nch, w.icc, w.iicc, w.mk)
+    a.set_precision(precision)
+    a.timing(True)
+    for L in lists:
+        a.gen_matrix(L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
+    used = a.timing_report()
+    h, acf = a.get_matrix(), a.get_acf()
+    a.close()
+    assert ("k_seg_apply" in used) == by_segment
+    assert ("k_scatter_dp" in used) != by_segment
+    ref, racf = oracle(w, lists)
+    check(h, ref, tol)
+    assert relmax(acf, racf) <= 1e-12
