@@ -1003,14 +1003,17 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
   if (c0 == c1 && nown_acf == 0) return DBSRG_OK;
   // tables of the case (cached after the first use)
   const double *tabs[4] = {nullptr, nullptr, nullptr, nullptr};
+  if (P.icase == 2 && P.factored && P.itype == 4 && (rc = ensure_r_band_tables(c, P.kpol)))
+    return rc;
   for (int a = 0; a < P.na; a++) {
     rc = DBSRG_OK;
     if (P.icase == 2) {
       // the factored path reads only the band |j-i| <= 16 of exchange
-      // tables and no table at all for the direct contraction
+      // tables (type 3 reads type 2's results) and no table at all for the
+      // direct contraction
       if (!P.factored)
         rc = get_rtable(c, a, P.kpol, &tabs[a]);
-      else if (P.itype == 4)
+      else if (P.itype == 4 && a < 3)
         rc = get_band_table(c, 0, a, P.kpol, &tabs[a]);
     } else {
       if (!P.factored)

@@ -244,8 +244,10 @@ void free_tables(dbsrg_ctx *c) {
     cache_free(c, p);
   c->rbtab.clear();
   c->sbtab.clear();
-  for (auto &cd : c->rcell)
-    cache_free(c, cd.lo1);
+  for (auto &r : c->rshare) {
+    cache_free(c, r.mom);
+    for (double *p : r.diag) cache_free(c, p);
+  }
   for (auto &cd : c->scell)
     cache_free(c, cd.lo1);
   free_orbital_products(c);
@@ -253,6 +255,7 @@ void free_tables(dbsrg_ctx *c) {
   c->stab.clear();
   c->quad.clear();
   c->rcell.clear();
+  c->rshare.clear();
   c->scell.clear();
 }
 

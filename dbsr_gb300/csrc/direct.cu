@@ -400,14 +400,8 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
   for (int a = 0; a < j.na; a++)
     if ((rc = get_celldata(c, j.family, j.types[a], j.kpol, &cd[a]))) return rc;
   if (j.prep) return DBSRG_OK;
-  const T *rows;
-  if (FF) {
-    const float2 *f;
-    if ((rc = ff_bound_rows(c, &f))) return rc;
-    rows = (const T *)f;
-  } else {
-    rows = (const T *)c->brows;
-  }
+  // both built before the first list of an assembly is prepared
+  const T *rows = FF ? (const T *)c->browsf : (const T *)c->brows;
   const bool two = j.family == 0;  // both fields (r1 < r2 and r1 > r2 cells)
   const int nset = ncs * (two ? 2 : 1);
   const size_t per = (size_t)ns * ncol;
@@ -462,13 +456,15 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
         ca.ed[s * nm2 + m] = ed;
         ca.comp[s * nm2 + m] = s;
       }
-      // cell integrals: float-float copy (first pair fastest, no padding) or rkd
-      const int n1 = npairs(tb.e1), n2 = npairs(tb.e2);
+      // cell integrals: float-float copy (first pair fastest, no padding) or
+      // rkd; the first pair is the second electron's where tr
+      const int n1 = npairs(x.tr ? tb.e2 : tb.e1), n2 = npairs(x.tr ? tb.e1 : tb.e2);
+      const bool ofirst = (j.icv == 1) != x.tr;
       p.R[o][t] = FF ? (const T *)x.rkf : (const T *)x.rkd;
       p.rcell[o][t] = FF ? (size_t)n1 * n2 : (size_t)kk * kk;
       const int r2 = FF ? n1 : kk;  // stride of the second pair
-      p.rpo[o][t] = j.icv == 1 ? 1 : r2;
-      p.rpd[o][t] = j.icv == 1 ? r2 : 1;
+      p.rpo[o][t] = ofirst ? 1 : r2;
+      p.rpd[o][t] = ofirst ? r2 : 1;
       p.L1[o][t] = j.icv == 1 ? x.lo1 : x.hi2;
       p.L2[o][t] = two ? x.hi1 : nullptr;
       p.comp[o][t] = s;

@@ -99,16 +99,18 @@ __device__ __forceinline__ void write_digit_row(__nv_bfloat16 *D, int NR, int ro
 // over its 32-row tiles
 constexpr int EXP_PER_ROWTILE = 33;
 
-// U (ns x nb, column-major), orbital chunk blockIdx.y (orbitals 32c ..
-// 32c+31) -> digit operand [chunk][slice][NR][TILE] and exponents
-// [chunk][NR*33]
+// Vectors U (blockIdx.z of them, each ns x nb column-major), orbital chunk
+// blockIdx.y (orbitals 32c .. 32c+31) -> digit operands
+// [vector][chunk][slice][NR][TILE] and exponents [vector][chunk][NR*33]
 __global__ void k_udigits(int ns, int nb, int NR, const double *U, __nv_bfloat16 *Dall,
                           int *euall) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int ck = blockIdx.y;
   if (x >= NR * 32) return;
-  __nv_bfloat16 *D = Dall + (size_t)ck * TS * NR * TILE;
-  int *eu = euall + (size_t)ck * NR * EXP_PER_ROWTILE;
+  const size_t op = (size_t)blockIdx.z * gridDim.y + ck;
+  U += (size_t)blockIdx.z * ns * nb;
+  __nv_bfloat16 *D = Dall + op * TS * NR * TILE;
+  int *eu = euall + op * NR * EXP_PER_ROWTILE;
   double vals[32];
   double m = 0.0;
 #pragma unroll
@@ -951,38 +953,33 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
   const int nbk = (nb + 31) / 32;  // chunks of 32 bound orbitals
   if (x.na < 1 || x.na > 4 || x.nm < 1 || (x.nxq < 1 && !x.prep)) return DBSRG_OK;
   cudaStream_t st = c->stream;
-  int rc0;
   const int ntx = (ns + 127) / 128, NR = 4 * ntx, nty = (ns + 31) / 32;
   const size_t sl = (size_t)NR * TILE;
-  // digits of U (and Ul) per table, cached with the far-field vectors
+  // digits of U (and Ul) per table, cached with the far-field vectors; of the
+  // four shared vectors of a k at once (R^k)
   for (int a = 0; a < x.na; a++) {
     FarField *f = const_cast<FarField *>(x.far[a]);
     if (f->Ud) continue;
-    void *d = nullptr;
-    const size_t bytes = 2 * (size_t)nbk * TS * sl * sizeof(__nv_bfloat16) +
-                         2 * (size_t)nbk * NR * EXP_PER_ROWTILE * sizeof(int);
-    if (!(d = cache_alloc(c, bytes))) {
-      return set_err(c, DBSRG_ENOMEM, "digit allocation failed");
-    }
-    f->Ud = d;
-    f->eu = (int *)((char *)d + 2 * (size_t)nbk * TS * sl * sizeof(__nv_bfloat16));
-    for (int m = 0; m < (f->Ul ? 2 : 1); m++)
+    if (x.lower && !f->Vl) return set_err(c, DBSRG_EINVAL, "split exchange: no lower field");
+    const int nvec = f->sh ? 4 : 1;
+    const size_t dn = (size_t)nbk * TS * sl, en = (size_t)nbk * NR * EXP_PER_ROWTILE;
+    void *d = f->sh ? f->sh->D : nullptr;
+    if (!d) {
+      if (!(d = cache_alloc(c, nvec * (dn * sizeof(__nv_bfloat16) + en * sizeof(int)))))
+        return set_err(c, DBSRG_ENOMEM, "digit allocation failed");
+      int *e = (int *)((__nv_bfloat16 *)d + nvec * dn);
+      if (f->sh) {
+        f->sh->D = d;
+        f->sh->e = e;
+      }
       DBSRG_RUN(c, "k_udigits",
-                k_udigits<<<dim3((unsigned)((NR * 32 + 127) / 128), (unsigned)nbk), 128, 0, st>>>(
-                    ns, nb, NR, m ? f->Ul : f->U,
-                    (__nv_bfloat16 *)f->Ud + (size_t)m * nbk * TS * sl,
-                    f->eu + (size_t)m * nbk * NR * EXP_PER_ROWTILE));
-  }
-  const size_t mv = (size_t)ns * nb;
-  if (x.prep) {  // float-float far-field vectors, then nothing per chunk
-    for (int a = 0; a < x.na; a++) {
-      const float2 *v;
-      if (x.lower && !x.far[a]->Vl) return set_err(c, DBSRG_EINVAL, "split exchange: no lower field");
-      if ((rc0 = ff_of(c, x.far[a]->V, mv, &v))) return rc0;
-      if (x.lower && (rc0 = ff_of(c, x.far[a]->Vl, mv, &v))) return rc0;
+                k_udigits<<<dim3((unsigned)(NR * 32 / 32), (unsigned)nbk, (unsigned)nvec), 32, 0,
+                            st>>>(ns, nb, NR, f->sh ? f->sh->W : f->U, (__nv_bfloat16 *)d, e));
     }
-    return DBSRG_OK;
+    f->Ud = (__nv_bfloat16 *)d + (size_t)f->first * dn;
+    f->eu = (f->sh ? f->sh->e : (int *)((__nv_bfloat16 *)d + nvec * dn)) + (size_t)f->first * en;
   }
+  if (x.prep) return DBSRG_OK;
   // per chunk: Z digits, exponents, band rows, error word
   const size_t zel = (size_t)x.na * 2 * x.nm * nbk * TS * sl;
   const size_t zex = (size_t)x.na * 2 * x.nm * nbk * NR * EXP_PER_ROWTILE;
@@ -1008,9 +1005,8 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
   z.lower = x.lower;
   if (!x.cdf) return set_err(c, DBSRG_EINVAL, "split exchange: no float-float coefficients");
   for (int a = 0; a < x.na; a++) {
-    if (x.lower && !x.far[a]->Vl) return set_err(c, DBSRG_EINVAL, "split exchange: no lower field");
-    if ((rc = ff_of(c, x.far[a]->V, mv, &z.V[a]))) return rc;
-    if (x.lower && (rc = ff_of(c, x.far[a]->Vl, mv, &z.Vl[a]))) return rc;
+    z.V[a] = x.far[a]->Vf;
+    z.Vl[a] = x.far[a]->Vlf;
     z.Kb[a] = x.Kbf[a];
   }
   z.members = x.members;

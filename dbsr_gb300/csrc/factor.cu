@@ -65,13 +65,17 @@ struct KdSet {
 };
 
 // ---------------------------------------------------------------------------
-// bound-orbital rows of one component: P[a*ns + x] = pq(x+1, comp, b2o[a])
-__global__ void k_bound_rows(int ns, int nb, const int *b2o, const double *pq, int comp,
-                             double *P) {
+// bound-orbital rows of both components (blockIdx.y):
+// P[a*ns + x] = pq(x+1, comp, b2o[a]), and as float-float pairs
+__global__ void k_bound_rows(int ns, int nb, const int *b2o, const double *pq, double *P,
+                             float2 *Pf) {
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= ns * nb) return;
-  int x = q % ns, a = q / ns;
-  P[q] = pq[(size_t)x + (size_t)ns * (comp - 1) + (size_t)2 * ns * (b2o[a] - 1)];
+  const int x = q % ns, a = q / ns, comp = blockIdx.y;
+  const double v = pq[(size_t)x + (size_t)ns * comp + (size_t)2 * ns * (b2o[a] - 1)];
+  const size_t o = (size_t)comp * ns * nb + q;
+  P[o] = v;
+  Pf[o] = ffa::split(v);
 }
 
 // ordered bound-orbital pair of every entry
@@ -90,13 +94,19 @@ __global__ void k_pair_index(int n, const int *k2, const int *k3, const int *bma
 
 // ---------------------------------------------------------------------------
 // far-field vectors of one electron: Ulo(x,a) = sum_iv sum_xc mlo(pair;iv) p_a(xc)
-// (and Uhi with mhi), x the output function, xc the contracted one.
-// both electrons' vectors in one launch (blockIdx.y)
+// (and Uhi with mhi), x the output function, xc the contracted one, and their
+// float-float copies where asked for.  Both electrons' vectors (R^k: those of
+// the P and Q pairs, which every type of the k shares) in one launch
+// (blockIdx.y).  A thread sums up to 9 cells of 9 functions, nine loads in
+// flight: bound by the latency of those loads.  ns 283, 20 orbitals: 19 us a k,
+// against 4 x 26 us (and 8 conversions of 6 us) with a launch per type that
+// loaded one value at a time.
 struct FarSide {
   PairSpec e;
   int out_first, ko, kc, ccomp;
   const double *mlo, *mhi;
   double *Ulo, *Uhi;
+  float2 *Flo, *Fhi;
 };
 
 __global__ void k_far_vectors(int ns, int nv, int kk, int nb, const int *b2o, const double *pq,
@@ -105,25 +115,34 @@ __global__ void k_far_vectors(int ns, int nv, int kk, int nb, const int *b2o, co
   const PairSpec e = sd.e;
   const int out_first = sd.out_first, ko = sd.ko, kc = sd.kc, ccomp = sd.ccomp;
   const double *mlo = sd.mlo, *mhi = sd.mhi;
-  double *Ulo = sd.Ulo, *Uhi = sd.Uhi;
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= ns * nb) return;
   int x = q % ns + 1, a = q / ns;
   const double *p = pq + (size_t)ns * (ccomp - 1) + (size_t)2 * ns * (b2o[a] - 1) - 1;
   double slo = 0.0, shi = 0.0;
   for (int iv = max(1, x - ko + 1); iv <= min(nv, x); iv++) {
-    int ho = x - iv + 1;
-    for (int hc = 1; hc <= kc; hc++) {
-      int xc = iv + hc - 1;
-      if (xc > ns) break;
-      int pi = out_first ? pidx(e, ho, hc) : pidx(e, hc, ho);
-      size_t o = (size_t)pi + (size_t)kk * (iv - 1);
-      slo = fma(mlo[o], p[xc], slo);
-      if (mhi) shi = fma(mhi[o], p[xc], shi);
+    const int ho = x - iv + 1;
+    double pv[9], lv[9], hv[9];
+#pragma unroll
+    for (int u = 0; u < 9; u++) {
+      const int hc = u + 1, xc = iv + u;
+      const bool ok = hc <= kc && xc <= ns;
+      const size_t o = (size_t)(out_first ? pidx(e, ho, hc) : pidx(e, hc, ho)) +
+                       (size_t)kk * (iv - 1);
+      pv[u] = ok ? p[xc] : 0.0;
+      lv[u] = ok ? mlo[o] : 0.0;
+      hv[u] = ok && mhi ? mhi[o] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 9; u++) {
+      slo = fma(lv[u], pv[u], slo);
+      shi = fma(hv[u], pv[u], shi);
     }
   }
-  Ulo[q] = slo;
-  if (Uhi) Uhi[q] = shi;
+  sd.Ulo[q] = slo;
+  if (sd.Uhi) sd.Uhi[q] = shi;
+  if (sd.Flo) sd.Flo[q] = ffa::split(slo);
+  if (sd.Fhi) sd.Fhi[q] = ffa::split(shi);
 }
 
 // Z(a,y) = sum_{e in segment, first orbital a} c_e V(y, second orbital), also Zl with Vl
@@ -214,12 +233,18 @@ __global__ void __launch_bounds__(256) k_far_field(int ns, int nb, const double 
 // Band table layout: rkb(i, j-i+BW+1, ip, jp) for |j - i| <= BW.
 // FF: the windows split once into float-float pairs, both stages as
 // float-float sums (ff.cuh), Kb written as float-float pairs (float2).
+// Kx: where the results of the table with the electrons exchanged go, element
+// (b a; y, x - y) for (a b; x, y - x).  R^k types 0 and 1 are unchanged under
+// the exchange (Kx = Kout): only the diagonals d >= 0 are computed.  Type 2
+// gives type 3's potentials this way (Kx theirs); S^k has none (Kx null).
+// ns 400, 20 orbitals: an R^k list's potentials 4 x 84 -> 3 launches of 47, 47
+// and 90 us.
 template <bool FF>
 __global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int mode,
                                                    const double *__restrict__ rkb,
                                                    const double *__restrict__ P1,
-                                                   const double *__restrict__ P2,
-                                                   void *__restrict__ Kout) {
+                                                   const double *__restrict__ P2, void *Kout,
+                                                   void *Kx) {
   using S = typename std::conditional<FF, float2, double>::type;
   extern __shared__ double smraw[];
   S *sm = reinterpret_cast<S *>(smraw);
@@ -228,7 +253,7 @@ __global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int m
   const int WLP = WL | 1;              // its stride (odd: no bank conflicts across orbitals)
   const int HX = W * nb + 1;           // stride of H per output row (odd)
   const int x0 = blockIdx.x * PXC + 1; // first output row (1-based)
-  const int d = (int)blockIdx.y - BAND;
+  const int d = Kx == Kout ? (int)blockIdx.y : (int)blockIdx.y - BAND;
   S *Wm = sm;                          // [PXC][W][W]
   S *p1w = Wm + PXC * W * W;           // [nb][WLP]: P1(a, x0-(ks-1)+t)
   S *p2w = p1w + nb * WLP;             // [nb][WLP]: P2(b, x0+d-(ks-1)+t)
@@ -302,14 +327,19 @@ __global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int m
     const S *p = p1w + (size_t)a * WLP + xl;
     const S *h = H + (size_t)xl * HX + b;
     const size_t o = (size_t)pr * per + (size_t)(x - 1) + (size_t)ns * (d + BAND);
+    // the exchanged element; on the diagonal of Kout another thread's own
+    const size_t o2 = (size_t)(b * nb + a) * per + (size_t)(y - 1) + (size_t)ns * (BAND - d);
+    const bool both = Kx && (Kx != Kout || d > 0);
     if constexpr (FF) {
       float sh = 0.0f, sl = 0.0f;
       for (int u = 0; u < W; u++) ffa::mac(p[u], h[(size_t)u * nb], sh, sl);
       static_cast<float2 *>(Kout)[o] = ffa::norm(sh, sl);
+      if (both) static_cast<float2 *>(Kx)[o2] = ffa::norm(sh, sl);
     } else {
       double s = 0.0;
       for (int u = 0; u < W; u++) s = fma(p[u], h[(size_t)u * nb], s);
       static_cast<double *>(Kout)[o] = s;
+      if (both) static_cast<double *>(Kx)[o2] = s;
     }
   }
 }
@@ -407,7 +437,7 @@ __global__ void k_pair_scan(int nv, int npair, double *S0, int suffix0, double *
 // [cv, cv+8], so cells of one phase never share an output.  Two stages:
 // H(po, g1, b) = sum_g2 R P2, then sum_g1 P1 H.
 template <bool FF>
-__global__ void __launch_bounds__(512) k_pair_diag(int ns, int ks, int kk, int nb, int icv,
+__global__ void __launch_bounds__(512) k_pair_diag(int ns, int ks, int kk, int nb, int ofirst,
                                                    char sym, PairSpec eo, PairSpec ed,
                                                    const double *__restrict__ rkd,
                                                    const double *__restrict__ P1,
@@ -453,10 +483,10 @@ __global__ void __launch_bounds__(512) k_pair_diag(int ns, int ks, int kk, int n
   }
   const double *rc = rkd + (size_t)kk * kk * (cv - 1);  // rkd(e1 pair, e2 pair; cv)
   // the cell's table slice: consecutive threads read consecutive table
-  // elements (po fastest for case 1, the density pair fastest otherwise)
+  // elements (ofirst: the output pair is rkd's first index)
   for (int q = threadIdx.x; q < npo * kd; q += blockDim.x) {
     int po, r;
-    if (icv == 1) {
+    if (ofirst) {
       po = q % npo;
       r = q / npo;
     } else {
@@ -466,7 +496,7 @@ __global__ void __launch_bounds__(512) k_pair_diag(int ns, int ks, int kk, int n
     const int g1 = r / k2 + 1, g2 = r % k2 + 1;
     const int pd = pidx(ed, g1, g2);
     Rt[(size_t)po * kd + r] =
-        sv(icv == 1 ? rc[(size_t)po + (size_t)kk * pd] : rc[(size_t)pd + (size_t)kk * po]);
+        sv(ofirst ? rc[(size_t)po + (size_t)kk * pd] : rc[(size_t)pd + (size_t)kk * po]);
   }
   __syncthreads();
   const int ph = (cv - 1) % FAR;
@@ -789,7 +819,8 @@ int pair_index(dbsrg_ctx *c, int n, const int *k2, const int *k3, int *pairs, in
   return DBSRG_OK;
 }
 
-// far-field vectors of (family, type, k, exchange case), cached
+// far-field vectors of (family, type, k, exchange case), cached; R^k (case 3
+// only): views of the four vectors that the types of the k share
 static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const FarField **out) {
   std::map<size_t, FarField> &v = family == 0 ? c->rfar : c->sfar;
   const size_t idx = ((size_t)k * (family == 0 ? 4 : 2) + type) * 2 + (cs == 4 ? 1 : 0);
@@ -799,34 +830,63 @@ static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const
     return DBSRG_OK;
   }
   const DeviceGrid &g = c->g;
-  const CellData *cd;
-  int rc = get_celldata(c, family, type, k, &cd);
-  if (rc) return rc;
   const int ns = g.ns, nb = c->nbound, kk = g.ks * g.ks;
-  size_t m = (size_t)ns * nb;
-  double *base = nullptr;
-  if (!(base = (double *)cache_alloc(c, 4 * m * sizeof(double))))
-    return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
-  FarField f;
-  f.U = base;
-  f.V = base + m;
-  f.Ul = family == 0 ? base + 2 * m : nullptr;
-  f.Vl = family == 0 ? base + 3 * m : nullptr;
-  TableBases tb = table_bases(g, family, type);
-  auto ord = [&](int b) { return b == 1 ? g.ksp : g.ksq; };
-  // electron 1: case 3 output = first function, contracted = second
-  int o1f = cs == 3 ? 1 : 0;
-  int ko1 = ord(cs == 3 ? tb.a1 : tb.a2), kc1 = ord(cs == 3 ? tb.a2 : tb.a1);
-  int cc1 = cs == 3 ? tb.a2 : tb.a1;
-  // electron 2: case 3 output = second function, contracted = first
-  int o2f = cs == 3 ? 0 : 1;
-  int ko2 = ord(cs == 3 ? tb.b2 : tb.b1), kc2 = ord(cs == 3 ? tb.b1 : tb.b2);
-  int cc2 = cs == 3 ? tb.b1 : tb.b2;
-  const FarSide s1{tb.e1, o1f, ko1, kc1, cc1, cd->lo1, family == 0 ? cd->hi1 : nullptr, f.U, f.Ul};
-  const FarSide s2{tb.e2, o2f, ko2, kc2, cc2, cd->hi2, family == 0 ? cd->lo2 : nullptr, f.V, f.Vl};
+  const size_t m = (size_t)ns * nb;
   const dim3 gv((unsigned)((m + 63) / 64), 2);
-  DBSRG_RUN(c, "k_far_vectors",
-            k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.nv, kk, nb, c->b2o, c->pq, s1, s2));
+  const TableBases tb = table_bases(g, family, type);
+  int rc;
+  FarField f;
+  if (family == 0) {
+    if (cs != 3) return set_err(c, DBSRG_EINVAL, "far field: R^k exchange is convol case 3");
+    RFar &r = c->rfarw[k];
+    if (!r.W) {
+      const CellData *pp, *qq;
+      if ((rc = get_celldata(c, 0, 0, k, &pp)) || (rc = get_celldata(c, 0, 1, k, &qq))) return rc;
+      double *W = (double *)cache_alloc(c, 8 * m * sizeof(double));
+      if (!W) return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
+      r.W = W;
+      r.Wf = (float2 *)(W + 4 * m);
+      auto side = [&](int comp, const CellData &cd) {
+        const int o = comp == 1 ? 0 : 2, ord = comp == 1 ? g.ksp : g.ksq;
+        return FarSide{{ord, ord, 1}, 1, ord, ord, comp, cd.lo1, cd.hi1, W + o * m,
+                       W + (o + 1) * m, r.Wf + o * m, r.Wf + (o + 1) * m};
+      };
+      DBSRG_RUN(c, "k_far_vectors",
+                k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.nv, kk, nb, c->b2o, c->pq,
+                                                        side(1, *pp), side(2, *qq)));
+    }
+    // U, Ul: lo and hi of electron 1's pairs; V, Vl: hi and lo of electron 2's
+    const int a = tb.a1 == 1 ? 0 : 2, b = tb.b1 == 1 ? 0 : 2;
+    f.U = r.W + a * m;
+    f.Ul = r.W + (a + 1) * m;
+    f.V = r.W + (b + 1) * m;
+    f.Vl = r.W + b * m;
+    f.Vf = r.Wf + (b + 1) * m;
+    f.Vlf = r.Wf + b * m;
+    f.sh = &r;
+    f.first = a;
+  } else {
+    const CellData *cd;
+    if ((rc = get_celldata(c, family, type, k, &cd))) return rc;
+    double *base = (double *)cache_alloc(c, 3 * m * sizeof(double));
+    if (!base) return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
+    f.U = base;
+    f.V = base + m;
+    f.Vf = (float2 *)(base + 2 * m);
+    auto ord = [&](int b) { return b == 1 ? g.ksp : g.ksq; };
+    // electron 1: case 3 output = first function, contracted = second
+    int o1f = cs == 3 ? 1 : 0;
+    int ko1 = ord(cs == 3 ? tb.a1 : tb.a2), kc1 = ord(cs == 3 ? tb.a2 : tb.a1);
+    int cc1 = cs == 3 ? tb.a2 : tb.a1;
+    // electron 2: case 3 output = second function, contracted = first
+    int o2f = cs == 3 ? 0 : 1;
+    int ko2 = ord(cs == 3 ? tb.b2 : tb.b1), kc2 = ord(cs == 3 ? tb.b1 : tb.b2);
+    int cc2 = cs == 3 ? tb.b1 : tb.b2;
+    const FarSide s1{tb.e1, o1f, ko1, kc1, cc1, cd->lo1, nullptr, f.U, nullptr, nullptr, nullptr};
+    const FarSide s2{tb.e2, o2f, ko2, kc2, cc2, cd->hi2, nullptr, f.V, nullptr, f.Vf, nullptr};
+    DBSRG_RUN(c, "k_far_vectors",
+              k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.nv, kk, nb, c->b2o, c->pq, s1, s2));
+  }
   v[idx] = f;
   *out = &v.at(idx);
   return DBSRG_OK;
@@ -837,12 +897,12 @@ static int ensure_brows(dbsrg_ctx *c) {
   if (c->brows) return DBSRG_OK;
   const int ns = c->g.ns, nb = c->nbound;
   const size_t m = (size_t)ns * nb;
-  if (!(c->brows = (double *)cache_alloc(c, 2 * m * sizeof(double))))
+  if (!(c->brows = (double *)cache_alloc(c, 4 * m * sizeof(double))))
     return set_err(c, DBSRG_ENOMEM, "bound-orbital rows allocation failed");
-  for (int comp = 1; comp <= 2; comp++)
-    DBSRG_RUN(c, "k_bound_rows",
-              k_bound_rows<<<(unsigned)((m + 255) / 256), 256, 0, c->stream>>>(
-                  ns, nb, c->b2o, c->pq, comp, c->brows + (size_t)(comp - 1) * m));
+  c->browsf = (float2 *)(c->brows + 2 * m);
+  DBSRG_RUN(c, "k_bound_rows",
+            k_bound_rows<<<dim3((unsigned)((m + 255) / 256), 2), 256, 0, c->stream>>>(
+                ns, nb, c->b2o, c->pq, c->brows, c->browsf));
   return DBSRG_OK;
 }
 
@@ -931,6 +991,7 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
   const double *lo1 = icv == 1 ? cd->lo1 : nullptr;
   const double *hi1 = (icv == 1 && family == 0) ? cd->hi1 : nullptr;
   dim3 gf((unsigned)((per + 127) / 128), (unsigned)npair);
+  const int ofirst = (icv == 1) != cd->tr;
   // executed work of the diagonal cells: per cell, stage 1 npo k1 k2 nb and
   // stage 2 npo nb k1 nb multiply-adds; the cell's table slice read and its
   // npo nb^2 outputs written.  The final potentials: per output element and
@@ -944,7 +1005,7 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
     if ((rc = set_smem(c, (const void *)k_pair_diag<true>, sm3))) return rc;
     DBSRG_RUN_W(c, "k_pair_diag", dbytes, dflops,
                 k_pair_diag<true><<<nv, 512, sm3, st>>>(
-                    ns, ks, kk, nb, icv, sym, eo, ed, cd->rkd, P1, P2, Dq, per));
+                    ns, ks, kk, nb, ofirst, sym, eo, ed, cd->rkd, P1, P2, Dq, per));
     DBSRG_RUN_W(c, "k_pair_direct_final", fbytes, fflops,
                 k_pair_direct_final<true><<<gf, 128, 0, st>>>(ns, ks, nv, kk, nb, icv, sym, eo,
                                                               lo1, hi1, cd->hi2, SA,
@@ -953,7 +1014,7 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
     if ((rc = set_smem(c, (const void *)k_pair_diag<false>, sm3))) return rc;
     DBSRG_RUN_W(c, "k_pair_diag", dbytes, dflops,
                 k_pair_diag<false><<<nv, 512, sm3, st>>>(
-                    ns, ks, kk, nb, icv, sym, eo, ed, cd->rkd, P1, P2, Dq, per));
+                    ns, ks, kk, nb, ofirst, sym, eo, ed, cd->rkd, P1, P2, Dq, per));
     DBSRG_RUN_W(c, "k_pair_direct_final", fbytes, fflops,
                 k_pair_direct_final<false><<<gf, 128, 0, st>>>(ns, ks, nv, kk, nb, icv, sym, eo,
                                                                lo1, hi1, cd->hi2, SA,
@@ -967,50 +1028,67 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
 // components jp1/jp2: Kb[pair][ns*17], cached
 // ff: both stages in float-float arithmetic, the result stored as
 // float-float pairs (float2, same bytes) for the split form's Z digits
+// (R^k: tabs of types 0..2 by type, type 3 comes with type 2; S^k: tabs[0])
 static int get_pairpot_band(dbsrg_ctx *c, int family, int type, int k, int cs, int jp1, int jp2,
-                            const double *tab, bool ff, const void **out) {
+                            const double *const *tabs, bool ff, const void **out) {
+  if (family == 0 && type == 3) {
+    type = 2;
+    std::swap(jp1, jp2);
+    const long long k3 = pairpot_key(1, 0, 3, k, cs, jp2, jp1, ff);
+    const int rc = c->ppot.count(k3)
+                       ? DBSRG_OK
+                       : get_pairpot_band(c, 0, 2, k, cs, jp1, jp2, tabs, ff, out);
+    if (rc) return rc;
+    *out = c->ppot.at(k3);
+    return DBSRG_OK;
+  }
   const long long key = pairpot_key(1, family, type, k, cs, jp1, jp2, ff);
   auto it = c->ppot.find(key);
   if (it != c->ppot.end()) {
     *out = it->second;
     return DBSRG_OK;
   }
+  const double *tab = tabs[family == 0 ? type : 0];
   const DeviceGrid &g = c->g;
   const int ns = g.ns, ks = g.ks, nb = c->nbound;
   const size_t npair = (size_t)nb * nb, per = (size_t)ns * NDB;
   int rc;
   if ((rc = ensure_brows(c))) return rc;
-  double *K = nullptr;
-  if (!(K = (double *)cache_alloc(c, npair * per * sizeof(double)))) {
-    cudaGetLastError();
-    return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
-  }
+  const size_t kbytes = npair * per * sizeof(double);
+  double *K = (double *)cache_alloc(c, kbytes), *Kx = nullptr;
+  if (!K) return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
   c->ppot[key] = K;
+  if (family == 0) {  // the results with the electrons exchanged
+    Kx = type == 2 ? (double *)cache_alloc(c, kbytes) : K;
+    if (!Kx) return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
+    if (type == 2) c->ppot[pairpot_key(1, 0, 3, k, cs, jp2, jp1, ff)] = Kx;
+  }
   // positions past the ends of the band are never written by k_pair_band
-  DBSRG_TRY(c, cudaMemsetAsync(K, 0, npair * per * sizeof(double), c->stream));
+  for (double *q : {K, Kx == K ? nullptr : Kx})
+    if (q) DBSRG_TRY(c, cudaMemsetAsync(q, 0, kbytes, c->stream));
   const double *P1 = c->brows + (size_t)(jp1 - 1) * nb * ns;
   const double *P2 = c->brows + (size_t)(jp2 - 1) * nb * ns;
   const int W = 2 * ks - 1, WLP = (PXC + W - 1) | 1;
   const size_t smem =
       ((size_t)PXC * W * W + 2 * (size_t)nb * WLP + (size_t)PXC * (W * nb + 1)) * sizeof(double);
   const int mode = family == 0 ? 0 : (cs == 3 ? 1 : 2);
-  dim3 gb((unsigned)((ns + PXC - 1) / PXC), (unsigned)NDB);
+  dim3 gb((unsigned)((ns + PXC - 1) / PXC), (unsigned)(Kx == K ? BAND + 1 : NDB));
   // executed work: per output row and band diagonal W^2 nb (stage 1) and
   // W nb^2 (stage 2) multiply-adds; the band table read, the potentials
   // written
   const double kb = family == 0 ? ks : W;
-  const double bflops = 2.0 * ns * NDB * ((double)W * W * nb + (double)W * nb * nb);
+  const double bflops = 2.0 * ns * gb.y * ((double)W * W * nb + (double)W * nb * nb);
   const double bbytes = 8.0 * ns * NDB * (kb * kb + (double)npair);
   if (ff) {
     if ((rc = set_smem(c, (const void *)k_pair_band<true>, smem))) return rc;
     DBSRG_RUN_W(c, "k_pair_band", bbytes, bflops,
-                k_pair_band<true><<<gb, 256, smem, c->stream>>>(ns, ks, nb, mode, tab, P1, P2,
-                                                                K));
+                k_pair_band<true><<<gb, 256, smem, c->stream>>>(ns, ks, nb, mode, tab, P1, P2, K,
+                                                                Kx));
   } else {
     if ((rc = set_smem(c, (const void *)k_pair_band<false>, smem))) return rc;
     DBSRG_RUN_W(c, "k_pair_band", bbytes, bflops,
-                k_pair_band<false><<<gb, 256, smem, c->stream>>>(ns, ks, nb, mode, tab, P1, P2,
-                                                                 K));
+                k_pair_band<false><<<gb, 256, smem, c->stream>>>(ns, ks, nb, mode, tab, P1, P2, K,
+                                                                 Kx));
   }
   *out = K;
   return DBSRG_OK;
@@ -1018,14 +1096,17 @@ static int get_pairpot_band(dbsrg_ctx *c, int family, int type, int k, int cs, i
 
 void free_orbital_products(dbsrg_ctx *c) {
   graph_drop(c);
-  if (!c->rfar.empty() || !c->sfar.empty() || !c->ppot.empty() || c->brows || c->vch ||
-      !c->ffc.empty())
+  if (!c->rfarw.empty() || !c->sfar.empty() || !c->ppot.empty() || c->brows || c->vch)
     cudaStreamSynchronize(c->stream);
-  for (auto *v : {&c->rfar, &c->sfar})
-    for (auto &kv : *v) {
-      cache_free(c, kv.second.U);
-      cache_free(c, kv.second.Ud);
-    }
+  for (auto &kv : c->rfarw) {
+    cache_free(c, kv.second.W);
+    cache_free(c, kv.second.D);
+  }
+  for (auto &kv : c->sfar) {
+    cache_free(c, kv.second.U);
+    cache_free(c, kv.second.Ud);
+  }
+  c->rfarw.clear();
   c->rfar.clear();
   c->sfar.clear();
   for (auto &kv : c->ppot)
@@ -1033,37 +1114,9 @@ void free_orbital_products(dbsrg_ctx *c) {
   c->ppot.clear();
   cache_free(c, c->brows);
   c->brows = nullptr;
+  c->browsf = nullptr;
   cache_free(c, c->vch);
   c->vch = nullptr;
-  for (auto &kv : c->ffc) cache_free(c, kv.second);
-  c->ffc.clear();
-}
-
-namespace {
-__global__ void k_to_ff(size_t n, const double *src, float2 *dst) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = ffa::split(src[i]);
-}
-}  // namespace
-
-int ff_of(dbsrg_ctx *c, const double *src, size_t n, const float2 **out) {
-  auto it = c->ffc.find(src);
-  if (it != c->ffc.end()) {
-    *out = it->second;
-    return DBSRG_OK;
-  }
-  float2 *d = (float2 *)cache_alloc(c, n * sizeof(float2));
-  if (!d) return set_err(c, DBSRG_ENOMEM, "float-float copy allocation failed");
-  c->ffc[src] = d;
-  DBSRG_RUN(c, "k_to_ff",
-            k_to_ff<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, src, d));
-  *out = d;
-  return DBSRG_OK;
-}
-
-int ff_bound_rows(dbsrg_ctx *c, const float2 **out) {
-  const int rc = ensure_brows(c);
-  return rc ? rc : ff_of(c, c->brows, (size_t)2 * c->nbound * c->g.ns, out);
 }
 
 int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
@@ -1093,8 +1146,8 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
       int c1 = cs == 3 ? tb.a2 : tb.a1, c2 = cs == 3 ? tb.b1 : tb.b2;
       if (c1 != j.jp1[a] || c2 != j.jp2[a])
         return set_err(c, DBSRG_EINVAL, "factored exchange: component mismatch");
-      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.jp1[a], j.jp2[a],
-                                 j.tabs[a], true, (const void **)&x.Kbf[a])))
+      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.jp1[a], j.jp2[a], j.tabs,
+                                 true, (const void **)&x.Kbf[a])))
         return rc;
     }
     x.members = j.members;
@@ -1115,7 +1168,7 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
       const void *Kb;
       if ((rc = get_farfield(c, j.family, j.types[a], j.kpol, j.icv, &f))) return rc;
       if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, j.icv, j.jp1[a], j.jp2[a],
-                                 j.tabs[a], false, &Kb)))
+                                 j.tabs, false, &Kb)))
         return rc;
     }
     return DBSRG_OK;
@@ -1134,8 +1187,8 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
       if (c1 != j.jp1[a] || c2 != j.jp2[a])
         return set_err(c, DBSRG_EINVAL, "factored exchange: component mismatch");
       const double *Kb;
-      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.jp1[a], j.jp2[a],
-                                 j.tabs[a], false, (const void **)&Kb)))
+      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.jp1[a], j.jp2[a], j.tabs,
+                                 false, (const void **)&Kb)))
         return rc;
       double *Ya = j.Y + (size_t)a * j.nm * per;
       dim3 gz((unsigned)((ns * nb + 127) / 128), (unsigned)j.nm);

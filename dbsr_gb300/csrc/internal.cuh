@@ -38,18 +38,42 @@ struct DeviceGrid {
   double *tri = nullptr;
 };
 
-// resident cell moments and diagonal-cell integrals of one table
+// resident cell moments and diagonal-cell integrals of one table.  The R^k
+// tables of one k share theirs: the moments of the P and Q pairs, and the
+// diagonal cells of types 2 and 3, which are the same integrals with the
+// electrons exchanged (tr: the second electron's pair is the first index).
 struct CellData {
   double *lo1 = nullptr, *hi1 = nullptr, *lo2 = nullptr, *hi2 = nullptr, *rkd = nullptr;
   // rkd as float-float pairs without padding, rkf[(pair1 + np1 pair2) + cell np1 np2]
   // (np1, np2 the numbers of pairs of the two electrons)
   float2 *rkf = nullptr;
+  bool tr = false;
+};
+
+// what the R^k tables of one k are made of
+struct RCells {
+  double *mom = nullptr;  // moments of P pairs r^k, r^-(k+1), of Q pairs r^k, r^-(k+1)
+  double *diag[3] = {nullptr, nullptr, nullptr};  // rkd and rkf of types 0, 1, 2
+};
+
+// far-field vectors of the R^k tables of one k: every type's U, Ul, V and Vl are
+// four of them, [lo P, hi P, lo Q, hi Q][ns*nbound] (lo/hi: moment-contracted
+// with r^k / r^-(k+1)), their float-float copies, and their split-BF16 digit
+// tiles and exponents (built on first use by the tensor-core exchange)
+struct RFar {
+  double *W = nullptr;
+  float2 *Wf = nullptr;
+  void *D = nullptr;
+  int *e = nullptr;
 };
 
 // far-field orbital vectors of one exchange table and contraction case:
 // U, V (upper field) and Ul, Vl (lower field, R^k only), each (ns, nbound)
 struct FarField {
   double *U = nullptr, *V = nullptr, *Ul = nullptr, *Vl = nullptr;
+  float2 *Vf = nullptr, *Vlf = nullptr;  // V and Vl as float-float pairs
+  RFar *sh = nullptr;                    // R^k: the shared vectors these are views of
+  int first = 0;                         // position of U among them
   // split-BF16 digit tiles of U (mode 0) and Ul (mode 1) and their row
   // exponents, built on first use by the tensor-core exchange
   void *Ud = nullptr;
@@ -90,20 +114,20 @@ struct dbsrg_ctx {
   std::vector<double *> rtab, stab;
   // band-limited tables (|j-i| <= DBSRG_TABLE_BAND) for the factored path
   std::vector<double *> rbtab, sbtab;
-  std::vector<CellData> rcell, scell;
+  std::vector<CellData> rcell, scell;  // rcell: views of rshare
+  std::vector<RCells> rshare;          // [k]
   // far-field vectors, keyed (k*4+type)*2+case34 (R) / (k*2+type)*2+case34 (S);
   // map nodes keep their addresses while other entries are added
   std::map<size_t, FarField> rfar, sfar;
+  std::map<int, RFar> rfarw;  // [k], what rfar's entries are views of
   // orbital-pair potentials of the factored contraction (direct band results
   // and exchange band results per ordered bound-orbital pair), keyed by
   // pairpot_key(); they depend on the tables and the orbitals
   std::map<long long, double *> ppot;
-  // float-float copies (hi, lo) of orbital products for the split form's
-  // gather-sums, keyed by the FP64 array they copy; dropped with the
-  // orbital products
-  std::map<const void *, float2 *> ffc;
   // bound-orbital rows brows[(comp-1)*nbound*ns + a*ns + x] = pq(x+1, comp, b2o[a])
+  // and the same as float-float pairs (behind them, one allocation)
   double *brows = nullptr;
+  float2 *browsf = nullptr;
   // overlap vectors V_ch of every orbital, vch[2 ns (orbital - 1)] = (fpbs P;
   // fqbs Q); an orbital product like the others, built on the contraction
   // stream by the first list of an assembly that reads it
@@ -335,18 +359,19 @@ int graph_launch(dbsrg_ctx *c, const double *pq);
 void graph_drop(dbsrg_ctx *c);
 // handles of the channel basis (basis.cu)
 void basis_release(dbsrg_ctx *c);
-// float-float copy of n doubles at src (cached until the orbital products go)
-int ff_of(dbsrg_ctx *c, const double *src, size_t n, const float2 **out);
-
 // ---- tables.cu ------------------------------------------------------------
 int build_grid(dbsrg_ctx *c, const double *t_host_or_dev);
 int compute_moments(dbsrg_ctx *c, int which, int k, double *rkm_dev);
-int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd_dev, float2 *rkf_dev = nullptr);
+int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd_dev);
 // returns device pointer of the cached table (building it if needed)
 int get_rtable(dbsrg_ctx *c, int type, int k, const double **out);
 int get_stable(dbsrg_ctx *c, int type, int k, const double **out);
 int get_quad(dbsrg_ctx *c, int k, const double **out);
 int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out);
+// the cell data of every R^k type of one k in two launches, and the band tables
+// of types 0, 1 and 2 in one (type 3's exchange reads type 2's)
+int ensure_r_cells(dbsrg_ctx *c, int k);
+int ensure_r_band_tables(dbsrg_ctx *c, int k);
 // (ns, 2*DBSRG_TABLE_BAND+1, kb, kb): rkb(i, j-i+DBSRG_TABLE_BAND+1, ip, jp)
 #define DBSRG_TABLE_BAND 16
 int get_band_table(dbsrg_ctx *c, int family, int type, int k, const double **out);
@@ -433,8 +458,6 @@ struct FactorJob {
   long long nent;    // entries of the member segments (executed-work statements)
 };
 int factored_contract(dbsrg_ctx *c, const FactorJob &job);
-// float-float copy of the bound-orbital rows (both components)
-int ff_bound_rows(dbsrg_ctx *c, const float2 **out);
 // ---- direct.cu: the direct cases segment by segment
 // whether a list of nseg segments and nent entries takes fewer operations that
 // way than through the pair potentials

@@ -9,6 +9,7 @@
 #include "internal.cuh"
 #include "pairs.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 #define IDX2(i, j, n1) ((size_t)(i) + (size_t)(n1) * (size_t)(j))
@@ -278,16 +279,22 @@ __global__ void k_triang_points(int nv, int ks, int ksp, int ksq, const double *
   for (int j = 0; j < ksq; j++) tb[2 * KS2 + (size_t)KS2 * ksp + (size_t)p * ksq + j] = v[j];
 }
 
-__global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, const double *tri,
-                         const double *grm, const double *grw, const double *pbsp,
-                         const double *qbsp, double *rkd, float2 *rkf) {
+// up to three types per launch (blockIdx.y)
+struct TriSet {
+  int type[3];
+  double *rkd[3];
+  float2 *rkf[3];
+};
+
+__global__ void k_triang(int nv, int ks, int ksp, int ksq, const TriSet ts, int k,
+                         const double *tri, const double *grm, const double *grw,
+                         const double *pbsp, const double *qbsp) {
   extern __shared__ double sm[];
   const int iv = blockIdx.x;  // 0-based interval
-  // this block's share of the interval's kk*kk output cells (blockIdx.y of
-  // gridDim.y, launched with one block per interval: the inner integrals
-  // would be repeated by every block of an interval)
-  const int nq = ks * ks * ks * ks, part = (nq + gridDim.y - 1) / gridDim.y;
-  const int q0 = blockIdx.y * part, q1 = min(nq, q0 + part);
+  const int type = ts.type[blockIdx.y];
+  double *rkd = ts.rkd[blockIdx.y];
+  float2 *rkf = ts.rkf[blockIdx.y];
+  const int nq = ks * ks * ks * ks;
   const int nw = nv + 1, kk = ks * ks;
   const int KS2 = ks * ks;
   const double *tb = tri + (size_t)iv * KS2 * (2 + ksp + ksq);  // x | w | BP | BQ
@@ -391,7 +398,7 @@ __global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, cons
       A[q] = s;
     }
     __syncthreads();
-    for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
       int ii = q % kk, jj = q / kk;
       const bool ok = ii < ik && jj < ik;
       const double v = ok ? __dadd_rn(A[ii + ik * jj], A[jj + ik * ii]) : 0.0;
@@ -400,7 +407,7 @@ __global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, cons
     }
   } else if (type == 2 || type == 3) {
     const int ikp = ksp * (ksp + 1) / 2, ikq = ksq * (ksq + 1) / 2;
-    for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
       int r = q % kk, cc = q / kk;
       int pp_ = type == 2 ? r : cc, qq_ = type == 2 ? cc : r;  // P pair, Q pair
       double v = 0.0;
@@ -420,7 +427,7 @@ __global__ void k_triang(int nv, int ks, int ksp, int ksq, int type, int k, cons
     }
   } else {
     const int np = ksp * ksq;
-    for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
       int jj = q % kk, ii = q / kk;  // rkd(jj,ii): jj inner (P,Q), ii outer
       double v = 0.0;
       if (jj < np && ii < np) {
@@ -448,7 +455,8 @@ static int build_triang_points(dbsrg_ctx *c) {
   return DBSRG_OK;
 }
 
-int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd, float2 *rkf) {
+// n (1..3) types in one launch
+static int compute_diag_set(dbsrg_ctx *c, int n, const TriSet &ts, int k) {
   const DeviceGrid &g = c->g;
   const int ks = g.ks, kk = ks * ks;
   size_t nsm = (size_t)ks * ks + (size_t)ks * ks * g.ksp + (size_t)ks * ks * g.ksq +
@@ -458,9 +466,17 @@ int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd, float2 *rkf) 
   int rc = raise_smem_limit(c, (const void *)k_triang, bytes);
   if (rc) return rc;
   DBSRG_RUN(c, "k_triang",
-            k_triang<<<dim3(g.nv, 1), 256, bytes, c->stream>>>(g.nv, ks, g.ksp, g.ksq, type, k, g.tri,
-                                                      g.grm, g.grw, g.pbsp, g.qbsp, rkd, rkf));
+            k_triang<<<dim3(g.nv, n), 256, bytes, c->stream>>>(g.nv, ks, g.ksp, g.ksq, ts, k,
+                                                               g.tri, g.grm, g.grw, g.pbsp,
+                                                               g.qbsp));
   return DBSRG_OK;
+}
+
+int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd) {
+  TriSet ts{};
+  ts.type[0] = type;
+  ts.rkd[0] = rkd;
+  return compute_diag_set(c, 1, ts, k);
 }
 
 // ----------------------------------------------------------------------------
@@ -475,9 +491,20 @@ __device__ __forceinline__ int tri_index(int h, int hp, int kx) {  // 1-based
 // band > 0: only the elements with |j - i| <= band, stored as
 // rkb(i, j-i+band+1, ip, jp) of shape (ns, 2*band+1, ks, ks) -- all that the
 // band part of the factored exchange reads.
-__global__ void k_fill_r(int ns, int ks, int nv, int ka, int kb, const double *lowA,
-                         const double *highA, const double *lowB, const double *highB,
-                         const double *rkd, double *rkb, int band) {
+// Up to three tables per launch (blockIdx.y); tr: rkd has the electron-2 pair
+// first.
+struct FillSet {
+  int ka[3], kb[3], tr[3];
+  const double *lowA[3], *highA[3], *lowB[3], *highB[3], *rkd[3];
+  double *rkb[3];
+};
+
+__global__ void k_fill_r(int ns, int ks, int nv, const FillSet fs, int band) {
+  const int y = blockIdx.y, ka = fs.ka[y], kb = fs.kb[y];
+  const double *lowA = fs.lowA[y], *highA = fs.highA[y], *lowB = fs.lowB[y], *highB = fs.highB[y],
+               *rkd = fs.rkd[y];
+  double *rkb = fs.rkb[y];
+  const bool tr = fs.tr[y];
   size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nj = band > 0 ? 2 * band + 1 : ns;
   size_t total = (size_t)ns * nj * ks * ks;
@@ -523,7 +550,8 @@ __global__ void k_fill_r(int ns, int ks, int nv, int ka, int kb, const double *l
       if (iv >= jvlo && iv <= jvhi) {  // the diagonal cell, then jv = iv joins the prefix
         const int ih = i - iv + 1, jh = j - iv + 1;
         const int ii = tri_index(ih, ih + ip - 1, ka), jj = tri_index(jh, jh + jp - 1, kb);
-        acc += rkd[(ii - 1) + (size_t)kk * ((jj - 1) + (size_t)kk * (iv - 1))];
+        const int r1 = tr ? jj : ii, r2 = tr ? ii : jj;
+        acc += rkd[(r1 - 1) + (size_t)kk * ((r2 - 1) + (size_t)kk * (iv - 1))];
         pre += lowB[jb(iv)];
       }
     }
@@ -588,51 +616,146 @@ static int ensure_slot(dbsrg_ctx *c, std::vector<double *> &v, size_t idx) {
 
 // Cell moments and diagonal-cell integrals of one table (family, type, k),
 // kept resident: the table fill and the factored contraction both read
-// them.  R: lo1/hi1 = moments of the electron-1 basis at r^k / r^-(k+1),
+// them (the R^k types of one k share theirs, ensure_r_cells).  R: lo1/hi1 = moments of the electron-1 basis at r^k / r^-(k+1),
 // lo2/hi2 the same for electron 2 (mrk_*: rkd1..rkd4).  S: lo1 =
 // moments_pq(k) of electron 1, hi2 = moments_pq or moments_qp(-(k+1)) of
 // electron 2 (msk_*: rkd1, rkd2); hi1 = lo2 = null (no r1 > r2 cells).
 int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out) {
   const DeviceGrid &g = c->g;
-  std::vector<CellData> &v = family == 0 ? c->rcell : c->scell;
-  size_t idx = (size_t)k * (family == 0 ? 4 : 2) + type;
+  const int nv = g.nv, kk = g.ks * g.ks;
+  const size_t m = (size_t)kk * nv, d = (size_t)kk * kk * nv;
+  int rc;
+  if (family == 0) {
+    if ((rc = ensure_r_cells(c, k))) return rc;
+    *out = &c->rcell[(size_t)k * 4 + type];
+    return DBSRG_OK;
+  }
+  std::vector<CellData> &v = c->scell;
+  const size_t idx = (size_t)k * 2 + type;
   if (v.size() <= idx) v.resize(idx + 1);
   if (v[idx].rkd) {
     *out = &v[idx];
     return DBSRG_OK;
   }
-  const int nv = g.nv, kk = g.ks * g.ks;
-  size_t m = (size_t)kk * nv, d = (size_t)kk * kk * nv;
   const TableBases tb = table_bases(g, family, type);
   const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
   double *base = nullptr;
-  if (!(base = (double *)cache_alloc(c, (4 * m + d + f) * sizeof(double))))
+  if (!(base = (double *)cache_alloc(c, (2 * m + d + f) * sizeof(double))))
     return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
   CellData cd;
   cd.lo1 = base;
-  cd.hi1 = base + m;
-  cd.lo2 = base + 2 * m;
-  cd.hi2 = base + 3 * m;
-  cd.rkd = base + 4 * m;
+  cd.hi2 = base + m;
+  cd.rkd = base + 2 * m;
   cd.rkf = (float2 *)(cd.rkd + d);
-  int rc;
-  if (family == 0) {
-    int wa = (type == 0 || type == 2) ? 0 : 1, wb = (type == 0 || type == 3) ? 0 : 1;
-    const int wh[4] = {wa, wa, wb, wb}, kp[4] = {k, -(k + 1), k, -(k + 1)};
-    double *const out[4] = {cd.lo1, cd.hi1, cd.lo2, cd.hi2};
-    if ((rc = compute_moment_set(c, 4, wh, kp, out))) return rc;
-    if ((rc = compute_diag_cells(c, type, k, cd.rkd, cd.rkf))) return rc;
-  } else {
-    const int wh[2] = {2, type == 0 ? 2 : 3}, kp[2] = {k, -(k + 1)};
-    double *const out[2] = {cd.lo1, cd.hi2};
-    if ((rc = compute_moment_set(c, 2, wh, kp, out))) return rc;
-    if ((rc = compute_diag_cells(c, type == 0 ? 4 : 5, k, cd.rkd, cd.rkf))) return rc;
-    cd.hi1 = nullptr;
-    cd.lo2 = nullptr;
-  }
+  const int wh[2] = {2, type == 0 ? 2 : 3}, kp[2] = {k, -(k + 1)};
+  double *const mo[2] = {cd.lo1, cd.hi2};
+  if ((rc = compute_moment_set(c, 2, wh, kp, mo))) return rc;
+  TriSet ts{};
+  ts.type[0] = type == 0 ? 4 : 5;
+  ts.rkd[0] = cd.rkd;
+  ts.rkf[0] = cd.rkf;
+  if ((rc = compute_diag_set(c, 1, ts, k))) return rc;
   v[idx] = cd;
   *out = &v[idx];
   return DBSRG_OK;
+}
+
+// The R^k tables of one k: the moments of the P and Q pairs (four arrays, one
+// launch; every type takes two of each) and the diagonal cells of types 0, 1
+// and 2 (one launch; type 3 reads type 2's with the electrons exchanged).  A
+// list takes all types of its k, so nothing is built that it does not read.
+// ns 283: moments 4 x 18 -> 18 us a k, diagonal cells 4 x 40 -> 95 us, band
+// tables (ensure_r_band_tables) 4 x 39 -> 87 us against a launch per type.
+int ensure_r_cells(dbsrg_ctx *c, int k) {
+  const DeviceGrid &g = c->g;
+  const int nv = g.nv, kk = g.ks * g.ks;
+  const size_t m = (size_t)kk * nv, d = (size_t)kk * kk * nv;
+  if ((int)c->rshare.size() <= k) c->rshare.resize(k + 1);
+  if (c->rcell.size() < (size_t)(k + 1) * 4) c->rcell.resize((size_t)(k + 1) * 4);
+  RCells &r = c->rshare[k];
+  if (c->rcell[(size_t)k * 4].rkd) return DBSRG_OK;
+  int rc;
+  if (!r.mom && !(r.mom = (double *)cache_alloc(c, 4 * m * sizeof(double))))
+    return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
+  const int wh[4] = {0, 0, 1, 1}, kp[4] = {k, -(k + 1), k, -(k + 1)};
+  double *const mo[4] = {r.mom, r.mom + m, r.mom + 2 * m, r.mom + 3 * m};
+  if ((rc = compute_moment_set(c, 4, wh, kp, mo))) return rc;
+  TriSet ts{};
+  for (int t = 0; t < 3; t++) {
+    const TableBases tb = table_bases(g, 0, t);
+    const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
+    if (!r.diag[t] && !(r.diag[t] = (double *)cache_alloc(c, (d + f) * sizeof(double))))
+      return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
+    ts.type[t] = t;
+    ts.rkd[t] = r.diag[t];
+    ts.rkf[t] = (float2 *)(r.diag[t] + d);
+  }
+  if ((rc = compute_diag_set(c, 3, ts, k))) return rc;
+  for (int t = 0; t < 4; t++) {
+    CellData cd;
+    const int wa = (t == 0 || t == 2) ? 0 : 1, wb = (t == 0 || t == 3) ? 0 : 1;
+    cd.lo1 = r.mom + 2 * wa * m;
+    cd.hi1 = cd.lo1 + m;
+    cd.lo2 = r.mom + 2 * wb * m;
+    cd.hi2 = cd.lo2 + m;
+    cd.rkd = r.diag[std::min(t, 2)];
+    cd.rkf = (float2 *)(cd.rkd + d);
+    cd.tr = t == 3;
+    c->rcell[(size_t)k * 4 + t] = cd;
+  }
+  return DBSRG_OK;
+}
+
+// fills n (1..3) R^k tables of one k, full (band 0) or band-limited
+static int fill_r(dbsrg_ctx *c, int n, const int *types, int k, double *const *tab, int band) {
+  const DeviceGrid &g = c->g;
+  const int nj = band ? 2 * band + 1 : g.ns;
+  const size_t nt = (size_t)g.ns * nj * g.ks * g.ks;
+  FillSet fs{};
+  for (int i = 0; i < n; i++) {
+    const CellData *cd;
+    int rc = get_celldata(c, 0, types[i], k, &cd);
+    if (rc) return rc;
+    const TableBases tb = table_bases(g, 0, types[i]);
+    fs.ka[i] = tb.e1.k1;
+    fs.kb[i] = tb.e2.k1;
+    fs.tr[i] = cd->tr;
+    fs.lowA[i] = cd->lo1;
+    fs.highA[i] = cd->hi1;
+    fs.lowB[i] = cd->lo2;
+    fs.highB[i] = cd->hi2;
+    fs.rkd[i] = cd->rkd;
+    fs.rkb[i] = tab[i];
+  }
+  DBSRG_RUN(c, "k_fill_r",
+            k_fill_r<<<dim3((unsigned)((nt + 255) / 256), n), 256, 0, c->stream>>>(
+                g.ns, g.ks, g.nv, fs, band));
+  return DBSRG_OK;
+}
+
+int ensure_r_band_tables(dbsrg_ctx *c, int k) {
+  const size_t i0 = (size_t)k * 4;
+  if (c->rbtab.size() < i0 + 4) c->rbtab.resize(i0 + 4, nullptr);
+  const size_t nt = (size_t)c->g.ns * (2 * DBSRG_TABLE_BAND + 1) * c->g.ks * c->g.ks;
+  int types[3], n = 0;
+  double *tab[3];
+  for (int t = 0; t < 3; t++) {
+    if (c->rbtab[i0 + t]) continue;
+    if (!(tab[n] = (double *)cache_alloc(c, nt * sizeof(double)))) {
+      for (int i = 0; i < n; i++) cache_free(c, tab[i]);
+      return set_err(c, DBSRG_ENOMEM, "table allocation failed");
+    }
+    types[n++] = t;
+  }
+  if (n == 0) return DBSRG_OK;
+  const int rc = fill_r(c, n, types, k, tab, DBSRG_TABLE_BAND);
+  for (int i = 0; i < n; i++) {
+    if (rc)
+      cache_free(c, tab[i]);
+    else
+      c->rbtab[i0 + types[i]] = tab[i];
+  }
+  return rc;
 }
 
 // full (band == 0) or band-limited table of (family, type, k), cached
@@ -655,14 +778,10 @@ static int get_table_any(dbsrg_ctx *c, int family, int type, int k, int band,
   double *tab = nullptr;
   if (!(tab = (double *)cache_alloc(c, nt * sizeof(double))))
     return set_err(c, DBSRG_ENOMEM, "table allocation failed");
-  unsigned nb = (unsigned)((nt + 255) / 256);
   if (family == 0) {
-    int wa = (type == 0 || type == 2) ? 0 : 1, wb = (type == 0 || type == 3) ? 0 : 1;
-    int ka = wa ? g.ksq : g.ksp, kbb = wb ? g.ksq : g.ksp;
-    DBSRG_RUN(c, "k_fill_r",
-              k_fill_r<<<nb, 256, 0, c->stream>>>(ns, ks, nv, ka, kbb, cd->lo1, cd->hi1, cd->lo2,
-                                                  cd->hi2, cd->rkd, tab, band));
+    if ((rc = fill_r(c, 1, &type, k, &tab, band))) return rc;
   } else {
+    const unsigned nb = (unsigned)((nt + 255) / 256);
     int kj1 = type == 0 ? g.ksp : g.ksq, kj2 = type == 0 ? g.ksq : g.ksp;
     DBSRG_RUN(c, "k_fill_s",
               k_fill_s<<<nb, 256, 0, c->stream>>>(ns, ks, nv, g.ksp, g.ksq, kj1, kj2, cd->lo1,
