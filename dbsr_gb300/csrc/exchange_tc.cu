@@ -34,6 +34,8 @@
 // Every wait is bounded (2 s): on a timeout the kernel records an error word,
 // waits (bounded) for its own copies and MMAs in flight, frees its TMEM and
 // returns.
+#include <type_traits>
+
 #include "internal.cuh"
 #include "tc_common.cuh"
 #include "ff.cuh"
@@ -138,93 +140,112 @@ struct ZArgs {
   double *Yb;         // [a][slot][ns*17]
 };
 
-// Per segment slot and atype, one thread per row y (ZROWS rows a block):
+// Per segment slot and atype, 32 rows y a block (one 32-row digit tile):
 //   Z_s(k,y) = sum_{e in s, first orbital k} c_e V(y, second orbital)  (Zl with Vl)
 //   Yb_s(y,d) = sum_e c_e Kb(pair_e; y, d)                             (near band)
 // as float-float sums (ff.cuh), then the digits of Z (and Zl) and their row
-// exponents.  The sums read the pair potentials of every entry: the kernel
-// is bound by those reads (L2 and HBM), not by its arithmetic.
-constexpr int ZROWS = 32;  // one warp per block: one 32-row digit tile
+// exponents.  The sums read the pair potentials of every entry, and an entry
+// costs a load latency: the four warps of a block share the 17 band diagonals
+// and the two fields, so that each has few enough values an entry to load those
+// of ZEB entries together.  Long lists are bound by the L2 reads of the
+// potentials, short ones by the chain of their entries.  One warp per block,
+// one entry at a time: 72 us a launch at ns 283 and 26 segments, 177 us at
+// ns 400 and 160.
+constexpr int ZROWS = 32, ZW = 4, ZEB = 4;
+constexpr int ZND = 5;  // most band diagonals of a warp
 // ONE: at most 32 bound orbitals (one chunk)
 template <bool ONE>
-__global__ void __launch_bounds__(ZROWS) k_zdigits(const ZArgs z) {
-  // [mode][nb][ZROWS] float-float: per thread one column; sized by the bound
+__global__ void __launch_bounds__(ZROWS * ZW) k_zdigits(const ZArgs z) {
+  // [mode][nb][ZROWS] float-float: per row one column; sized by the bound
   // orbitals (and the modes) in use, which sets how many blocks share an SM
   extern __shared__ float2 zs[];
-  const int t = threadIdx.x, y = blockIdx.x * ZROWS + t, slot = blockIdx.y, a = blockIdx.z;
+  const int t = threadIdx.x % ZROWS, w = threadIdx.x / ZROWS;
+  const int y = blockIdx.x * ZROWS + t, slot = blockIdx.y, a = blockIdx.z;
   const int ns = z.ns, nb = z.nb;
   float2 *z0 = zs, *z1 = zs + nb * ZROWS;
-  for (int k = 0; k < nb; k++) {
-    z0[k * ZROWS + t] = make_float2(0.0f, 0.0f);
-    if (z.lower) z1[k * ZROWS + t] = make_float2(0.0f, 0.0f);
-  }
+  // diagonals of this warp, and the field whose Z it sums (warps 0 and 1)
+  const int d0 = w < 2 ? 4 * w : 8 + 5 * (w - 2), dn = w < 2 ? 4 : w == 2 ? 5 : 4;
+  const bool field = w == 0 || (w == 1 && z.lower);
+  float2 *zf = w == 0 ? z0 : z1;
+  if (field)
+    for (int k = 0; k < nb; k++) zf[k * ZROWS + t] = make_float2(0.0f, 0.0f);
   const SegInfo si = z.info[z.members[slot]];
-  const float2 *V = z.V[a], *Vl = z.lower ? z.Vl[a] : nullptr, *Kb = z.Kb[a];
   const size_t kper = (size_t)ns * NDB;
-  float bh[NDB], bl[NDB];
-#pragma unroll
-  for (int d = 0; d < NDB; d++) bh[d] = bl[d] = 0.0f;
   if (y < ns) {
-    // the next entry's pair index and coefficient are loaded while this
-    // entry's potentials are summed
-    int pr_n = si.start < si.end ? z.pairs[si.start] : 0;
-    float2 c_n = si.start < si.end ? z.cd[si.start] : make_float2(0.0f, 0.0f);
-    for (int e = si.start; e < si.end; e++) {
-      const int pr = pr_n, oa = pr / nb, ob = pr - oa * nb;
-      const float2 c = c_n;
-      if (e + 1 < si.end) {
-        pr_n = z.pairs[e + 1];
-        c_n = z.cd[e + 1];
-      }
-      const float2 *kb = Kb + (size_t)pr * kper + y;
-      float2 kv[NDB];
+    const float2 *V = (w == 0 ? z.V[a] : z.Vl[a]) + y;
+    const float2 *Kb = z.Kb[a] + (size_t)ns * d0 + y;
+    float bh[ZND], bl[ZND];
 #pragma unroll
-      for (int d = 0; d < NDB; d++) kv[d] = kb[(size_t)ns * d];
-      {
-        float2 acc = z0[oa * ZROWS + t];
-        ffa::mac(c, V[(size_t)y + (size_t)ns * ob], acc.x, acc.y);
-        z0[oa * ZROWS + t] = acc;
-      }
-      if (Vl) {
-        float2 acc = z1[oa * ZROWS + t];
-        ffa::mac(c, Vl[(size_t)y + (size_t)ns * ob], acc.x, acc.y);
-        z1[oa * ZROWS + t] = acc;
+    for (int d = 0; d < ZND; d++) bh[d] = bl[d] = 0.0f;
+    int e = si.start;
+    auto batch = [&](auto nc) {
+      constexpr int N = decltype(nc)::value;
+      int oa[N];
+      float2 c[N], kv[N][ZND], vv[N];
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+        const int pr = z.pairs[e + u];
+        oa[u] = pr / nb;
+        c[u] = z.cd[e + u];
+        const float2 *kb = Kb + (size_t)pr * kper;
+#pragma unroll
+        for (int d = 0; d < ZND; d++)
+          if (d < 4 || dn == 5) kv[u][d] = kb[(size_t)ns * d];
+        if (field) vv[u] = V[(size_t)ns * (pr - oa[u] * nb)];
       }
 #pragma unroll
-      for (int d = 0; d < NDB; d++) ffa::mac(c, kv[d], bh[d], bl[d]);
-    }
-    double *yb = z.Yb + ((size_t)a * z.nm + slot) * kper + y;
+      for (int u = 0; u < N; u++) {
+        if (field) {
+          float2 acc = zf[oa[u] * ZROWS + t];
+          ffa::mac(c[u], vv[u], acc.x, acc.y);
+          zf[oa[u] * ZROWS + t] = acc;
+        }
 #pragma unroll
-    for (int d = 0; d < NDB; d++) yb[(size_t)ns * d] = ffa::value(bh[d], bl[d]);
+        for (int d = 0; d < ZND; d++)
+          if (d < 4 || dn == 5) ffa::mac(c[u], kv[u][d], bh[d], bl[d]);
+      }
+      e += N;
+    };
+    while (e + ZEB <= si.end) batch(std::integral_constant<int, ZEB>());
+    while (e < si.end) batch(std::integral_constant<int, 1>());
+    double *yb = z.Yb + ((size_t)a * z.nm + slot) * kper + (size_t)ns * d0 + y;
+#pragma unroll
+    for (int d = 0; d < ZND; d++)
+      if (d < dn) yb[(size_t)ns * d] = ffa::value(bh[d], bl[d]);
   }
+  __syncthreads();
+  // digits: warps 0, 1 the first field, 2, 3 the second, half of the 8-column
+  // groups each
   const size_t sl = (size_t)z.NR * TILE;
-  for (int mode = 0; mode < (z.lower ? 2 : 1); mode++) {
-    float2 *zz = mode ? z1 : z0;
-    // per chunk of 32 orbitals: each sum renormalised in place (TwoSum:
-    // hi + lo unchanged, |lo| at most half an ulp of hi), the row exponent
-    // from the high words, the digits 8 columns at a time
-    for (int ck = 0; ck < (ONE ? 1 : z.nbk); ck++) {
-      float m = 0.0f;
-      for (int k = 32 * ck; k < (ONE ? nb : min(nb, 32 * ck + 32)); k++) {
-        const float2 v = zz[k * ZROWS + t];
-        const float s = v.x + v.y, bp = s - v.x;
-        zz[k * ZROWS + t] = make_float2(s, (v.x - (s - bp)) + (v.y - bp));
-        m = fmaxf(m, fabsf(s));
-      }
-      const int e = scale_exp_ff(m);
-      const size_t op = ((size_t)(a * 2 + mode) * z.nm + slot) * (ONE ? 1 : z.nbk) + ck;
+  const int mode = w / 2;
+  if (mode && !z.lower) return;
+  const float2 *zz = mode ? z1 : z0;
+  // per chunk of 32 orbitals: each sum renormalised (TwoSum: hi + lo
+  // unchanged, |lo| at most half an ulp of hi), the row exponent from the high
+  // words, the digits 8 columns at a time
+  auto renorm = [&](float2 v) {
+    const float s = v.x + v.y, bp = s - v.x;
+    return make_float2(s, (v.x - (s - bp)) + (v.y - bp));
+  };
+  for (int ck = 0; ck < (ONE ? 1 : z.nbk); ck++) {
+    float m = 0.0f;
+    for (int k = 32 * ck; k < (ONE ? nb : min(nb, 32 * ck + 32)); k++)
+      m = fmaxf(m, fabsf(renorm(zz[k * ZROWS + t]).x));
+    const int e = scale_exp_ff(m);
+    const size_t op = ((size_t)(a * 2 + mode) * z.nm + slot) * (ONE ? 1 : z.nbk) + ck;
+    if (w % 2 == 0) {
       z.ez[op * z.NR * EXP_PER_ROWTILE + y] = e;
       const int et = __reduce_max_sync(0xffffffffu, e);  // a warp is one 32-row tile
-      if ((t & 31) == 0) z.ez[op * z.NR * EXP_PER_ROWTILE + z.NR * 32 + y / 32] = et;
-      for (int kg = 0; kg < 4; kg++) {
-        float2 vals[8];
+      if (t == 0) z.ez[op * z.NR * EXP_PER_ROWTILE + z.NR * 32 + y / 32] = et;
+    }
+    for (int kg = w % 2; kg < 4; kg += 2) {
+      float2 vals[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int k = 32 * ck + 8 * kg + u;
-          vals[u] = k < nb ? zz[k * ZROWS + t] : make_float2(0.0f, 0.0f);
-        }
-        write_digit_group_ff(z.Zd + op * TS * sl, z.NR, y, kg, vals, e);
+      for (int u = 0; u < 8; u++) {
+        const int k = 32 * ck + 8 * kg + u;
+        vals[u] = k < nb ? renorm(zz[k * ZROWS + t]) : make_float2(0.0f, 0.0f);
       }
+      write_digit_group_ff(z.Zd + op * TS * sl, z.NR, y, kg, vals, e);
     }
   }
 }
@@ -1030,9 +1051,9 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
   // every row of the operand, zeros past ns
   const dim3 gz((unsigned)(NR * 32 / ZROWS), (unsigned)x.nm, (unsigned)x.na);
   if (nbk == 1)
-    DBSRG_RUN_W(c, "k_zdigits", zb, zf, k_zdigits<true><<<gz, ZROWS, zsm, st>>>(z));
+    DBSRG_RUN_W(c, "k_zdigits", zb, zf, k_zdigits<true><<<gz, ZROWS * ZW, zsm, st>>>(z));
   else
-    DBSRG_RUN_W(c, "k_zdigits", zb, zf, k_zdigits<false><<<gz, ZROWS, zsm, st>>>(z));
+    DBSRG_RUN_W(c, "k_zdigits", zb, zf, k_zdigits<false><<<gz, ZROWS * ZW, zsm, st>>>(z));
   XArgs p{};
   p.ns = ns;
   p.NR = NR;
