@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(ZROWS * ZW) k_zdigits(const ZArgs z) {
 struct XArgs {
   int ns, NR, ntx, nty, nm, na, lower;
   int nbk;                     // chunks of 32 bound orbitals (products per term and field)
-  int nrows;                   // (quadrant record, x tile) rows of 128 x ns
+  int nrows;                   // work items: y segments of (quadrant record, x tile) strips
+  int ysplit;                  // y segments per 128 x ns strip
   const __nv_bfloat16 *Ud[4];  // per atype: [mode][chunk][slice][NR][TILE]
   const int *eu[4];            // per atype: [mode][chunk][NR*33]
   const __nv_bfloat16 *Zd;     // [a][mode][slot][chunk][slice][NR][TILE]
@@ -270,10 +271,16 @@ struct XArgs {
 // t = atype | transposed << 2 | member slot << 3
 struct Row {
   int blk, qr, qc, nt, half, tx;
+  int ty0, ty1;  // y tiles of the item
   int tc[MAXT];
 };
 
 __device__ __forceinline__ void load_row(const XArgs &p, int row, Row &r) {
+  const int seg = row % p.ysplit;
+  row /= p.ysplit;
+  const int per = (p.nty + p.ysplit - 1) / p.ysplit;
+  r.ty0 = seg * per;
+  r.ty1 = min(p.nty, r.ty0 + per);
   const int4 *q = reinterpret_cast<const int4 *>(p.xq + row / p.ntx);
   const int4 v0 = q[0], v1 = q[1], v2 = q[2];  // blk qr qc nt | half t0 t1 t2 | t3 . . .
   r.tx = row % p.ntx;
@@ -337,11 +344,11 @@ __device__ __forceinline__ bool prod_next(const XArgs &p, int nbk, ProdIt &it) {
   it.ck = 0;
   it.pc++;
   while (it.pc >= it.np) {
-    if (++it.ty >= p.nty) {
+    if (++it.ty >= it.r.ty1) {
       it.row += gridDim.x;
       if (it.row >= p.nrows) return false;
       load_row(p, it.row, it.r);
-      it.ty = 0;
+      it.ty = it.r.ty0;
     }
     bool band;
     it.codes = tile_products(p, it.r, it.ty, it.np, band);
@@ -365,6 +372,7 @@ __device__ __forceinline__ void prod_operands(const XArgs &p, int nbk, const Pro
   Bs = (tra ? Ub : Zb) + (size_t)it.ty * TILE;
 }
 
+constexpr int XITEMS = 8;               // work items an SM (split_exchange)
 constexpr int NCW = 16;               // consumer (epilogue) warps
 constexpr int CPT = 32 / (NCW / 4);   // tile columns per consumer thread
 constexpr int WPROD = NCW;            // producer warp
@@ -473,7 +481,8 @@ __global__ void __maxnreg__(96) k_xfused(const XArgs p) {
     if (lane == 0) {
       ProdIt it;
       it.row = (int)blockIdx.x - (int)gridDim.x;
-      it.ty = p.nty - 1;
+      it.ty = 0;
+      it.r.ty1 = 0;
       it.pc = 0;
       it.np = 0;
       it.ck = nbk - 1;  // the first prod_next moves to the first product
@@ -606,7 +615,7 @@ __global__ void __maxnreg__(96) k_xfused(const XArgs p) {
         const int x0 = r.tx * 128, nrow = min(128, p.ns - x0);
         const double *hq = p.hch + (size_t)(r.blk - 1) * ms * ms + (size_t)(r.qr - 1) * p.ns +
                            ms * (size_t)(r.qc - 1) * p.ns;
-        for (int ty = 0; ty < p.nty; ty++) {
+        for (int ty = r.ty0; ty < r.ty1; ty++) {
           int np;
           bool band;
           tile_products(p, r, ty, np, band);
@@ -717,7 +726,7 @@ __global__ void __maxnreg__(96) k_xfused(const XArgs p) {
       const bool row_ok = x < p.ns;
       const double *hq = p.hch + (size_t)(r.blk - 1) * ms * ms + (size_t)(r.qr - 1) * p.ns +
                          ms * (size_t)(r.qc - 1) * p.ns;
-      for (int ty = 0; ty < p.nty; ty++) {
+      for (int ty = r.ty0; ty < r.ty1; ty++) {
         int np;
         bool band;
         const uint32_t codes = tile_products(p, r, ty, np, band);
@@ -1063,7 +1072,18 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
   p.na = x.na;
   p.lower = x.lower;
   p.nbk = nbk;
-  p.nrows = x.nxq * ntx;
+  // Items of a launch: a strip of 128 rows whole (its A operands are loaded
+  // once) where the strips keep every SM busy for several rounds, otherwise
+  // its y tiles split so that they do: XITEMS items an SM, at least one tile
+  // each.  One channel at ns 300 (12 strips): 82 -> 22 us a launch; ns 283, 26
+  // segments (312 strips on 152 SMs): 98 us whole, 95, 82, 82, 73, 69 and 69 us
+  // at 1, 2, 4, 8, 16 and 32 items; ns 400, 80 channels: 494 us up to 8 items,
+  // 522 and 596 us at 16 and 32 (more loads of A operands).
+  const int strips = x.nxq * ntx;
+  p.ysplit = std::max(1, std::min(nty, (XITEMS * c->nsm + strips - 1) / strips));
+  const int per = (nty + p.ysplit - 1) / p.ysplit;
+  p.ysplit = (nty + per - 1) / per;  // no empty segment
+  p.nrows = strips * p.ysplit;
   for (int a = 0; a < x.na; a++) {
     p.Ud[a] = (const __nv_bfloat16 *)x.far[a]->Ud;
     p.eu[a] = x.far[a]->eu;
