@@ -7,8 +7,8 @@
 //   UPDATE_HS/HW/HX   DBSR_MAT3/updates.f90:79-216
 //
 // Work decomposition (one Gen_matrix call):
-//   1. the list is copied to the device in Add_matrix (IPT) order;
-//   2. k_segments marks the runs of equal K1 (one channel pair each) --
+//   1. k_list_entries gathers the list into Add_matrix (IPT) order;
+//   2. k_list_segments marks the runs of equal K1 (one channel pair each) --
 //      the reference flushes a segment when the next K1 differs;
 //   3. k_density_acc forms xx = sum_e c_e * density(e) for every segment
 //      and atype, entries in list order;
@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <functional>
 
 namespace {
@@ -34,104 +35,162 @@ constexpr int kSegChunk = 256;  // segments per pass of the plain contraction
 
 
 // ---------------------------------------------------------------------------
-// list gather into IPT order
-__global__ void k_gather(int n, const int *ipt, const int *k1, const int *k2, const int *k3,
-                         const double *c, int *o1, int *o2, int *o3, double *oc) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  int i = ipt ? ipt[e] - 1 : e;
-  o1[e] = k1[i];
-  o2[e] = k2[i];
-  o3[e] = k3[i];
-  oc[e] = c[i];
-}
-
-// segment starts: positions where K1 differs from the previous entry.
-// Single thread block; counts per thread chunk, block scan, then writes.
-__global__ void k_segments(int n, const int *k1, int *seg_start, int *nseg_out) {
-  __shared__ int cnt[1024];
-  int tid = threadIdx.x, nt = blockDim.x;
-  int chunk = (n + nt - 1) / nt;
-  int lo = tid * chunk, hi = min(n, lo + chunk);
-  int c = 0;
-  for (int p = lo; p < hi; p++)
-    if (p == 0 || k1[p] != k1[p - 1]) c++;
-  cnt[tid] = c;
-  __syncthreads();
-  // inclusive scan (Hillis-Steele)
-  for (int off = 1; off < nt; off <<= 1) {
-    int v = tid >= off ? cnt[tid - off] : 0;
-    __syncthreads();
-    cnt[tid] += v;
-    __syncthreads();
-  }
-  int base = cnt[tid] - c;
-  for (int p = lo; p < hi; p++)
-    if (p == 0 || k1[p] != k1[p - 1]) seg_start[base++] = p;
-  if (tid == nt - 1) {
-    seg_start[cnt[tid]] = n;
-    *nseg_out = cnt[tid];
-  }
-}
-
-// the coefficients as float-float pairs (split form gather-sums)
-__global__ void k_cd_ff(int n, const double *cd, float2 *cdf) {
+// Set-up of a list in two launches and one read-back.  The host waits for it
+// once a list, so its length is what a wave of short lists costs: six launches
+// and two read-backs took 130 to 170 us of a list's issue, this takes 65 to 90
+// (ns 283, 32 channels, 59 lists: 18.9 -> 16.5 ms a wave, with four list buffers
+// instead of two and the set-up stream at the highest priority).
+//
+// (1) The entries: gathered into IPT order, the coefficients as float-float
+// pairs too (split form gather-sums), and checked: IPT, K2 and K3 must address
+// the list and pq(:,:,1:nbf) (err 1), coefficients be finite (err 3).  With bmap
+// (factored forms) the ordered pair of bound orbitals of every entry (pair_err
+// where one is not bound).
+__global__ void k_list_entries(int n, const int *ipt, const int *k1, const int *k2,
+                               const int *k3, const double *c, int nbf, const int *bmap, int nb,
+                               int check, int *o1, int *o2, int *o3, double *oc, float2 *ocf,
+                               int *pairs, int *err, int *pair_err) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < n) cdf[e] = ffa::split(cd[e]);
-}
-
-// bound-orbital indices of every entry must address pq(:,:,1:nbf) (err 1),
-// and every coefficient must be finite (err 3)
-__global__ void k_check_orbitals(int n, const int *k2, const int *k3, const double *cd, int nbf,
-                                 int *err) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
-  if (k2[e] < 1 || k2[e] > nbf || k3[e] < 1 || k3[e] > nbf) atomicExch(err, 1);
-  if (!isfinite(cd[e])) atomicExch(err, 3);
+  const int i = ipt ? ipt[e] - 1 : e;
+  if (i < 0 || i >= n) {
+    atomicExch(err, 1);
+    return;
+  }
+  const int a = k2[i], b = k3[i];
+  const double v = c[i];
+  o1[e] = k1[i];
+  o2[e] = a;
+  o3[e] = b;
+  oc[e] = v;
+  ocf[e] = ffa::split(v);
+  if (!check) return;
+  if (!isfinite(v)) atomicExch(err, 3);
+  if (a < 1 || a > nbf || b < 1 || b > nbf) {
+    atomicExch(err, 1);
+    return;
+  }
+  if (bmap) {
+    const int x = bmap[a - 1], y = bmap[b - 1];
+    if (x < 0 || y < 0) atomicExch(pair_err, 3);
+    pairs[e] = x < 0 || y < 0 ? 0 : x * nb + y;
+  }
 }
 
-// decode segments, look up blocks, pair up segments of the same block
-__global__ void k_seg_info(int nseg, const int *seg_start, const int *k1, int nch, int iicc,
-                           const int *icc, SegInfo *info, int *err) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  SegInfo si;
-  si.start = seg_start[s];
-  si.end = seg_start[s + 1];
-  int key = k1[si.start];
-  si.ich = key / DBSRG_IBO;
-  si.jch = key % DBSRG_IBO;
-  si.blk = 0;
-  si.partner = -1;
-  si.owner = 1;
-  if (si.ich < 1 || si.jch < 1 || si.ich > nch || si.jch > nch) {
-    atomicExch(err, 1);
-  } else {
-    int b = icc[(si.ich - 1) + (size_t)nch * (si.jch - 1)];
-    if (b < 1 || b > iicc)
-      atomicExch(err, 2);
-    else
-      si.blk = b;
-    if (si.ich != si.jch) {
-      // the swapped pair maps to the same block; binary search its K1
-      int want = si.jch * DBSRG_IBO + si.ich;
-      int lo = 0, hi = nseg - 1;
-      while (lo <= hi) {
-        int mid = (lo + hi) >> 1;
-        int v = k1[seg_start[mid]];
-        if (v == want) {
-          si.partner = mid;
-          break;
-        }
-        if (v < want)
-          lo = mid + 1;
-        else
-          hi = mid - 1;
-      }
-      if (si.partner >= 0 && si.partner < s) si.owner = 0;
+// (2) The segments (runs of equal K1, one channel pair each), their blocks and
+// the pairing of segments of one block, by one thread block: eight entries a
+// thread and round, counted and placed by warp and block scans; then one
+// thread per segment decodes its K1 and finds the swapped pair by binary
+// search over the segments' keys (in shared memory up to SEGKEYS of them).
+// A list of one segment: 6.7 us, 6.5 + 6.5 us as two kernels with a read-back
+// between them, one run of entries per thread and the keys looked up in the list.
+constexpr int SEGKEYS = 4096;
+
+// dscal: [0] number of segments, [1] error (set here or by the entries)
+__global__ void __launch_bounds__(1024) k_list_segments(int n, const int *__restrict__ k1,
+                                                        int nch, int iicc, const int *icc,
+                                                        int *seg_start, SegInfo *info,
+                                                        int *dscal) {
+  __shared__ int wsum[32];
+  __shared__ int keys[SEGKEYS];
+  __shared__ int base;
+  const int tid = threadIdx.x, lane = tid % 32, w = tid / 32;
+  if (tid == 0) base = 0;
+  __syncthreads();
+  for (int p0 = 0; p0 < n; p0 += 8 * 1024) {
+    const int p = p0 + 8 * tid;
+    int v[8], prev = 0;
+    unsigned flag = 0;
+    if (p > 0 && p < n) prev = k1[p - 1];
+    if (p + 8 <= n) {  // k1 is 256-byte aligned, p a multiple of 8
+      const int4 x = *reinterpret_cast<const int4 *>(k1 + p),
+                 y = *reinterpret_cast<const int4 *>(k1 + p + 4);
+      v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+      v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = p + u < n ? k1[p + u] : 0;
     }
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (p + u < n && (p + u == 0 || v[u] != (u ? v[u - 1] : prev))) flag |= 1u << u;
+    int cnt = __popc(flag), incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+      int x = wsum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      wsum[lane] = x;
+    }
+    __syncthreads();
+    int at = base + (w ? wsum[w - 1] : 0) + incl - cnt;
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (flag >> u & 1) {
+        seg_start[at] = p + u;
+        if (at < SEGKEYS) keys[at] = v[u];
+        at++;
+      }
+    __syncthreads();
+    if (tid == 0) base += wsum[31];
+    __syncthreads();
   }
-  info[s] = si;
+  const int nseg = base;
+  if (tid == 0) {
+    seg_start[nseg] = n;
+    dscal[0] = nseg;
+  }
+  __threadfence_block();
+  __syncthreads();
+  const bool cached = nseg <= SEGKEYS;
+  auto key_of = [&](int s) { return cached ? keys[s] : k1[seg_start[s]]; };
+  for (int s = tid; s < nseg; s += 1024) {
+    SegInfo si;
+    si.start = seg_start[s];
+    si.end = seg_start[s + 1];
+    const int key = key_of(s);
+    si.ich = key / DBSRG_IBO;
+    si.jch = key % DBSRG_IBO;
+    si.blk = 0;
+    si.partner = -1;
+    si.owner = 1;
+    if (si.ich < 1 || si.jch < 1 || si.ich > nch || si.jch > nch) {
+      atomicExch(dscal + 1, 1);
+    } else {
+      const int b = icc[(si.ich - 1) + (size_t)nch * (si.jch - 1)];
+      if (b < 1 || b > iicc)
+        atomicExch(dscal + 2, 2);
+      else
+        si.blk = b;
+      if (si.ich != si.jch) {
+        // the swapped pair maps to the same block; binary search its K1
+        const int want = si.jch * DBSRG_IBO + si.ich;
+        int lo = 0, hi = nseg - 1;
+        while (lo <= hi) {
+          const int mid = (lo + hi) >> 1, x = key_of(mid);
+          if (x == want) {
+            si.partner = mid;
+            break;
+          }
+          if (x < want)
+            lo = mid + 1;
+          else
+            hi = mid - 1;
+        }
+        if (si.partner >= 0 && si.partner < s) si.owner = 0;
+      }
+    }
+    info[s] = si;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -675,8 +734,8 @@ size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 size_t plan_bytes(const dbsrg_ctx *c, int icase, int itype, int n) {
   if (is_structure_list(icase, itype)) return structure_plan_bytes(c, icase, itype, n);
   const size_t ib = sizeof(int) * (size_t)n, db = sizeof(double) * (size_t)n;
-  size_t t = 8 * al256(ib) + 2 * al256(db) + al256(sizeof(int) * (n + 2)) + al256(64) +
-             al256(sizeof(SegInfo) * (size_t)(n + 1)) + al256(sizeof(int) * (size_t)(7 * (n + 1))) +
+  size_t t = 8 * al256(ib) + 2 * al256(db) + al256(sizeof(int) * (n + 2)) +
+             al256(64 + sizeof(SegInfo) * (size_t)(n + 1)) + al256(sizeof(int) * (size_t)(7 * (n + 1))) +
              al256(sizeof(XQuad) * 4 * (size_t)(n + 1)) + al256(sizeof(float2) * (size_t)n);
   if (icase == 0)
     t += al256(sizeof(int) * (2 * (size_t)(c->iicc + 2) + n));
@@ -728,24 +787,44 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
   P.lcd = (double *)take(dbytes);
   P.lpair = (int *)take(ibytes);  // factored path: bound-orbital pair of each entry
   int *seg_start = (int *)take(sizeof(int) * (size_t)(n + 2));
-  int *dscal = (int *)take(64);  // [0]=nseg [1]=err [2]=- [3]=pair err
-  P.info = (SegInfo *)take(sizeof(SegInfo) * (size_t)(n + 1));
+  // [0] segments [1] error [2] block error [3] pair error, and behind them the
+  // segment table: read back together
+  constexpr size_t HDR = 64;
+  int *dscal = (int *)take(HDR + sizeof(SegInfo) * (size_t)(n + 1));
+  P.info = (SegInfo *)((char *)dscal + HDR);
   // per chunk member segment ids and owner slots (at most 6 ints per
   // segment), then the acf owners (one per segment)
   P.work = (int *)take(sizeof(int) * (size_t)(7 * (n + 1)));
   P.dxq = (XQuad *)take(sizeof(XQuad) * 4 * (size_t)(n + 1));
   P.lcdf = (float2 *)take(sizeof(float2) * (size_t)n);
-  if ((rc = copy_in_s(c, dk1, k1, ibytes, ss))) return rc;
-  if ((rc = copy_in_s(c, dk2, k2, ibytes, ss))) return rc;
-  if ((rc = copy_in_s(c, dk3, k3, ibytes, ss))) return rc;
-  if ((rc = copy_in_s(c, dcd, cdata, dbytes, ss))) return rc;
-  if (ipt && (rc = copy_in_s(c, dipt, ipt, ibytes, ss))) return rc;
-  DBSRG_TRY(c, cudaMemsetAsync(dscal, 0, 64, ss));
-  DBSRG_RUN_S(c, ss, "k_gather",
-              k_gather<<<(n + 255) / 256, 256, 0, ss>>>(n, ipt ? dipt : nullptr, dk1, dk2, dk3,
-                                                        dcd, P.lk1, P.lk2, P.lk3, P.lcd));
-  DBSRG_RUN_S(c, ss, "k_cd_ff",
-              k_cd_ff<<<(n + 255) / 256, 256, 0, ss>>>(n, P.lcd, P.lcdf));
+  P.factored = c->precision != DBSRG_PLAIN_FP64;
+  if (icase != 0 && P.factored) {
+    // the factored contraction works with ordered pairs of bound orbitals
+    if (c->nbound < 1) return set_err(c, DBSRG_ESTATE, "no bound orbitals (ipbs = 0)");
+    if (c->nbound > 128)
+      return set_err(c, DBSRG_EINVAL, "factored contraction: 1..128 bound orbitals (ipbs = 0)");
+  }
+  if ((rc = ensure_pinned(c, HDR + sizeof(SegInfo) * 2048))) return rc;
+  // lists resident and aligned on this device are read where they are (the
+  // read-back below waits for that), others copied in
+  const int *src[4] = {k1, k2, k3, ipt};
+  int *dst[4] = {dk1, dk2, dk3, dipt};
+  for (int q = 0; q < 4; q++)
+    if (src[q] && !device_readable(c, src[q], alignof(int))) {
+      if ((rc = copy_in_s(c, dst[q], src[q], ibytes, ss))) return rc;
+      src[q] = dst[q];
+    }
+  const double *srcc = cdata;
+  if (!device_readable(c, cdata, alignof(double))) {
+    if ((rc = copy_in_s(c, dcd, cdata, dbytes, ss))) return rc;
+    srcc = dcd;
+  }
+  DBSRG_TRY(c, cudaMemsetAsync(dscal, 0, HDR, ss));
+  DBSRG_RUN_S(c, ss, "k_list_entries",
+              k_list_entries<<<(n + 255) / 256, 256, 0, ss>>>(
+                  n, src[3], src[0], src[1], src[2], srcc, c->nbf,
+                  P.factored && icase != 0 ? c->bmap : nullptr, c->nbound, icase != 0, P.lk1,
+                  P.lk2, P.lk3, P.lcd, P.lcdf, P.lpair, dscal + 1, dscal + 3));
 
   // ---- overlaps: entries grouped by block on the host (counting sort, list
   // order kept within a block); entries below eps_c are dropped
@@ -758,10 +837,13 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
     P.order = P.tlist + (iicc + 2);
     std::vector<int> hk1(n), hk2(n);
     std::vector<double> hcd(n);
+    int oerr = 0;
+    DBSRG_TRY(c, cudaMemcpyAsync(&oerr, dscal + 1, sizeof(int), cudaMemcpyDeviceToHost, ss));
     DBSRG_TRY(c, cudaMemcpyAsync(hk1.data(), P.lk1, ibytes, cudaMemcpyDeviceToHost, ss));
     DBSRG_TRY(c, cudaMemcpyAsync(hk2.data(), P.lk2, ibytes, cudaMemcpyDeviceToHost, ss));
     DBSRG_TRY(c, cudaMemcpyAsync(hcd.data(), P.lcd, dbytes, cudaMemcpyDeviceToHost, ss));
     DBSRG_TRY(c, cudaStreamSynchronize(ss));
+    if (oerr) return set_err(c, DBSRG_ERANGE, "IPT entry out of range");
     std::vector<int> eblk(n, 0), hstart(iicc + 2, 0), hlist, horder(n);
     for (int e = 0; e < n; e++) {
       if (!std::isfinite(hcd[e])) return set_err(c, DBSRG_EINVAL, "non-finite coefficient in list");
@@ -805,25 +887,7 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
     return DBSRG_OK;
   }
 
-  // ---- segments (orbital check and segment count read back together)
-  DBSRG_RUN_S(c, ss, "k_check_orbitals",
-              k_check_orbitals<<<(n + 255) / 256, 256, 0, ss>>>(n, P.lk2, P.lk3, P.lcd, c->nbf,
-                                                                dscal + 1));
-  DBSRG_RUN_S(c, ss, "k_segments", k_segments<<<1, 1024, 0, ss>>>(n, P.lk1, seg_start, dscal));
-  int hs[4] = {0, 0, 0, 0};  // nseg, error, -, bound-pair error
-  DBSRG_TRY(c, cudaMemcpyAsync(hs, dscal, 2 * sizeof(int), cudaMemcpyDeviceToHost, ss));
-  DBSRG_TRY(c, cudaStreamSynchronize(ss));
-  if (hs[1] == 3) return set_err(c, DBSRG_EINVAL, "non-finite coefficient in list");
-  if (hs[1]) return set_err(c, DBSRG_ERANGE, "channel or orbital index out of range in list");
-  const int nseg = hs[0];
-  if (nseg < 1 || nseg > n) return set_err(c, DBSRG_ECUDA, "inconsistent segment count");
-  P.nseg = nseg;
-  DBSRG_RUN_S(c, ss, "k_seg_info",
-              k_seg_info<<<(nseg + 127) / 128, 128, 0, ss>>>(nseg, seg_start, P.lk1, c->nch,
-                                                             c->iicc, c->icc, P.info, dscal + 1));
-
   // ---- the case: PQ types, storage and convol case
-  P.factored = c->precision != DBSRG_PLAIN_FP64;
   if (icase == 2) {
     if (itype != 3 && itype != 4) return set_err(c, DBSRG_EINVAL, "R_data: unknown itype");
     if (kpol < 0 || kpol > c->mk) return set_err(c, DBSRG_ERANGE, "R_data: kpol out of range");
@@ -885,19 +949,32 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
   P.per = (size_t)ns * P.ncol;
   P.split_x = P.factored && P.icv >= 3 && c->precision == DBSRG_SPLIT_BF16;
 
-  if (P.factored) {
-    // the factored contraction works with ordered pairs of bound orbitals
-    if (c->nbound < 1) return set_err(c, DBSRG_ESTATE, "no bound orbitals (ipbs = 0)");
-    if ((rc = pair_index(c, n, P.lk2, P.lk3, P.lpair, dscal + 3, ss))) return rc;
-  }
-  // segment table, segment errors and bound-pair errors in one read-back
-  std::vector<SegInfo> hinfo(nseg);
-  DBSRG_TRY(c, cudaMemcpyAsync(hs, dscal, 4 * sizeof(int), cudaMemcpyDeviceToHost, ss));
-  DBSRG_TRY(c, cudaMemcpyAsync(hinfo.data(), P.info, sizeof(SegInfo) * nseg,
+  // ---- segments: count, errors and the table in one read-back into pinned
+  // memory (of as many segments as there are channel pairs, at most 2048; a
+  // longer table takes a second one)
+  DBSRG_RUN_S(c, ss, "k_list_segments",
+              k_list_segments<<<1, 1024, 0, ss>>>(n, P.lk1, c->nch, c->iicc, c->icc, seg_start,
+                                                  P.info, dscal));
+  const size_t nfirst = std::min<size_t>({(size_t)n, (size_t)c->nch * c->nch, (size_t)2048});
+  DBSRG_TRY(c, cudaMemcpyAsync(c->pinned, dscal, HDR + sizeof(SegInfo) * nfirst,
                                cudaMemcpyDeviceToHost, ss));
   DBSRG_TRY(c, cudaStreamSynchronize(ss));
-  if (hs[1] == 1) return set_err(c, DBSRG_ERANGE, "channel or orbital index out of range in list");
-  if (hs[1] == 2) return set_err(c, DBSRG_ERANGE, "channel pair has no block in icc");
+  int hs[4];
+  std::memcpy(hs, c->pinned, sizeof(hs));
+  if (hs[1] == 3) return set_err(c, DBSRG_EINVAL, "non-finite coefficient in list");
+  if (hs[1]) return set_err(c, DBSRG_ERANGE, "channel or orbital index out of range in list");
+  const int nseg = hs[0];
+  if (nseg < 1 || nseg > n) return set_err(c, DBSRG_ECUDA, "inconsistent segment count");
+  P.nseg = nseg;
+  std::vector<SegInfo> hinfo(nseg);
+  std::memcpy(hinfo.data(), (char *)c->pinned + HDR,
+              sizeof(SegInfo) * std::min<size_t>(nseg, nfirst));
+  if ((size_t)nseg > nfirst) {
+    DBSRG_TRY(c, cudaMemcpyAsync(hinfo.data() + nfirst, P.info + nfirst,
+                                 sizeof(SegInfo) * (nseg - nfirst), cudaMemcpyDeviceToHost, ss));
+    DBSRG_TRY(c, cudaStreamSynchronize(ss));
+  }
+  if (hs[2]) return set_err(c, DBSRG_ERANGE, "channel pair has no block in icc");
   if (hs[3]) return set_err(c, DBSRG_EINVAL, "factored contraction: K2/K3 must be bound orbitals");
   for (int s = 0; s < nseg; s++) {
     const SegInfo &si = hinfo[s];
@@ -1240,12 +1317,12 @@ int gen_matrix_plain(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const 
   if (!c->pq) return set_err(c, DBSRG_ESTATE, "no orbitals set");
   cudaStream_t st = c->stream;
   int rc;
-  // The list state lives in one of two buffers; in the asynchronous mode the
-  // set-up runs on the set-up stream once the kernels of the call two back
-  // are done with the buffer, while the previous call's kernels run.
+  // The list state lives in one of NLSTATE buffers; in the asynchronous mode
+  // the set-up runs on the set-up stream once the kernels of the call NLSTATE
+  // back are done with the buffer, while the kernels of the calls between run.
   const bool pipe = c->async;
-  const int par = c->lpar;
-  c->lpar ^= 1;
+  const int par = pipe ? c->lpar : 0;
+  if (pipe) c->lpar = (c->lpar + 1) % dbsrg_ctx::NLSTATE;
   cudaStream_t ss = pipe ? c->sstream : st;
   if ((rc = ensure_lstate(c, par, plan_bytes(c, icase, itype, n)))) return rc;
   if (pipe) DBSRG_TRY(c, cudaStreamWaitEvent(ss, c->lfree[par], 0));

@@ -36,6 +36,17 @@ bool is_device_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+bool device_readable(const dbsrg_ctx *c, const void *p, size_t align) {
+  if (!p || reinterpret_cast<uintptr_t>(p) % align) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return (a.type == cudaMemoryTypeDevice && a.device == c->device) ||
+         a.type == cudaMemoryTypeManaged;
+}
+
 int copy_in_s(dbsrg_ctx *c, void *dst, const void *src, size_t n, cudaStream_t s) {
   if (n == 0) return DBSRG_OK;
   if (!src) return set_err(c, DBSRG_EINVAL, "null input pointer");
@@ -296,7 +307,7 @@ int dbsrg_create(dbsrg_ctx **out, const dbsrg_grid_desc *d) {
   }
   int prio_lo = 0, prio_hi = 0;
   cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
-  if (cudaStreamCreateWithFlags(&c->sstream, cudaStreamNonBlocking) != cudaSuccess ||
+  if (cudaStreamCreateWithPriority(&c->sstream, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->cstream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithPriority(&c->bstream[0], cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
       cudaStreamCreateWithPriority(&c->bstream[1], cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
@@ -306,13 +317,17 @@ int dbsrg_create(dbsrg_ctx **out, const dbsrg_grid_desc *d) {
       cudaEventCreateWithFlags(&c->cdone[0], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->cdone[1], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->wdone, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->lfree[0], cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->lfree[1], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->lready, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
     dbsrg_destroy(c);
     return DBSRG_ECUDA;
   }
+  for (cudaEvent_t &e : c->lfree)
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      dbsrg_destroy(c);
+      return DBSRG_ECUDA;
+    }
   DeviceGrid &g = c->g;
   g.ns = d->ns;
   g.ks = d->ks;
@@ -360,7 +375,7 @@ int dbsrg_destroy(dbsrg_ctx *c) {
   if (c->tcscratch) cudaFree(c->tcscratch);
   for (void *p : c->pscratch)
     if (p) cudaFree(p);
-  for (int i = 0; i < 2; i++) {
+  for (int i = 0; i < dbsrg_ctx::NLSTATE; i++) {
     if (c->lstate[i]) cudaFree(c->lstate[i]);
     if (c->lfree[i]) cudaEventDestroy(c->lfree[i]);
   }

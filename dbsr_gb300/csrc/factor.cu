@@ -78,20 +78,6 @@ __global__ void k_bound_rows(int ns, int nb, const int *b2o, const double *pq, d
   Pf[o] = ffa::split(v);
 }
 
-// ordered bound-orbital pair of every entry
-__global__ void k_pair_index(int n, const int *k2, const int *k3, const int *bmap, int nb,
-                             int *pairs, int *err) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  int a = bmap[k2[e] - 1], b = bmap[k3[e] - 1];
-  if (a < 0 || b < 0) {
-    atomicExch(err, 3);
-    pairs[e] = 0;
-    return;
-  }
-  pairs[e] = a * nb + b;
-}
-
 // ---------------------------------------------------------------------------
 // far-field vectors of one electron: Ulo(x,a) = sum_iv sum_xc mlo(pair;iv) p_a(xc)
 // (and Uhi with mhi), x the output function, xc the contracted one, and their
@@ -806,17 +792,6 @@ __global__ void k_scatter_dp(int ns, int ks, char sym, QuadSpec sp, KdSet kd,
 
 int ensure_fscratch(dbsrg_ctx *c, size_t bytes) {
   return grow_buffer(c, &c->fscratch, &c->fscratch_bytes, bytes);
-}
-
-int pair_index(dbsrg_ctx *c, int n, const int *k2, const int *k3, int *pairs, int *derr,
-               cudaStream_t s) {
-  if (n <= 0) return DBSRG_OK;
-  if (c->nbound < 1 || c->nbound > NB_MAX)
-    return set_err(c, DBSRG_EINVAL, "factored contraction: 1..128 bound orbitals (ipbs = 0)");
-  DBSRG_RUN_S(c, s, "k_pair_index",
-              k_pair_index<<<(n + 255) / 256, 256, 0, s>>>(n, k2, k3, c->bmap, c->nbound, pairs,
-                                                           derr));
-  return DBSRG_OK;
 }
 
 // far-field vectors of (family, type, k, exchange case), cached; R^k (case 3

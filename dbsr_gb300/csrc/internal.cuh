@@ -154,15 +154,17 @@ struct dbsrg_ctx {
   void *pscratch[2] = {nullptr, nullptr};
   size_t pscratch_bytes[2] = {0, 0};
   // List pipeline.  The state of one Gen_matrix call (the list in IPT order,
-  // segments, chunk members, quadrant records) lives in one of two buffers,
-  // alternating per call.  Its set-up (copies, segment kernels, read-backs)
-  // runs on sstream once the kernels of the call two back have released the
-  // buffer (lfree), and the contraction on stream waits for it (lready), so
+  // segments, chunk members, quadrant records) lives in one of NLSTATE buffers,
+  // taken in turn.  Its set-up (copies, segment kernels, read-back) runs on
+  // sstream (of the highest priority: the host waits for it) once the kernels
+  // of the call NLSTATE back have released the buffer (lfree), and the
+  // contraction on stream waits for it (lready), so
   // the host plans one list while the kernels of the previous one run.
   cudaStream_t sstream = nullptr;
-  void *lstate[2] = {nullptr, nullptr};
-  size_t lstate_bytes[2] = {0, 0};
-  cudaEvent_t lfree[2] = {nullptr, nullptr};
+  static constexpr int NLSTATE = 4;
+  void *lstate[NLSTATE] = {};
+  size_t lstate_bytes[NLSTATE] = {};
+  cudaEvent_t lfree[NLSTATE] = {};
   cudaEvent_t lready = nullptr;
   int lpar = 0;
   // Table streams.  The tables, cell data, far fields, digits and pair
@@ -317,6 +319,9 @@ bool sync_check_enabled();
 #define DBSRG_RUN_S(ctx, strm, name, ...) DBSRG_RUN_SW(ctx, strm, name, 0, 0, __VA_ARGS__)
 
 bool is_device_ptr(const void *p);
+// a kernel of this context can read p in place: memory of its device (or
+// managed), at a multiple of align
+bool device_readable(const dbsrg_ctx *c, const void *p, size_t align);
 // copies n bytes from a host-or-device pointer into device memory dst
 int copy_in(dbsrg_ctx *c, void *dst, const void *src, size_t n);
 int copy_in_s(dbsrg_ctx *c, void *dst, const void *src, size_t n, cudaStream_t s);
@@ -514,10 +519,6 @@ int get_pairpot_direct_ff(dbsrg_ctx *c, int family, int type, int k, int icv, in
                           const float2 **out);
 int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1, int jp2,
                            bool ff, const void **out);
-// pairs[e] = bmap[K2]*nbound + bmap[K3]; sets *derr when an orbital is not bound
-int pair_index(dbsrg_ctx *c, int n, const int *k2, const int *k3, int *pairs, int *derr,
-               cudaStream_t s);
-
 // ---- device helpers ---------------------------------------------------------
 // Values of the kx B-splines that are nonzero on the interval starting at
 // knot tx(kg) (1-based), at point x: the ni=1, nderiv=1 path of zbsplvd /

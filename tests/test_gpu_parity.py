@@ -172,3 +172,38 @@ def test_band_contraction_tiles_by_segment_count(ns, nch):
     a, m = run_both(w)
     check_blocks(a, m, w)
     a.close()
+
+
+@pytest.mark.parametrize("nch,per", [(65, 1), (2, 2731), (1, 8192)])
+def test_list_setup_sizes(nch, per):
+    """The set-up of a list at its sizes: more segments than one read-back
+    holds (2145 channel pairs), entry counts just above and at a round of the
+    segment scan (3 x 2731 = 8193, 8192), host and device lists with the same
+    bits, the coefficients also at an address that is no multiple of eight."""
+    import torch
+
+    w = synth.small(ns=32, nch=nch, mk=0, n_entries=4, breit=False, seed=61)
+    rng = np.random.default_rng(7)
+    pairs = [(i, j) for i in range(1, nch + 1) for j in range(1, i + 1)]
+    k1 = np.repeat(np.array([i * synth.IBO + j for i, j in pairs], np.int32), per)
+    k2 = rng.integers(1, w.nbound + 1, k1.size).astype(np.int32)
+    k3 = rng.integers(1, w.nbound + 1, k1.size).astype(np.int32)
+    c = rng.uniform(-1, 1, k1.size)
+    L = synth.CList(2, 3, 0, k1, k2, k3, np.zeros_like(k1), c)
+    a, m = run_both(w, [L])
+    check_blocks(a, m, w)
+    h = a.get_matrix()
+    raw = torch.zeros(8 * c.size + 4, dtype=torch.uint8, device="cuda")
+    raw[4:] = torch.from_numpy(c.view(np.uint8)).cuda()
+
+    dev = [torch.from_numpy(x).cuda() for x in (k1, k2, k3, L.k4, c)]
+    torch.cuda.synchronize()
+    import ctypes as C
+
+    for coef in (dev[4].data_ptr(), raw.data_ptr() + 4):
+        a.zero_matrix()
+        rc = a._L.dbsrg_gen_matrix(a._h, 2, 3, 0, k1.size, None,
+                                   *[C.c_void_p(x.data_ptr()) for x in dev[:4]], C.c_void_p(coef))
+        assert rc == 0
+        assert np.array_equal(a.get_matrix(), h)
+    a.close()
