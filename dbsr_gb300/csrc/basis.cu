@@ -297,19 +297,18 @@ extern "C" int dbsrg_channel_basis(dbsrg_ctx *c, const double *sol, const int *n
     }
     D = dD;
   }
-  if (cudaMalloc(&dWt, blk * 8)) {
-    cudaGetLastError();
-    if (dD) cudaFree(dD);
-    return set_err(c, DBSRG_ENOMEM, "channel_basis: allocation failed");
-  }
   if (c->precision == DBSRG_SPLIT_BF16) {  // split-BF16 tensor-core products (sgemm.cu)
     rc = split_channel_basis(c, D, nsol);
     cudaStreamSynchronize(st);
-    cudaFree(dWt);
     if (dD) cudaFree(dD);
     if (rc) return rc;
     if (out) return copy_out(c, out, c->hch, blk * c->iicc * 8);
     return DBSRG_OK;
+  }
+  if (cudaMalloc(&dWt, blk * 8)) {
+    cudaGetLastError();
+    if (dD) cudaFree(dD);
+    return set_err(c, DBSRG_ENOMEM, "channel_basis: allocation failed");
   }
   const double one = 1.0, zero = 0.0;
   int bad = 0;

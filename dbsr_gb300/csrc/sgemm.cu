@@ -50,10 +50,23 @@ constexpr int NO_EXP = -100000;   // the empty sum
 
 // digits of R vectors of K elements (vector r at X + r ldx, contiguous),
 // rows padded to NR*32 and K to nk*32 with zeros: out [nk][TS][NR][TILE],
-// chunk exponents ex[nk][NR*32].  One warp per vector; lanes 4q..4q+3 hold
-// the four groups of 8 elements of one chunk.
-__global__ void k_vec_digits(int R, int K, const double *X, size_t ldx, int NR, int nk,
-                             __nv_bfloat16 *out, int *ex) {
+// chunk exponents ex[nk][NR*32]; the matrices of a whole batch in one launch
+// (blockIdx.y: a launch per matrix of ms 500 took 12 us for 2 us of traffic).
+// One warp per vector; lanes 4q..4q+3 hold the four groups of 8 elements of
+// one chunk.
+struct VecJob {
+  const double *X;
+  __nv_bfloat16 *out;
+  int *ex;
+  int R, pad;
+};
+
+__global__ void k_vec_digits(const VecJob *jobs, int K, size_t ldx, int NR, int nk) {
+  const VecJob J = jobs[blockIdx.y];
+  const int R = J.R;
+  const double *X = J.X;
+  __nv_bfloat16 *out = J.out;
+  int *ex = J.ex;
   const int r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
   if (r >= NR * 32) return;  // whole warps
   const double *x = X + (size_t)r * ldx;
@@ -96,6 +109,7 @@ struct GemmJob {
   double *C;                   // C(r, c) at C[r*sr + c*sc]
   long long sr, sc;
   int M, N, NRa, NRb;
+  int Mz, Nz;  // zeros where M <= r < Mz or N <= c < Nz (0: none)
 };
 
 __device__ __forceinline__ void mbar_arrive1(uint32_t mbar) {
@@ -111,10 +125,16 @@ __global__ void __launch_bounds__(NTHR) k_sgemm(const GemmJob *jobs, int nk, int
   __shared__ uint32_t tmem_base;
   __shared__ int s_abort;
   const GemmJob jb = jobs[blockIdx.y];
-  const int ntn = (jb.N + 31) / 32;
+  const int ntn = (max(jb.N, jb.Nz) + 31) / 32;
   const int mt = blockIdx.x / ntn, nt = blockIdx.x % ntn;
-  if (mt * 128 >= jb.M || nt * 32 >= jb.N) return;  // uniform per CTA, before any barrier
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  if (mt * 128 >= jb.M || nt * 32 >= jb.N) {  // uniform per CTA, before any barrier
+    for (int q = tid; q < 128 * 32; q += NTHR) {
+      const int r = mt * 128 + q % 128, cc = nt * 32 + q / 128;
+      if (r < jb.Mz && cc < jb.Nz) jb.C[(long long)r * jb.sr + (long long)cc * jb.sc] = 0.0;
+    }
+    return;
+  }
   if (tid == 0) {
     for (int b = 0; b < 2; b++) {
       mbar_init(smem_u32(&bar_ld[b]), 1);
@@ -279,13 +299,13 @@ __global__ void __launch_bounds__(NTHR) k_sgemm(const GemmJob *jobs, int nk, int
         if (sh < 63) acc[c] += I >> sh;
       }
     }
-    if (!dead && r < jb.M) {
+    if (!dead && r < max(jb.M, jb.Mz)) {
 #pragma unroll
       for (int c = 0; c < 16; c++) {
         const int cc = nt * 32 + ch * 16 + c;
-        if (cc < jb.N)
-          jb.C[(long long)r * jb.sr + (long long)cc * jb.sc] =
-              i64_to_f64(acc[c], cur[c] - 8 * (TS + 1) + SHIFT);
+        if (cc >= max(jb.N, jb.Nz)) continue;
+        jb.C[(long long)r * jb.sr + (long long)cc * jb.sc] =
+            r < jb.M && cc < jb.N ? i64_to_f64(acc[c], cur[c] - 8 * (TS + 1) + SHIFT) : 0.0;
       }
     }
   }
@@ -294,21 +314,6 @@ __global__ void __launch_bounds__(NTHR) k_sgemm(const GemmJob *jobs, int nk, int
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(512));
 }
-
-struct Buf {
-  void *p = nullptr;
-  ~Buf() {
-    if (p) cudaFree(p);
-  }
-  bool alloc(size_t n) {
-    if (cudaMalloc(&p, std::max<size_t>(n, 16)) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-      return false;
-    }
-    return true;
-  }
-};
 
 }  // namespace
 
@@ -333,109 +338,83 @@ int split_channel_basis(dbsrg_ctx *c, const double *D, const int *nsol) {
       bk.push_back(k);
     }
   if (bk.empty()) return DBSRG_OK;
-  // digits of every channel's solutions (columns of D_ch)
-  Buf dD, eD, err;
+  // workspace: digits of every channel's solutions (columns of D_ch), and per
+  // block of a batch the digits of H's columns, W^T (ms x ni) and the digits
+  // of W's rows; batches of at most 32 blocks (each fills the SMs several
+  // times over by itself)
   const size_t esz = (size_t)nk * NR * 32;  // chunk exponents of one operand
-  if (!dD.alloc(dsz * 2 * nch) || !eD.alloc(sizeof(int) * esz * nch) || !err.alloc(4))
-    return set_err(c, DBSRG_ENOMEM, "channel_basis: digit allocation failed");
-  __nv_bfloat16 *Dd = (__nv_bfloat16 *)dD.p;
-  int *De = (int *)eD.p;
-  cudaMemsetAsync(err.p, 0, 4, st);
-  const unsigned gv = (unsigned)((NR * 32 + 7) / 8);  // 8 vectors (warps) a block
-  for (int ch = 1; ch <= nch; ch++)
-    DBSRG_RUN(c, "k_vec_digits",
-              k_vec_digits<<<gv, 256, 0, st>>>(nsol[ch - 1], ms, D + (size_t)(ch - 1) * blk, ms,
-                                                NR, nk, Dd + dsz * (ch - 1),
-                                                De + esz * (ch - 1)));
-  // blocks in batches: digits of H's columns, W^T (ms x ni), digits of W's rows
-  const size_t per_blk = 2 * dsz * 2 + blk * 8 + 2 * sizeof(int) * esz;
-  size_t freeb = 0, totb = 0;
-  cudaMemGetInfo(&freeb, &totb);
-  int nb = (int)std::max<size_t>(1, std::min<size_t>(256, (freeb / 4) / per_blk));
-  nb = std::min<int>(nb, (int)bk.size());
-  Buf dH, dW, dWd, eH, eW, dJ;
-  if (!dH.alloc(dsz * 2 * nb) || !dW.alloc(blk * 8 * nb) || !dWd.alloc(dsz * 2 * nb) ||
-      !eH.alloc(sizeof(int) * esz * nb) || !eW.alloc(sizeof(int) * esz * nb) ||
-      !dJ.alloc(sizeof(GemmJob) * nb))
-    return set_err(c, DBSRG_ENOMEM, "channel_basis: product allocation failed");
-  const size_t smem = 2 * TS * (A_BYTES + B_BYTES);
+  const int nb = std::min<int>(32, (int)bk.size());
+  size_t total = 0;
+  auto part = [&](size_t bytes) {
+    const size_t o = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return o;
+  };
+  const size_t oD = part(dsz * 2 * nch), oeD = part(sizeof(int) * esz * nch), oErr = part(4),
+               oVD = part(sizeof(VecJob) * nch), oH = part(dsz * 2 * nb), oW = part(blk * 8 * nb),
+               oWd = part(dsz * 2 * nb), oeH = part(sizeof(int) * esz * nb),
+               oeW = part(sizeof(int) * esz * nb), oV = part(sizeof(VecJob) * 2 * nb),
+               oJ = part(sizeof(GemmJob) * 2 * nb);
   int rc;
+  if ((rc = ensure_fscratch(c, total))) return rc;
+  char *ws = (char *)c->fscratch;
+  __nv_bfloat16 *Dd = (__nv_bfloat16 *)(ws + oD), *dH = (__nv_bfloat16 *)(ws + oH),
+                *dWd = (__nv_bfloat16 *)(ws + oWd);
+  int *De = (int *)(ws + oeD), *eH = (int *)(ws + oeH), *eW = (int *)(ws + oeW),
+      *err = (int *)(ws + oErr);
+  double *dW = (double *)(ws + oW);
+  VecJob *dvd = (VecJob *)(ws + oVD), *dv = (VecJob *)(ws + oV);
+  GemmJob *dj = (GemmJob *)(ws + oJ);
+  DBSRG_TRY(c, cudaMemsetAsync(err, 0, 4, st));
+  const unsigned gv = (unsigned)((NR * 32 + 7) / 8);  // 8 vectors (warps) a block
+  std::vector<VecJob> vd(nch), vj(2 * (size_t)nb);
+  for (int ch = 0; ch < nch; ch++)
+    vd[ch] = {D + (size_t)ch * blk, Dd + dsz * ch, De + esz * ch, nsol[ch], 0};
+  if ((rc = copy_in(c, dvd, vd.data(), sizeof(VecJob) * nch))) return rc;
+  for (int c0 = 0; c0 < nch; c0 += 65535)  // grid y limit
+    DBSRG_RUN(c, "k_vec_digits",
+              k_vec_digits<<<dim3(gv, (unsigned)std::min(65535, nch - c0)), 256, 0, st>>>(
+                  dvd + c0, ms, ms, NR, nk));
+  const size_t smem = 2 * TS * (A_BYTES + B_BYTES);
   if ((rc = raise_smem_limit(c, (const void *)k_sgemm, smem))) return rc;
-  std::vector<GemmJob> jobs(nb);
+  std::vector<GemmJob> jobs(2 * (size_t)nb);
   const int tiles = ((ms + 127) / 128) * ((ms + 31) / 32);
   for (size_t b0 = 0; b0 < bk.size(); b0 += nb) {
     const int n = (int)std::min<size_t>(nb, bk.size() - b0);
-    // H columns -> digits (B of the first product)
+    int j1 = 0;
     for (int q = 0; q < n; q++) {
+      const int ich = bi[b0 + q], jch = bj[b0 + q], ni = nsol[ich - 1], nj = nsol[jch - 1];
       double *H = c->hch + (size_t)(bk[b0 + q] - 1) * blk;
-      DBSRG_RUN(c, "k_vec_digits",
-                k_vec_digits<<<gv, 256, 0, st>>>(ms, ms, H, ms, NR, nk,
-                                                  (__nv_bfloat16 *)dH.p + dsz * q,
-                                                  (int *)eH.p + esz * q));
+      // H columns (B of the first product) and W rows (columns of W^T, A of the
+      // second) to digits
+      vj[q] = {H, dH + dsz * q, eH + esz * q, ms, 0};
+      vj[nb + q] = {dW + blk * q, dWd + dsz * q, eW + esz * q, ni, 0};
+      // W^T(k, r) = sum_m H(m, k) D_ich(m, r): A = D_ich^T (rows r), B = H
+      // (columns k), stored transposed: element (r, k) at Wt[k + ms r]
+      if (ni > 0)
+        jobs[j1++] = {Dd + dsz * (ich - 1), dH + dsz * q, De + esz * (ich - 1), eH + esz * q,
+                      dW + blk * q, ms, 1, ni, ms, NR, NR, 0, 0};
+      // c = W D_jch into the block (column-major, ld ms), zeros outside ni x nj
+      jobs[nb + q] = {dWd + dsz * q, Dd + dsz * (jch - 1), eW + esz * q, De + esz * (jch - 1),
+                      H, 1, ms, nj > 0 ? ni : 0, ni > 0 ? nj : 0, NR, NR, ms, ms};
     }
-    // W^T(k, r) = sum_m H(m, k) D_ich(m, r): A = D_ich^T (rows r), B = H (columns k),
-    // stored transposed: element (r, k) at Wt[k + ms r]
-    int jn = 0;
-    for (int q = 0; q < n; q++) {
-      const int ich = bi[b0 + q], ni = nsol[ich - 1];
-      if (ni == 0) continue;
-      GemmJob &j = jobs[jn++];
-      j.A = Dd + dsz * (ich - 1);
-      j.ea = De + esz * (ich - 1);
-      j.B = (__nv_bfloat16 *)dH.p + dsz * q;
-      j.eb = (int *)eH.p + esz * q;
-      j.C = (double *)dW.p + blk * q;
-      j.sr = ms;
-      j.sc = 1;
-      j.M = ni;
-      j.N = ms;
-      j.NRa = NR;
-      j.NRb = NR;
-    }
-    if (jn > 0) {
-      if ((rc = copy_in(c, dJ.p, jobs.data(), sizeof(GemmJob) * jn))) return rc;
+    // the tables are rewritten only after the batch before has read them (same
+    // stream); pageable sources are staged before the calls return
+    if ((rc = copy_in(c, dv, vj.data(), sizeof(VecJob) * 2 * nb)) ||
+        (rc = copy_in(c, dj, jobs.data(), sizeof(GemmJob) * 2 * nb)))
+      return rc;
+    DBSRG_RUN(c, "k_vec_digits",
+              k_vec_digits<<<dim3(gv, (unsigned)n), 256, 0, st>>>(dv, ms, ms, NR, nk));
+    if (j1 > 0)
       DBSRG_RUN(c, "k_sgemm",
-                k_sgemm<<<dim3((unsigned)tiles, (unsigned)jn), NTHR, smem, st>>>(
-                    (const GemmJob *)dJ.p, nk, (int *)err.p));
-    }
-    // W rows (columns of W^T) -> digits (A of the second product)
-    for (int q = 0; q < n; q++) {
-      const int ni = nsol[bi[b0 + q] - 1];
-      DBSRG_RUN(c, "k_vec_digits",
-                k_vec_digits<<<gv, 256, 0, st>>>(ni, ms, (double *)dW.p + blk * q, ms, NR, nk,
-                                                  (__nv_bfloat16 *)dWd.p + dsz * q,
-                                                  (int *)eW.p + esz * q));
-    }
-    // c = W D_jch into the zeroed block (column-major, ld ms)
-    jn = 0;
-    for (int q = 0; q < n; q++) {
-      double *H = c->hch + (size_t)(bk[b0 + q] - 1) * blk;
-      cudaMemsetAsync(H, 0, blk * 8, st);
-      const int ni = nsol[bi[b0 + q] - 1], jch = bj[b0 + q], nj = nsol[jch - 1];
-      if (ni == 0 || nj == 0) continue;
-      GemmJob &j = jobs[jn++];
-      j.A = (__nv_bfloat16 *)dWd.p + dsz * q;
-      j.ea = (int *)eW.p + esz * q;
-      j.B = Dd + dsz * (jch - 1);
-      j.eb = De + esz * (jch - 1);
-      j.C = H;
-      j.sr = 1;
-      j.sc = ms;
-      j.M = ni;
-      j.N = nj;
-      j.NRa = NR;
-      j.NRb = NR;
-    }
-    if (jn > 0) {
-      // the job table is rewritten only after the first product has read it
-      if ((rc = copy_in(c, dJ.p, jobs.data(), sizeof(GemmJob) * jn))) return rc;
-      DBSRG_RUN(c, "k_sgemm",
-                k_sgemm<<<dim3((unsigned)tiles, (unsigned)jn), NTHR, smem, st>>>(
-                    (const GemmJob *)dJ.p, nk, (int *)err.p));
-    }
+                k_sgemm<<<dim3((unsigned)tiles, (unsigned)j1), NTHR, smem, st>>>(dj, nk, err));
+    DBSRG_RUN(c, "k_vec_digits",
+              k_vec_digits<<<dim3(gv, (unsigned)n), 256, 0, st>>>(dv + nb, ms, ms, NR, nk));
+    DBSRG_RUN(c, "k_sgemm",
+              k_sgemm<<<dim3((unsigned)tiles, (unsigned)n), NTHR, smem, st>>>(dj + nb, nk, err));
   }
   int herr = 0;
-  cudaMemcpyAsync(&herr, err.p, 4, cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st);
   if (cudaStreamSynchronize(st) != cudaSuccess)
     return set_err(c, DBSRG_ECUDA, "channel_basis: tensor-core products failed");
   if (herr) return set_err(c, DBSRG_ETIMEOUT, "channel_basis: a product pipeline wait ran out");

@@ -215,3 +215,36 @@ def test_split_transform_sizes(ns, nch):
                 assert not got[ni:, :].any() and not got[:, nj:].any()
         prev = out.copy()
     a.close()
+
+
+@pytest.mark.parametrize("nch,empty", [(9, ()), (9, (0, 4)), (2, (1,))])
+def test_channel_basis_batches_and_empty_channels(nch, empty):
+    """More blocks than a batch of the split products holds (36), ni x nj
+    corners with the rest of the block zeroed, channels without solutions;
+    against plain products (split bound 1e-10 of each block's largest
+    element)."""
+    import torch
+
+    w = synth.small(ns=50, nch=nch, mk=1, n_entries=200, breit=False, seed=93)
+    a = Assembler(w.t, w.ks, w.ksp, w.ksq)
+    a.set_orbitals(w.pq, w.ipbs)
+    a.alloc_matrix(w.nch, w.icc, w.iicc, w.mk)
+    a.set_precision(SPLIT_BF16)
+    for L in w.lists:
+        a.gen_matrix(L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
+    h = a.get_matrix()
+    rng = np.random.default_rng(4)
+    ms = a.ms
+    sol = np.asfortranarray(rng.standard_normal((ms, ms, nch)))
+    nsol = rng.integers(1, ms + 1, nch).astype(np.int32)
+    nsol[list(empty)] = 0
+    out = a.channel_basis(torch.from_numpy(np.ascontiguousarray(sol.transpose(2, 1, 0))).cuda(),
+                          nsol, out=True)
+    a.close()
+    for i in range(nch):
+        for j in range(i):
+            b = w.icc[i, j] - 1
+            ref = np.zeros((ms, ms))
+            ni, nj = int(nsol[i]), int(nsol[j])
+            ref[:ni, :nj] = sol[:, :ni, i].T @ h[:, :, b] @ sol[:, :nj, j]
+            assert np.abs(out[:, :, b] - ref).max() <= 1e-10 * max(np.abs(ref).max(), 1e-300), (i, j)
