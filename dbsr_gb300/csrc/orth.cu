@@ -19,6 +19,8 @@
 //     X'  = X - W_a T1' - T2 W_b^T      (= X - W_a T1 - T2 W_b^T + W_a S W_b^T)
 // FP64 throughout; every sum runs in a fixed order (no atomics), so the
 // result is deterministic.
+#include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -27,8 +29,7 @@ namespace {
 
 constexpr int OCH = 4;  // orbitals per chunk of the dot-product kernels
 
-// one stored block and its two channels' orbital lists (indices into the
-// V/W columns) and scratch offsets
+// one stored block and its two channels' orbital lists (columns of V and W) and scratch offsets
 struct OrthBlock {
   int blk;     // 1-based block number
   int a0, na;  // row channel: orbitals olist[a0 .. a0+na)
@@ -36,20 +37,23 @@ struct OrthBlock {
   long long t1, t2;  // scratch offsets (doubles) of T1 (na x ms) and T2 (ms x nb)
 };
 
-// V(:,u) = (P; Q) of bound orbital orb[u], W(:,u) = fppqq V(:,u); one
-// thread per (row r, orbital u)
-__global__ void k_orth_vw(int ns, int nu, const int *orb, const double *pq, const double *fppqq,
-                          double *V, double *W) {
-  const int ms = 2 * ns;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ms * nu) return;
-  const int r = q % ms, u = q / ms;
-  const double *p = pq + (size_t)2 * ns * (orb[u] - 1);  // (P; Q) are contiguous
-  V[q] = p[r];
-  double acc = 0.0;
-  for (int c = 0; c < ms; c++) acc = fma(fppqq[r + (size_t)ms * c], p[c], acc);
-  W[q] = acc;
+// f(N, u0) for every group of N = OCH, then the remaining 1..OCH-1, of n orbitals:
+// the FP64 pipe is what bounds the three passes over a block, so no group
+// computes orbitals that are not there.  136 blocks of ms 500, 1 to 4 orbitals a
+// channel: T1 366 -> 233 us, T2 295 -> 186 us (with its columns in four runs; one
+// run a thread 292), update 366 -> 288 us (a subtraction less an element)
+template <class F>
+__device__ __forceinline__ void orb_groups(int n, F f) {
+  int u0 = 0;
+  for (; u0 + OCH <= n; u0 += OCH) f(std::integral_constant<int, OCH>(), u0);
+  switch (n - u0) {
+    case 1: f(std::integral_constant<int, 1>(), u0); break;
+    case 2: f(std::integral_constant<int, 2>(), u0); break;
+    case 3: f(std::integral_constant<int, 3>(), u0); break;
+    default: break;
+  }
 }
+static_assert(OCH == 4, "orb_groups lists the remainders of four");
 
 // T1(j,c) = sum_r V(r, a_j) X(r,c): one warp per column c, lanes over rows,
 // a fixed shuffle tree per sum
@@ -62,52 +66,72 @@ __global__ void k_orth_t1(int ms, const OrthBlock *bl, const int *olist, const d
   if (c >= ms) return;
   const double *x = hch + (size_t)(B.blk - 1) * ms * ms + (size_t)ms * c;
   double *t1 = scr + B.t1;
-  for (int j0 = 0; j0 < B.na; j0 += OCH) {
-    double acc[OCH] = {0.0, 0.0, 0.0, 0.0};
-    const double *v[OCH];
+  orb_groups(B.na, [&](auto nc, int j0) {
+    constexpr int N = decltype(nc)::value;
+    double acc[N];
+    const double *v[N];
 #pragma unroll
-    for (int u = 0; u < OCH; u++)
-      v[u] = V + (size_t)ms * olist[B.a0 + min(j0 + u, B.na - 1)];
+    for (int u = 0; u < N; u++) {
+      acc[u] = 0.0;
+      v[u] = V + (size_t)ms * olist[B.a0 + j0 + u];
+    }
+#pragma unroll 4
     for (int r = lane; r < ms; r += 32) {
       const double xv = x[r];
 #pragma unroll
-      for (int u = 0; u < OCH; u++) acc[u] = fma(v[u][r], xv, acc[u]);
+      for (int u = 0; u < N; u++) acc[u] = fma(v[u][r], xv, acc[u]);
     }
 #pragma unroll
-    for (int u = 0; u < OCH; u++) {
+    for (int u = 0; u < N; u++) {
       double s = acc[u];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0 && j0 + u < B.na) t1[(size_t)(j0 + u) + (size_t)B.na * c] = s;
+      if (lane == 0) t1[(size_t)(j0 + u) + (size_t)B.na * c] = s;
     }
-  }
+  });
 }
 
-// T2(r,l) = sum_c X(r,c) V(c, b_l): one thread per row, columns in order
-// (consecutive threads read consecutive rows of a column)
-__global__ void k_orth_t2(int ms, const OrthBlock *bl, const int *olist, const double *V,
-                          const double *hch, double *scr) {
+// T2(r,l) = sum_c X(r,c) V(c, b_l): T2R rows a block (consecutive threads read
+// consecutive rows of a column), the columns in T2S runs summed side by side
+// and then added in order
+constexpr int T2R = 64, T2S = 4;
+__global__ void __launch_bounds__(T2R * T2S) k_orth_t2(int ms, const OrthBlock *bl,
+                                                       const int *olist, const double *V,
+                                                       const double *hch, double *scr) {
+  __shared__ double part[T2S][OCH][T2R];
   const OrthBlock B = bl[blockIdx.y];
   if (B.nb == 0) return;
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= ms) return;
-  const double *x = hch + (size_t)(B.blk - 1) * ms * ms + r;
+  const int tr = threadIdx.x % T2R, sl = threadIdx.x / T2R;
+  const int r = blockIdx.x * T2R + tr;
+  const int per = (ms + T2S - 1) / T2S, c0 = sl * per, c1 = min(ms, c0 + per);
+  const double *x = hch + (size_t)(B.blk - 1) * ms * ms + min(r, ms - 1);
   double *t2 = scr + B.t2;
-  for (int l0 = 0; l0 < B.nb; l0 += OCH) {
-    double acc[OCH] = {0.0, 0.0, 0.0, 0.0};
-    const double *v[OCH];
+  orb_groups(B.nb, [&](auto nc, int l0) {
+    constexpr int N = decltype(nc)::value;
+    double acc[N];
+    const double *v[N];
 #pragma unroll
-    for (int u = 0; u < OCH; u++)
-      v[u] = V + (size_t)ms * olist[B.b0 + min(l0 + u, B.nb - 1)];
-    for (int c = 0; c < ms; c++) {
+    for (int u = 0; u < N; u++) {
+      acc[u] = 0.0;
+      v[u] = V + (size_t)ms * olist[B.b0 + l0 + u];
+    }
+#pragma unroll 8
+    for (int c = c0; c < c1; c++) {
       const double xv = x[(size_t)ms * c];
 #pragma unroll
-      for (int u = 0; u < OCH; u++) acc[u] = fma(xv, v[u][c], acc[u]);
+      for (int u = 0; u < N; u++) acc[u] = fma(xv, v[u][c], acc[u]);
     }
 #pragma unroll
-    for (int u = 0; u < OCH; u++)
-      if (l0 + u < B.nb) t2[r + (size_t)ms * (l0 + u)] = acc[u];
-  }
+    for (int u = 0; u < N; u++) part[sl][u][tr] = acc[u];
+    __syncthreads();
+    for (int u = sl; u < N; u += T2S) {
+      double s = part[0][u][tr];
+#pragma unroll
+      for (int k = 1; k < T2S; k++) s += part[k][u][tr];
+      if (r < ms) t2[r + (size_t)ms * (l0 + u)] = s;
+    }
+    __syncthreads();
+  });
 }
 
 // T1' = T1 - S W_b^T with S = T1 V_b (na x nb), per block: one CTA, S in
@@ -154,15 +178,15 @@ __global__ void k_orth_update(int ms, const OrthBlock *bl, const int *olist, con
   const double *t1 = scr + B.t1 + (size_t)B.na * c0, *t2 = scr + B.t2 + r;
   double d[UCOLS];
 #pragma unroll
-  for (int k = 0; k < UCOLS; k++) d[k] = 0.0;
+  for (int k = 0; k < UCOLS; k++) d[k] = k < nc ? x[(size_t)ms * k] : 0.0;
   for (int j = 0; j < B.na; j++) {
-    const double w = W[r + (size_t)ms * olist[B.a0 + j]];
+    const double w = -W[r + (size_t)ms * olist[B.a0 + j]];
 #pragma unroll
     for (int k = 0; k < UCOLS; k++)
       if (k < nc) d[k] = fma(w, t1[(size_t)j + (size_t)B.na * k], d[k]);
   }
   for (int l = 0; l < B.nb; l++) {
-    const double t = t2[(size_t)ms * l];
+    const double t = -t2[(size_t)ms * l];
     const double *wb = W + (size_t)ms * olist[B.b0 + l] + c0;
 #pragma unroll
     for (int k = 0; k < UCOLS; k++)
@@ -170,7 +194,7 @@ __global__ void k_orth_update(int ms, const OrthBlock *bl, const int *olist, con
   }
 #pragma unroll
   for (int k = 0; k < UCOLS; k++)
-    if (k < nc) x[(size_t)ms * k] -= d[k];
+    if (k < nc) x[(size_t)ms * k] = d[k];
 }
 
 }  // namespace
@@ -185,9 +209,9 @@ extern "C" int dbsrg_orth_channels(dbsrg_ctx *c, const int *iort) {
   cudaSetDevice(c->device);
   int rc = drain(c);
   if (rc) return rc;
-  const int ns = c->g.ns, ms = c->g.ms, nch = c->nch, nbf = c->nbf;
-  // orbitals used by any channel, and each channel's list of them
-  std::vector<int> ucol(nbf, -1), orb;
+  const int ms = c->g.ms, nch = c->nch, nbf = c->nbf;
+  // each channel's orbitals (0-based); V is the orbitals themselves, W = B V the
+  // overlap vectors of every orbital
   std::vector<int> cstart(nch + 1, 0), olist;
   for (int ich = 0; ich < nch; ich++) {
     cstart[ich] = (int)olist.size();
@@ -195,17 +219,13 @@ extern "C" int dbsrg_orth_channels(dbsrg_ctx *c, const int *iort) {
       if (!iort[j + (size_t)nbf * ich]) continue;
       if (c->h_ipbs[j] != 0)
         return set_err(c, DBSRG_EINVAL, "orth_channels: orthogonality to a non-bound orbital");
-      if (ucol[j] < 0) {
-        ucol[j] = (int)orb.size();
-        orb.push_back(j + 1);
-      }
-      olist.push_back(ucol[j]);
+      olist.push_back(j);
     }
     if ((int)olist.size() - cstart[ich] > MAXO)
       return set_err(c, DBSRG_ERANGE, "orth_channels: more than 32 orbitals for one channel");
   }
   cstart[nch] = (int)olist.size();
-  if (orb.empty()) return DBSRG_OK;
+  if (olist.empty()) return DBSRG_OK;
   // stored blocks with a condition on either side
   std::vector<OrthBlock> blocks;
   long long off = 0;
@@ -228,7 +248,6 @@ extern "C" int dbsrg_orth_channels(dbsrg_ctx *c, const int *iort) {
     }
   if (blocks.empty()) return DBSRG_OK;
   cudaStream_t st = c->stream;
-  const int nu = (int)orb.size();
   // chunks of at most 65535 blocks (grid y/z limit) whose scratch stays below
   // 1 GB (a block needs at most 2 x 32 x ms doubles), offsets rebased to each
   // chunk's first element
@@ -249,33 +268,16 @@ extern "C" int dbsrg_orth_channels(dbsrg_ctx *c, const int *iort) {
       blocks[i].t2 -= base;
     }
   }
-  int *dorb = nullptr, *dol = nullptr;
-  double *dV = nullptr, *dW = nullptr, *dscr = nullptr;
-  OrthBlock *dbl = nullptr;
-  auto cleanup = [&]() {
-    for (void *p : {(void *)dorb, (void *)dol, (void *)dV, (void *)dW, (void *)dscr, (void *)dbl})
-      if (p) cudaFree(p);
-  };
-  if (cudaMalloc(&dorb, sizeof(int) * nu) || cudaMalloc(&dol, sizeof(int) * olist.size()) ||
-      cudaMalloc(&dV, sizeof(double) * ms * nu) || cudaMalloc(&dW, sizeof(double) * ms * nu) ||
-      cudaMalloc(&dscr, sizeof(double) * cap) ||
-      cudaMalloc(&dbl, sizeof(OrthBlock) * blocks.size())) {
-    cudaGetLastError();
-    cleanup();
-    return set_err(c, DBSRG_ENOMEM, "orth_channels: allocation failed");
-  }
-  auto fail = [&](int code, const char *msg) {
-    cudaStreamSynchronize(st);
-    cleanup();
-    return set_err(c, code, msg);
-  };
-  if ((rc = copy_in(c, dorb, orb.data(), sizeof(int) * nu))) return fail(rc, "copy");
-  if ((rc = copy_in(c, dol, olist.data(), sizeof(int) * olist.size()))) return fail(rc, "copy");
-  if ((rc = copy_in(c, dbl, blocks.data(), sizeof(OrthBlock) * blocks.size())))
-    return fail(rc, "copy");
-  DBSRG_RUN(c, "k_orth_vw",
-            k_orth_vw<<<(unsigned)((ms * nu + 255) / 256), 256, 0, st>>>(ns, nu, dorb, c->pq,
-                                                                         c->g.fppqq, dV, dW));
+  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t sb = al(sizeof(double) * cap), lb = al(sizeof(int) * olist.size());
+  if ((rc = ensure_fscratch(c, sb + lb + sizeof(OrthBlock) * blocks.size()))) return rc;
+  double *dscr = (double *)c->fscratch;
+  int *dol = (int *)((char *)c->fscratch + sb);
+  OrthBlock *dbl = (OrthBlock *)((char *)c->fscratch + sb + lb);
+  const double *dV = c->pq, *dW;
+  if ((rc = get_vch(c, &dW)) || (rc = copy_in(c, dol, olist.data(), sizeof(int) * olist.size())) ||
+      (rc = copy_in(c, dbl, blocks.data(), sizeof(OrthBlock) * blocks.size())))
+    return rc;
   for (size_t k = 0; k + 1 < cuts.size(); k++) {
     const OrthBlock *cb = dbl + cuts[k];
     const unsigned nbk = (unsigned)(cuts[k + 1] - cuts[k]);
@@ -283,15 +285,14 @@ extern "C" int dbsrg_orth_channels(dbsrg_ctx *c, const int *iort) {
               k_orth_t1<<<dim3((unsigned)((ms + 7) / 8), nbk), 256, 0, st>>>(ms, cb, dol, dV,
                                                                               c->hch, dscr));
     DBSRG_RUN(c, "k_orth_t2",
-              k_orth_t2<<<dim3((unsigned)((ms + 127) / 128), nbk), 128, 0, st>>>(ms, cb, dol, dV,
-                                                                                 c->hch, dscr));
+              k_orth_t2<<<dim3((unsigned)((ms + T2R - 1) / T2R), nbk), T2R * T2S, 0, st>>>(
+                  ms, cb, dol, dV, c->hch, dscr));
     DBSRG_RUN(c, "k_orth_s", k_orth_s<<<nbk, 256, 0, st>>>(ms, cb, dol, dV, dW, dscr));
     DBSRG_RUN(c, "k_orth_update",
               k_orth_update<<<dim3((unsigned)((ms + 127) / 128),
                                    (unsigned)((ms + UCOLS - 1) / UCOLS), nbk),
                               128, 0, st>>>(ms, cb, dol, dW, dscr, c->hch));
   }
-  if (cudaStreamSynchronize(st) != cudaSuccess) return fail(DBSRG_ECUDA, "orth_channels");
-  cleanup();
+  DBSRG_TRY(c, cudaStreamSynchronize(st));
   return DBSRG_OK;
 }
