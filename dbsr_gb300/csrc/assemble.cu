@@ -532,8 +532,9 @@ __global__ void k_scatter(int ns, int ks, int mode, ScatterSpec sp, int nm, cons
 // segment (the owner, then its partner) the lanes sum every 32nd entry and
 // a butterfly combines the lanes, and the sum is added to acf in that order.
 constexpr int ACF_WARPS = 4;  // warps per block
-__global__ void k_acf(int nseg_owner, const int *owners, const SegInfo *info, int kpol,
-                      int nbf, const int *k2, const int *k3, const double *cd,
+// (quad over n orbitals: pairs, or K2 and K3 themselves where pairs is null)
+__global__ void k_acf(int nseg_owner, const int *owners, const SegInfo *info, int kpol, int n,
+                      const int *pairs, const int *k2, const int *k3, const double *cd,
                       const double *quad, double *acf, int iicc) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * ACF_WARPS + threadIdx.x / 32;
@@ -549,9 +550,8 @@ __global__ void k_acf(int nseg_owner, const int *owners, const SegInfo *info, in
       const SegInfo sj = info[ss];
       double CA = 0.0;
       for (int e = sj.start + lane; e < sj.end; e += 32) {
-        const double S =
-            quad[(size_t)(k2[e] - 1) + (size_t)nbf * ((k3[e] - 1) + (size_t)nbf * a)];
-        CA = CA + cd[e] * S;
+        const int pr = pairs ? pairs[e] : (k2[e] - 1) * n + k3[e] - 1;
+        CA = CA + cd[e] * quad[(size_t)pr + (size_t)n * n * a];
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) CA += __shfl_xor_sync(0xffffffffu, CA, o);
@@ -1180,12 +1180,13 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
     if ((rc = run_chunk(P.chunks[k]))) return rc;
   if (nown_acf > 0) {
     const double *quad;
-    if ((rc = get_quad(c, P.kpol, &quad))) return rc;
+    if ((rc = get_quad(c, P.kpol, P.factored, &quad))) return rc;
     if (prep) return DBSRG_OK;
     DBSRG_RUN(c, "k_acf",
               k_acf<<<(nown_acf + ACF_WARPS - 1) / ACF_WARPS, 32 * ACF_WARPS, 0, st>>>(
-                  nown_acf, P.work + P.own_off + o0, P.info, P.kpol, c->nbf, P.lk2, P.lk3, P.lcd,
-                  quad, c->acf, c->iicc));
+                  nown_acf, P.work + P.own_off + o0, P.info, P.kpol,
+                  P.factored ? c->nbound : c->nbf, P.factored ? P.lpair : nullptr, P.lk2, P.lk3,
+                  P.lcd, quad, c->acf, c->iicc));
   }
   return DBSRG_OK;
 }

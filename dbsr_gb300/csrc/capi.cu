@@ -247,8 +247,8 @@ void free_tables(dbsrg_ctx *c) {
     cache_free(c, p);
   for (double *p : c->stab)
     cache_free(c, p);
-  for (double *p : c->quad)
-    cache_free(c, p);
+  for (auto *v : {&c->quad, &c->quadb})
+    for (double *p : *v) cache_free(c, p);
   for (double *p : c->rbtab)
     cache_free(c, p);
   for (double *p : c->sbtab)
@@ -265,6 +265,7 @@ void free_tables(dbsrg_ctx *c) {
   c->rtab.clear();
   c->stab.clear();
   c->quad.clear();
+  c->quadb.clear();
   c->rcell.clear();
   c->rshare.clear();
   c->scell.clear();
@@ -534,8 +535,10 @@ int dbsrg_set_orbitals(dbsrg_ctx *c, int nbf, const double *pq, const int *ipbs)
   if (c->ipbs) cudaFree(c->ipbs);
   c->pq = nullptr;
   c->ipbs = nullptr;
-  for (double *p : c->quad) cache_free(c, p);
-  c->quad.clear();
+  for (auto *v : {&c->quad, &c->quadb}) {
+    for (double *p : *v) cache_free(c, p);
+    v->clear();
+  }
   size_t n = (size_t)2 * c->g.ns * nbf;
   DBSRG_TRY(c, cudaMalloc((void **)&c->pq, n * sizeof(double)));
   DBSRG_TRY(c, cudaMalloc((void **)&c->ipbs, nbf * sizeof(int)));

@@ -83,7 +83,7 @@ __global__ void k_bound_rows(int ns, int nb, const int *b2o, const double *pq, d
 // (and Uhi with mhi), x the output function, xc the contracted one, and their
 // float-float copies where asked for.  Both electrons' vectors (R^k: those of
 // the P and Q pairs, which every type of the k shares) in one launch
-// (blockIdx.y).  A thread sums up to 9 cells of 9 functions, nine loads in
+// (blockIdx.y).  A thread sums up to ks cells of ks functions, nine loads in
 // flight: bound by the latency of those loads.  ns 283, 20 orbitals: 19 us a k,
 // against 4 x 26 us (and 8 conversions of 6 us) with a launch per type that
 // loaded one value at a time.
@@ -104,25 +104,27 @@ __global__ void k_far_vectors(int ns, int nv, int kk, int nb, const int *b2o, co
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= ns * nb) return;
   int x = q % ns + 1, a = q / ns;
-  const double *p = pq + (size_t)ns * (ccomp - 1) + (size_t)2 * ns * (b2o[a] - 1) - 1;
+  const double *p = pq + (size_t)ns * (ccomp - 1) + (size_t)2 * ns * (b2o ? b2o[a] - 1 : a) - 1;
   double slo = 0.0, shi = 0.0;
   for (int iv = max(1, x - ko + 1); iv <= min(nv, x); iv++) {
     const int ho = x - iv + 1;
-    double pv[9], lv[9], hv[9];
+    for (int u0 = 0; u0 < kc; u0 += 9) {
+      double pv[9], lv[9], hv[9];
 #pragma unroll
-    for (int u = 0; u < 9; u++) {
-      const int hc = u + 1, xc = iv + u;
-      const bool ok = hc <= kc && xc <= ns;
-      const size_t o = (size_t)(out_first ? pidx(e, ho, hc) : pidx(e, hc, ho)) +
-                       (size_t)kk * (iv - 1);
-      pv[u] = ok ? p[xc] : 0.0;
-      lv[u] = ok ? mlo[o] : 0.0;
-      hv[u] = ok && mhi ? mhi[o] : 0.0;
-    }
+      for (int u = 0; u < 9; u++) {
+        const int hc = u0 + u + 1, xc = iv + u0 + u;
+        const bool ok = hc <= kc && xc <= ns;
+        const size_t o = (size_t)(out_first ? pidx(e, ho, hc) : pidx(e, hc, ho)) +
+                         (size_t)kk * (iv - 1);
+        pv[u] = ok ? p[xc] : 0.0;
+        lv[u] = ok ? mlo[o] : 0.0;
+        hv[u] = ok && mhi ? mhi[o] : 0.0;
+      }
 #pragma unroll
-    for (int u = 0; u < 9; u++) {
-      slo = fma(lv[u], pv[u], slo);
-      shi = fma(hv[u], pv[u], shi);
+      for (int u = 0; u < 9; u++) {
+        slo = fma(lv[u], pv[u], slo);
+        shi = fma(hv[u], pv[u], shi);
+      }
     }
   }
   sd.Ulo[q] = slo;
@@ -794,6 +796,55 @@ int ensure_fscratch(dbsrg_ctx *c, size_t bytes) {
   return grow_buffer(c, &c->fscratch, &c->fscratch_bytes, bytes);
 }
 
+// the four R^k vectors of one k over nb orbitals (b2o null: all of them)
+static int r_far_vectors(dbsrg_ctx *c, int k, int nb, const int *b2o, double *W, float2 *Wf) {
+  const DeviceGrid &g = c->g;
+  const int ns = g.ns, kk = g.ks * g.ks;
+  const size_t m = (size_t)ns * nb;
+  const CellData *pp, *qq;
+  int rc;
+  if ((rc = get_celldata(c, 0, 0, k, &pp)) || (rc = get_celldata(c, 0, 1, k, &qq))) return rc;
+  auto side = [&](int comp, const CellData &cd) {
+    const int o = comp == 1 ? 0 : 2, ord = comp == 1 ? g.ksp : g.ksq;
+    return FarSide{{ord, ord, 1}, 1, ord, ord, comp, cd.lo1, cd.hi1, W + o * m, W + (o + 1) * m,
+                   Wf ? Wf + o * m : nullptr, Wf ? Wf + (o + 1) * m : nullptr};
+  };
+  const dim3 gv((unsigned)((m + 63) / 64), 2);
+  DBSRG_RUN(c, "k_far_vectors",
+            k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.nv, kk, nb, b2o, c->pq, side(1, *pp),
+                                                    side(2, *qq)));
+  return DBSRG_OK;
+}
+
+int far_vectors_all(dbsrg_ctx *c, int k, double *W) {
+  return r_far_vectors(c, k, c->nbf, nullptr, W, nullptr);
+}
+
+static int ensure_rfar(dbsrg_ctx *c, int k, RFar **out) {
+  RFar &r = c->rfarw[k];
+  if (!r.W) {
+    const size_t m = (size_t)c->g.ns * c->nbound;
+    double *W = (double *)cache_alloc(c, 8 * m * sizeof(double));
+    if (!W) return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
+    const int rc = r_far_vectors(c, k, c->nbound, c->b2o, W, (float2 *)(W + 4 * m));
+    if (rc) {
+      cache_free(c, W);
+      return rc;
+    }
+    r.W = W;
+    r.Wf = (float2 *)(W + 4 * m);
+  }
+  *out = &r;
+  return DBSRG_OK;
+}
+
+int get_rfar(dbsrg_ctx *c, int k, const double **W) {
+  RFar *r;
+  const int rc = ensure_rfar(c, k, &r);
+  if (!rc) *W = r->W;
+  return rc;
+}
+
 // far-field vectors of (family, type, k, exchange case), cached; R^k (case 3
 // only): views of the four vectors that the types of the k share
 static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const FarField **out) {
@@ -813,23 +864,9 @@ static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const
   FarField f;
   if (family == 0) {
     if (cs != 3) return set_err(c, DBSRG_EINVAL, "far field: R^k exchange is convol case 3");
-    RFar &r = c->rfarw[k];
-    if (!r.W) {
-      const CellData *pp, *qq;
-      if ((rc = get_celldata(c, 0, 0, k, &pp)) || (rc = get_celldata(c, 0, 1, k, &qq))) return rc;
-      double *W = (double *)cache_alloc(c, 8 * m * sizeof(double));
-      if (!W) return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
-      r.W = W;
-      r.Wf = (float2 *)(W + 4 * m);
-      auto side = [&](int comp, const CellData &cd) {
-        const int o = comp == 1 ? 0 : 2, ord = comp == 1 ? g.ksp : g.ksq;
-        return FarSide{{ord, ord, 1}, 1, ord, ord, comp, cd.lo1, cd.hi1, W + o * m,
-                       W + (o + 1) * m, r.Wf + o * m, r.Wf + (o + 1) * m};
-      };
-      DBSRG_RUN(c, "k_far_vectors",
-                k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.nv, kk, nb, c->b2o, c->pq,
-                                                        side(1, *pp), side(2, *qq)));
-    }
+    RFar *rp;
+    if ((rc = ensure_rfar(c, k, &rp))) return rc;
+    RFar &r = *rp;
     // U, Ul: lo and hi of electron 1's pairs; V, Vl: hi and lo of electron 2's
     const int a = tb.a1 == 1 ? 0 : 2, b = tb.b1 == 1 ? 0 : 2;
     f.U = r.W + a * m;

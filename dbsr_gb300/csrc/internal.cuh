@@ -138,7 +138,7 @@ struct dbsrg_ctx {
   int *b2o = nullptr;   // (nbound): 1-based orbital of each bound index
   std::vector<int> h_bmap;
   // <a|r^k|b> per component for the asymptotic coefficients, [k]
-  std::vector<double *> quad;
+  std::vector<double *> quad, quadb;  // over all orbitals, over the bound ones
   // scratch arena (grown on demand, reused across calls)
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
@@ -368,10 +368,15 @@ void basis_release(dbsrg_ctx *c);
 int build_grid(dbsrg_ctx *c, const double *t_host_or_dev);
 int compute_moments(dbsrg_ctx *c, int which, int k, double *rkm_dev);
 int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd_dev);
+// far-field vectors of the R^k tables of one k (factor.cu): of the bound
+// orbitals (cached, [lo P, hi P, lo Q, hi Q][ns*nbound]), or of all nbf orbitals
+// into W (4 ns nbf values, same order)
+int get_rfar(dbsrg_ctx *c, int k, const double **W);
+int far_vectors_all(dbsrg_ctx *c, int k, double *W);
 // returns device pointer of the cached table (building it if needed)
 int get_rtable(dbsrg_ctx *c, int type, int k, const double **out);
 int get_stable(dbsrg_ctx *c, int type, int k, const double **out);
-int get_quad(dbsrg_ctx *c, int k, const double **out);
+int get_quad(dbsrg_ctx *c, int k, bool bound, const double **out);
 int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out);
 // the cell data of every R^k type of one k in two launches, and the band tables
 // of types 0, 1 and 2 in one (type 3's exchange reads type 2's)

@@ -803,107 +803,63 @@ int get_band_table(dbsrg_ctx *c, int family, int type, int k, const double **out
 }
 
 // ----------------------------------------------------------------------------
-// <a|r^k|b> split by component for all orbital pairs: quadr
-// (dbsr_lib_dbs.f90:3940-3976), used for the asymptotic coefficients
-// (QUADR_PQ at R_data.f90:224, which selects the component by atype).
-// First the banded matrix G(i,i+d) = sum over intervals and Gauss points of
-// r^k w B_i B_{i+d} (d = 0..kx-1) per component, then quad(a,b,comp) =
-// sum_{i,j} G(i,j) p_a(i) p_b(j) as W = G P per orbital and the products
-// P^T W of all orbital pairs.
-// blockIdx.y 0: the P basis (order kp, values bp, into Gp); 1: the Q basis
-__global__ void k_rk_gram(int ns, int nv, int ks, int kp, int kq, int k, const double *bp,
-                          const double *bq, const double *gr, const double *grw, double *Gp,
-                          double *Gq) {
-  const int kx = blockIdx.y ? kq : kp;
-  const double *bs = blockIdx.y ? bq : bp;
-  double *G = blockIdx.y ? Gq : Gp;
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ns * kx) return;
-  int i = q % ns + 1, d = q / ns, j = i + d;  // 1-based i, j = i + d
-  const int nw = nv + 1;
-  double acc = 0.0;
-  if (j <= ns) {
-    int lo = max(1, j - kx + 1), hi = min(nv, i);
-    for (int iv = lo; iv <= hi; iv++) {
-      int ith = i - iv, jth = j - iv;
-      double s = 0.0;
-      for (int m = 0; m < ks; m++) {
-        double wk = __dmul_rn(ipow_d(gr[IDX2(iv - 1, m, nv)], k), grw[IDX2(iv - 1, m, nv)]);
-        s = __dadd_rn(s, __dmul_rn(bs[IDX3(iv - 1, m, jth, nw, ks)],
-                                   __dmul_rn(wk, bs[IDX3(iv - 1, m, ith, nw, ks)])));
-      }
-      acc = __dadd_rn(acc, s);
-    }
-  }
-  G[q] = acc;
+// <a|r^k|b> split by component: quadr (dbsr_lib_dbs.f90:3940-3976), used for
+// the asymptotic coefficients (QUADR_PQ at R_data.f90:224, which selects the
+// component by atype).  With G(i,j) = sum over cells of the moments <B_i|r^k|B_j>
+// and w_b = G p_b -- the far-field vectors of the R^k tables of this k, which
+// the exchange lists need as well -- it is p_a . w_b.
+// quad[comp][pair]: one warp per pair (a, b), pair = a n + b.  ns 80: 6 us a k;
+// as a Gram matrix from the Gauss points, a banded product and 32 x 32 tiles of
+// all orbitals (channel ones too) 55 + 8 + 31 us (ns 283: 62 + 10 + 95).
+__global__ void k_quad_dot(int n, int ns, const double *P, size_t pstride, const int *b2o,
+                           const double *W, size_t wcomp, double *quad) {
+  const int q = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int comp = blockIdx.y;
+  if (q >= n * n) return;
+  const int a = q / n, b = q % n;
+  const double *p = P + (size_t)(b2o ? b2o[a] - 1 : a) * pstride + (size_t)ns * comp;
+  const double *w = W + (size_t)comp * wcomp + (size_t)ns * b;
+  double s = 0.0;
+#pragma unroll 4
+  for (int i = lane; i < ns; i += 32) s = fma(p[i], w[i], s);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) quad[(size_t)comp * n * n + q] = s;
 }
 
-// W(b, comp)(i) = sum_j G(i,j) p_b(j) over the symmetric band G (d = 0..kx-1
-// stored as G(i, i+d))
-__global__ void k_quad_w(int nbf, int ns, int ksp, int ksq, const double *pq, const double *GP,
-                         const double *GQ, double *W) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= 2 * nbf * ns) return;
-  const int i = q % ns, b = (q / ns) % nbf, comp = q / (ns * nbf);
-  const int kx = comp == 0 ? ksp : ksq;
-  const double *G = comp == 0 ? GP : GQ;
-  const double *pb = pq + (size_t)ns * comp + (size_t)2 * ns * b;
-  double s = G[i] * pb[i];
-  for (int d = 1; d < kx; d++) {
-    if (i + d < ns) s += G[(size_t)i + (size_t)ns * d] * pb[i + d];
-    if (i - d >= 0) s += G[(size_t)(i - d) + (size_t)ns * d] * pb[i - d];
-  }
-  W[q] = s;
-}
-
-// quad(a, b, comp) = sum_i p_a(i) W(b, comp)(i): 32 x 32 tiles of (a, b)
-__global__ void k_quad_dot(int nbf, int ns, const double *pq, const double *W, double *quad) {
-  __shared__ double sa[32][33], sw[32][33];
-  const int comp = blockIdx.z, a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
-  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;  // 256 threads: 8 rows
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int i0 = 0; i0 < ns; i0 += 32) {
-    for (int r = ty; r < 32; r += 8) {
-      const int a = a0 + r, b = b0 + r, i = i0 + tx;
-      sa[r][tx] = (a < nbf && i < ns) ? pq[(size_t)i + (size_t)ns * comp + (size_t)2 * ns * a] : 0.0;
-      sw[r][tx] = (b < nbf && i < ns) ? W[(size_t)i + (size_t)ns * (b + (size_t)nbf * comp)] : 0.0;
-    }
-    __syncthreads();
-    for (int k = 0; k < 4; k++) {
-      const int ar = ty + 8 * k;
-      double s = acc[k];
-      for (int ii = 0; ii < 32; ii++) s += sa[ar][ii] * sw[tx][ii];
-      acc[k] = s;
-    }
-    __syncthreads();
-  }
-  for (int k = 0; k < 4; k++) {
-    const int a = a0 + ty + 8 * k, b = b0 + tx;
-    if (a < nbf && b < nbf) quad[(size_t)a + (size_t)nbf * (b + (size_t)nbf * comp)] = acc[k];
-  }
-}
-
-int get_quad(dbsrg_ctx *c, int k, const double **out) {
-  if ((int)c->quad.size() <= k) c->quad.resize(k + 1, nullptr);
-  if (c->quad[k]) {
-    *out = c->quad[k];
+// bound: over the bound orbitals (pairs as in the factored forms' lists),
+// otherwise over all nbf
+int get_quad(dbsrg_ctx *c, int k, bool bound, const double **out) {
+  std::vector<double *> &v = bound ? c->quadb : c->quad;
+  if ((int)v.size() <= k) v.resize(k + 1, nullptr);
+  if (v[k]) {
+    *out = v[k];
     return DBSRG_OK;
   }
   const DeviceGrid &g = c->g;
-  double *q = nullptr;
-  size_t n = (size_t)c->nbf * c->nbf * 2;
-  size_t gp = (size_t)g.ns * g.ksp, gq = (size_t)g.ns * g.ksq, nw = (size_t)2 * c->nbf * g.ns;
-  if (!(q = (double *)cache_alloc(c, (n + gp + gq + nw) * sizeof(double))))
-    return set_err(c, DBSRG_ENOMEM, "quad allocation failed");
-  double *GP = q + n, *GQ = GP + gp, *W = GQ + gq;
-  DBSRG_RUN(c, "k_rk_gram",
-            k_rk_gram<<<dim3((unsigned)((std::max(gp, gq) + 63) / 64), 2), 64, 0, c->stream>>>(
-                g.ns, g.nv, g.ks, g.ksp, g.ksq, k, g.pbsp, g.qbsp, g.gr, g.grw, GP, GQ));
-  DBSRG_RUN(c, "k_quad_w", k_quad_w<<<(unsigned)((nw + 255) / 256), 256, 0, c->stream>>>(
-                               c->nbf, g.ns, g.ksp, g.ksq, c->pq, GP, GQ, W));
-  dim3 gd((unsigned)((c->nbf + 31) / 32), (unsigned)((c->nbf + 31) / 32), 2);
-  DBSRG_RUN(c, "k_quad_dot", k_quad_dot<<<gd, 256, 0, c->stream>>>(c->nbf, g.ns, c->pq, W, q));
-  c->quad[k] = q;
+  const int n = bound ? c->nbound : c->nbf;
+  const size_t m = (size_t)g.ns * n, nq = (size_t)2 * n * n;
+  int rc;
+  const double *W;
+  double *q;
+  if (bound) {
+    if ((rc = get_rfar(c, k, &W))) return rc;
+    q = (double *)cache_alloc(c, nq * sizeof(double));
+  } else {
+    q = (double *)cache_alloc(c, (nq + 4 * m) * sizeof(double));
+  }
+  if (!q) return set_err(c, DBSRG_ENOMEM, "quad allocation failed");
+  if (!bound) {
+    if ((rc = far_vectors_all(c, k, q + nq))) {
+      cache_free(c, q);
+      return rc;
+    }
+    W = q + nq;
+  }
+  v[k] = q;
+  DBSRG_RUN(c, "k_quad_dot",
+            k_quad_dot<<<dim3((unsigned)(((size_t)n * n + 7) / 8), 2), 256, 0, c->stream>>>(
+                n, g.ns, c->pq, (size_t)2 * g.ns, bound ? c->b2o : nullptr, W, 2 * m, q));
   *out = q;
   return DBSRG_OK;
 }

@@ -207,3 +207,31 @@ def test_list_setup_sizes(nch, per):
         assert rc == 0
         assert np.array_equal(a.get_matrix(), h)
     a.close()
+
+
+@pytest.mark.parametrize("ks,ksp,ksq", [(7, 6, 7), (9, 8, 9), (11, 10, 11)])
+def test_asymptotic_coefficients_at_other_spline_orders(ks, ksp, ksq):
+    """acf of the direct R^k lists from the moments: orders below, at and above
+    the nine functions loaded together (plain form: any order), channel
+    orbitals of the list with zero coefficients."""
+    w = synth.small(ns=45, nch=2, mk=2, n_entries=60, breit=False, seed=37)
+    rng = np.random.default_rng(3)
+    t = np.concatenate([np.zeros(ks - 1), np.linspace(0.0, 1.0, 46 - ks) ** 3 * 12.0,
+                        np.full(ks - 1, 12.0)])
+    ns = t.size - ks
+    pq = np.zeros((ns, 2, w.nbf), order="F")
+    pq[: ns - ks + ksp, 0, : w.nbound] = rng.uniform(-1, 1, (ns - ks + ksp, w.nbound))
+    pq[: ns - ks + ksq, 1, : w.nbound] = rng.uniform(-1, 1, (ns - ks + ksq, w.nbound))
+    a = Assembler(t, ks, ksp, ksq)
+    a.set_orbitals(pq, w.ipbs)
+    a.alloc_matrix(w.nch, w.icc, w.iicc, w.mk)
+    g = O.Grid(t, ks, ksp, ksq)
+    m = O.Matrix(g, pq, w.ipbs, w.nch, w.icc, w.mk)
+    for L in w.lists:
+        if (L.icase, L.itype) == (2, 3):
+            a.gen_matrix(L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
+            m.gen_matrix(L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
+    acf, h = a.get_acf(), a.get_matrix()
+    a.close()
+    assert np.abs(m.acf).max() > 0 and relmax(acf, m.acf) <= PLAIN
+    assert relmax(h, m.hch) <= PLAIN
