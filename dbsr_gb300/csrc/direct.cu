@@ -37,6 +37,13 @@ struct Val<true> {
   float h = 0.0f, l = 0.0f;
   __device__ void mac(float2 a, float2 b) { ffa::mac(a, b, h, l); }
   __device__ void add_value(float2 o) { ffa::add(o, h, l); }
+  // the low sum back below half an ulp of the high one: its own rounding errors
+  // grow with its size, which is a random walk over the terms added
+  __device__ void renorm() {
+    const float2 v = ffa::norm(h, l);
+    h = v.x;
+    l = v.y;
+  }
   __device__ float2 get() const { return ffa::norm(h, l); }
   __device__ double value() const { return ffa::value(h, l); }
   __device__ static float2 zero() { return make_float2(0.0f, 0.0f); }
@@ -54,6 +61,7 @@ struct Val<false> {
   double v = 0.0;
   __device__ void mac(double a, double b) { v = fma(a, b, v); }
   __device__ void add_value(double o) { v += o; }
+  __device__ void renorm() {}
   __device__ double get() const { return v; }
   __device__ double value() const { return v; }
   __device__ static double zero() { return 0.0; }
@@ -216,6 +224,10 @@ __global__ void __launch_bounds__(32 * SCW) k_seg_scan(int nv, int nmp, unsigned
 // order.  In the split form bound by the twelve FP32 instructions of a
 // float-float multiply-add, otherwise by the FP64 pipe.  ns 400, 78 segments,
 // R^k (201 M multiply-adds): 274 us; 352 us with one warp per output diagonal.
+// A chain is renormalised after each row of up to nine terms: over 30 drawn
+// matrices the error against 64 bits is 1.5e-14 in the mean and 3.2e-14 at most
+// of a block's norm, 1.7e-14 and 5.5e-14 without (pair potentials 1.6e-14 and
+// 3.9e-14).
 template <bool FF>
 struct ApplyArgs {
   int ns, nv, ks, kk, nm, nmp, ncol, icv, sym;
@@ -307,6 +319,8 @@ __global__ void __launch_bounds__(SYM ? 160 : 288, SYM ? 4 : 2) k_seg_apply(cons
 #pragma unroll
             for (int q = 0; q < N; q++) acc[q].mac(r[q], dv);
           }
+#pragma unroll
+          for (int q = 0; q < N; q++) acc[q].renorm();
         }
       };
       switch (nr) {
