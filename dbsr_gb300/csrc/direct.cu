@@ -11,9 +11,9 @@
 // S^k, whose tables hold no r1 > r2 cells).  The two PQ types of an R^k list
 // that fill the same quadrant are summed in Y.  The work is per segment --
 // npo kd multiply-adds a cell, ns ncol an entry -- and there is none per
-// orbital pair: factor.cu's pair potentials take npo k1 nb^2 a cell and table
-// whatever the list holds, and pay where a list has many segments
-// (direct_by_segment compares the two).
+// orbital pair: factor.cu's pair potentials cost the same whatever the list
+// holds, and pay where a list has many segments (direct_by_segment compares the
+// two).
 //
 // Segments lie along the lanes of a warp: every table value is uniform across
 // a warp, densities are stored segment-fastest.  In the split form the
@@ -28,47 +28,6 @@
 #include "pairs.cuh"
 
 namespace {
-
-template <bool FF>
-struct Val;
-template <>
-struct Val<true> {
-  using T = float2;
-  float h = 0.0f, l = 0.0f;
-  __device__ void mac(float2 a, float2 b) { ffa::mac(a, b, h, l); }
-  __device__ void add_value(float2 o) { ffa::add(o, h, l); }
-  // the low sum back below half an ulp of the high one: its own rounding errors
-  // grow with its size, which is a random walk over the terms added
-  __device__ void renorm() {
-    const float2 v = ffa::norm(h, l);
-    h = v.x;
-    l = v.y;
-  }
-  __device__ float2 get() const { return ffa::norm(h, l); }
-  __device__ double value() const { return ffa::value(h, l); }
-  __device__ static float2 zero() { return make_float2(0.0f, 0.0f); }
-  __device__ static float2 of(double v) { return ffa::split(v); }
-  __device__ static double dbl(float2 v) { return ffa::value(v.x, v.y); }
-  __device__ static float2 mul(float2 a, float2 b) {
-    const float p = a.x * b.x;
-    const float e = fmaf(a.x, b.x, -p);
-    return ffa::norm(p, fmaf(a.x, b.y, fmaf(a.y, b.x, e)));
-  }
-};
-template <>
-struct Val<false> {
-  using T = double;
-  double v = 0.0;
-  __device__ void mac(double a, double b) { v = fma(a, b, v); }
-  __device__ void add_value(double o) { v += o; }
-  __device__ void renorm() {}
-  __device__ double get() const { return v; }
-  __device__ double value() const { return v; }
-  __device__ static double zero() { return 0.0; }
-  __device__ static double of(double x) { return x; }
-  __device__ static double dbl(double x) { return x; }
-  __device__ static double mul(double a, double b) { return a * b; }
-};
 
 constexpr int NC3 = 3;  // band columns per thread of the density kernel
 constexpr int DSL = 8;  // segments per block of the density kernel
@@ -185,14 +144,14 @@ __global__ void __launch_bounds__(32 * CW) k_seg_cells(const CellArgs<FF> a) {
 }
 
 // Exclusive sums over the later (bit set in sufmask) or earlier cells, in
-// place: 32 segments a block, each warp a run of cells
-constexpr int SCW = 16;
-__global__ void __launch_bounds__(32 * SCW) k_seg_scan(int nv, int nmp, unsigned sufmask,
+// place: eight segments a block, each with sixteen runs of cells
+constexpr int SCW = 16, SCL = 8;
+__global__ void __launch_bounds__(SCL * SCW) k_seg_scan(int nv, int nmp, unsigned sufmask,
                                                        double *S) {
-  __shared__ double tot[SCW][32];
-  const int lane = threadIdx.x % 32, w = threadIdx.x / 32, set = blockIdx.y;
+  __shared__ double tot[SCW][SCL];
+  const int lane = threadIdx.x % SCL, w = threadIdx.x / SCL, set = blockIdx.y;
   const bool suf = (sufmask >> set) & 1;
-  double *s = S + (size_t)set * nv * nmp + blockIdx.x * 32 + lane;
+  double *s = S + (size_t)set * nv * nmp + blockIdx.x * SCL + lane;
   const int run = (nv + SCW - 1) / SCW, lo = min(nv, w * run), hi = min(nv, lo + run);
   double t = 0.0;
 #pragma unroll 8
@@ -204,12 +163,21 @@ __global__ void __launch_bounds__(32 * SCW) k_seg_scan(int nv, int nmp, unsigned
     for (int k = SCW - 1; k > w; k--) acc += tot[k][lane];
   else
     for (int k = 0; k < w; k++) acc += tot[k][lane];
-#pragma unroll 8
-  for (int i = lo; i < hi; i++) {
-    double *x = s + (size_t)(suf ? hi - 1 - (i - lo) : i) * nmp;
-    const double v = *x;
-    *x = acc;
-    acc += v;
+  // (loads of eight cells before their stores: the array is overwritten)
+  for (int i0 = lo; i0 < hi; i0 += 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int i = i0 + u;
+      v[u] = i < hi ? s[(size_t)(suf ? hi - 1 - (i - lo) : i) * nmp] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int i = i0 + u;
+      if (i >= hi) break;
+      s[(size_t)(suf ? hi - 1 - (i - lo) : i) * nmp] = acc;
+      acc += v[u];
+    }
   }
 }
 
@@ -501,7 +469,7 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
             k_seg_cells<FF><<<dim3((unsigned)(nmp / 32), (unsigned)((nv + CW - 1) / CW),
                                    (unsigned)nset),
                               32 * CW, 0, st>>>(ca));
-  DBSRG_RUN(c, "k_seg_scan", k_seg_scan<<<dim3((unsigned)(nmp / 32), (unsigned)nset), 32 * SCW, 0,
+  DBSRG_RUN(c, "k_seg_scan", k_seg_scan<<<dim3((unsigned)(nmp / SCL), (unsigned)nset), SCL * SCW, 0,
                                           st>>>(nv, nmp, sufmask, S));
   p.nm = nm;
   p.icv = j.icv;
@@ -532,12 +500,15 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
 
 // Multiply-adds of the two ways over a whole list (all its segments, whatever
 // the window or chunk, so that a block's result does not depend on them), the
-// pair way with the potentials it builds whether or not they are cached.
-// k_seg_apply and k_pair_diag run at about the same rate per multiply-add (0.4 to
-// 1.0 T/s).  Assemblies with the line at half and at twice the count: ns 400, 80
-// channels (R^k lists of 78 segments by segment, S^k lists of 350 by pairs)
-// 66.3 and 61.8 ms against 61.6; ns 222, 14 channels in FP64 15.3 and 16.7
-// against 15.4; all lists by segment 86 ms and 16.7 ms, none 66.1 and 17.3.
+// pair way with the potentials it builds whether or not they are cached.  Per
+// cell and segment the apply kernel takes npo kd of them, the cell moments
+// about 24 kd (FP64); a pair potential about 4000 an output for its small
+// matrix, 120 per second orbital and 14 per pair; both ways one an entry and
+// band element.  Assemblies by the rule, all lists by pairs, and with the line
+// before the pair potentials were built a row at a time (mostly by segment):
+// ns 80, 2 channels 1.86 / 1.99 / 1.86 ms; ns 200, 12 channels 4.96 / 5.12 / 5.14;
+// ns 283, 32 channels 14.0 / 14.2 / 14.2; ns 400, 80 channels 47.5 / 47.6 / 49.7;
+// four waves of 6 to 28 channels in turn 34.0 / 35.0 / 34.5.
 // The lists of a one-channel matrix (the SCF potentials) hold one segment each
 // and come once per orbital, so the pair potentials of an iteration serve all
 // of them: 30 orbitals at ns 300 took 76 ms by segment, 66 ms by pairs.
@@ -545,17 +516,18 @@ bool direct_by_segment(const dbsrg_ctx *c, int family, int icv, int na, const in
                        long long nseg, long long nent) {
   const DeviceGrid &g = c->g;
   if (c->nch == 1) return false;
-  const double nb = c->nbound, ns = g.ns, nv = g.nv, nd = 2.0 * g.ks - 1.0;
+  const double nb = c->nbound, ns = g.ns, nv = g.nv;
+  const double ncol = family == 0 ? g.ks : 2.0 * g.ks - 1.0;
   double seg = 0.0, pair = 0.0;
   for (int a = 0; a < na; a++) {
     const TableBases tb = table_bases(g, family, types[a]);
     const PairSpec eo = icv == 1 ? tb.e1 : tb.e2, ed = icv == 1 ? tb.e2 : tb.e1;
-    const double npo = npairs(eo), kd = npairs(ed);
-    seg += (double)nseg * nv * npo * kd;
-    pair += nv * npo * ed.k1 * (ed.k2 * nb + nb * nb) + nb * nb * ns * nd * 2.0;
-    pair += (double)nent * ns * nd;
+    const double npo = npairs(eo), kd = npairs(ed), np = family == 0 ? nb * (nb + 1) / 2 : nb * nb;
+    seg += (double)nseg * nv * kd * (npo + 24.0);
+    pair += ns * ncol * (4000.0 + 120.0 * nb + 14.0 * np);
+    pair += (double)nent * ns * ncol;
   }
-  seg += (double)nent * ns * nd * (na > 1 ? 2.0 : 1.0);
+  seg += (double)nent * ns * ncol * (na > 1 ? 2.0 : 1.0);
   return seg < pair;
 }
 

@@ -49,7 +49,6 @@ constexpr int FAR = 9;            // |y - x| >= FAR is far field (spline orders 
 constexpr int BAND = FAR - 1;     // near band |y - x| <= 8
 constexpr int NDB = 2 * BAND + 1; // band diagonals
 constexpr int PXC = 4;            // output rows per block of the band pair potentials
-constexpr int PBC = 4;            // second-orbital chunk of the diagonal-cell stage
 
 // target quadrants of the atypes of one list (UPDATE_HS)
 struct QuadSpec {
@@ -225,8 +224,7 @@ __global__ void __launch_bounds__(256) k_far_field(int ns, int nb, const double 
 // (b a; y, x - y) for (a b; x, y - x).  R^k types 0 and 1 are unchanged under
 // the exchange (Kx = Kout): only the diagonals d >= 0 are computed.  Type 2
 // gives type 3's potentials this way (Kx theirs); S^k has none (Kx null).
-// ns 400, 20 orbitals: an R^k list's potentials 4 x 84 -> 3 launches of 47, 47
-// and 90 us.
+// ns 400, 20 orbitals: an R^k list's potentials 4 x 84 us, 3 launches now.
 template <bool FF>
 __global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int mode,
                                                    const double *__restrict__ rkb,
@@ -337,9 +335,19 @@ __global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int m
 // output electron.  Pair densities of a symmetric storage give every ordered
 // (h1, h2) the moment of the unordered pair (pidx orders them).
 //
+// Pairs are numbered a + nb b, or, where exchanging the orbitals changes
+// nothing (symab: packed symmetric density pairs of equal components), by the
+// pairs a <= b alone, a + b (b + 1) / 2.
+__host__ __device__ inline int pair_count(int nb, int symab) {
+  return symab ? nb * (nb + 1) / 2 : nb * nb;
+}
+__device__ __forceinline__ int pair_number(int nb, int symab, int a, int b) {
+  return a + (symab ? b * (b + 1) / 2 : b * nb);
+}
+
 // (1) cell sums, one block per cell cv:
-//   S1(ab, cv) = sum_{h1,h2} M1(h1,h2;cv) P1(a, cv+h1-1) P2(b, cv+h2-1), S2 with M2
-__global__ void k_pair_cellsum(int ns, int nv, int kk, int nb, PairSpec ed, const double *M1,
+//   S1(cv, pair) = sum_{h1,h2} M1(h1,h2;cv) P1(a, cv+h1-1) P2(b, cv+h2-1), S2 with M2
+__global__ void k_pair_cellsum(int ns, int kk, int nb, int symab, PairSpec ed, const double *M1,
                                const double *M2, const double *P1, const double *P2, double *S1,
                                double *S2) {
   extern __shared__ double sm[];
@@ -367,243 +375,266 @@ __global__ void k_pair_cellsum(int ns, int nv, int kk, int nb, PairSpec ed, cons
     t2[q] = s2;
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < nb * nb; q += blockDim.x) {
-    const int a = q / nb, b = q % nb;
+  const int np = pair_count(nb, symab);
+  for (int q = threadIdx.x; q < np; q += blockDim.x) {
+    int a, b;
+    if (symab) {
+      b = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);
+      while (b * (b + 1) / 2 > q) b--;
+      while ((b + 1) * (b + 2) / 2 <= q) b++;
+      a = q - b * (b + 1) / 2;
+    } else {
+      b = q / nb;
+      a = q - b * nb;
+    }
     double s1 = 0.0, s2 = 0.0;
     for (int h = 0; h < k1; h++) {
       const double p = w1[a * k1 + h];
       s1 = fma(p, t1[b * k1 + h], s1);
-      s2 = fma(p, t2[b * k1 + h], s2);
+      if (M2) s2 = fma(p, t2[b * k1 + h], s2);
     }
-    S1[(size_t)q * nv + cv - 1] = s1;
-    if (S2) S2[(size_t)q * nv + cv - 1] = s2;
+    S1[(size_t)(cv - 1) * np + q] = s1;
+    if (M2) S2[(size_t)(cv - 1) * np + q] = s2;
   }
 }
 
-// (2) exclusive suffix (sum over later cells) or prefix sums per pair, one
-// warp per pair: every lane scans a run of cells, the run totals are
-// scanned across the warp by shuffles
-// (blockIdx.y 1: a second array S1 with its own direction, same launch)
-__global__ void k_pair_scan(int nv, int npair, double *S0, int suffix0, double *S1, int suffix1) {
-  double *S = blockIdx.y ? S1 : S0;
-  const int suffix = blockIdx.y ? suffix1 : suffix0;
-  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 32), lane = threadIdx.x % 32;
-  if (warp >= npair) return;
-  double *s = S + (size_t)warp * nv;
-  const int run = (nv + 31) / 32;
-  const int lo = min(nv, lane * run), hi = min(nv, lo + run);
-  double tot = 0.0;
-  for (int i = lo; i < hi; i++) tot += s[i];
-  double incl = tot;
-  for (int off = 1; off < 32; off <<= 1) {
-    const double v = suffix ? __shfl_down_sync(0xffffffffu, incl, off)
-                            : __shfl_up_sync(0xffffffffu, incl, off);
-    if (suffix ? lane + off < 32 : lane >= off) incl += v;
-  }
-  const double nb1 = suffix ? __shfl_down_sync(0xffffffffu, incl, 1)
-                            : __shfl_up_sync(0xffffffffu, incl, 1);
-  double acc = suffix ? (lane == 31 ? 0.0 : nb1) : (lane == 0 ? 0.0 : nb1);
-  if (suffix) {
-    for (int i = hi - 1; i >= lo; i--) {
-      const double v = s[i];
-      s[i] = acc;
-      acc += v;
-    }
-  } else {
-    for (int i = lo; i < hi; i++) {
-      const double v = s[i];
-      s[i] = acc;
-      acc += v;
-    }
-  }
-}
-
-// (3) diagonal cells, one block per cell cv:
-//   Dq[ph][ab][q(po)] = sum_{g1,g2} R(po; g1,g2; cv) P1(a, cv+g1-1) P2(b, cv+g2-1)
-// with po an output pair of the cell, q its position in the ns x ncol result
-// and ph = (cv-1) mod 9: a cell touches outputs with first index in
-// [cv, cv+8], so cells of one phase never share an output.  Two stages:
-// H(po, g1, b) = sum_g2 R P2, then sum_g1 P1 H.
+// (2) exclusive suffix (sum over later cells) or prefix sums per pair, in place
+// (as float-float pairs in the split form): eight pairs a block, each with
+// sixteen runs of cells (blockIdx.y 1: the second array, prefix sums).  Bound by
+// the FP64 instructions, so the pairs are spread over many blocks: ns 300, 30
+// orbitals, split form 23 us with 32 pairs a block.
+constexpr int PSW = 16, PSP = 8;
 template <bool FF>
-__global__ void __launch_bounds__(512) k_pair_diag(int ns, int ks, int kk, int nb, int ofirst,
-                                                   char sym, PairSpec eo, PairSpec ed,
-                                                   const double *__restrict__ rkd,
-                                                   const double *__restrict__ P1,
-                                                   const double *__restrict__ P2,
-                                                   double *__restrict__ Dq, size_t per) {
-  using S = typename std::conditional<FF, float2, double>::type;
-  extern __shared__ double smraw[];
-  S *sm = reinterpret_cast<S *>(smraw);
-  auto sv = [](double v) -> S {
-    if constexpr (FF) return ffa::split(v); else return v;
+__global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, int np, int suffix0, double *S0,
+                                                        double *S1) {
+  __shared__ double tot[PSW][PSP];
+  const int lane = threadIdx.x % PSP, w = threadIdx.x / PSP, q = blockIdx.x * PSP + lane;
+  double *s = (blockIdx.y ? S1 : S0) + q;
+  const bool suf = blockIdx.y == 0 && suffix0, ok = q < np;
+  const int run = (nv + PSW - 1) / PSW, lo = min(nv, w * run), hi = min(nv, lo + run);
+  double t = 0.0;
+  if (ok)
+#pragma unroll 8
+    for (int i = lo; i < hi; i++) t += s[(size_t)(suf ? hi - 1 - (i - lo) : i) * np];
+  tot[w][lane] = t;
+  __syncthreads();
+  if (!ok) return;
+  double acc = 0.0;
+  if (suf)
+    for (int k = PSW - 1; k > w; k--) acc += tot[k][lane];
+  else
+    for (int k = 0; k < w; k++) acc += tot[k][lane];
+  // (loads of eight cells before their stores: the array is overwritten)
+  for (int i0 = lo; i0 < hi; i0 += 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int i = i0 + u;
+      v[u] = i < hi ? s[(size_t)(suf ? hi - 1 - (i - lo) : i) * np] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int i = i0 + u;
+      if (i >= hi) break;
+      double *x = s + (size_t)(suf ? hi - 1 - (i - lo) : i) * np;
+      if constexpr (FF)
+        *reinterpret_cast<float2 *>(x) = ffa::split(acc);
+      else
+        *x = acc;
+      acc += v[u];
+    }
+  }
+}
+
+// (3) the potentials.  An output (f, f+dl) belongs to the cells lo .. hi that
+// hold both functions.  Everything the density does inside those cells goes
+// through one small matrix per output, the table's elements without the far
+// cells,
+//   W(x,y) = sum_cv [ R(po(cv); x,y; cv) + M1(x,y;cv) sum_{cv' before} L1(po(cv'))
+//                     + M2(x,y;cv) sum_{cv' after} L2(po(cv')) ],
+// (x, y within the cells' functions, at most 17 x 17 at order 9, banded), and
+//   Kd_ab = sum_x P1_a(x) H_b(x) + SA_ab sum_cv L1 + SB_ab sum_cv L2,
+//   H_b(x) = sum_y W(x,y) P2_b(y),
+// with SA/SB the scanned sums beyond the window (L1 = lo1, SA after the window;
+// case 2: L1 = hi2, SA before it and the sum over cv' after).  Per pair an
+// output takes up to 17 + 2 multiply-adds; contracting every diagonal cell by
+// itself and adding the separable terms cell by cell takes up to 81 + 18.
+// A block forms PDX consecutive f (a full sector of the result) of one dl
+// for PDB second orbitals; a thread takes two second orbitals at once.  The
+// small matrix is summed in FP64 and rebuilt by every block, so blocks of 16
+// second orbitals lose more than they gain (106 us for 78).  Bound by the FP64
+// pipe, in the split form by the latency of the small matrix's loads.  Cell by
+// cell with partial sums in memory against this: ns 300, 30 orbitals, R^k, FP64
+// 325 -> 78 us; ns 400, 20 orbitals, split form (R^k and S^k) 217 -> 66 us.
+constexpr int PDX = 4, PDB = 32, PDT = 256;
+template <bool FF>
+struct PairDirArgs {
+  int ns, nv, kk, nb, np, symab, suf, dl0;  // dl0: dl of column 0
+  PairSpec eo, ed;
+  const double *rkd;
+  int rpo, rpd;
+  const double *L1, *L2, *M1, *M2;
+  const typename Val<FF>::T *P1, *P2, *SA, *SB;
+  typename Val<FF>::T *K;
+  size_t per;
+};
+
+__host__ __device__ inline int pair_row_stride(int n) {  // 8 mod 16: rows on other banks
+  return (n + 7) / 16 * 16 + 8;
+}
+
+// KM: the largest spline order the shared arrays are laid out for (9, or 16 for
+// the orders above: the energy functional takes them all)
+constexpr int pair_window(int km) { return 2 * km - 1; }
+constexpr int pair_rows(int km) { return PDX - 1 + pair_window(km); }
+
+template <bool FF, int KM>
+__global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
+  constexpr int PDW = pair_window(KM), PDR = pair_rows(KM);
+  using V = Val<FF>;
+  using T = typename V::T;
+  struct alignas(16) T2 {
+    T a, b;
   };
-  const int cv = blockIdx.x + 1, k1 = ed.k1, k2 = ed.k2, kd = k1 * k2;
-  const int npo = eo.sym ? eo.k1 * (eo.k1 + 1) / 2 : eo.k1 * eo.k2;
-  const size_t npair = (size_t)nb * nb;
-  S *w1 = sm, *w2 = w1 + nb * k1, *Rt = w2 + nb * k2;
-  S *H = Rt + (size_t)npo * kd;
-  int *poq = (int *)(H + (size_t)npo * k1 * PBC);
-  for (int q = threadIdx.x; q < nb * k1; q += blockDim.x) {
-    const int a = q / k1, x = cv + q % k1;
-    w1[q] = sv(x <= ns ? P1[(size_t)a * ns + x - 1] : 0.0);
-  }
-  for (int q = threadIdx.x; q < nb * k2; q += blockDim.x) {
-    const int b = q / k2, x = cv + q % k2;
-    w2[q] = sv(x <= ns ? P2[(size_t)b * ns + x - 1] : 0.0);
-  }
-  for (int po = threadIdx.x; po < npo; po += blockDim.x) {
-    int h1, h2;
-    if (eo.sym) {
-      int r = po, row = 0;
-      while (r >= eo.k1 - row) {
-        r -= eo.k1 - row;
-        row++;
-      }
-      h1 = row + 1;
-      h2 = row + 1 + r;
-    } else {
-      h1 = po / eo.k2 + 1;
-      h2 = po % eo.k2 + 1;
+  extern __shared__ __align__(16) unsigned char smdir[];
+  T *W = reinterpret_cast<T *>(smdir);     // [PDX][PDW][PDW]
+  T *H = W + PDX * PDW * PDW;              // [PDX][PDW][PDB]
+  T *p2w = H + PDX * PDW * PDB;            // [PDR][PDB]
+  T *p1w = p2w + PDR * PDB;                // [PDR][pstr]
+  __shared__ double c1[PDX][KM], c2[PDX][KM];
+  __shared__ T t1[PDX], t2[PDX];
+  __shared__ int los[PDX], his[PDX], pos[PDX][KM];
+  const int ns = p.ns, nb = p.nb, pstr = pair_row_stride(nb);
+  const PairSpec eo = p.eo, ed = p.ed;
+  const int f0 = blockIdx.x * PDX + 1, dl = p.dl0 + (int)blockIdx.y, zb = blockIdx.z * PDB;
+  const int bc = min(PDB, nb - zb), na = p.symab ? zb + bc : nb;
+  const int rb = f0 + max(1 - eo.k1, dl + 1 - eo.k2);  // first row of the windows
+  if (threadIdx.x < PDX) {
+    const int fl = threadIdx.x, f = f0 + fl, s2 = f + dl;
+    int lo = max(1, rb + fl), hi = min(p.nv, min(f, s2));
+    if (f > ns || s2 < 1 || s2 > ns) hi = lo - 1;
+    double l1[KM], l2[KM], s1 = 0.0, s2s = 0.0;
+#pragma unroll
+    for (int k = 0; k < KM; k++) {
+      const int cv = lo + k;
+      const bool ok = cv <= hi;
+      const int po = ok ? pidx(eo, f - cv + 1, s2 - cv + 1) : 0;
+      const size_t o = (size_t)po + (size_t)p.kk * (ok ? cv - 1 : 0);
+      l1[k] = ok ? p.L1[o] : 0.0;
+      l2[k] = ok && p.L2 ? p.L2[o] : 0.0;
+      pos[fl][k] = po;
     }
-    const int f = cv + h1 - 1, s2 = cv + h2 - 1;
-    poq[po] = (f > ns || s2 > ns) ? -1
-              : (sym == 's' ? (f - 1) + ns * (s2 - f) : (f - 1) + ns * (s2 - f + ks - 1));
-  }
-  const double *rc = rkd + (size_t)kk * kk * (cv - 1);  // rkd(e1 pair, e2 pair; cv)
-  // the cell's table slice: consecutive threads read consecutive table
-  // elements (ofirst: the output pair is rkd's first index)
-  for (int q = threadIdx.x; q < npo * kd; q += blockDim.x) {
-    int po, r;
-    if (ofirst) {
-      po = q % npo;
-      r = q / npo;
-    } else {
-      po = q / kd;
-      r = q % kd;
+    // sums over the window's cells before (c1 where suf) or after a cell
+#pragma unroll
+    for (int k = 0; k < KM; k++) {
+      if (p.suf) c1[fl][k] = s1;
+      s1 += l1[k];
     }
-    const int g1 = r / k2 + 1, g2 = r % k2 + 1;
-    const int pd = pidx(ed, g1, g2);
-    Rt[(size_t)po * kd + r] =
-        sv(ofirst ? rc[(size_t)po + (size_t)kk * pd] : rc[(size_t)pd + (size_t)kk * po]);
+    double r1 = 0.0;
+#pragma unroll
+    for (int k = KM - 1; k >= 0; k--) {
+      c2[fl][k] = s2s;
+      s2s += l2[k];
+      if (!p.suf) c1[fl][k] = r1;
+      r1 += l1[k];
+    }
+    t1[fl] = V::of(s1);
+    t2[fl] = V::of(s2s);
+    los[fl] = lo;
+    his[fl] = hi;
+  }
+  for (int q = threadIdx.x; q < PDR * na; q += PDT) {
+    const int a = q / PDR, r = q - a * PDR, x = rb + r;
+    p1w[r * pstr + a] = x >= 1 && x <= ns ? p.P1[(size_t)a * ns + x - 1] : V::zero();
+  }
+  for (int q = threadIdx.x; q < PDR * PDB; q += PDT) {
+    const int b = q / PDR, r = q - b * PDR, y = rb + r;
+    p2w[r * PDB + b] =
+        b < bc && y >= 1 && y <= ns ? p.P2[(size_t)(zb + b) * ns + y - 1] : V::zero();
   }
   __syncthreads();
-  const int ph = (cv - 1) % FAR;
-  for (int b0 = 0; b0 < nb; b0 += PBC) {  // chunks of second orbitals
-    const int bc = min(PBC, nb - b0);
-    // stage 1: a thread forms H(po, g1, b) for the bc second orbitals of the
-    // chunk at once (independent sums sharing each table load)
-    for (int q = threadIdx.x; q < npo * k1; q += blockDim.x) {
-      const int g1 = q % k1, po = q / k1;
-      const S *rt = Rt + (size_t)po * kd + (size_t)g1 * k2;
-      S *hq = H + ((size_t)po * k1 + g1) * PBC;
-      if constexpr (FF) {
-        float sh[PBC], sl[PBC];
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++) sh[bb] = sl[bb] = 0.0f;
-        for (int g2 = 0; g2 < k2; g2++) {
-          const S r = rt[g2];
-#pragma unroll
-          for (int bb = 0; bb < PBC; bb++)
-            if (bb < bc) ffa::mac(r, w2[(size_t)(b0 + bb) * k2 + g2], sh[bb], sl[bb]);
-        }
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++)
-          if (bb < bc) hq[bb] = ffa::norm(sh[bb], sl[bb]);
-      } else {
-        double acc[PBC];
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++) acc[bb] = 0.0;
-        for (int g2 = 0; g2 < k2; g2++) {
-          const S r = rt[g2];
-#pragma unroll
-          for (int bb = 0; bb < PBC; bb++)
-            if (bb < bc) acc[bb] = fma(r, w2[(size_t)(b0 + bb) * k2 + g2], acc[bb]);
-        }
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++)
-          if (bb < bc) hq[bb] = acc[bb];
-      }
+  // one item per element, diagonal by diagonal (symmetric: the upper ones)
+  const int u0 = ed.sym ? 0 : 1 - ed.k1, ndg = ed.k2 - u0;
+  for (int q = threadIdx.x; q < PDX * PDW * ndg; q += PDT) {
+    const int r = q / PDW, t = q - r * PDW, fl = r % PDX, u = t + u0 + r / PDX;
+    const int lo = los[fl], hi = his[fl], x = lo + t, y = lo + u;
+    const int ca = max(lo, max(x - ed.k1, y - ed.k2) + 1), cb = min(hi, min(x, y));
+    if (ca > cb) continue;
+    double v = 0.0;
+#pragma unroll 9
+    for (int cv = ca; cv <= cb; cv++) {
+      const int pd = pidx(ed, x - cv + 1, y - cv + 1);
+      const size_t o = (size_t)pd + (size_t)p.kk * (cv - 1);
+      v += p.rkd[(size_t)p.kk * p.kk * (cv - 1) + (size_t)p.rpo * pos[fl][cv - lo] +
+                 (size_t)p.rpd * pd];
+      v = fma(p.M1[o], c1[fl][cv - lo], v);
+      if (p.M2) v = fma(p.M2[o], c2[fl][cv - lo], v);
     }
-    __syncthreads();
-    // stage 2: Dq for the bc second orbitals at once
-    for (int q = threadIdx.x; q < npo * nb; q += blockDim.x) {
-      const int a = q % nb, po = q / nb;
-      const int qp = poq[po];
-      if (qp < 0) continue;
-      const S *p = w1 + (size_t)a * k1;
-      const S *h = H + (size_t)po * k1 * PBC;
-      const size_t d0 = ((size_t)ph * npair + (size_t)a * nb + b0) * per + qp;
-      if constexpr (FF) {  // kept as float-float pairs (no FP64 conversion)
-        float sh[PBC], sl[PBC];
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++) sh[bb] = sl[bb] = 0.0f;
-        for (int g1 = 0; g1 < k1; g1++) {
-          const S pv = p[g1];
-#pragma unroll
-          for (int bb = 0; bb < PBC; bb++)
-            if (bb < bc) ffa::mac(pv, h[(size_t)g1 * PBC + bb], sh[bb], sl[bb]);
-        }
-        float2 *D = reinterpret_cast<float2 *>(Dq);
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++)
-          if (bb < bc) D[d0 + (size_t)bb * per] = ffa::norm(sh[bb], sl[bb]);
-      } else {
-        double s[PBC];
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++) s[bb] = 0.0;
-        for (int g1 = 0; g1 < k1; g1++) {
-          const S pv = p[g1];
-#pragma unroll
-          for (int bb = 0; bb < PBC; bb++)
-            if (bb < bc) s[bb] = fma(pv, h[(size_t)g1 * PBC + bb], s[bb]);
-        }
-#pragma unroll
-        for (int bb = 0; bb < PBC; bb++)
-          if (bb < bc) Dq[d0 + (size_t)bb * per] = s[bb];
-      }
-    }
-    __syncthreads();
+    const T wv = V::of(v);
+    W[(fl * PDW + t) * PDW + u] = wv;
+    if (ed.sym) W[(fl * PDW + u) * PDW + t] = wv;
   }
-}
-
-// (4) the pair potential: separable terms from the scanned cell sums plus the
-// diagonal-cell parts, cells in order (the output loop of k_direct)
-template <bool FF>
-__global__ void k_pair_direct_final(int ns, int ks, int nv, int kk, int nb, int icv, char sym,
-                                    PairSpec eo, const double *lo1, const double *hi1,
-                                    const double *hi2, const double *SA, const double *SB,
-                                    const double *Dq, void *Kout, size_t per) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= per) return;
-  const int pair = blockIdx.y;
-  const size_t npair = (size_t)nb * nb;
-  const int f = (int)(t % ns) + 1, col = (int)(t / ns) + 1;
-  const int s2 = sym == 's' ? f + col - 1 : f + col - ks;
-  double acc = 0.0;
-  float dh = 0.0f, dl = 0.0f;  // float-float diagonal-cell parts (FF)
-  if (s2 >= 1 && s2 <= ns) {
-    const int lo = max(max(1, f - eo.k1 + 1), s2 - eo.k2 + 1), hi = min(min(nv, f), s2);
-    const double *sa = SA + (size_t)pair * nv;
-    const double *sb = SB ? SB + (size_t)pair * nv : nullptr;
-    for (int cv = lo; cv <= hi; cv++) {
-      const size_t o = (size_t)pidx(eo, f - cv + 1, s2 - cv + 1) + (size_t)kk * (cv - 1);
-      if (icv == 1) {
-        acc = fma(lo1[o], sa[cv - 1], acc);
-        if (sb) acc = fma(hi1[o], sb[cv - 1], acc);
-      } else {
-        acc = fma(hi2[o], sa[cv - 1], acc);
-      }
-      const size_t dq = ((size_t)((cv - 1) % FAR) * npair + pair) * per + t;
-      if constexpr (FF)
-        ffa::add(reinterpret_cast<const float2 *>(Dq)[dq], dh, dl);
-      else
-        acc += Dq[dq];
+  __syncthreads();
+  const int ng = (bc + 1) / 2;  // groups of two second orbitals
+  for (int q = threadIdx.x; q < PDX * PDW * ng; q += PDT) {
+    const int r = q / ng, g = q - r * ng, fl = r / PDW, t = r - fl * PDW;
+    const int lo = los[fl], hi = his[fl], x = lo + t;
+    const int ca = max(lo, x - ed.k1 + 1), cb = min(hi, x);
+    if (ca > cb) continue;
+    const T *w = W + r * PDW;
+    const T *pp = p2w + (lo - rb) * PDB + 2 * g;
+    V s0, s1;
+    for (int u = ca - lo; u < cb + ed.k2 - lo; u++) {
+      const T wv = w[u];
+      const T2 v = *reinterpret_cast<const T2 *>(pp + u * PDB);
+      s0.mac(wv, v.a);
+      s1.mac(wv, v.b);
     }
+    *reinterpret_cast<T2 *>(H + r * PDB + 2 * g) = {s0.get(), s1.get()};
   }
-  if constexpr (FF)
-    static_cast<float2 *>(Kout)[(size_t)pair * per + t] = ffa::split(acc + ffa::value(dh, dl));
-  else
-    static_cast<double *>(Kout)[(size_t)pair * per + t] = acc;
+  __syncthreads();
+  // items: fl fastest, then the first orbital, then the group
+  const int nitem = p.symab ? ng * zb + ng * (ng + 1) : ng * na;
+  for (int q = threadIdx.x; q < PDX * nitem; q += PDT) {
+    const int fl = q % PDX, f = f0 + fl;
+    int a = q / PDX, g = 0;
+    if (p.symab) {  // group g holds the first orbitals up to its second one
+      while (a >= zb + 2 * g + 2) a -= zb + 2 * g + 2, g++;
+      if (a >= na) continue;
+    } else {
+      g = a / na;
+      a -= g * na;
+    }
+    if (f > ns) continue;
+    const int lo = los[fl], hi = his[fl], b0 = zb + 2 * g;
+    V s0, s1;
+    if (lo <= hi) {
+      const T *pa = p1w + (lo - rb) * pstr + a, *h = H + fl * PDW * PDB + 2 * g;
+      const int nt = hi - lo + ed.k1;
+      for (int t = 0; t < nt; t++) {
+        const T pv = pa[t * pstr];
+        const T2 v = *reinterpret_cast<const T2 *>(h + t * PDB);
+        s0.mac(pv, v.a);
+        s1.mac(pv, v.b);
+      }
+      const size_t ra = (size_t)((p.suf ? hi : lo) - 1) * p.np, rl = (size_t)(lo - 1) * p.np;
+      const int q0 = pair_number(nb, p.symab, p.symab ? min(a, b0) : a, b0);
+      const int q1 = pair_number(nb, p.symab, a, min(b0 + 1, nb - 1));
+      s0.mac(t1[fl], p.SA[ra + q0]);
+      s1.mac(t1[fl], p.SA[ra + q1]);
+      if (p.SB) {
+        s0.mac(t2[fl], p.SB[rl + q0]);
+        s1.mac(t2[fl], p.SB[rl + q1]);
+      }
+    }
+    const size_t o = (size_t)(f - 1) + (size_t)ns * blockIdx.y;
+    auto put = [&](int b, T v) {
+      p.K[((size_t)a * nb + b) * p.per + o] = v;
+      if (p.symab && a < b) p.K[((size_t)b * nb + a) * p.per + o] = v;
+    };
+    if (!p.symab || a <= b0) put(b0, s0.get());
+    if (b0 + 1 < nb) put(b0 + 1, s1.get());
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -976,12 +1007,12 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
   const double *P2 = c->brows + (size_t)(jp2 - 1) * nb * ns;
   const double *M1 = icv == 1 ? cd->hi2 : cd->lo1;
   const double *M2 = (icv == 1 && family == 0) ? cd->lo2 : nullptr;
-  // scratch: SA, SB (npair x nv), Dq (9 x npair x per)
-  const size_t sbytes = (2 * npair * nv + (size_t)FAR * npair * per) * sizeof(double);
+  const int symab = ed.sym && jp1 == jp2, np = pair_count(nb, symab);
+  // scratch: SA, SB (nv x np)
   const int ps = c->stream == c->bstream[1] ? 1 : 0;  // scratch of this stream
   if (c->stream != c->bstream[0] && c->stream != c->bstream[1]) c->stream_built = true;
-  if ((rc = ensure_pscratch(c, ps, sbytes))) return rc;
-  double *SA = (double *)c->pscratch[ps], *SB = SA + npair * nv, *Dq = SB + npair * nv;
+  if ((rc = ensure_pscratch(c, ps, 2 * (size_t)np * nv * sizeof(double)))) return rc;
+  double *SA = (double *)c->pscratch[ps], *SB = M2 ? SA + (size_t)np * nv : nullptr;
   double *K = nullptr;  // doubles, or as many float2 pairs (same bytes)
   if (!(K = (double *)cache_alloc(c, npair * per * sizeof(double)))) {
     cudaGetLastError();
@@ -992,46 +1023,68 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
   const size_t sm1 = (size_t)nb * (3 * ed.k1 + ed.k2) * sizeof(double);
   if ((rc = set_smem(c, (const void *)k_pair_cellsum, sm1))) return rc;
   DBSRG_RUN(c, "k_pair_cellsum",
-            k_pair_cellsum<<<nv, 256, sm1, st>>>(ns, nv, kk, nb, ed, M1, M2, P1, P2, SA,
-                                                 M2 ? SB : nullptr));
-  const unsigned gp = (unsigned)((npair * 32 + 255) / 256);
-  DBSRG_RUN(c, "k_pair_scan", k_pair_scan<<<dim3(gp, M2 ? 2 : 1), 256, 0, st>>>(
-                                  nv, (int)npair, SA, icv == 1, SB, 0));
-  const int npo = eo.sym ? eo.k1 * (eo.k1 + 1) / 2 : eo.k1 * eo.k2;
-  const size_t sm3 = ((size_t)nb * (ed.k1 + ed.k2) + (size_t)npo * ed.k1 * ed.k2 +
-                      (size_t)npo * ed.k1 * PBC) * sizeof(double) + (size_t)npo * sizeof(int);
-  const double *lo1 = icv == 1 ? cd->lo1 : nullptr;
-  const double *hi1 = (icv == 1 && family == 0) ? cd->hi1 : nullptr;
-  dim3 gf((unsigned)((per + 127) / 128), (unsigned)npair);
+            k_pair_cellsum<<<nv, 256, sm1, st>>>(ns, kk, nb, symab, ed, M1, M2, P1, P2, SA, SB));
   const int ofirst = (icv == 1) != cd->tr;
-  // executed work of the diagonal cells: per cell, stage 1 npo k1 k2 nb and
-  // stage 2 npo nb k1 nb multiply-adds; the cell's table slice read and its
-  // npo nb^2 outputs written.  The final potentials: per output element and
-  // pair a few separable terms (about 4 multiply-adds) and the nine
-  // diagonal-cell phases read, the potential written.
-  const double dflops = 2.0 * nv * npo * ed.k1 * ((double)ed.k2 * nb + (double)nb * nb);
-  const double dbytes = 8.0 * nv * ((double)npo * ed.k1 * ed.k2 + (double)npo * nb * nb);
-  const double fflops = 8.0 * (double)per * npair;
-  const double fbytes = 8.0 * (double)per * npair * (FAR + 1);
-  if (ff) {
-    if ((rc = set_smem(c, (const void *)k_pair_diag<true>, sm3))) return rc;
-    DBSRG_RUN_W(c, "k_pair_diag", dbytes, dflops,
-                k_pair_diag<true><<<nv, 512, sm3, st>>>(
-                    ns, ks, kk, nb, ofirst, sym, eo, ed, cd->rkd, P1, P2, Dq, per));
-    DBSRG_RUN_W(c, "k_pair_direct_final", fbytes, fflops,
-                k_pair_direct_final<true><<<gf, 128, 0, st>>>(ns, ks, nv, kk, nb, icv, sym, eo,
-                                                              lo1, hi1, cd->hi2, SA,
-                                                              M2 ? SB : nullptr, Dq, K, per));
-  } else {
-    if ((rc = set_smem(c, (const void *)k_pair_diag<false>, sm3))) return rc;
-    DBSRG_RUN_W(c, "k_pair_diag", dbytes, dflops,
-                k_pair_diag<false><<<nv, 512, sm3, st>>>(
-                    ns, ks, kk, nb, ofirst, sym, eo, ed, cd->rkd, P1, P2, Dq, per));
-    DBSRG_RUN_W(c, "k_pair_direct_final", fbytes, fflops,
-                k_pair_direct_final<false><<<gf, 128, 0, st>>>(ns, ks, nv, kk, nb, icv, sym, eo,
-                                                               lo1, hi1, cd->hi2, SA,
-                                                               M2 ? SB : nullptr, Dq, K, per));
-  }
+  auto potentials = [&](auto ff_c, auto km_c) -> int {
+    constexpr bool F = decltype(ff_c)::value;
+    constexpr int KM = decltype(km_c)::value, PDW = pair_window(KM), PDR = pair_rows(KM);
+    using T = typename Val<F>::T;
+    DBSRG_RUN(c, "k_pair_scan",
+              k_pair_scan<F><<<dim3((unsigned)((np + PSP - 1) / PSP), M2 ? 2 : 1), PSP * PSW, 0, st>>>(
+                  nv, np, icv == 1, SA, SB));
+    PairDirArgs<F> d{};
+    d.ns = ns;
+    d.nv = nv;
+    d.kk = kk;
+    d.nb = nb;
+    d.np = np;
+    d.symab = symab;
+    d.suf = icv == 1;
+    d.dl0 = sym == 's' ? 0 : 1 - ks;
+    d.eo = eo;
+    d.ed = ed;
+    d.rkd = cd->rkd;
+    d.rpo = ofirst ? 1 : kk;
+    d.rpd = ofirst ? kk : 1;
+    d.L1 = icv == 1 ? cd->lo1 : cd->hi2;
+    d.L2 = M2 ? cd->hi1 : nullptr;
+    d.M1 = M1;
+    d.M2 = M2;
+    const T *rows = F ? (const T *)c->browsf : (const T *)c->brows;
+    d.P1 = rows + (size_t)(jp1 - 1) * nb * ns;
+    d.P2 = rows + (size_t)(jp2 - 1) * nb * ns;
+    d.SA = (const T *)SA;
+    d.SB = (const T *)SB;
+    d.K = (T *)K;
+    d.per = per;
+    const size_t smem = sizeof(T) * ((size_t)PDX * PDW * (PDW + PDB) + PDR * PDB +
+                                     (size_t)PDR * pair_row_stride(nb));
+    const int frc = set_smem(c, (const void *)k_pair_direct<F, KM>, smem);
+    if (frc) return frc;
+    // executed work: an output's n = k - |dl| cells hold r = n + k - 1 functions
+    // and a banded matrix of r^2 - n (n - 1) elements: as many multiply-adds per
+    // second orbital, r + 2 per pair; the potentials written
+    const int ncol = (int)(per / ns);
+    double fl = 0.0;
+    for (int col = 0; col < ncol; col++) {
+      const int dl = d.dl0 + col, n = std::min(eo.k1, eo.k2) - std::abs(dl);
+      if (n <= 0) continue;
+      const double r = n + ed.k1 - 1;
+      fl += 2.0 * ns * ((r * r - n * (n - 1.0)) * nb + (r + 2.0) * np);
+    }
+    const dim3 gd((unsigned)((ns + PDX - 1) / PDX), (unsigned)ncol,
+                  (unsigned)((nb + PDB - 1) / PDB));
+    DBSRG_RUN_W(c, "k_pair_direct", 8.0 * (double)per * npair, fl,
+                (k_pair_direct<F, KM><<<gd, PDT, smem, st>>>(d)));
+    return DBSRG_OK;
+  };
+  const std::integral_constant<int, FAR> k9;
+  const std::integral_constant<int, DBSRG_MAXK> kmax;
+  if (ks <= FAR)
+    rc = ff ? potentials(std::true_type(), k9) : potentials(std::false_type(), k9);
+  else
+    rc = ff ? potentials(std::true_type(), kmax) : potentials(std::false_type(), kmax);
+  if (rc) return rc;
   *out = K;
   return DBSRG_OK;
 }

@@ -52,3 +52,45 @@ __device__ __forceinline__ float2 norm(float sh, float sl) {
 }
 
 }  // namespace ffa
+
+// a sum and its terms in either arithmetic: float-float (FF) or FP64
+template <bool FF>
+struct Val;
+template <>
+struct Val<true> {
+  using T = float2;
+  float h = 0.0f, l = 0.0f;
+  __device__ void mac(float2 a, float2 b) { ffa::mac(a, b, h, l); }
+  __device__ void add_value(float2 o) { ffa::add(o, h, l); }
+  // the low sum back below half an ulp of the high one: its own rounding errors
+  // grow with its size, which is a random walk over the terms added
+  __device__ void renorm() {
+    const float2 v = ffa::norm(h, l);
+    h = v.x;
+    l = v.y;
+  }
+  __device__ float2 get() const { return ffa::norm(h, l); }
+  __device__ double value() const { return ffa::value(h, l); }
+  __device__ static float2 zero() { return make_float2(0.0f, 0.0f); }
+  __device__ static float2 of(double v) { return ffa::split(v); }
+  __device__ static double dbl(float2 v) { return ffa::value(v.x, v.y); }
+  __device__ static float2 mul(float2 a, float2 b) {
+    const float p = a.x * b.x;
+    const float e = fmaf(a.x, b.x, -p);
+    return ffa::norm(p, fmaf(a.x, b.y, fmaf(a.y, b.x, e)));
+  }
+};
+template <>
+struct Val<false> {
+  using T = double;
+  double v = 0.0;
+  __device__ void mac(double a, double b) { v = fma(a, b, v); }
+  __device__ void add_value(double o) { v += o; }
+  __device__ void renorm() {}
+  __device__ double get() const { return v; }
+  __device__ double value() const { return v; }
+  __device__ static double zero() { return 0.0; }
+  __device__ static double of(double x) { return x; }
+  __device__ static double dbl(double x) { return x; }
+  __device__ static double mul(double a, double b) { return a * b; }
+};

@@ -161,3 +161,27 @@ def test_backward_row_chunks_and_pair_lists(ns, norb, n):
     for e in (E, E0):
         assert abs(e - Er) <= 1e-12 * max(abs(Er), 1.0)
     assert np.abs(G - Gr).max() <= 1e-12 * np.abs(Gr).max()
+
+
+@pytest.mark.parametrize("ks,ksp,ksq,ns,norb", [(9, 8, 9, 41, 33), (9, 8, 9, 10, 2), (4, 3, 4, 19, 7),
+                                                (3, 2, 2, 7, 1), (11, 10, 11, 30, 4)])
+def test_pair_potentials_at_other_sizes(ks, ksp, ksq, ns, norb):
+    """The pair potentials' blocks: rows that four does not divide, odd numbers
+    of orbitals, more than one block of second orbitals, windows cut by both
+    ends of the grid, orders up to and above nine.  FP64 sums of at most a few
+    hundred terms: the 1e-12 of the other cases."""
+    rng = np.random.default_rng(100 * ks + ns)
+    t = synth.knots(ns, 1.0 if ns < 40 else 10.0, 7.0, ks)
+    orbitals = (synth.TARGET_ORBITALS * 2)[:norb]
+    pq = synth.orbital_coefficients(t, ks, ksp, ksq, 7.0, orbitals, rng)
+    n = 40
+    k = rng.integers(0, 3, n).astype(np.int32)
+    i1, i2, i3, i4 = (rng.integers(1, norb + 1, n).astype(np.int32) for _ in range(4))
+    coef = rng.uniform(-1.0, 1.0, n)
+    a = Assembler(t, ks, ksp, ksq)
+    a.set_orbitals(pq, np.zeros(norb, dtype=np.int32))
+    E, G = a.backward(k, i1, i2, i3, i4, coef)
+    a.close()
+    Er, Gr = O.Grid(t, ks, ksp, ksq).rk_energy_grad(k, i1, i2, i3, i4, coef, pq)
+    assert abs(E - Er) <= 1e-12 * max(abs(Er), 1.0)
+    assert np.abs(G - Gr).max() <= 1e-12 * np.abs(Gr).max()
