@@ -18,9 +18,34 @@
 
 namespace ffa {
 
+// Conversions between double and float-float in integer arithmetic: the 64-bit
+// conversion instructions run on the FP64 pipe at about two a clock and SM, and
+// a split takes three of its instructions, a sum of two floats three more.
+// hi: the bits rounded to 24 (ties away from zero); lo: what is left, a signed
+// integer of 29 bits, converted and scaled by v's power of two in two exact
+// steps.  Values outside the normal floats (but for zero) take the conversions.
 __device__ __forceinline__ float2 split(double v) {
-  const float h = __double2float_rn(v);
-  return make_float2(h, __double2float_rn(v - (double)h));
+  const unsigned hw = (unsigned)__double2hiint(v), lw = (unsigned)__double2loint(v);
+  const unsigned e = hw >> 20 & 0x7ffu, sign = hw & 0x80000000u;
+  if (e - 898u > 251u) {
+    if (((hw ^ sign) | lw) == 0) return make_float2(__uint_as_float(sign), 0.0f);
+    const float h = __double2float_rn(v);
+    return make_float2(h, __double2float_rn(v - (double)h));
+  }
+  const unsigned lr = lw + 0x10000000u, hr = hw + (lr < lw ? 1u : 0u);
+  // the exponent field's low nine bits above the 23 of the mantissa, 1023 - 127
+  // taken off modulo 512
+  const unsigned h = ((hr << 3 | lr >> 29) - 0xC0000000u) | sign;
+  const int rem = (int)(lr & 0x1fffffffu) - 0x10000000;
+  const float p2 = __uint_as_float((e - 896u) << 23 | sign);
+  return make_float2(__uint_as_float(h), (float)rem * 0x1p-52f * p2);
+}
+
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), a = b & 0x7fffffffu;
+  if (a - 0x00800000u >= 0x7f000000u && a != 0) return (double)f;
+  const unsigned h = a ? (a >> 3) + 0x38000000u : 0u;
+  return __hiloint2double((int)(h | (b & 0x80000000u)), (int)(b << 29));
 }
 
 __device__ __forceinline__ void mac(float2 c, float2 k, float &sh, float &sl) {
@@ -43,7 +68,7 @@ __device__ __forceinline__ void add(float2 v, float &sh, float &sl) {
   sl = sl + (e + v.y);
 }
 
-__device__ __forceinline__ double value(float sh, float sl) { return (double)sh + (double)sl; }
+__device__ __forceinline__ double value(float sh, float sl) { return widen(sh) + widen(sl); }
 
 // (hi, lo) renormalised so that lo is below half an ulp of hi (Fast2Sum)
 __device__ __forceinline__ float2 norm(float sh, float sl) {
