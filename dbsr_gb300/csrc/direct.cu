@@ -438,13 +438,13 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
         ca.ed[s * nm2 + m] = ed;
         ca.comp[s * nm2 + m] = s;
       }
-      // cell integrals: float-float copy (first pair fastest, no padding) or
-      // rkd; the first pair is the second electron's where tr
+      // cell integrals (float-float copy or FP64): first pair fastest; it is the
+      // second electron's where tr
       const int n1 = npairs(x.tr ? tb.e2 : tb.e1), n2 = npairs(x.tr ? tb.e1 : tb.e2);
       const bool ofirst = (j.icv == 1) != x.tr;
       p.R[o][t] = FF ? (const T *)x.rkf : (const T *)x.rkd;
-      p.rcell[o][t] = FF ? (size_t)n1 * n2 : (size_t)kk * kk;
-      const int r2 = FF ? n1 : kk;  // stride of the second pair
+      p.rcell[o][t] = (size_t)n1 * n2;
+      const int r2 = n1;  // stride of the second pair
       p.rpo[o][t] = ofirst ? 1 : r2;
       p.rpd[o][t] = ofirst ? r2 : 1;
       p.L1[o][t] = j.icv == 1 ? x.lo1 : x.hi2;

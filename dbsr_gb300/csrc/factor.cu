@@ -471,7 +471,8 @@ template <bool FF>
 struct PairDirArgs {
   int ns, nv, kk, nb, np, symab, suf, dl0;  // dl0: dl of column 0
   PairSpec eo, ed;
-  const double *rkd;
+  const double *rkd;  // element (po, pd; cell) at rpo po + rpd pd + rcell cell
+  size_t rcell;
   int rpo, rpd;
   const double *L1, *L2, *M1, *M2;
   const typename Val<FF>::T *P1, *P2, *SA, *SB;
@@ -565,7 +566,7 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
     for (int cv = ca; cv <= cb; cv++) {
       const int pd = pidx(ed, x - cv + 1, y - cv + 1);
       const size_t o = (size_t)pd + (size_t)p.kk * (cv - 1);
-      v += p.rkd[(size_t)p.kk * p.kk * (cv - 1) + (size_t)p.rpo * pos[fl][cv - lo] +
+      v += p.rkd[p.rcell * (cv - 1) + (size_t)p.rpo * pos[fl][cv - lo] +
                  (size_t)p.rpd * pd];
       v = fma(p.M1[o], c1[fl][cv - lo], v);
       if (p.M2) v = fma(p.M2[o], c2[fl][cv - lo], v);
@@ -1044,8 +1045,9 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
     d.eo = eo;
     d.ed = ed;
     d.rkd = cd->rkd;
-    d.rpo = ofirst ? 1 : kk;
-    d.rpd = ofirst ? kk : 1;
+    d.rcell = (size_t)npairs(eo) * npairs(ed);
+    d.rpo = ofirst ? 1 : npairs(ed);
+    d.rpd = ofirst ? npairs(eo) : 1;
     d.L1 = icv == 1 ? cd->lo1 : cd->hi2;
     d.L2 = M2 ? cd->hi1 : nullptr;
     d.M1 = M1;

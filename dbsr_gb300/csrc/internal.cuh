@@ -44,8 +44,8 @@ struct DeviceGrid {
 // electrons exchanged (tr: the second electron's pair is the first index).
 struct CellData {
   double *lo1 = nullptr, *hi1 = nullptr, *lo2 = nullptr, *hi2 = nullptr, *rkd = nullptr;
-  // rkd as float-float pairs without padding, rkf[(pair1 + np1 pair2) + cell np1 np2]
-  // (np1, np2 the numbers of pairs of the two electrons)
+  // rkd[(pair1 + np1 pair2) + cell np1 np2] (np1, np2 the numbers of pairs of the
+  // two indices) and the same as float-float pairs
   float2 *rkf = nullptr;
   bool tr = false;
 };

@@ -279,37 +279,48 @@ __global__ void k_triang_points(int nv, int ks, int ksp, int ksq, const double *
   for (int j = 0; j < ksq; j++) tb[2 * KS2 + (size_t)KS2 * ksp + (size_t)p * ksq + j] = v[j];
 }
 
-// up to three types per launch (blockIdx.y)
+// up to three types per launch (blockIdx.y); out: element (pair 1, pair 2; cell)
+// at p1 + ld p2 + cell size, no padding where ld is 0 (float-float copy: never
+// padded)
 struct TriSet {
   int type[3];
   double *rkd[3];
   float2 *rkf[3];
 };
 
-__global__ void k_triang(int nv, int ks, int ksp, int ksq, const TriSet ts, int k,
-                         const double *tri, const double *grm, const double *grw,
-                         const double *pbsp, const double *qbsp) {
+// One block per interval and type.  INT (inner integrals) and OB (outer weight
+// times two functions) are arrays [pair][outer point] of the type's pairs, of
+// odd stride so that a warp's pairs fall on different banks; an element of the
+// result is a dot product (types 2 and 3: two) over the outer points.  Bound by
+// the FP64 pipe once the integer work per element is small and no padding is
+// written: ns 400, R^k (three types) and S^k launches 98 us in the mean with the
+// functions' square for INT, the pair's two functions searched for at every
+// element and ks^2 x ks^2 results; 69 us here (ns 283: 59 and 50).
+__global__ void __launch_bounds__(256) k_triang(int nv, int ks, int ksp, int ksq, const TriSet ts,
+                                                int ld, int k, const double *tri,
+                                                const double *grm, const double *grw,
+                                                const double *pbsp, const double *qbsp) {
   extern __shared__ double sm[];
   const int iv = blockIdx.x;  // 0-based interval
   const int type = ts.type[blockIdx.y];
-  double *rkd = ts.rkd[blockIdx.y];
   float2 *rkf = ts.rkf[blockIdx.y];
-  const int nq = ks * ks * ks * ks;
-  const int nw = nv + 1, kk = ks * ks;
-  const int KS2 = ks * ks;
+  const int nw = nv + 1, KS2 = ks * ks, kr = ks | 1;
+  const int ikp = ksp * (ksp + 1) / 2, ikq = ksq * (ksq + 1) / 2, npq = ksp * ksq;
+  const bool needP = type != 1, needQ = type != 0;
+  // the pairs of the two arrays: 1 for the first family, 2 for the second (types
+  // 2 and 3: P and Q)
+  const int m1 = type == 1 ? ikq : (type >= 4 ? npq : ikp), m2 = type == 2 || type == 3 ? ikq : 0;
   const double *tb = tri + (size_t)iv * KS2 * (2 + ksp + ksq);  // x | w | BP | BQ
   double *wk = sm;                 // (m,i) inner weight * r^k       [ks*ks]
   double *BP = wk + KS2;           // (m,i,j) P values at inner pts  [ks*ks*ksp]
   double *BQ = BP + KS2 * ksp;     // (m,i,j) Q values               [ks*ks*ksq]
-  double *INTP = BQ + KS2 * ksq;   // (j,jp,m) over P x P            [ksp*ksp*ks]
-  double *INTQ = INTP + ksp * ksp * ks;  // Q x Q                    [ksq*ksq*ks]
-  double *INTPQ = INTQ + ksq * ksq * ks; // P x Q                    [ksp*ksq*ks]
-  double *gxo = INTPQ + ksp * ksq * ks;  // outer weights            [ks]
-  double *A = gxo + ks;                  // a(ii,jj) for pppp/qqqq   [kk*kk]
-  // outer products b1(m,i) b2(m,ip) gxo(m) per pair and outer point, formed
-  // once per interval: OB1 for the first pair family, OB2 for the second
-  double *OB1 = A + kk * kk;             //                          [kk*ks]
-  double *OB2 = OB1 + kk * ks;           //                          [kk*ks]
+  double *gxo = BQ + KS2 * ksq;    // outer weights                  [ks]
+  double *INT1 = gxo + ks;         //                                [m1][kr]
+  double *OB1 = INT1 + m1 * kr;    //                                [m1][kr]
+  double *INT2 = OB1 + m1 * kr;    //                                [m2][kr]
+  double *OB2 = INT2 + m2 * kr;    //                                [m2][kr]
+  double *A = OB2 + m2 * kr;       // weighted functions, then types 0/1: a(ii,jj)
+  __shared__ unsigned char fn[2][2][DBSRG_MAXK * (DBSRG_MAXK + 1) / 2];  // pairs' functions
 
   // phase 1: inner points, weights and B-spline values (k_triang_points)
   for (int q = threadIdx.x; q < KS2; q += blockDim.x)
@@ -318,128 +329,102 @@ __global__ void k_triang(int nv, int ks, int ksp, int ksq, const TriSet ts, int 
     BP[q] = tb[2 * KS2 + q];  // BQ follows BP in both layouts
   for (int m = threadIdx.x; m < ks; m += blockDim.x)
     gxo[m] = __dmul_rn(grw[IDX2(iv, m, nv)], ipow_d(grm[IDX2(iv, m, nv)], k + 1));
-  __syncthreads();
-  // phase 2: INT(j,jp,m) = sum_i (wk*Ba_j)*Bb_jp
-  // (the weighted first factors wk*Ba are formed once per call in A, which
-  // phase 3 fills only after the last call)
-  auto inner = [&](const double *Ba, int ka, const double *Bb, int kb, double *INT) {
-    double *WB = A;
-    for (int q = threadIdx.x; q < KS2 * ka; q += blockDim.x) WB[q] = __dmul_rn(wk[q / ka], Ba[q]);
-    __syncthreads();
-    for (int q = threadIdx.x; q < ka * kb * ks; q += blockDim.x) {
-      int j = q % ka, jp = (q / ka) % kb, m = q / (ka * kb);
-      double s = 0.0;
-      for (int i = 0; i < ks; i++) {
-        int p = m * ks + i;
-        s = fma(WB[(size_t)p * ka + j], Bb[(size_t)p * kb + jp], s);
-      }
-      INT[j + ka * (jp + kb * m)] = s;
-    }
-    __syncthreads();
-  };
-  if (type == 0) inner(BP, ksp, BP, ksp, INTP);
-  if (type == 1) inner(BQ, ksq, BQ, ksq, INTQ);
-  if (type == 2 || type == 3) {
-    inner(BP, ksp, BP, ksp, INTP);
-    inner(BQ, ksq, BQ, ksq, INTQ);
-  }
-  if (type == 4 || type == 5) inner(BP, ksp, BQ, ksq, INTPQ);
-  __syncthreads();
-
-  double *out = rkd + (size_t)kk * kk * iv;
-  auto ob = [&](const double *b1, int i, const double *b2, int ip, int m) -> double {
-    return __dmul_rn(__dmul_rn(b1[IDX3(iv, m, i, nw, ks)], b2[IDX3(iv, m, ip, nw, ks)]), gxo[m]);
-  };
-  auto pair_of = [](int ii, int kx, int *i, int *ip) {
-    int r = ii, row = 0;
+  for (int q = threadIdx.x; q < ikp + ikq; q += blockDim.x) {
+    const int w = q >= ikp, kx = w ? ksq : ksp;
+    int r = w ? q - ikp : q, row = 0;
+    const int at = r;
     while (r >= kx - row) {
       r -= kx - row;
       row++;
     }
-    *i = row;
-    *ip = row + r;
-  };
-  // triangular pairs (i <= ip) of one basis: OB[ii*ks + m]
-  auto fill_tri = [&](const double *bs, int kx, double *OB) {
-    const int ik = kx * (kx + 1) / 2;
-    for (int q = threadIdx.x; q < ik * ks; q += blockDim.x) {
-      const int ii = q / ks, m = q % ks;
-      int i, ip;
-      pair_of(ii, kx, &i, &ip);
-      OB[q] = ob(bs, i, bs, ip, m);
-    }
-  };
-  if (type == 0) fill_tri(pbsp, ksp, OB1);
-  if (type == 1) fill_tri(qbsp, ksq, OB1);
-  if (type == 2 || type == 3) {
-    fill_tri(pbsp, ksp, OB1);
-    fill_tri(qbsp, ksq, OB2);
-  }
-  if (type == 4 || type == 5) {  // outer (P,Q) pairs ii = i*ksq + ip, or (Q,P) ii = i*ksp + ip
-    const int np = ksp * ksq;
-    for (int q = threadIdx.x; q < np * ks; q += blockDim.x) {
-      const int ii = q / ks, m = q % ks;
-      OB1[q] = type == 4 ? ob(pbsp, ii / ksq, qbsp, ii % ksq, m)
-                         : ob(qbsp, ii / ksp, pbsp, ii % ksp, m);
-    }
+    fn[w][0][at] = (unsigned char)row;
+    fn[w][1][at] = (unsigned char)(row + r);
   }
   __syncthreads();
-  if (type == 0 || type == 1) {
-    const int kx = type == 0 ? ksp : ksq;
-    const double *INT = type == 0 ? INTP : INTQ;
-    const int ik = kx * (kx + 1) / 2;
-    for (int q = threadIdx.x; q < ik * ik; q += blockDim.x) {
-      int ii = q % ik, jj = q / ik;
-      int j, jp;
-      pair_of(jj, kx, &j, &jp);
-      const double *o = OB1 + ii * ks;
+  // phase 2: INT(pair, m) = sum_i (wk*Ba_j)*Bb_jp
+  // (the weighted first factors wk*Ba are formed once per call in A, which
+  // phase 3 fills only after the last call); w: packed symmetric pairs of P (0)
+  // or Q (1), 2: (P, Q) pairs
+  auto inner = [&](const double *Ba, int ka, const double *Bb, int kb, int w, int np,
+                   double *INT) {
+    double *WB = A;
+    for (int q = threadIdx.x; q < KS2 * ka; q += blockDim.x) WB[q] = __dmul_rn(wk[q / ka], Ba[q]);
+    __syncthreads();
+    for (int q = threadIdx.x; q < np * ks; q += blockDim.x) {
+      const int pr = q / ks, m = q - pr * ks;
+      const int j = w < 2 ? fn[w][0][pr] : pr / kb, jp = w < 2 ? fn[w][1][pr] : pr % kb;
+      const double *a = WB + (size_t)m * ks * ka + j, *b = Bb + (size_t)m * ks * kb + jp;
       double s = 0.0;
-      for (int m = 0; m < ks; m++) s = fma(o[m], INT[j + kx * (jp + kx * m)], s);
+      for (int i = 0; i < ks; i++) s = fma(a[i * ka], b[i * kb], s);
+      INT[pr * kr + m] = s;
+    }
+    __syncthreads();
+  };
+  if (type >= 4) {
+    inner(BP, ksp, BQ, ksq, 2, npq, INT1);
+  } else {
+    if (needP) inner(BP, ksp, BP, ksp, 0, ikp, INT1);
+    if (needQ) inner(BQ, ksq, BQ, ksq, 1, ikq, type == 1 ? INT1 : INT2);
+  }
+  // outer products b1(m,i) b2(m,ip) gxo(m) per pair and outer point
+  auto ob = [&](const double *b1, int i, const double *b2, int ip, int m) -> double {
+    return __dmul_rn(__dmul_rn(b1[IDX3(iv, m, i, nw, ks)], b2[IDX3(iv, m, ip, nw, ks)]), gxo[m]);
+  };
+  auto outer = [&](int w, int np, double *OB) {
+    const double *bs = w ? qbsp : pbsp;
+    for (int q = threadIdx.x; q < np * ks; q += blockDim.x) {
+      const int pr = q / ks, m = q - pr * ks;
+      OB[pr * kr + m] = ob(bs, fn[w][0][pr], bs, fn[w][1][pr], m);
+    }
+  };
+  if (type >= 4) {  // outer (P,Q) pairs ii = i*ksq + ip, or (Q,P) ii = i*ksp + ip
+    for (int q = threadIdx.x; q < npq * ks; q += blockDim.x) {
+      const int ii = q / ks, m = q - ii * ks;
+      OB1[ii * kr + m] = type == 4 ? ob(pbsp, ii / ksq, qbsp, ii % ksq, m)
+                                   : ob(qbsp, ii / ksp, pbsp, ii % ksp, m);
+    }
+  } else {
+    if (needP) outer(0, ikp, OB1);
+    if (needQ) outer(1, ikq, type == 1 ? OB1 : OB2);
+  }
+  __syncthreads();
+  // element (r, cc) of the result, n1 x n2
+  const int n1 = type == 3 ? ikq : m1, n2 = type == 2 ? ikq : m1;
+  const int l2 = ld ? ld : n1;
+  double *out = ts.rkd[blockIdx.y] + (size_t)(ld ? ld * ld : n1 * n2) * iv;
+  if (rkf) rkf += (size_t)n1 * n2 * iv;
+  if (type < 2) {
+    for (int q = threadIdx.x; q < n1 * n1; q += blockDim.x) {
+      const int jj = q / n1, ii = q - jj * n1;
+      const double *o = OB1 + ii * kr, *t = INT1 + jj * kr;
+      double s = 0.0;
+      for (int m = 0; m < ks; m++) s = fma(o[m], t[m], s);
       A[q] = s;
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-      int ii = q % kk, jj = q / kk;
-      const bool ok = ii < ik && jj < ik;
-      const double v = ok ? __dadd_rn(A[ii + ik * jj], A[jj + ik * ii]) : 0.0;
-      out[q] = v;
-      if (rkf && ok) rkf[(size_t)iv * ik * ik + ii + (size_t)ik * jj] = ffa::split(v);
-    }
-  } else if (type == 2 || type == 3) {
-    const int ikp = ksp * (ksp + 1) / 2, ikq = ksq * (ksq + 1) / 2;
-    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-      int r = q % kk, cc = q / kk;
-      int pp_ = type == 2 ? r : cc, qq_ = type == 2 ? cc : r;  // P pair, Q pair
-      double v = 0.0;
-      if (pp_ < ikp && qq_ < ikq) {
-        int i, ip, j, jp;
-        pair_of(pp_, ksp, &i, &ip);
-        pair_of(qq_, ksq, &j, &jp);
-        const double *o1 = OB1 + pp_ * ks, *o2 = OB2 + qq_ * ks;
-        double s1 = 0.0, s2 = 0.0;
-        for (int m = 0; m < ks; m++) s1 = fma(o1[m], INTQ[j + ksq * (jp + ksq * m)], s1);
-        for (int m = 0; m < ks; m++) s2 = fma(o2[m], INTP[i + ksp * (ip + ksp * m)], s2);
-        v = __dadd_rn(s1, s2);
-        const int n1 = type == 2 ? ikp : ikq;  // pairs of the first electron
-        if (rkf) rkf[(size_t)iv * ikp * ikq + r + (size_t)n1 * cc] = ffa::split(v);
+  }
+  for (int q = threadIdx.x; q < n1 * n2; q += blockDim.x) {
+    const int cc = q / n1, r = q - cc * n1;
+    double v;
+    if (type < 2) {
+      v = __dadd_rn(A[q], A[cc + n1 * r]);
+    } else if (type < 4) {
+      const int pp = type == 2 ? r : cc, qq = type == 2 ? cc : r;  // P pair, Q pair
+      const double *o1 = OB1 + pp * kr, *t2 = INT2 + qq * kr;
+      const double *o2 = OB2 + qq * kr, *t1 = INT1 + pp * kr;
+      double s1 = 0.0, s2 = 0.0;
+      for (int m = 0; m < ks; m++) {
+        s1 = fma(o1[m], t2[m], s1);
+        s2 = fma(o2[m], t1[m], s2);
       }
-      out[q] = v;
+      v = __dadd_rn(s1, s2);
+    } else {  // rkd(jj,ii): jj inner (P,Q), ii outer
+      const double *o = OB1 + cc * kr, *t = INT1 + r * kr;
+      v = 0.0;
+      for (int m = 0; m < ks; m++) v = fma(o[m], t[m], v);
     }
-  } else {
-    const int np = ksp * ksq;
-    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-      int jj = q % kk, ii = q / kk;  // rkd(jj,ii): jj inner (P,Q), ii outer
-      double v = 0.0;
-      if (jj < np && ii < np) {
-        int j = jj / ksq, jp = jj % ksq;
-        const double *o = OB1 + ii * ks;
-        double s = 0.0;
-        for (int m = 0; m < ks; m++) s = fma(o[m], INTPQ[j + ksp * (jp + ksq * m)], s);
-        v = s;
-        if (rkf) rkf[(size_t)iv * np * np + jj + (size_t)np * ii] = ffa::split(v);
-      }
-      out[q] = v;
-    }
+    out[r + (size_t)l2 * cc] = v;
+    if (rkf) rkf[q] = ffa::split(v);
   }
 }
 
@@ -455,28 +440,34 @@ static int build_triang_points(dbsrg_ctx *c) {
   return DBSRG_OK;
 }
 
-// n (1..3) types in one launch
-static int compute_diag_set(dbsrg_ctx *c, int n, const TriSet &ts, int k) {
+// n (1..3) types in one launch; ld: as in TriSet
+static int compute_diag_set(dbsrg_ctx *c, int n, const TriSet &ts, int k, int ld = 0) {
   const DeviceGrid &g = c->g;
-  const int ks = g.ks, kk = ks * ks;
-  size_t nsm = (size_t)ks * ks + (size_t)ks * ks * g.ksp + (size_t)ks * ks * g.ksq +
-               (size_t)g.ksp * g.ksp * ks + (size_t)g.ksq * g.ksq * ks +
-               (size_t)g.ksp * g.ksq * ks + ks + (size_t)kk * kk + 2 * (size_t)kk * ks;
-  size_t bytes = nsm * sizeof(double);
+  const size_t ks = g.ks, kr = ks | 1, ikp = g.ksp * (g.ksp + 1) / 2,
+               ikq = g.ksq * (g.ksq + 1) / 2, kmax = std::max(g.ksp, g.ksq);
+  // the largest type's arrays (k_triang): pairs of both families or the (P,Q)
+  // pairs; weighted functions or the square of the larger family's pairs
+  const size_t pairs = std::max(ikp + ikq, (size_t)g.ksp * g.ksq);
+  const size_t am = std::max(std::max(ikp * ikp, ikq * ikq), ks * ks * kmax);
+  const size_t bytes =
+      sizeof(double) * (ks * ks * (1 + g.ksp + g.ksq) + ks + 2 * pairs * kr + am);
   int rc = raise_smem_limit(c, (const void *)k_triang, bytes);
   if (rc) return rc;
   DBSRG_RUN(c, "k_triang",
-            k_triang<<<dim3(g.nv, n), 256, bytes, c->stream>>>(g.nv, ks, g.ksp, g.ksq, ts, k,
+            k_triang<<<dim3(g.nv, n), 256, bytes, c->stream>>>(g.nv, g.ks, g.ksp, g.ksq, ts, ld, k,
                                                                g.tri, g.grm, g.grw, g.pbsp,
                                                                g.qbsp));
   return DBSRG_OK;
 }
 
+// one type's cells as ks^2 x ks^2 arrays, zeros past the pairs
 int compute_diag_cells(dbsrg_ctx *c, int type, int k, double *rkd) {
+  const int kk = c->g.ks * c->g.ks;
   TriSet ts{};
   ts.type[0] = type;
   ts.rkd[0] = rkd;
-  return compute_diag_set(c, 1, ts, k);
+  DBSRG_TRY(c, cudaMemsetAsync(rkd, 0, sizeof(double) * kk * kk * c->g.nv, c->stream));
+  return compute_diag_set(c, 1, ts, k, kk);
 }
 
 // ----------------------------------------------------------------------------
@@ -537,6 +528,8 @@ __global__ void k_fill_r(int ns, int ks, int nv, const FillSet fs, int band) {
     // B-spline products are positive), suffix sums with iv descending and
     // prefix sums with iv ascending, so every element keeps full relative
     // precision with O(ka + kb) operations instead of O(ka kb).
+    const int na = ka * (ka + 1) / 2, nbp = kb * (kb + 1) / 2;
+    const size_t n1 = tr ? nbp : na, n2 = tr ? na : nbp;  // pairs of rkd's two indices
     double suf = 0.0;
     for (int jv = jvhi; jv >= max(jvlo, ivhi + 1); jv--) suf += highB[jb(jv)];
     for (int iv = ivhi; iv >= ivlo; iv--) {
@@ -551,7 +544,7 @@ __global__ void k_fill_r(int ns, int ks, int nv, const FillSet fs, int band) {
         const int ih = i - iv + 1, jh = j - iv + 1;
         const int ii = tri_index(ih, ih + ip - 1, ka), jj = tri_index(jh, jh + jp - 1, kb);
         const int r1 = tr ? jj : ii, r2 = tr ? ii : jj;
-        acc += rkd[(r1 - 1) + (size_t)kk * ((r2 - 1) + (size_t)kk * (iv - 1))];
+        acc += rkd[(r1 - 1) + n1 * ((r2 - 1) + n2 * (iv - 1))];
         pre += lowB[jb(iv)];
       }
     }
@@ -597,12 +590,13 @@ __global__ void k_fill_s(int ns, int ks, int nv, int ksp, int ksq, int kj1, int 
   };
   // cells iv < jv: r1(iv) times the suffix sum of r2 over jv > iv (positive
   // moments, additions only, iv descending); the diagonal cells iv = jv
+  const size_t npq = (size_t)ksp * ksq;  // pairs of either electron
   double suf = 0.0;
   for (int jv = jvhi; jv >= max(jvlo, ivhi + 1); jv--) suf += r2[jb(jv) + (size_t)kk * (jv - 1)];
   for (int iv = ivhi; iv >= ivlo; iv--) {
     acc = fma(r1[ia(iv) + (size_t)kk * (iv - 1)], suf, acc);
     if (iv >= jvlo && iv <= jvhi) {
-      acc += rkd[ia(iv) + (size_t)kk * (jb(iv) + (size_t)kk * (iv - 1))];
+      acc += rkd[ia(iv) + npq * (jb(iv) + npq * (iv - 1))];
       suf += r2[jb(iv) + (size_t)kk * (iv - 1)];
     }
   }
@@ -623,7 +617,7 @@ static int ensure_slot(dbsrg_ctx *c, std::vector<double *> &v, size_t idx) {
 int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out) {
   const DeviceGrid &g = c->g;
   const int nv = g.nv, kk = g.ks * g.ks;
-  const size_t m = (size_t)kk * nv, d = (size_t)kk * kk * nv;
+  const size_t m = (size_t)kk * nv;
   int rc;
   if (family == 0) {
     if ((rc = ensure_r_cells(c, k))) return rc;
@@ -640,13 +634,13 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
   const TableBases tb = table_bases(g, family, type);
   const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
   double *base = nullptr;
-  if (!(base = (double *)cache_alloc(c, (2 * m + d + f) * sizeof(double))))
+  if (!(base = (double *)cache_alloc(c, (2 * m + 2 * f) * sizeof(double))))
     return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
   CellData cd;
   cd.lo1 = base;
   cd.hi2 = base + m;
   cd.rkd = base + 2 * m;
-  cd.rkf = (float2 *)(cd.rkd + d);
+  cd.rkf = (float2 *)(cd.rkd + f);
   const int wh[2] = {2, type == 0 ? 2 : 3}, kp[2] = {k, -(k + 1)};
   double *const mo[2] = {cd.lo1, cd.hi2};
   if ((rc = compute_moment_set(c, 2, wh, kp, mo))) return rc;
@@ -669,7 +663,7 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
 int ensure_r_cells(dbsrg_ctx *c, int k) {
   const DeviceGrid &g = c->g;
   const int nv = g.nv, kk = g.ks * g.ks;
-  const size_t m = (size_t)kk * nv, d = (size_t)kk * kk * nv;
+  const size_t m = (size_t)kk * nv;
   if ((int)c->rshare.size() <= k) c->rshare.resize(k + 1);
   if (c->rcell.size() < (size_t)(k + 1) * 4) c->rcell.resize((size_t)(k + 1) * 4);
   RCells &r = c->rshare[k];
@@ -684,11 +678,11 @@ int ensure_r_cells(dbsrg_ctx *c, int k) {
   for (int t = 0; t < 3; t++) {
     const TableBases tb = table_bases(g, 0, t);
     const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
-    if (!r.diag[t] && !(r.diag[t] = (double *)cache_alloc(c, (d + f) * sizeof(double))))
+    if (!r.diag[t] && !(r.diag[t] = (double *)cache_alloc(c, 2 * f * sizeof(double))))
       return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
     ts.type[t] = t;
     ts.rkd[t] = r.diag[t];
-    ts.rkf[t] = (float2 *)(r.diag[t] + d);
+    ts.rkf[t] = (float2 *)(r.diag[t] + f);
   }
   if ((rc = compute_diag_set(c, 3, ts, k))) return rc;
   for (int t = 0; t < 4; t++) {
@@ -699,7 +693,8 @@ int ensure_r_cells(dbsrg_ctx *c, int k) {
     cd.lo2 = r.mom + 2 * wb * m;
     cd.hi2 = cd.lo2 + m;
     cd.rkd = r.diag[std::min(t, 2)];
-    cd.rkf = (float2 *)(cd.rkd + d);
+    const TableBases tb = table_bases(g, 0, t);
+    cd.rkf = (float2 *)(cd.rkd + (size_t)npairs(tb.e1) * npairs(tb.e2) * nv);
     cd.tr = t == 3;
     c->rcell[(size_t)k * 4 + t] = cd;
   }
