@@ -49,6 +49,8 @@ constexpr int FAR = 9;            // |y - x| >= FAR is far field (spline orders 
 constexpr int BAND = FAR - 1;     // near band |y - x| <= 8
 constexpr int NDB = 2 * BAND + 1; // band diagonals
 constexpr int PXC = 4;            // output rows per block of the band pair potentials
+constexpr int PDB = 32;           // second orbitals per block of the pair potentials
+constexpr int PDT = 256;          // their threads
 
 // target quadrants of the atypes of one list (UPDATE_HS)
 struct QuadSpec {
@@ -207,6 +209,10 @@ __global__ void __launch_bounds__(256) k_far_field(int ns, int nb, const double 
   }
 }
 
+__host__ __device__ inline int pair_row_stride(int n) {  // 8 mod 16: rows on other banks
+  return (n + 7) / 16 * 16 + 8;
+}
+
 // ---------------------------------------------------------------------------
 // band pair potentials of an exchange table, one block per PXC output rows
 // and one band diagonal d = y - x:
@@ -218,56 +224,79 @@ __global__ void __launch_bounds__(256) k_far_field(int ns, int nb, const double 
 //   Kb(ab; x, y) = sum_i P1(a, i) H(x; i, b)
 // mode 0: R table 's','s' case 3; 1: S 'n','n' case 3; 2: S 'n','n' case 4.
 // Band table layout: rkb(i, j-i+BW+1, ip, jp) for |j - i| <= BW.
-// FF: the windows split once into float-float pairs, both stages as
+// FF: the table elements split into float-float pairs, both stages as
 // float-float sums (ff.cuh), Kb written as float-float pairs (float2).
 // Kx: where the results of the table with the electrons exchanged go, element
 // (b a; y, x - y) for (a b; x, y - x).  R^k types 0 and 1 are unchanged under
 // the exchange (Kx = Kout): only the diagonals d >= 0 are computed.  Type 2
 // gives type 3's potentials this way (Kx theirs); S^k has none (Kx null).
-// ns 400, 20 orbitals: an R^k list's potentials 4 x 84 us, 3 launches now.
+// Positions past the ends of the grid are set to zero.
+//
+// PXC rows are a full sector of the results and of the table's rows; a block
+// takes PDB second orbitals, a thread two of them at once, so that a value read
+// from shared memory meets two sums.  Bound by the twelve FP32 instructions of a
+// float-float multiply-add, otherwise by the FP64 pipe.  ns 283, 20 orbitals:
+// 63 us a list in the mean over R^k and S^k; 86 us with one sum a thread (two
+// loads a multiply-add), FP64 windows split by every block and a launch per
+// table, and launches before to clear the results.
+// The three tables of an R^k list are one launch (blockIdx.y: table and d), so
+// that short grids fill the SMs too.
 template <bool FF>
-__global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int mode,
-                                                   const double *__restrict__ rkb,
-                                                   const double *__restrict__ P1,
-                                                   const double *__restrict__ P2, void *Kout,
-                                                   void *Kx) {
-  using S = typename std::conditional<FF, float2, double>::type;
-  extern __shared__ double smraw[];
-  S *sm = reinterpret_cast<S *>(smraw);
-  const int W = 2 * ks - 1;            // offsets -(ks-1) .. ks-1
-  const int WL = PXC + W - 1;          // window of the row vectors
-  const int WLP = WL | 1;              // its stride (odd: no bank conflicts across orbitals)
-  const int HX = W * nb + 1;           // stride of H per output row (odd)
-  const int x0 = blockIdx.x * PXC + 1; // first output row (1-based)
-  const int d = Kx == Kout ? (int)blockIdx.y : (int)blockIdx.y - BAND;
-  S *Wm = sm;                          // [PXC][W][W]
-  S *p1w = Wm + PXC * W * W;           // [nb][WLP]: P1(a, x0-(ks-1)+t)
-  S *p2w = p1w + nb * WLP;             // [nb][WLP]: P2(b, x0+d-(ks-1)+t)
-  S *H = p2w + nb * WLP;               // [PXC][HX]: H(xl; u, b) at u*nb + b
-  auto sv = [](double v) -> S {
-    if constexpr (FF) return ffa::split(v); else return v;
+struct PairBandArgs {
+  int ns, ks, nb, mode, bw;  // bw: stride of the second orbitals' arrays
+  int y0[4];                 // first blockIdx.y of each table, and their end
+  const double *rkb[3];
+  const typename Val<FF>::T *P1[3], *P2[3];
+  typename Val<FF>::T *Kout[3], *Kx[3];
+};
+constexpr int PBW = 2 * FAR - 1;         // window of one output, at most
+constexpr int PBR = PXC - 1 + PBW;       // rows of a block's windows
+
+template <bool FF>
+__global__ void __launch_bounds__(PDT) k_pair_band(const PairBandArgs<FF> p) {
+  using V = Val<FF>;
+  using T = typename V::T;
+  struct alignas(16) T2 {
+    T a, b;
   };
-  const int kb = mode == 0 ? ks : 2 * ks - 1;
+  extern __shared__ __align__(16) unsigned char smband[];
+  T *Wm = reinterpret_cast<T *>(smband);  // [PXC][PBW][PBW]: (i, j) at (i-x+ks-1, j-y+ks-1)
+  const int bw = p.bw;
+  T *H = Wm + PXC * PBW * PBW;            // [PXC][PBW][bw]
+  T *p2w = H + PXC * PBW * bw;            // [PBR][bw]: P2(b, x0+d-(ks-1)+row)
+  T *p1w = p2w + PBR * bw;                // [PBR][pstr]: P1(a, x0-(ks-1)+row)
+  const int ns = p.ns, ks = p.ks, nb = p.nb, pstr = pair_row_stride(nb);
+  const int W = 2 * ks - 1;               // offsets -(ks-1) .. ks-1
+  const int x0 = blockIdx.x * PXC + 1;    // first output row (1-based)
+  const int ty = ((int)blockIdx.y >= p.y0[1]) + ((int)blockIdx.y >= p.y0[2]);
+  T *Kout = p.Kout[ty], *Kx = p.Kx[ty];
+  const int d = (int)blockIdx.y - p.y0[ty] - (Kx == Kout ? 0 : BAND);
+  const double *rkb = p.rkb[ty];
+  const int zb = blockIdx.z * PDB, bc = min(PDB, nb - zb), ng = (bc + 1) / 2;
+  const int kb = p.mode == 0 ? ks : W;
   constexpr int BW = DBSRG_TABLE_BAND, NJ = 2 * DBSRG_TABLE_BAND + 1;
-  auto TB = [&](int i, int j, int ip, int jp) -> double {
-    return rkb[(size_t)(i - 1) + (size_t)ns * ((size_t)(j - i + BW) +
-               (size_t)NJ * ((size_t)(ip - 1) + (size_t)kb * (size_t)(jp - 1)))];
+  auto TB = [&](int i, int j, int ip, int jp) -> T {
+    return V::of(rkb[(size_t)(i - 1) + (size_t)ns * ((size_t)(j - i + BW) +
+               (size_t)NJ * ((size_t)(ip - 1) + (size_t)kb * (size_t)(jp - 1)))]);
   };
-  for (int q = threadIdx.x; q < PXC * W * W; q += blockDim.x) Wm[q] = sv(0.0);
-  for (int q = threadIdx.x; q < nb * WL; q += blockDim.x) {
-    const int a = q / WL, t = q % WL;
-    const int xi = x0 - (ks - 1) + t, yi = x0 + d - (ks - 1) + t;
-    p1w[a * WLP + t] = sv((xi >= 1 && xi <= ns) ? P1[(size_t)a * ns + xi - 1] : 0.0);
-    p2w[a * WLP + t] = sv((yi >= 1 && yi <= ns) ? P2[(size_t)a * ns + yi - 1] : 0.0);
+  for (int q = threadIdx.x; q < PXC * PBW * PBW; q += PDT) Wm[q] = V::zero();
+  for (int q = threadIdx.x; q < PBR * nb; q += PDT) {
+    const int a = q / PBR, r = q - a * PBR, x = x0 - (ks - 1) + r;
+    p1w[r * pstr + a] = x >= 1 && x <= ns ? p.P1[ty][(size_t)a * ns + x - 1] : V::zero();
+  }
+  for (int q = threadIdx.x; q < PBR * bw; q += PDT) {
+    const int b = q / PBR, r = q - b * PBR, y = x0 + d - (ks - 1) + r;
+    p2w[r * bw + b] =
+        b < bc && y >= 1 && y <= ns ? p.P2[ty][(size_t)(zb + b) * ns + y - 1] : V::zero();
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < PXC * kb * kb; q += blockDim.x) {
-    const int xl = q / (kb * kb), r = q % (kb * kb), ip = r % kb + 1, jp = r / kb + 1;
+  for (int q = threadIdx.x; q < PXC * kb * kb; q += PDT) {
+    const int xl = q % PXC, r = q / PXC, ip = r % kb + 1, jp = r / kb + 1;
     const int x = x0 + xl, y = x + d;
     if (x > ns || y < 1 || y > ns) continue;
-    S *w = Wm + (size_t)xl * W * W;
-    auto put = [&](int i, int j, double v) { w[(i - x + ks - 1) * W + (j - y + ks - 1)] = sv(v); };
-    if (mode == 0) {
+    T *w = Wm + (size_t)xl * PBW * PBW;
+    auto put = [&](int i, int j, T v) { w[(i - x + ks - 1) * PBW + (j - y + ks - 1)] = v; };
+    if (p.mode == 0) {
       if (y - jp + 1 >= 1 && x + ip - 1 <= ns)
         put(x + ip - 1, y - jp + 1, TB(x, y - jp + 1, ip, jp));
       if (ip > 1 && x - ip + 1 >= 1 && y - jp + 1 >= 1)
@@ -276,7 +305,7 @@ __global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int m
         put(x + ip - 1, y + jp - 1, TB(x, y, ip, jp));
       if (ip > 1 && jp > 1 && x - ip + 1 >= 1 && y + jp - 1 <= ns)
         put(x - ip + 1, y + jp - 1, TB(x - ip + 1, y, ip, jp));
-    } else if (mode == 1) {
+    } else if (p.mode == 1) {
       const int j = y - jp + ks, ii = x + ip - ks;
       if (j < max(1, 1 + ks - jp) || j > min(ns, ns + ks - jp)) continue;
       if (x < max(1, 1 + ks - ip) || x > min(ns, ns + ks - ip)) continue;
@@ -289,44 +318,49 @@ __global__ void __launch_bounds__(256) k_pair_band(int ns, int ks, int nb, int m
     }
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < PXC * W * nb; q += blockDim.x) {
-    const int b = q % nb, r = q / nb, u = r % W, xl = r / W;
-    const S *w = Wm + ((size_t)xl * W + u) * W;
-    const S *p = p2w + (size_t)b * WLP + xl;
-    S *hq = H + (size_t)xl * HX + (size_t)u * nb + b;
-    if constexpr (FF) {
-      float sh = 0.0f, sl = 0.0f;
-      for (int v = 0; v < W; v++) ffa::mac(w[v], p[v], sh, sl);
-      *hq = ffa::norm(sh, sl);
-    } else {
-      double s = 0.0;
-      for (int v = 0; v < W; v++) s = fma(w[v], p[v], s);
-      *hq = s;
+  for (int q = threadIdx.x; q < PXC * W * ng; q += PDT) {
+    const int r = q / ng, g = q - r * ng, xl = r / W, u = r - xl * W;
+    const T *w = Wm + (xl * PBW + u) * PBW;
+    const T *pp = p2w + xl * bw + 2 * g;
+    V s0, s1;
+    for (int v = 0; v < W; v++) {
+      const T wv = w[v];
+      const T2 b2 = *reinterpret_cast<const T2 *>(pp + v * bw);
+      s0.mac(wv, b2.a);
+      s1.mac(wv, b2.b);
     }
+    *reinterpret_cast<T2 *>(H + (xl * PBW + u) * bw + 2 * g) = {s0.get(), s1.get()};
   }
   __syncthreads();
   const size_t per = (size_t)ns * NDB;
-  for (int q = threadIdx.x; q < PXC * nb * nb; q += blockDim.x) {
-    const int xl = q % PXC, pr = q / PXC, b = pr % nb, a = pr / nb;
-    const int x = x0 + xl, y = x + d;
-    if (x > ns || y < 1 || y > ns) continue;
-    const S *p = p1w + (size_t)a * WLP + xl;
-    const S *h = H + (size_t)xl * HX + b;
-    const size_t o = (size_t)pr * per + (size_t)(x - 1) + (size_t)ns * (d + BAND);
-    // the exchanged element; on the diagonal of Kout another thread's own
-    const size_t o2 = (size_t)(b * nb + a) * per + (size_t)(y - 1) + (size_t)ns * (BAND - d);
-    const bool both = Kx && (Kx != Kout || d > 0);
-    if constexpr (FF) {
-      float sh = 0.0f, sl = 0.0f;
-      for (int u = 0; u < W; u++) ffa::mac(p[u], h[(size_t)u * nb], sh, sl);
-      static_cast<float2 *>(Kout)[o] = ffa::norm(sh, sl);
-      if (both) static_cast<float2 *>(Kx)[o2] = ffa::norm(sh, sl);
-    } else {
-      double s = 0.0;
-      for (int u = 0; u < W; u++) s = fma(p[u], h[(size_t)u * nb], s);
-      static_cast<double *>(Kout)[o] = s;
-      if (both) static_cast<double *>(Kx)[o2] = s;
+  const bool both = Kx && (Kx != Kout || d > 0);
+  // items: xl fastest, then the first orbital, then the group of two second ones
+  for (int q = threadIdx.x; q < PXC * nb * ng; q += PDT) {
+    const int xl = q % PXC, r = q / PXC, g = r / nb, a = r - g * nb;
+    const int x = x0 + xl, y = x + d, b = zb + 2 * g;
+    if (x > ns) continue;
+    V s0, s1;
+    int xx = y;  // row of the exchanged element
+    if (y >= 1 && y <= ns) {
+      const T *pa = p1w + xl * pstr + a, *h = H + xl * PBW * bw + 2 * g;
+      for (int u = 0; u < W; u++) {
+        const T pv = pa[u * pstr];
+        const T2 h2 = *reinterpret_cast<const T2 *>(h + u * bw);
+        s0.mac(pv, h2.a);
+        s1.mac(pv, h2.b);
+      }
+    } else {  // no element: as many are missing from the exchanged diagonal's other end
+      const int m = abs(d);
+      xx = m >= ns ? x : (d > 0 ? x - (ns - m) : x + (ns - m));
     }
+    const size_t o = (size_t)(x - 1) + (size_t)ns * (d + BAND);
+    const size_t ox = (size_t)(xx - 1) + (size_t)ns * (BAND - d);
+    auto put = [&](int bb, T v) {
+      Kout[((size_t)a * nb + bb) * per + o] = v;
+      if (both) Kx[((size_t)bb * nb + a) * per + ox] = v;
+    };
+    put(b, s0.get());
+    if (b + 1 < nb) put(b + 1, s1.get());
   }
 }
 
@@ -465,11 +499,12 @@ __global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, int np, int suf
 // second orbitals lose more than they gain (106 us for 78).  Bound by the FP64
 // pipe, in the split form by the latency of the small matrix's loads.  Cell by
 // cell with partial sums in memory against this: ns 300, 30 orbitals, R^k, FP64
-// 325 -> 78 us; ns 400, 20 orbitals, split form (R^k and S^k) 217 -> 66 us.
-constexpr int PDX = 4, PDB = 32, PDT = 256;
+// 325 -> 78 us; ns 400, 20 orbitals, split form (R^k and S^k) 217 -> 55 us.
+constexpr int PDX = 4;
 template <bool FF>
 struct PairDirArgs {
   int ns, nv, kk, nb, np, symab, suf, dl0;  // dl0: dl of column 0
+  int bw;  // stride of the second orbitals' arrays
   PairSpec eo, ed;
   const double *rkd;  // element (po, pd; cell) at rpo po + rpd pd + rcell cell
   size_t rcell;
@@ -479,10 +514,6 @@ struct PairDirArgs {
   typename Val<FF>::T *K;
   size_t per;
 };
-
-__host__ __device__ inline int pair_row_stride(int n) {  // 8 mod 16: rows on other banks
-  return (n + 7) / 16 * 16 + 8;
-}
 
 // KM: the largest spline order the shared arrays are laid out for (9, or 16 for
 // the orders above: the energy functional takes them all)
@@ -499,9 +530,10 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
   };
   extern __shared__ __align__(16) unsigned char smdir[];
   T *W = reinterpret_cast<T *>(smdir);     // [PDX][PDW][PDW]
-  T *H = W + PDX * PDW * PDW;              // [PDX][PDW][PDB]
-  T *p2w = H + PDX * PDW * PDB;            // [PDR][PDB]
-  T *p1w = p2w + PDR * PDB;                // [PDR][pstr]
+  const int bw = p.bw;
+  T *H = W + PDX * PDW * PDW;              // [PDX][PDW][bw]
+  T *p2w = H + PDX * PDW * bw;             // [PDR][bw]
+  T *p1w = p2w + PDR * bw;                 // [PDR][pstr]
   __shared__ double c1[PDX][KM], c2[PDX][KM];
   __shared__ T t1[PDX], t2[PDX];
   __shared__ int los[PDX], his[PDX], pos[PDX][KM];
@@ -548,9 +580,9 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
     const int a = q / PDR, r = q - a * PDR, x = rb + r;
     p1w[r * pstr + a] = x >= 1 && x <= ns ? p.P1[(size_t)a * ns + x - 1] : V::zero();
   }
-  for (int q = threadIdx.x; q < PDR * PDB; q += PDT) {
+  for (int q = threadIdx.x; q < PDR * bw; q += PDT) {
     const int b = q / PDR, r = q - b * PDR, y = rb + r;
-    p2w[r * PDB + b] =
+    p2w[r * bw + b] =
         b < bc && y >= 1 && y <= ns ? p.P2[(size_t)(zb + b) * ns + y - 1] : V::zero();
   }
   __syncthreads();
@@ -583,15 +615,15 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
     const int ca = max(lo, x - ed.k1 + 1), cb = min(hi, x);
     if (ca > cb) continue;
     const T *w = W + r * PDW;
-    const T *pp = p2w + (lo - rb) * PDB + 2 * g;
+    const T *pp = p2w + (lo - rb) * bw + 2 * g;
     V s0, s1;
     for (int u = ca - lo; u < cb + ed.k2 - lo; u++) {
       const T wv = w[u];
-      const T2 v = *reinterpret_cast<const T2 *>(pp + u * PDB);
+      const T2 v = *reinterpret_cast<const T2 *>(pp + u * bw);
       s0.mac(wv, v.a);
       s1.mac(wv, v.b);
     }
-    *reinterpret_cast<T2 *>(H + r * PDB + 2 * g) = {s0.get(), s1.get()};
+    *reinterpret_cast<T2 *>(H + r * bw + 2 * g) = {s0.get(), s1.get()};
   }
   __syncthreads();
   // items: fl fastest, then the first orbital, then the group
@@ -610,11 +642,11 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
     const int lo = los[fl], hi = his[fl], b0 = zb + 2 * g;
     V s0, s1;
     if (lo <= hi) {
-      const T *pa = p1w + (lo - rb) * pstr + a, *h = H + fl * PDW * PDB + 2 * g;
+      const T *pa = p1w + (lo - rb) * pstr + a, *h = H + fl * PDW * bw + 2 * g;
       const int nt = hi - lo + ed.k1;
       for (int t = 0; t < nt; t++) {
         const T pv = pa[t * pstr];
-        const T2 v = *reinterpret_cast<const T2 *>(h + t * PDB);
+        const T2 v = *reinterpret_cast<const T2 *>(h + t * bw);
         s0.mac(pv, v.a);
         s1.mac(pv, v.b);
       }
@@ -1059,7 +1091,8 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
     d.SB = (const T *)SB;
     d.K = (T *)K;
     d.per = per;
-    const size_t smem = sizeof(T) * ((size_t)PDX * PDW * (PDW + PDB) + PDR * PDB +
+    d.bw = (std::min(nb, PDB) + 1) & ~1;
+    const size_t smem = sizeof(T) * ((size_t)PDX * PDW * (PDW + d.bw) + PDR * d.bw +
                                      (size_t)PDR * pair_row_stride(nb));
     const int frc = set_smem(c, (const void *)k_pair_direct<F, KM>, smem);
     if (frc) return frc;
@@ -1091,73 +1124,89 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
   return DBSRG_OK;
 }
 
-// exchange band pair potentials of (family, type, k, case) with density
-// components jp1/jp2: Kb[pair][ns*17], cached
-// ff: both stages in float-float arithmetic, the result stored as
-// float-float pairs (float2, same bytes) for the split form's Z digits
-// (R^k: tabs of types 0..2 by type, type 3 comes with type 2; S^k: tabs[0])
-static int get_pairpot_band(dbsrg_ctx *c, int family, int type, int k, int cs, int jp1, int jp2,
+// exchange band pair potentials of (family, type, k, case), cached:
+// Kb[pair][ns*17], in FP64 or float-float pairs (ff: both stages in that
+// arithmetic, same bytes; the split form's Z digits read those).  An R^k table's
+// come with those of all types of its k (tabs of types 0..2 by type, type 3 from
+// type 2), as a list takes them all; S^k: tabs[0].  The density components are
+// the contracted functions' (factored_contract checks them).
+static int get_pairpot_band(dbsrg_ctx *c, int family, int type, int k, int cs,
                             const double *const *tabs, bool ff, const void **out) {
-  if (family == 0 && type == 3) {
-    type = 2;
-    std::swap(jp1, jp2);
-    const long long k3 = pairpot_key(1, 0, 3, k, cs, jp2, jp1, ff);
-    const int rc = c->ppot.count(k3)
-                       ? DBSRG_OK
-                       : get_pairpot_band(c, 0, 2, k, cs, jp1, jp2, tabs, ff, out);
-    if (rc) return rc;
-    *out = c->ppot.at(k3);
-    return DBSRG_OK;
-  }
-  const long long key = pairpot_key(1, family, type, k, cs, jp1, jp2, ff);
-  auto it = c->ppot.find(key);
+  auto key_of = [&](int t) {
+    const TableBases tb = table_bases(c->g, family, t);
+    return pairpot_key(1, family, t, k, cs, cs == 3 ? tb.a2 : tb.a1, cs == 3 ? tb.b1 : tb.b2, ff);
+  };
+  auto it = c->ppot.find(key_of(type));
   if (it != c->ppot.end()) {
     *out = it->second;
     return DBSRG_OK;
   }
-  const double *tab = tabs[family == 0 ? type : 0];
   const DeviceGrid &g = c->g;
   const int ns = g.ns, ks = g.ks, nb = c->nbound;
   const size_t npair = (size_t)nb * nb, per = (size_t)ns * NDB;
   int rc;
   if ((rc = ensure_brows(c))) return rc;
   const size_t kbytes = npair * per * sizeof(double);
-  double *K = (double *)cache_alloc(c, kbytes), *Kx = nullptr;
-  if (!K) return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
-  c->ppot[key] = K;
-  if (family == 0) {  // the results with the electrons exchanged
-    Kx = type == 2 ? (double *)cache_alloc(c, kbytes) : K;
-    if (!Kx) return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
-    if (type == 2) c->ppot[pairpot_key(1, 0, 3, k, cs, jp2, jp1, ff)] = Kx;
-  }
-  // positions past the ends of the band are never written by k_pair_band
-  for (double *q : {K, Kx == K ? nullptr : Kx})
-    if (q) DBSRG_TRY(c, cudaMemsetAsync(q, 0, kbytes, c->stream));
-  const double *P1 = c->brows + (size_t)(jp1 - 1) * nb * ns;
-  const double *P2 = c->brows + (size_t)(jp2 - 1) * nb * ns;
-  const int W = 2 * ks - 1, WLP = (PXC + W - 1) | 1;
-  const size_t smem =
-      ((size_t)PXC * W * W + 2 * (size_t)nb * WLP + (size_t)PXC * (W * nb + 1)) * sizeof(double);
-  const int mode = family == 0 ? 0 : (cs == 3 ? 1 : 2);
-  dim3 gb((unsigned)((ns + PXC - 1) / PXC), (unsigned)(Kx == K ? BAND + 1 : NDB));
-  // executed work: per output row and band diagonal W^2 nb (stage 1) and
-  // W nb^2 (stage 2) multiply-adds; the band table read, the potentials
-  // written
-  const double kb = family == 0 ? ks : W;
-  const double bflops = 2.0 * ns * gb.y * ((double)W * W * nb + (double)W * nb * nb);
-  const double bbytes = 8.0 * ns * NDB * (kb * kb + (double)npair);
-  if (ff) {
-    if ((rc = set_smem(c, (const void *)k_pair_band<true>, smem))) return rc;
+  const int n = family == 0 ? 3 : 1;
+  void *K[3], *Kx[3] = {nullptr, nullptr, nullptr};
+  // the results, S^k one, R^k those of types 0..2 and of type 3 (type 2's with the
+  // electrons exchanged)
+  void *buf[4];
+  for (int i = 0; i < n + (n == 3); i++)
+    if (!(buf[i] = cache_alloc(c, kbytes))) {
+      while (i > 0) cache_free(c, buf[--i]);
+      return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
+    }
+  for (int i = 0; i < n; i++) K[i] = buf[i];
+  if (n == 3) Kx[0] = K[0], Kx[1] = K[1], Kx[2] = buf[3];
+  const int W = 2 * ks - 1, mode = family == 0 ? 0 : (cs == 3 ? 1 : 2);
+  const int bw = (std::min(nb, PDB) + 1) & ~1;
+  auto potentials = [&](auto ff_c) -> int {
+    constexpr bool F = decltype(ff_c)::value;
+    using T = typename Val<F>::T;
+    const T *rows = F ? (const T *)c->browsf : (const T *)c->brows;
+    PairBandArgs<F> p{};
+    p.ns = ns;
+    p.ks = ks;
+    p.nb = nb;
+    p.mode = mode;
+    p.bw = bw;
+    for (int i = 0; i < n; i++) {
+      const TableBases tb = table_bases(g, family, family == 0 ? i : type);
+      p.rkb[i] = tabs[i];
+      p.P1[i] = rows + (size_t)((cs == 3 ? tb.a2 : tb.a1) - 1) * nb * ns;
+      p.P2[i] = rows + (size_t)((cs == 3 ? tb.b1 : tb.b2) - 1) * nb * ns;
+      p.Kout[i] = (T *)K[i];
+      p.Kx[i] = (T *)Kx[i];
+      p.y0[i + 1] = p.y0[i] + (Kx[i] == K[i] ? BAND + 1 : NDB);
+    }
+    for (int i = n; i < 3; i++) p.y0[i + 1] = p.y0[i];
+    const int ny = p.y0[n];
+    if (n == 1) p.y0[1] = p.y0[2] = ny;
+    const dim3 gb((unsigned)((ns + PXC - 1) / PXC), (unsigned)ny, (unsigned)((nb + PDB - 1) / PDB));
+    // executed work: per output row and band diagonal W^2 nb (stage 1) and
+    // W nb^2 (stage 2) multiply-adds; the band tables read, the potentials
+    // written
+    const double kb = family == 0 ? ks : W;
+    const double bflops = 2.0 * ns * ny * ((double)W * W * nb + (double)W * nb * nb);
+    const double bbytes = 8.0 * ns * NDB * (n * kb * kb + (n == 3 ? 4 : 1) * (double)npair);
+    const size_t smem = sizeof(T) * ((size_t)PXC * PBW * (PBW + bw) + PBR * bw +
+                                     (size_t)PBR * pair_row_stride(nb));
+    const int brc = set_smem(c, (const void *)k_pair_band<F>, smem);
+    if (brc) return brc;
     DBSRG_RUN_W(c, "k_pair_band", bbytes, bflops,
-                k_pair_band<true><<<gb, 256, smem, c->stream>>>(ns, ks, nb, mode, tab, P1, P2, K,
-                                                                Kx));
-  } else {
-    if ((rc = set_smem(c, (const void *)k_pair_band<false>, smem))) return rc;
-    DBSRG_RUN_W(c, "k_pair_band", bbytes, bflops,
-                k_pair_band<false><<<gb, 256, smem, c->stream>>>(ns, ks, nb, mode, tab, P1, P2, K,
-                                                                 Kx));
+                k_pair_band<F><<<gb, PDT, smem, c->stream>>>(p));
+    return DBSRG_OK;
+  };
+  rc = ff ? potentials(std::true_type()) : potentials(std::false_type());
+  for (int i = 0; i < n + (n == 3); i++) {
+    if (rc)
+      cache_free(c, buf[i]);
+    else
+      c->ppot[key_of(n == 3 ? i : type)] = (double *)buf[i];
   }
-  *out = K;
+  if (rc) return rc;
+  *out = c->ppot.at(key_of(type));
   return DBSRG_OK;
 }
 
@@ -1213,8 +1262,8 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
       int c1 = cs == 3 ? tb.a2 : tb.a1, c2 = cs == 3 ? tb.b1 : tb.b2;
       if (c1 != j.jp1[a] || c2 != j.jp2[a])
         return set_err(c, DBSRG_EINVAL, "factored exchange: component mismatch");
-      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.jp1[a], j.jp2[a], j.tabs,
-                                 true, (const void **)&x.Kbf[a])))
+      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.tabs, true,
+                                 (const void **)&x.Kbf[a])))
         return rc;
     }
     x.members = j.members;
@@ -1234,8 +1283,7 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
       const FarField *f;
       const void *Kb;
       if ((rc = get_farfield(c, j.family, j.types[a], j.kpol, j.icv, &f))) return rc;
-      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, j.icv, j.jp1[a], j.jp2[a],
-                                 j.tabs, false, &Kb)))
+      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, j.icv, j.tabs, false, &Kb)))
         return rc;
     }
     return DBSRG_OK;
@@ -1254,8 +1302,8 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
       if (c1 != j.jp1[a] || c2 != j.jp2[a])
         return set_err(c, DBSRG_EINVAL, "factored exchange: component mismatch");
       const double *Kb;
-      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.jp1[a], j.jp2[a], j.tabs,
-                                 false, (const void **)&Kb)))
+      if ((rc = get_pairpot_band(c, j.family, j.types[a], j.kpol, cs, j.tabs, false,
+                                 (const void **)&Kb)))
         return rc;
       double *Ya = j.Y + (size_t)a * j.nm * per;
       dim3 gz((unsigned)((ns * nb + 127) / 128), (unsigned)j.nm);

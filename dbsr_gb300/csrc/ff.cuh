@@ -23,13 +23,16 @@ namespace ffa {
 // a split takes three of its instructions, a sum of two floats three more.
 // hi: the bits rounded to 24 (ties away from zero); lo: what is left, a signed
 // integer of 29 bits, converted and scaled by v's power of two in two exact
-// steps.  Values outside the normal floats (but for zero) take the conversions.
+// steps.  Values past the ends of the normal floats take the conversion.
 __device__ __forceinline__ float2 split(double v) {
   const unsigned hw = (unsigned)__double2hiint(v), lw = (unsigned)__double2loint(v);
   const unsigned e = hw >> 20 & 0x7ffu, sign = hw & 0x80000000u;
   if (e - 898u > 251u) {
-    if (((hw ^ sign) | lw) == 0) return make_float2(__uint_as_float(sign), 0.0f);
+    // below half the smallest float: zero; below 2^-125 the rest of the rounded
+    // value is less than half the smallest float
+    if (e < 873u) return make_float2(__uint_as_float(sign), 0.0f);
     const float h = __double2float_rn(v);
+    if (e < 898u) return make_float2(h, 0.0f);
     return make_float2(h, __double2float_rn(v - (double)h));
   }
   const unsigned lr = lw + 0x10000000u, hr = hw + (lr < lw ? 1u : 0u);

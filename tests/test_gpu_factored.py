@@ -206,3 +206,26 @@ def test_exchange_strips_and_entry_batches(ns, nch, norb, per_slot):
     h, _ = run(w, SPLIT_BF16, lists)
     ref, _ = oracle(w, lists)
     check(h, ref, 1e-10)
+
+
+@pytest.mark.parametrize("precision,tol", [(FACTOR_FP64, 1e-12), (SPLIT_BF16, 1e-10)])
+@pytest.mark.parametrize("ks,ksp,ksq,ns", [(3, 2, 3, 5), (4, 3, 4, 7), (6, 5, 5, 11),
+                                           (8, 7, 8, 21), (9, 8, 9, 17)])
+def test_pair_potentials_on_small_grids(precision, tol, ks, ksp, ksq, ns):
+    """The band and direct pair potentials at orders below nine and on grids with
+    fewer functions than band diagonals (windows cut at both ends, rows that four
+    does not divide, diagonals with no element at all): every list kind against
+    the oracle."""
+    w = synth.small(ns=45, nch=3, mk=2, n_entries=90, breit=True, seed=90 + ks)
+    rng = np.random.default_rng(ks)
+    w.t = np.concatenate([np.zeros(ks - 1), np.linspace(0.0, 1.0, ns - ks + 2) ** 2 * 5.0,
+                          np.full(ks - 1, 5.0)])
+    w.ks, w.ksp, w.ksq = ks, ksp, ksq
+    w.pq = np.zeros((ns, 2, w.nbf), order="F")
+    w.pq[: ns - ks + ksp, 0, : w.nbound] = rng.uniform(-1, 1, (ns - ks + ksp, w.nbound))
+    w.pq[: ns - ks + ksq, 1, : w.nbound] = rng.uniform(-1, 1, (ns - ks + ksq, w.nbound))
+    lists = [L for L in w.lists if L.icase in (2, 3)]
+    h, acf = run(w, precision, lists)
+    ref, racf = oracle(w, lists)
+    check(h, ref, tol)
+    assert relmax(acf, racf) <= 1e-12
