@@ -62,6 +62,21 @@ extern "C" int dbsrg_hf_matrix(dbsrg_ctx *c, int iorb, int kmax, const double *a
   int rc = dbsrg_zero_matrix(c);
   if (rc) return rc;
   const int nbf = c->nbf;
+  // the lists of an orbital are queued as in the asynchronous mode (the set-up
+  // of one overlaps the kernels of the one before); the block's read-out waits.
+  // 30 orbitals at ns 300: 18.9 ms, 30.4 with a wait after every list
+  struct Pipeline {
+    dbsrg_ctx *c;
+    bool was, done = false;
+    explicit Pipeline(dbsrg_ctx *x) : c(x), was(x->async) { c->async = true; }
+    ~Pipeline() {
+      c->async = was;
+      if (done || !c->pending) return;
+      const std::string e = c->err;  // a list failed: that error stands
+      drain(c);
+      c->err = e;
+    }
+  } pipeline(c);
   std::vector<int> k1, k2, k4;
   std::vector<double> cd;
   for (int k = 0; k <= kmax; k++)
@@ -126,6 +141,7 @@ extern "C" int dbsrg_hf_matrix(dbsrg_ctx *c, int iorb, int kmax, const double *a
       }
   if (dhl && (rc = dbsrg_update_hx(c, 1, 1, dhl, qsum))) return rc;
   if ((rc = dbsrg_get_block(c, 1, 1, hfm))) return rc;
+  pipeline.done = true;
   const size_t n = (size_t)c->g.ms * c->g.ms;
   if (is_device_ptr(hfm)) {
     DBSRG_RUN(c, "k_div", k_div<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, qsum, hfm));
