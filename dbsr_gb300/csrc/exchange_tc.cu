@@ -34,7 +34,9 @@
 // Every wait is bounded (2 s): on a timeout the kernel records an error word,
 // waits (bounded) for its own copies and MMAs in flight, frees its TMEM and
 // returns.
+#include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "internal.cuh"
 #include "tc_common.cuh"
@@ -250,11 +252,13 @@ __global__ void __launch_bounds__(ZROWS * ZW) k_zdigits(const ZArgs z) {
   }
 }
 
+constexpr int MAXBLK = 256;  // blocks of a launch, at most
+
 struct XArgs {
   int ns, NR, ntx, nty, nm, na, lower;
   int nbk;                     // chunks of 32 bound orbitals (products per term and field)
-  int nrows;                   // work items: y segments of (quadrant record, x tile) strips
-  int ysplit;                  // y segments per 128 x ns strip
+  int nstrips;                 // (quadrant record, x tile) strips of 128 x ns (tile_ranges)
+  int start[MAXBLK + 1];       // first tile (strip nty + y tile) of every block
   const __nv_bfloat16 *Ud[4];  // per atype: [mode][chunk][slice][NR][TILE]
   const int *eu[4];            // per atype: [mode][chunk][NR*33]
   const __nv_bfloat16 *Zd;     // [a][mode][slot][chunk][slice][NR][TILE]
@@ -275,12 +279,18 @@ struct Row {
   int tc[MAXT];
 };
 
+// first strip of a block and the next one; a strip of p.nstrips or more: done
+__device__ __forceinline__ int first_row(const XArgs &p) {
+  const int t0 = p.start[blockIdx.x];
+  return t0 < p.start[blockIdx.x + 1] ? t0 / p.nty : p.nstrips;
+}
+__device__ __forceinline__ int next_row(const XArgs &p, int row) {
+  return (row + 1) * p.nty < p.start[blockIdx.x + 1] ? row + 1 : p.nstrips;
+}
+
 __device__ __forceinline__ void load_row(const XArgs &p, int row, Row &r) {
-  const int seg = row % p.ysplit;
-  row /= p.ysplit;
-  const int per = (p.nty + p.ysplit - 1) / p.ysplit;
-  r.ty0 = seg * per;
-  r.ty1 = min(p.nty, r.ty0 + per);
+  r.ty0 = max(0, p.start[blockIdx.x] - row * p.nty);
+  r.ty1 = min(p.nty, p.start[blockIdx.x + 1] - row * p.nty);
   const int4 *q = reinterpret_cast<const int4 *>(p.xq + row / p.ntx);
   const int4 v0 = q[0], v1 = q[1], v2 = q[2];  // blk qr qc nt | half t0 t1 t2 | t3 . . .
   r.tx = row % p.ntx;
@@ -339,14 +349,14 @@ struct ProdIt {
 // advance to the next product (orbital chunks innermost); false when the
 // CTA's rows are done
 __device__ __forceinline__ bool prod_next(const XArgs &p, int nbk, ProdIt &it) {
-  if (it.row >= p.nrows) return false;
+  if (it.row >= p.nstrips) return false;
   if (++it.ck < nbk) return true;
   it.ck = 0;
   it.pc++;
   while (it.pc >= it.np) {
     if (++it.ty >= it.r.ty1) {
-      it.row += gridDim.x;
-      if (it.row >= p.nrows) return false;
+      it.row = it.row < 0 ? first_row(p) : next_row(p, it.row);
+      if (it.row >= p.nstrips) return false;
       load_row(p, it.row, it.r);
       it.ty = it.r.ty0;
     }
@@ -372,7 +382,6 @@ __device__ __forceinline__ void prod_operands(const XArgs &p, int nbk, const Pro
   Bs = (tra ? Ub : Zb) + (size_t)it.ty * TILE;
 }
 
-constexpr int XITEMS = 8;               // work items an SM (split_exchange)
 constexpr int NCW = 16;               // consumer (epilogue) warps
 constexpr int CPT = 32 / (NCW / 4);   // tile columns per consumer thread
 constexpr int WPROD = NCW;            // producer warp
@@ -405,7 +414,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 }
 
 // Warp-specialised, one CTA per SM walking rows (quadrant record, x tile)
-// of 128 x ns; every role walks the same tile sequence.
+// of 128 x ns within its range of tiles (tile_ranges); every role walks the
+// same tile sequence.
 //  * producer (warp NCW, one lane): issues the bulk loads of the next
 //    product (once the MMAs of the previous one completed; the 128-row A
 //    operand only when neither A slot holds it already), then waits for this
@@ -480,7 +490,7 @@ __global__ void __maxnreg__(96) k_xfused(const XArgs p) {
     // theirs, so the copies of two products are in flight at once.
     if (lane == 0) {
       ProdIt it;
-      it.row = (int)blockIdx.x - (int)gridDim.x;
+      it.row = -1;
       it.ty = 0;
       it.r.ty1 = 0;
       it.pc = 0;
@@ -610,7 +620,7 @@ __global__ void __maxnreg__(96) k_xfused(const XArgs p) {
         __syncwarp();
       };
       Row r;
-      for (int row = blockIdx.x; row < p.nrows && !fail; row += gridDim.x) {
+      for (int row = first_row(p); row < p.nstrips && !fail; row = next_row(p, row)) {
         load_row(p, row, r);
         const int x0 = r.tx * 128, nrow = min(128, p.ns - x0);
         const double *hq = p.hch + (size_t)(r.blk - 1) * ms * ms + (size_t)(r.qr - 1) * p.ns +
@@ -720,7 +730,7 @@ __global__ void __maxnreg__(96) k_xfused(const XArgs p) {
     uint32_t q = 0, ntile = 0;
     Row r;
     long long Iacc[CPT];
-    for (int row = blockIdx.x; row < p.nrows; row += gridDim.x) {
+    for (int row = first_row(p); row < p.nstrips; row = next_row(p, row)) {
       load_row(p, row, r);
       const int x = r.tx * 128 + xl, x0 = r.tx * 128;
       const bool row_ok = x < p.ns;
@@ -976,6 +986,63 @@ static void xfused_work(const XQuad *hxq, int nxq, int ns, int lower, int nbk, d
   }
 }
 
+// How the tiles of a launch are divided among the blocks: block b takes the tiles
+// start[b] .. start[b+1] - 1 (strip by strip, the 128-row A operand kept along a
+// strip and from strip to strip where it repeats), cut where the products and
+// tiles before them have b of nblk equal costs, so that every block ends at about
+// the same time whatever a record's strips cost (S^k: products on one side of the
+// diagonal only).  Strips in turn -- block b takes strips b, b + nblk, .., cut
+// into y segments where there are few -- left the busiest SM with up to 1.6 times
+// the mean: ns 283, 26 segments a list 73 -> 67 us, ns 351 106 -> 93, ns 400,
+// 80 channels 494 -> 429 us.  (Changing the blocks' places from round to round
+// instead loads an A operand for every strip: 87 us at ns 283.)
+constexpr int TILE_COST = 1, PROD_COST = 12;  // reading and writing a tile, one product
+
+// fills p.start; the number of blocks
+static int tile_ranges(XArgs &p, const XQuad *hxq, int nxq, int maxblk) {
+  const int nt = p.ntx * p.nty;
+  std::vector<long long> pre[MAXT + 1][MAXT + 1];  // cost before each tile, by terms
+  auto costs = [&](const XQuad &r) -> const std::vector<long long> & {
+    int ntr = 0;
+    const int n = std::min(r.nt, MAXT);
+    for (int t = 0; t < n; t++) ntr += (r.term[t] >> 2) & 1;
+    std::vector<long long> &v = pre[n - ntr][ntr];
+    if (v.empty()) {
+      v.resize(nt + 1, 0);
+      for (int i = 0; i < nt; i++) {
+        const int x0 = i / p.nty * 128, y0 = i % p.nty * 32;
+        const bool up = (y0 + 31) - x0 >= FAR, lo = (x0 + 127) - y0 >= FAR;
+        const bool band = (y0 + 31) - x0 >= -BAND && y0 - (x0 + 127) <= BAND;
+        int np = 0;
+        if (up) np += n - ntr + (p.lower ? ntr : 0);
+        if (lo) np += ntr + (p.lower ? n - ntr : 0);
+        v[i + 1] = v[i] + (np || band ? TILE_COST + PROD_COST * np * p.nbk : 0);
+      }
+    }
+    return v;
+  };
+  long long total = 0;
+  for (int i = 0; i < nxq; i++) total += costs(hxq[i])[nt];
+  const int nblk = (int)std::min<long long>(maxblk, (long long)nxq * nt);
+  int b = 1;
+  long long before = 0;
+  p.start[0] = 0;
+  for (int i = 0; i < nxq; i++) {
+    const std::vector<long long> &v = costs(hxq[i]);
+    // the cut nearest to b of nblk parts, if it falls into this record
+    for (; b < nblk; b++) {
+      const long long want = total * b / nblk - before;
+      if (want > v[nt]) break;
+      int t = (int)(std::lower_bound(v.begin(), v.end(), want) - v.begin());
+      if (t > 0 && want - v[t - 1] < v[t] - want) t--;
+      p.start[b] = std::max(p.start[b - 1], i * nt + t);
+    }
+    before += v[nt];
+  }
+  for (; b <= nblk; b++) p.start[b] = nxq * nt;
+  return nblk;
+}
+
 int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
   const int ns = c->g.ns, nb = c->nbound;
   if (nb < 1 || nb > 32 * MAX_NBK)
@@ -1072,18 +1139,10 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
   p.na = x.na;
   p.lower = x.lower;
   p.nbk = nbk;
-  // Items of a launch: a strip of 128 rows whole (its A operands are loaded
-  // once) where the strips keep every SM busy for several rounds, otherwise
-  // its y tiles split so that they do: XITEMS items an SM, at least one tile
-  // each.  One channel at ns 300 (12 strips): 82 -> 22 us a launch; ns 283, 26
-  // segments (312 strips on 152 SMs): 98 us whole, 95, 82, 82, 73, 69 and 69 us
-  // at 1, 2, 4, 8, 16 and 32 items; ns 400, 80 channels: 494 us up to 8 items,
-  // 522 and 596 us at 16 and 32 (more loads of A operands).
-  const int strips = x.nxq * ntx;
-  p.ysplit = std::max(1, std::min(nty, (XITEMS * c->nsm + strips - 1) / strips));
-  const int per = (nty + p.ysplit - 1) / p.ysplit;
-  p.ysplit = (nty + per - 1) / per;  // no empty segment
-  p.nrows = strips * p.ysplit;
+  p.nstrips = x.nxq * ntx;
+  const int maxblk = std::min(MAXBLK, std::max(1, c->nsm));
+  if (!x.hxq) return set_err(c, DBSRG_EINVAL, "split exchange: no host records");
+  const int nblk = tile_ranges(p, x.hxq, x.nxq, maxblk);
   for (int a = 0; a < x.na; a++) {
     p.Ud[a] = (const __nv_bfloat16 *)x.far[a]->Ud;
     p.eu[a] = x.far[a]->eu;
@@ -1100,7 +1159,6 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
                       ((size_t)2 * MAXT * NDB * BR + 2 * 32 * 128) * sizeof(double);
   const void *xk = nbk == 1 ? (const void *)k_xfused<true> : (const void *)k_xfused<false>;
   if ((rc = raise_smem_limit(c, xk, smem))) return rc;
-  const int nblk = std::min(p.nrows, std::max(1, c->nsm));
   double wbytes = 0.0, wflops = 0.0;
   if (c->timing) xfused_work(x.hxq, x.nxq, ns, x.lower, nbk, wbytes, wflops);
   if (nbk == 1)
