@@ -292,10 +292,12 @@ extern "C" int dbsrg_backward(dbsrg_ctx *c, int n, const int *k, const int *i1, 
     const int i0 = kitem[kp], ni = kitem[kp + 1] - i0;
     if (ni == 0) continue;
     KdTypes kd{};
+    PairPotKey want[4];
     for (int t = 0; t < 4; t++) {
       const int comp = (t == 0 || t == 3) ? 1 : 2;  // electron-2 basis of the table
-      if ((rc = get_pairpot_direct(c, 0, t, kp, 1, comp, comp, &kd.K[t]))) return rc;
+      want[t] = {0, t, kp, 1, comp, comp};
     }
+    if ((rc = get_pairpots_direct(c, 4, want, false, (const void **)kd.K))) return rc;
     DBSRG_RUN(c, "k_rk_vsum",
               k_rk_vsum<<<dim3((unsigned)((per + 255) / 256), (unsigned)nup, 2), 256, 0, st>>>(
                   per, nup, dup, kd, dV));

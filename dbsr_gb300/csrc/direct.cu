@@ -501,14 +501,15 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
 // Multiply-adds of the two ways over a whole list (all its segments, whatever
 // the window or chunk, so that a block's result does not depend on them), the
 // pair way with the potentials it builds whether or not they are cached.  Per
-// cell and segment the apply kernel takes npo kd of them, the cell moments
-// about 24 kd (FP64); a pair potential about 4000 an output for its small
-// matrix, 120 per second orbital and 14 per pair; both ways one an entry and
-// band element.  Assemblies by the rule, all lists by pairs, and with the line
-// before the pair potentials were built a row at a time (mostly by segment):
-// ns 80, 2 channels 1.86 / 1.99 / 1.86 ms; ns 200, 12 channels 4.96 / 5.12 / 5.14;
-// ns 283, 32 channels 14.0 / 14.2 / 14.2; ns 400, 80 channels 47.5 / 47.6 / 49.7;
-// four waves of 6 to 28 channels in turn 34.0 / 35.0 / 34.5.
+// cell and lane of 32 segments (used or not) the apply kernel takes npo kd of
+// them, counted 1.6 times since its blocks are few (0.7 T/s against the pair
+// potentials' 1.2 where both are long), the cell moments about 40 kd (FP64); a pair
+// potential about 4000 an output for its small matrix, 120 per second orbital and
+// 14 per pair; both ways one an entry and band element.  So pairs up to some 28
+// orbitals, segments above unless a list has many.  Assemblies by pairs and mostly
+// by segment: ns 80, 2 channels 1.41 and 1.63 ms; ns 200, 12 channels 4.56 and 4.92;
+// ns 222, 14 channels in FP64 10.4 and 10.9; ns 283, 32 channels 11.8 and 12.4;
+// ns 400, 80 channels 47.6 and 49.7 (before the tensor-core kernel's ranges).
 // The lists of a one-channel matrix (the SCF potentials) hold one segment each
 // and come once per orbital, so the pair potentials of an iteration serve all
 // of them: 30 orbitals at ns 300 took 76 ms by segment, 66 ms by pairs.
@@ -518,12 +519,13 @@ bool direct_by_segment(const dbsrg_ctx *c, int family, int icv, int na, const in
   if (c->nch == 1) return false;
   const double nb = c->nbound, ns = g.ns, nv = g.nv;
   const double ncol = family == 0 ? g.ks : 2.0 * g.ks - 1.0;
+  const double lanes = (double)((nseg + 31) / 32 * 32);
   double seg = 0.0, pair = 0.0;
   for (int a = 0; a < na; a++) {
     const TableBases tb = table_bases(g, family, types[a]);
     const PairSpec eo = icv == 1 ? tb.e1 : tb.e2, ed = icv == 1 ? tb.e2 : tb.e1;
     const double npo = npairs(eo), kd = npairs(ed), np = family == 0 ? nb * (nb + 1) / 2 : nb * nb;
-    seg += (double)nseg * nv * kd * (npo + 24.0);
+    seg += lanes * nv * kd * (1.6 * npo + 40.0);
     pair += ns * ncol * (4000.0 + 120.0 * nb + 14.0 * np);
     pair += (double)nent * ns * ncol;
   }

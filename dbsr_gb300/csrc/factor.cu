@@ -379,11 +379,24 @@ __device__ __forceinline__ int pair_number(int nb, int symab, int a, int b) {
   return a + (symab ? b * (b + 1) / 2 : b * nb);
 }
 
-// (1) cell sums, one block per cell cv:
+// The potentials of up to four tables (an R^k list's types) are built together:
+// one launch of each of the three kernels.  ns 80, 5 orbitals: k_pair_direct 4 x 18
+// -> 23 us, the three kernels of a list about 143 -> 40; energy functional, ns 300,
+// 30 orbitals: 312 -> 249 us a multipole (6.2 -> 5.4 ms).
+struct PairCellArgs {
+  PairSpec ed[4];
+  int symab[4];
+  const double *M1[4], *M2[4], *P1[4], *P2[4];
+  double *S1[4], *S2[4];  // S2 (with M2): null where one field only
+};
+
+// (1) cell sums, one block per cell cv and table:
 //   S1(cv, pair) = sum_{h1,h2} M1(h1,h2;cv) P1(a, cv+h1-1) P2(b, cv+h2-1), S2 with M2
-__global__ void k_pair_cellsum(int ns, int kk, int nb, int symab, PairSpec ed, const double *M1,
-                               const double *M2, const double *P1, const double *P2, double *S1,
-                               double *S2) {
+__global__ void k_pair_cellsum(int ns, int kk, int nb, const PairCellArgs g) {
+  const int ty = blockIdx.y, symab = g.symab[ty];
+  const PairSpec ed = g.ed[ty];
+  const double *M1 = g.M1[ty], *M2 = g.M2[ty], *P1 = g.P1[ty], *P2 = g.P2[ty];
+  double *S1 = g.S1[ty], *S2 = g.S2[ty];
   extern __shared__ double sm[];
   const int cv = blockIdx.x + 1, k1 = ed.k1, k2 = ed.k2;
   double *w1 = sm, *w2 = w1 + nb * k1, *t1 = w2 + nb * k2, *t2 = t1 + nb * k1;
@@ -434,17 +447,23 @@ __global__ void k_pair_cellsum(int ns, int kk, int nb, int symab, PairSpec ed, c
 
 // (2) exclusive suffix (sum over later cells) or prefix sums per pair, in place
 // (as float-float pairs in the split form): eight pairs a block, each with
-// sixteen runs of cells (blockIdx.y 1: the second array, prefix sums).  Bound by
+// sixteen runs of cells (blockIdx.y: twice the table, odd ones its second array,
+// prefix sums).  Bound by
 // the FP64 instructions, so the pairs are spread over many blocks: ns 300, 30
 // orbitals, split form 23 us with 32 pairs a block.
 constexpr int PSW = 16, PSP = 8;
+struct PairScanArgs {
+  int np[4], suffix0[4];
+  double *S[4][2];
+};
 template <bool FF>
-__global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, int np, int suffix0, double *S0,
-                                                        double *S1) {
+__global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, const PairScanArgs g) {
   __shared__ double tot[PSW][PSP];
   const int lane = threadIdx.x % PSP, w = threadIdx.x / PSP, q = blockIdx.x * PSP + lane;
-  double *s = (blockIdx.y ? S1 : S0) + q;
-  const bool suf = blockIdx.y == 0 && suffix0, ok = q < np;
+  const int ty = blockIdx.y / 2, which = blockIdx.y % 2, np = g.np[ty];
+  if (!g.S[ty][which]) return;
+  double *s = g.S[ty][which] + q;
+  const bool suf = which == 0 && g.suffix0[ty], ok = q < np;
   const int run = (nv + PSW - 1) / PSW, lo = min(nv, w * run), hi = min(nv, lo + run);
   double t = 0.0;
   if (ok)
@@ -502,9 +521,8 @@ __global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, int np, int suf
 // 325 -> 78 us; ns 400, 20 orbitals, split form (R^k and S^k) 217 -> 55 us.
 constexpr int PDX = 4;
 template <bool FF>
-struct PairDirArgs {
-  int ns, nv, kk, nb, np, symab, suf, dl0;  // dl0: dl of column 0
-  int bw;  // stride of the second orbitals' arrays
+struct PairDirTable {
+  int np, symab, suf;
   PairSpec eo, ed;
   const double *rkd;  // element (po, pd; cell) at rpo po + rpd pd + rcell cell
   size_t rcell;
@@ -512,7 +530,13 @@ struct PairDirArgs {
   const double *L1, *L2, *M1, *M2;
   const typename Val<FF>::T *P1, *P2, *SA, *SB;
   typename Val<FF>::T *K;
+};
+template <bool FF>
+struct PairDirArgs {
+  int ns, nv, kk, nb, ncol, dl0;  // dl0: dl of column 0
+  int bw;                         // stride of the second orbitals' arrays
   size_t per;
+  PairDirTable<FF> t[4];          // blockIdx.y: table ncol + column
 };
 
 // KM: the largest spline order the shared arrays are laid out for (9, or 16 for
@@ -521,7 +545,8 @@ constexpr int pair_window(int km) { return 2 * km - 1; }
 constexpr int pair_rows(int km) { return PDX - 1 + pair_window(km); }
 
 template <bool FF, int KM>
-__global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
+__global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
+  const PairDirTable<FF> &p = g.t[blockIdx.y / g.ncol];
   constexpr int PDW = pair_window(KM), PDR = pair_rows(KM);
   using V = Val<FF>;
   using T = typename V::T;
@@ -530,21 +555,22 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
   };
   extern __shared__ __align__(16) unsigned char smdir[];
   T *W = reinterpret_cast<T *>(smdir);     // [PDX][PDW][PDW]
-  const int bw = p.bw;
+  const int bw = g.bw;
   T *H = W + PDX * PDW * PDW;              // [PDX][PDW][bw]
   T *p2w = H + PDX * PDW * bw;             // [PDR][bw]
   T *p1w = p2w + PDR * bw;                 // [PDR][pstr]
   __shared__ double c1[PDX][KM], c2[PDX][KM];
   __shared__ T t1[PDX], t2[PDX];
   __shared__ int los[PDX], his[PDX], pos[PDX][KM];
-  const int ns = p.ns, nb = p.nb, pstr = pair_row_stride(nb);
+  const size_t per = g.per;
+  const int ns = g.ns, nb = g.nb, kk = g.kk, pstr = pair_row_stride(nb);
   const PairSpec eo = p.eo, ed = p.ed;
-  const int f0 = blockIdx.x * PDX + 1, dl = p.dl0 + (int)blockIdx.y, zb = blockIdx.z * PDB;
+  const int f0 = blockIdx.x * PDX + 1, col = blockIdx.y % g.ncol, dl = g.dl0 + col, zb = blockIdx.z * PDB;
   const int bc = min(PDB, nb - zb), na = p.symab ? zb + bc : nb;
   const int rb = f0 + max(1 - eo.k1, dl + 1 - eo.k2);  // first row of the windows
   if (threadIdx.x < PDX) {
     const int fl = threadIdx.x, f = f0 + fl, s2 = f + dl;
-    int lo = max(1, rb + fl), hi = min(p.nv, min(f, s2));
+    int lo = max(1, rb + fl), hi = min(g.nv, min(f, s2));
     if (f > ns || s2 < 1 || s2 > ns) hi = lo - 1;
     double l1[KM], l2[KM], s1 = 0.0, s2s = 0.0;
 #pragma unroll
@@ -552,7 +578,7 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
       const int cv = lo + k;
       const bool ok = cv <= hi;
       const int po = ok ? pidx(eo, f - cv + 1, s2 - cv + 1) : 0;
-      const size_t o = (size_t)po + (size_t)p.kk * (ok ? cv - 1 : 0);
+      const size_t o = (size_t)po + (size_t)kk * (ok ? cv - 1 : 0);
       l1[k] = ok ? p.L1[o] : 0.0;
       l2[k] = ok && p.L2 ? p.L2[o] : 0.0;
       pos[fl][k] = po;
@@ -597,7 +623,7 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
 #pragma unroll 9
     for (int cv = ca; cv <= cb; cv++) {
       const int pd = pidx(ed, x - cv + 1, y - cv + 1);
-      const size_t o = (size_t)pd + (size_t)p.kk * (cv - 1);
+      const size_t o = (size_t)pd + (size_t)kk * (cv - 1);
       v += p.rkd[p.rcell * (cv - 1) + (size_t)p.rpo * pos[fl][cv - lo] +
                  (size_t)p.rpd * pd];
       v = fma(p.M1[o], c1[fl][cv - lo], v);
@@ -660,10 +686,10 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> p) {
         s1.mac(t2[fl], p.SB[rl + q1]);
       }
     }
-    const size_t o = (size_t)(f - 1) + (size_t)ns * blockIdx.y;
+    const size_t o = (size_t)(f - 1) + (size_t)ns * col;
     auto put = [&](int b, T v) {
-      p.K[((size_t)a * nb + b) * p.per + o] = v;
-      if (p.symab && a < b) p.K[((size_t)b * nb + a) * p.per + o] = v;
+      p.K[((size_t)a * nb + b) * per + o] = v;
+      if (p.symab && a < b) p.K[((size_t)b * nb + a) * per + o] = v;
     };
     if (!p.symab || a <= b0) put(b0, s0.get());
     if (b0 + 1 < nb) put(b0 + 1, s1.get());
@@ -811,6 +837,11 @@ __global__ void k_scatter_dp(int ns, int ks, char sym, QuadSpec sp, KdSet kd,
         for (int u = 0; u < EB; u++) kv[u] = K[(size_t)pairs[e + u] * per + p];
 #pragma unroll
         for (int u = 0; u < EB; u++) ffa::mac(cdf[e + u], kv[u], sh, sl);
+        // the low sum back below half an ulp of the high one, so that its own
+        // rounding does not grow with the entries
+        const float2 r = ffa::norm(sh, sl);
+        sh = r.x;
+        sl = r.y;
       }
       for (; e < sj.end; e++) ffa::mac(cdf[e], K[(size_t)pairs[e] * per + p], sh, sl);
       return ffa::value(sh, sl);
@@ -1003,113 +1034,144 @@ bool pair_potentials_fit(const dbsrg_ctx *c) {
   return c->g.ks <= FAR && c->nbound >= 1 && c->nbound <= 64;
 }
 
-// direct pair potentials of (family, type, k, case icv) with density
-// components jp1/jp2: Kd[pair][ns*ncol], cached
-int get_pairpot_direct(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1,
-                              int jp2, const double **out) {
-  return get_pairpot_direct_any(c, family, type, k, icv, jp1, jp2, false, (const void **)out);
-}
-
-int get_pairpot_direct_ff(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1, int jp2,
-                          const float2 **out) {
-  return get_pairpot_direct_any(c, family, type, k, icv, jp1, jp2, true, (const void **)out);
-}
-
-// ff: the diagonal-cell contraction in float-float arithmetic and the result
-// stored as float-float pairs (the split form's gather-sums read those)
-int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1,
-                           int jp2, bool ff, const void **out) {
-  const long long key = pairpot_key(0, family, type, k, icv, jp1, jp2, ff);
-  auto it = c->ppot.find(key);
-  if (it != c->ppot.end()) {
-    *out = it->second;
-    return DBSRG_OK;
-  }
+// direct pair potentials of up to four tables of one family, cached: Kd[pair][ns*ncol]
+// of (type, k, case icv) with density components jp1/jp2.  ff: the small
+// matrices' contraction in float-float arithmetic and the results stored as
+// float-float pairs (the split form's gather-sums read those).
+int get_pairpots_direct(dbsrg_ctx *c, int n, const PairPotKey *want, bool ff, const void **out) {
   const DeviceGrid &g = c->g;
   const int ns = g.ns, ks = g.ks, nv = g.nv, kk = ks * ks, nb = c->nbound;
   const size_t npair = (size_t)nb * nb;
-  const char sym = family == 0 ? 's' : 'n';
-  const size_t per = (size_t)ns * (sym == 's' ? ks : 2 * ks - 1);
-  int rc;
-  const CellData *cd;
-  if ((rc = get_celldata(c, family, type, k, &cd))) return rc;
+  int rc, m = 0, at[4];  // at: what builds want[i], -1 if cached
+  long long keys[4];
+  const PairPotKey *req[4];  // those to build
+  for (int i = 0; i < n; i++) {
+    const PairPotKey &w = want[i];
+    const long long key = pairpot_key(0, w.family, w.type, w.k, w.icv, w.jp1, w.jp2, ff);
+    auto it = c->ppot.find(key);
+    at[i] = -1;
+    if (it != c->ppot.end()) {
+      out[i] = it->second;
+      continue;
+    }
+    at[i] = (int)(std::find(keys, keys + m, key) - keys);
+    if (at[i] < m) continue;  // wanted twice
+    keys[m] = key;
+    req[m++] = &w;
+  }
+  if (m == 0) return DBSRG_OK;
   if ((rc = ensure_brows(c))) return rc;
-  TableBases tb = table_bases(g, family, type);
-  const PairSpec eo = icv == 1 ? tb.e1 : tb.e2, ed = icv == 1 ? tb.e2 : tb.e1;
-  const double *P1 = c->brows + (size_t)(jp1 - 1) * nb * ns;
-  const double *P2 = c->brows + (size_t)(jp2 - 1) * nb * ns;
-  const double *M1 = icv == 1 ? cd->hi2 : cd->lo1;
-  const double *M2 = (icv == 1 && family == 0) ? cd->lo2 : nullptr;
-  const int symab = ed.sym && jp1 == jp2, np = pair_count(nb, symab);
-  // scratch: SA, SB (nv x np)
+  const int family = req[0]->family;
+  const char sym = family == 0 ? 's' : 'n';
+  const int ncol = sym == 's' ? ks : 2 * ks - 1;
+  const size_t per = (size_t)ns * ncol;
+  const CellData *cd[4];
+  TableBases tb[4];
+  int np[4], symab[4], npmax = 0, k12 = 0;
+  size_t sall = 0;  // scanned sums: SA, SB (nv x np) a table
+  for (int i = 0; i < m; i++) {
+    const PairPotKey &w = *req[i];
+    if ((rc = get_celldata(c, family, w.type, w.k, &cd[i]))) return rc;
+    tb[i] = table_bases(g, family, w.type);
+    const PairSpec ed = w.icv == 1 ? tb[i].e2 : tb[i].e1;
+    symab[i] = ed.sym && w.jp1 == w.jp2;
+    np[i] = pair_count(nb, symab[i]);
+    npmax = std::max(npmax, np[i]);
+    k12 = std::max(k12, 3 * ed.k1 + ed.k2);
+    sall += 2 * (size_t)np[i] * nv;
+  }
   const int ps = c->stream == c->bstream[1] ? 1 : 0;  // scratch of this stream
   if (c->stream != c->bstream[0] && c->stream != c->bstream[1]) c->stream_built = true;
-  if ((rc = ensure_pscratch(c, ps, 2 * (size_t)np * nv * sizeof(double)))) return rc;
-  double *SA = (double *)c->pscratch[ps], *SB = M2 ? SA + (size_t)np * nv : nullptr;
-  double *K = nullptr;  // doubles, or as many float2 pairs (same bytes)
-  if (!(K = (double *)cache_alloc(c, npair * per * sizeof(double)))) {
-    cudaGetLastError();
-    return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
-  }
-  c->ppot[key] = K;
+  if ((rc = ensure_pscratch(c, ps, sall * sizeof(double)))) return rc;
+  double *K[4];  // doubles, or as many float2 pairs (same bytes)
+  for (int i = 0; i < m; i++)
+    if (!(K[i] = (double *)cache_alloc(c, npair * per * sizeof(double)))) {
+      cudaGetLastError();
+      while (i > 0) cache_free(c, K[--i]);
+      return set_err(c, DBSRG_ENOMEM, "pair potential allocation failed");
+    }
   cudaStream_t st = c->stream;
-  const size_t sm1 = (size_t)nb * (3 * ed.k1 + ed.k2) * sizeof(double);
-  if ((rc = set_smem(c, (const void *)k_pair_cellsum, sm1))) return rc;
-  DBSRG_RUN(c, "k_pair_cellsum",
-            k_pair_cellsum<<<nv, 256, sm1, st>>>(ns, kk, nb, symab, ed, M1, M2, P1, P2, SA, SB));
-  const int ofirst = (icv == 1) != cd->tr;
+  PairCellArgs ca{};
+  PairScanArgs sa{};
+  double *S = (double *)c->pscratch[ps];
+  for (int i = 0; i < m; i++) {
+    const PairPotKey &w = *req[i];
+    const bool one = w.icv == 1;
+    ca.ed[i] = one ? tb[i].e2 : tb[i].e1;
+    ca.symab[i] = symab[i];
+    ca.M1[i] = one ? cd[i]->hi2 : cd[i]->lo1;
+    ca.M2[i] = one && family == 0 ? cd[i]->lo2 : nullptr;
+    ca.P1[i] = c->brows + (size_t)(w.jp1 - 1) * nb * ns;
+    ca.P2[i] = c->brows + (size_t)(w.jp2 - 1) * nb * ns;
+    ca.S1[i] = S;
+    ca.S2[i] = ca.M2[i] ? S + (size_t)np[i] * nv : nullptr;
+    S += 2 * (size_t)np[i] * nv;
+    sa.np[i] = np[i];
+    sa.suffix0[i] = one;
+    sa.S[i][0] = ca.S1[i];
+    sa.S[i][1] = ca.S2[i];
+  }
   auto potentials = [&](auto ff_c, auto km_c) -> int {
     constexpr bool F = decltype(ff_c)::value;
     constexpr int KM = decltype(km_c)::value, PDW = pair_window(KM), PDR = pair_rows(KM);
     using T = typename Val<F>::T;
-    DBSRG_RUN(c, "k_pair_scan",
-              k_pair_scan<F><<<dim3((unsigned)((np + PSP - 1) / PSP), M2 ? 2 : 1), PSP * PSW, 0, st>>>(
-                  nv, np, icv == 1, SA, SB));
+    const size_t sm1 = (size_t)nb * k12 * sizeof(double);
     PairDirArgs<F> d{};
     d.ns = ns;
     d.nv = nv;
     d.kk = kk;
     d.nb = nb;
-    d.np = np;
-    d.symab = symab;
-    d.suf = icv == 1;
+    d.ncol = ncol;
     d.dl0 = sym == 's' ? 0 : 1 - ks;
-    d.eo = eo;
-    d.ed = ed;
-    d.rkd = cd->rkd;
-    d.rcell = (size_t)npairs(eo) * npairs(ed);
-    d.rpo = ofirst ? 1 : npairs(ed);
-    d.rpd = ofirst ? npairs(eo) : 1;
-    d.L1 = icv == 1 ? cd->lo1 : cd->hi2;
-    d.L2 = M2 ? cd->hi1 : nullptr;
-    d.M1 = M1;
-    d.M2 = M2;
-    const T *rows = F ? (const T *)c->browsf : (const T *)c->brows;
-    d.P1 = rows + (size_t)(jp1 - 1) * nb * ns;
-    d.P2 = rows + (size_t)(jp2 - 1) * nb * ns;
-    d.SA = (const T *)SA;
-    d.SB = (const T *)SB;
-    d.K = (T *)K;
-    d.per = per;
     d.bw = (std::min(nb, PDB) + 1) & ~1;
+    d.per = per;
+    const T *rows = F ? (const T *)c->browsf : (const T *)c->brows;
+    double fl = 0.0;
+    for (int i = 0; i < m; i++) {
+      const PairPotKey &w = *req[i];
+      const bool one = w.icv == 1, ofirst = one != cd[i]->tr;
+      PairDirTable<F> &t = d.t[i];
+      t.np = np[i];
+      t.symab = symab[i];
+      t.suf = one;
+      t.eo = one ? tb[i].e1 : tb[i].e2;
+      t.ed = one ? tb[i].e2 : tb[i].e1;
+      t.rkd = cd[i]->rkd;
+      t.rcell = (size_t)npairs(t.eo) * npairs(t.ed);
+      t.rpo = ofirst ? 1 : npairs(t.ed);
+      t.rpd = ofirst ? npairs(t.eo) : 1;
+      t.L1 = one ? cd[i]->lo1 : cd[i]->hi2;
+      t.L2 = ca.M2[i] ? cd[i]->hi1 : nullptr;
+      t.M1 = ca.M1[i];
+      t.M2 = ca.M2[i];
+      t.P1 = rows + (size_t)(w.jp1 - 1) * nb * ns;
+      t.P2 = rows + (size_t)(w.jp2 - 1) * nb * ns;
+      t.SA = (const T *)ca.S1[i];
+      t.SB = (const T *)ca.S2[i];
+      t.K = (T *)K[i];
+      // executed work: an output's n = k - |dl| cells hold r = n + k - 1 functions
+      // and a banded matrix of r^2 - n (n - 1) elements: as many multiply-adds per
+      // second orbital, r + 2 per pair; the potentials written
+      for (int col = 0; col < ncol; col++) {
+        const int x = std::min(t.eo.k1, t.eo.k2) - std::abs(d.dl0 + col);
+        if (x <= 0) continue;
+        const double r = x + t.ed.k1 - 1;
+        fl += 2.0 * ns * ((r * r - x * (x - 1.0)) * nb + (r + 2.0) * np[i]);
+      }
+    }
     const size_t smem = sizeof(T) * ((size_t)PDX * PDW * (PDW + d.bw) + PDR * d.bw +
                                      (size_t)PDR * pair_row_stride(nb));
-    const int frc = set_smem(c, (const void *)k_pair_direct<F, KM>, smem);
+    int frc = set_smem(c, (const void *)k_pair_cellsum, sm1);
+    if (!frc) frc = set_smem(c, (const void *)k_pair_direct<F, KM>, smem);
     if (frc) return frc;
-    // executed work: an output's n = k - |dl| cells hold r = n + k - 1 functions
-    // and a banded matrix of r^2 - n (n - 1) elements: as many multiply-adds per
-    // second orbital, r + 2 per pair; the potentials written
-    const int ncol = (int)(per / ns);
-    double fl = 0.0;
-    for (int col = 0; col < ncol; col++) {
-      const int dl = d.dl0 + col, n = std::min(eo.k1, eo.k2) - std::abs(dl);
-      if (n <= 0) continue;
-      const double r = n + ed.k1 - 1;
-      fl += 2.0 * ns * ((r * r - n * (n - 1.0)) * nb + (r + 2.0) * np);
-    }
-    const dim3 gd((unsigned)((ns + PDX - 1) / PDX), (unsigned)ncol,
+    DBSRG_RUN(c, "k_pair_cellsum",
+              k_pair_cellsum<<<dim3(nv, m), 256, sm1, st>>>(ns, kk, nb, ca));
+    DBSRG_RUN(c, "k_pair_scan",
+              k_pair_scan<F><<<dim3((unsigned)((npmax + PSP - 1) / PSP), 2 * m), PSP * PSW, 0,
+                               st>>>(nv, sa));
+    const dim3 gd((unsigned)((ns + PDX - 1) / PDX), (unsigned)(ncol * m),
                   (unsigned)((nb + PDB - 1) / PDB));
-    DBSRG_RUN_W(c, "k_pair_direct", 8.0 * (double)per * npair, fl,
+    DBSRG_RUN_W(c, "k_pair_direct", 8.0 * (double)per * npair * m, fl,
                 (k_pair_direct<F, KM><<<gd, PDT, smem, st>>>(d)));
     return DBSRG_OK;
   };
@@ -1119,8 +1181,15 @@ int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, i
     rc = ff ? potentials(std::true_type(), k9) : potentials(std::false_type(), k9);
   else
     rc = ff ? potentials(std::true_type(), kmax) : potentials(std::false_type(), kmax);
+  for (int i = 0; i < m; i++) {
+    if (rc)
+      cache_free(c, K[i]);
+    else
+      c->ppot[keys[i]] = K[i];
+  }
   if (rc) return rc;
-  *out = K;
+  for (int i = 0; i < n; i++)
+    if (at[i] >= 0) out[i] = K[at[i]];
   return DBSRG_OK;
 }
 
@@ -1328,14 +1397,17 @@ int factored_contract(dbsrg_ctx *c, const FactorJob &j) {
   if (j.dseg) return direct_segments(c, j);
   // direct, from the pair potentials
   KdSet kd{};
+  const bool ff = j.split && j.cdf;
+  PairPotKey want[4];
+  const void *got[4];
+  for (int a = 0; a < j.na; a++)
+    want[a] = {j.family, j.types[a], j.kpol, j.icv, j.jp1[a], j.jp2[a]};
+  if ((rc = get_pairpots_direct(c, j.na, want, ff, got))) return rc;
   for (int a = 0; a < j.na; a++) {
-    if (j.split && j.cdf)
-      rc = get_pairpot_direct_ff(c, j.family, j.types[a], j.kpol, j.icv, j.jp1[a], j.jp2[a],
-                                 &kd.Kf[a]);
+    if (ff)
+      kd.Kf[a] = (const float2 *)got[a];
     else
-      rc = get_pairpot_direct(c, j.family, j.types[a], j.kpol, j.icv, j.jp1[a], j.jp2[a],
-                              &kd.K[a]);
-    if (rc) return rc;
+      kd.K[a] = (const double *)got[a];
   }
   if (j.prep) return DBSRG_OK;
   const size_t space = (size_t)4 * ns * (2 * ks - 1);

@@ -515,15 +515,12 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x);
 bool pair_potentials_fit(const dbsrg_ctx *c);
 // Direct pair potentials of table (family, type, k) for convol case icv with
 // density components jp1/jp2: Kd[pair][ns*ncol] over the ordered bound-orbital
-// pairs (pair = a*nbound + b), cached until release_tables/set_orbitals.
-int get_pairpot_direct(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1, int jp2,
-                       const double **out);
-// the same potentials as float-float pairs, the diagonal cells contracted in
-// float-float arithmetic (the split form's direct sums)
-int get_pairpot_direct_ff(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1, int jp2,
-                          const float2 **out);
-int get_pairpot_direct_any(dbsrg_ctx *c, int family, int type, int k, int icv, int jp1, int jp2,
-                           bool ff, const void **out);
+// pairs (pair = a*nbound + b), cached until release_tables/set_orbitals; up to
+// four tables of one family, in FP64 or (ff) as float-float pairs
+struct PairPotKey {
+  int family, type, k, icv, jp1, jp2;
+};
+int get_pairpots_direct(dbsrg_ctx *c, int n, const PairPotKey *want, bool ff, const void **out);
 // ---- device helpers ---------------------------------------------------------
 // Values of the kx B-splines that are nonzero on the interval starting at
 // knot tx(kg) (1-based), at point x: the ni=1, nderiv=1 path of zbsplvd /

@@ -916,21 +916,22 @@ int exec_structures(dbsrg_ctx *c, const StructPlan &P, int w, bool prep) {
   const double *tabs[4] = {nullptr, nullptr, nullptr, nullptr};
   StPots pt{};
   pt.na = P.na;
-  if (P.family >= 0)
+  if (P.family >= 0 && P.fact) {
+    // convol case 2 of an R^k table is case 1 of the table with the electrons
+    // exchanged (types 2 and 3 swapped)
+    const bool sw = P.family == 0 && P.icv == 2;
+    PairPotKey want[4];
+    for (int a = 0; a < P.na; a++)
+      want[a] = {P.family, sw && P.ttype[a] >= 2 ? 5 - P.ttype[a] : P.ttype[a], P.kpol,
+                 sw ? 1 : P.icv, P.dc1[a], P.dc2[a]};
+    if ((rc = get_pairpots_direct(c, P.na, want, false, (const void **)pt.Y))) return rc;
+  } else if (P.family >= 0) {
     for (int a = 0; a < P.na; a++) {
-      if (P.fact) {
-        // convol case 2 of an R^k table is case 1 of the table with the
-        // electrons exchanged (types 2 and 3 swapped)
-        const bool sw = P.family == 0 && P.icv == 2;
-        const int t = sw && P.ttype[a] >= 2 ? 5 - P.ttype[a] : P.ttype[a];
-        rc = get_pairpot_direct(c, P.family, t, P.kpol, sw ? 1 : P.icv, P.dc1[a], P.dc2[a],
-                                &pt.Y[a]);
-      } else {
-        rc = P.family == 0 ? get_rtable(c, P.ttype[a], P.kpol, &tabs[a])
-                           : get_stable(c, P.ttype[a], P.kpol, &tabs[a]);
-      }
+      rc = P.family == 0 ? get_rtable(c, P.ttype[a], P.kpol, &tabs[a])
+                         : get_stable(c, P.ttype[a], P.kpol, &tabs[a]);
       if (rc) return rc;
     }
+  }
   if (prep) return DBSRG_OK;
   if (P.nlv > 0 && !c->hd) return set_err(c, DBSRG_ESTATE, "L_data: no one-electron matrices");
   const double *vch;

@@ -162,14 +162,16 @@ def test_bound_orbital_limit_of_the_factored_forms():
 
 
 @pytest.mark.parametrize("precision,tol", [(FACTOR_FP64, 1e-12), (SPLIT_BF16, 1e-10)])
-@pytest.mark.parametrize("ns,nch,norb,routes", [(61, 9, 20, "both"), (64, 3, 20, "segment"),
-                                                (62, 8, 30, "segment"), (60, 13, 4, "both")])
+@pytest.mark.parametrize("ns,nch,norb,routes", [(61, 9, 60, "segment"), (64, 3, 60, "segment"),
+                                                (62, 8, 20, "pairs"), (60, 13, 4, "pairs")])
 def test_direct_lists_by_segment_and_by_pairs(precision, tol, ns, nch, norb, routes):
     """The direct lists (R^k, S^k structures 6, 7, 16 and 17, channel pairs in
     both orders) segment by segment -- more segments than the 32 of a warp,
     fewer, odd and even ns -- and through the pair potentials, whichever the
     list's counts select; every block against the oracle."""
-    w = synth.small(ns=ns, nch=nch, mk=2, n_entries=60 * nch, breit=True, seed=71, norb=norb)
+    orbs = [(n + 1 + i // 30, k) for i, (n, k) in enumerate(synth.TARGET_ORBITALS * 2)][:norb]
+    kappas = [-1, 1, -2, 2, -3, 3, -4, 4, -5, 5, -6, 6, -7][:nch]
+    w = synth._build("direct", 700 + ns, ns, 20.0, 8.0, orbs, kappas, 2, 60 * nch, 1.0, breit=True)
     lists = [L for L in w.lists if (L.icase, L.itype) in ((2, 3), (3, 6), (3, 16))]
     for L in list(lists):
         if L.icase == 3 and L.kpol % 2:  # the density on the first electron
@@ -184,8 +186,8 @@ def test_direct_lists_by_segment_and_by_pairs(precision, tol, ns, nch, norb, rou
     used = a.timing_report()
     h, acf = a.get_matrix(), a.get_acf()
     a.close()
-    assert "k_seg_apply" in used
-    assert ("k_scatter_dp" in used) == (routes == "both")
+    assert ("k_seg_apply" in used) == (routes == "segment")
+    assert ("k_scatter_dp" in used) == (routes == "pairs")
     ref, racf = oracle(w, lists)
     check(h, ref, tol)
     assert relmax(acf, racf) <= 1e-12
