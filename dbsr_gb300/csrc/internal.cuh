@@ -47,12 +47,15 @@ struct CellData {
   // rkd[(pair1 + np1 pair2) + cell np1 np2] (np1, np2 the numbers of pairs of the
   // two indices) and the same as float-float pairs
   float2 *rkf = nullptr;
+  // sums of the four moment arrays over all cells, per function pair (built with
+  // the first table that is filled from them, moment_sums)
+  double *tlo1 = nullptr, *thi1 = nullptr, *tlo2 = nullptr, *thi2 = nullptr;
   bool tr = false;
 };
 
 // what the R^k tables of one k are made of
 struct RCells {
-  double *mom = nullptr;  // moments of P pairs r^k, r^-(k+1), of Q pairs r^k, r^-(k+1)
+  double *mom = nullptr;  // moments of P pairs r^k, r^-(k+1), of Q pairs r^k, r^-(k+1), their sums
   double *diag[3] = {nullptr, nullptr, nullptr};  // rkd and rkf of types 0, 1, 2
 };
 

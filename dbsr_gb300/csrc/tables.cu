@@ -479,14 +479,51 @@ __device__ __forceinline__ int tri_index(int h, int hp, int kx) {  // 1-based
   return (h - 1) * kx - ((h - 1) * (h - 2)) / 2 + (hp - h + 1);
 }
 
+// Sums over all cells of a function pair's moments, [i + ns ip] for the pair
+// (i, i+ip) of one basis ('s', ip = 0..ks-1) or (i, i+ip-ks+1) of two: a table
+// element whose two electrons' pairs share no cell is the product of two of them.
+// up to four arrays per launch (blockIdx.y)
+struct TotalSet {
+  int k1[4], k2[4], sym[4];
+  const double *M[4];
+  double *T[4];
+};
+
+__global__ void k_moment_sums(int ns, int ks, int nv, const TotalSet ts) {
+  const int y = blockIdx.y, k1 = ts.k1[y], k2 = ts.k2[y], sym = ts.sym[y], kk = ks * ks;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= ns * (sym ? ks : 2 * ks - 1)) return;
+  const int i = q % ns + 1, off = q / ns - (sym ? 0 : ks - 1);  // second function i + off
+  const double *M = ts.M[y];
+  double s = 0.0;
+  // (first function's places nine at a time, their loads in flight together)
+  for (int h0 = max(1, 1 - off); h0 <= min(k1, k2 - off); h0 += 9) {
+    double v[9];
+#pragma unroll
+    for (int u = 0; u < 9; u++) {
+      const int h = h0 + u, iv = i - h + 1;
+      const bool ok = h <= min(k1, k2 - off) && iv >= 1 && iv <= nv;
+      const int p = sym ? (h - 1) * k1 - ((h - 1) * (h - 2)) / 2 + off : (h - 1) * k2 + h + off - 1;
+      v[u] = ok ? M[(size_t)p + (size_t)kk * (iv - 1)] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 9; u++) s += v[u];
+  }
+  ts.T[y][q] = s;
+}
+
 // band > 0: only the elements with |j - i| <= band, stored as
 // rkb(i, j-i+band+1, ip, jp) of shape (ns, 2*band+1, ks, ks) -- all that the
 // band part of the factored exchange reads.
 // Up to three tables per launch (blockIdx.y); tr: rkd has the electron-2 pair
-// first.
+// first.  Bound by the FP64 pipe in the elements whose pairs share cells; the
+// others, two thirds of a band and most of a whole table, are one product of
+// k_moment_sums' sums.  ns 283, bands of three types 86 -> 44 us (S^k, one type
+// 55 -> 33), ns 400 120 -> 59 (77 -> 45), against a loop over the cells each.
 struct FillSet {
   int ka[3], kb[3], tr[3];
   const double *lowA[3], *highA[3], *lowB[3], *highB[3], *rkd[3];
+  const double *TlowA[3], *ThighA[3], *TlowB[3], *ThighB[3];  // k_moment_sums
   double *rkb[3];
 };
 
@@ -512,6 +549,15 @@ __global__ void k_fill_r(int ns, int ks, int nv, const FillSet fs, int band) {
   if (ip <= ka && jp <= kb && j >= 1 && j <= ns) {
     const int ivlo = max(1, i - ka + ip), ivhi = min(nv, i);
     const int jvlo = max(1, j - kb + jp), jvhi = min(nv, j);
+    const int ti = i - 1 + ns * (ip - 1), tj = j - 1 + ns * (jp - 1);
+    if (ivhi < jvlo) {
+      rkb[q] = fs.TlowA[y][ti] * fs.ThighB[y][tj];
+      return;
+    }
+    if (jvhi < ivlo) {
+      rkb[q] = fs.ThighA[y][ti] * fs.TlowB[y][tj];
+      return;
+    }
     // moment positions of the electron-1 pair in cell iv and the electron-2
     // pair in cell jv
     auto ia = [&](int iv) {
@@ -555,8 +601,8 @@ __global__ void k_fill_r(int ns, int ks, int nv, const FillSet fs, int band) {
 // S^k table fill: msk_ppqq / msk_pqqp, dbsr_lib_dbs.f90:3601-3662,
 // 3771-3833.  Only cells iv <= jv; band offsets ip = ihp-ih+ks.
 __global__ void k_fill_s(int ns, int ks, int nv, int ksp, int ksq, int kj1, int kj2,
-                         const double *r1, const double *r2, const double *rkd, double *rkb,
-                         int band) {
+                         const double *r1, const double *r2, const double *T1, const double *T2,
+                         const double *rkd, double *rkb, int band) {
   const int kb2 = 2 * ks - 1, kk = ks * ks;
   size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nj = band > 0 ? 2 * band + 1 : ns;
@@ -580,6 +626,14 @@ __global__ void k_fill_s(int ns, int ks, int nv, int ksp, int ksq, int kj1, int 
   const int jhlo = max(1, ks - jp + 1), jhhi = min(kj1, ks - jp + kj2);
   const int ivlo = max(1, i - ihhi + 1), ivhi = min(nv, i - ihlo + 1);
   const int jvlo = max(1, j - jhhi + 1), jvhi = min(nv, j - jhlo + 1);
+  if (ivlo > ivhi || jvlo > jvhi || jvhi < ivlo) {
+    rkb[q] = 0.0;
+    return;
+  }
+  if (ivhi < jvlo) {
+    rkb[q] = T1[i - 1 + ns * (ip - 1)] * T2[j - 1 + ns * (jp - 1)];
+    return;
+  }
   auto ia = [&](int iv) {  // (ii - 1) and the cell offset of electron 1
     const int ih = i - iv + 1;
     return (size_t)((ih - 1) * ksq + ip + ih - ks - 1);
@@ -633,8 +687,9 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
   }
   const TableBases tb = table_bases(g, family, type);
   const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
+  const size_t ts1 = (size_t)g.ns * (2 * g.ks - 1);  // sums of one moment array
   double *base = nullptr;
-  if (!(base = (double *)cache_alloc(c, (2 * m + 2 * f) * sizeof(double))))
+  if (!(base = (double *)cache_alloc(c, (2 * m + 2 * f + 2 * ts1) * sizeof(double))))
     return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
   CellData cd;
   cd.lo1 = base;
@@ -669,7 +724,8 @@ int ensure_r_cells(dbsrg_ctx *c, int k) {
   RCells &r = c->rshare[k];
   if (c->rcell[(size_t)k * 4].rkd) return DBSRG_OK;
   int rc;
-  if (!r.mom && !(r.mom = (double *)cache_alloc(c, 4 * m * sizeof(double))))
+  const size_t ts1 = (size_t)g.ns * g.ks;  // sums of one moment array
+  if (!r.mom && !(r.mom = (double *)cache_alloc(c, 4 * (m + ts1) * sizeof(double))))
     return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
   const int wh[4] = {0, 0, 1, 1}, kp[4] = {k, -(k + 1), k, -(k + 1)};
   double *const mo[4] = {r.mom, r.mom + m, r.mom + 2 * m, r.mom + 3 * m};
@@ -701,6 +757,52 @@ int ensure_r_cells(dbsrg_ctx *c, int k) {
   return DBSRG_OK;
 }
 
+// the sums of table (family, type, k)'s moments, R^k those of all types of the k
+static int moment_sums(dbsrg_ctx *c, int family, int type, int k) {
+  const DeviceGrid &g = c->g;
+  TotalSet ts{};
+  int n;
+  auto set = [&](int i, const PairSpec &e, const double *M, double *T) {
+    ts.k1[i] = e.k1;
+    ts.k2[i] = e.k2;
+    ts.sym[i] = e.sym;
+    ts.M[i] = M;
+    ts.T[i] = T;
+  };
+  if (family == 0) {
+    CellData *cd = &c->rcell[(size_t)k * 4];
+    if (cd[0].tlo1) return DBSRG_OK;
+    n = 4;
+    const size_t per = (size_t)g.ns * g.ks;
+    double *T = c->rshare[k].mom + 4 * (size_t)g.ks * g.ks * g.nv;
+    for (int t = 0; t < 4; t++) {
+      const bool pa = t == 0 || t == 2, pb = t == 0 || t == 3;
+      cd[t].tlo1 = T + (pa ? 0 : 2 * per);
+      cd[t].thi1 = cd[t].tlo1 + per;
+      cd[t].tlo2 = T + (pb ? 0 : 2 * per);
+      cd[t].thi2 = cd[t].tlo2 + per;
+    }
+    for (int b = 0; b < 2; b++) {  // electron 1 of types 0 and 1: the P and Q pairs
+      const PairSpec e = table_bases(g, 0, b).e1;
+      set(2 * b, e, cd[b].lo1, cd[b].tlo1);
+      set(2 * b + 1, e, cd[b].hi1, cd[b].thi1);
+    }
+  } else {
+    CellData &cd = c->scell[(size_t)k * 2 + type];
+    if (cd.tlo1) return DBSRG_OK;
+    n = 2;
+    const TableBases tb = table_bases(g, 1, type);
+    cd.tlo1 = (double *)(cd.rkf + (size_t)npairs(tb.e1) * npairs(tb.e2) * g.nv);
+    cd.thi2 = cd.tlo1 + (size_t)g.ns * (2 * g.ks - 1);
+    set(0, tb.e1, cd.lo1, cd.tlo1);
+    set(1, tb.e2, cd.hi2, cd.thi2);
+  }
+  const int m = g.ns * (family == 0 ? g.ks : 2 * g.ks - 1);
+  DBSRG_RUN(c, "k_moment_sums", k_moment_sums<<<dim3((m + 127) / 128, n), 128, 0, c->stream>>>(
+                                    g.ns, g.ks, g.nv, ts));
+  return DBSRG_OK;
+}
+
 // fills n (1..3) R^k tables of one k, full (band 0) or band-limited
 static int fill_r(dbsrg_ctx *c, int n, const int *types, int k, double *const *tab, int band) {
   const DeviceGrid &g = c->g;
@@ -710,8 +812,12 @@ static int fill_r(dbsrg_ctx *c, int n, const int *types, int k, double *const *t
   for (int i = 0; i < n; i++) {
     const CellData *cd;
     int rc = get_celldata(c, 0, types[i], k, &cd);
-    if (rc) return rc;
+    if (rc || (rc = moment_sums(c, 0, types[i], k))) return rc;
     const TableBases tb = table_bases(g, 0, types[i]);
+    fs.TlowA[i] = cd->tlo1;
+    fs.ThighA[i] = cd->thi1;
+    fs.TlowB[i] = cd->tlo2;
+    fs.ThighB[i] = cd->thi2;
     fs.ka[i] = tb.e1.k1;
     fs.kb[i] = tb.e2.k1;
     fs.tr[i] = cd->tr;
@@ -776,11 +882,16 @@ static int get_table_any(dbsrg_ctx *c, int family, int type, int k, int band,
   if (family == 0) {
     if ((rc = fill_r(c, 1, &type, k, &tab, band))) return rc;
   } else {
+    if ((rc = moment_sums(c, 1, type, k))) {
+      cache_free(c, tab);
+      return rc;
+    }
     const unsigned nb = (unsigned)((nt + 255) / 256);
     int kj1 = type == 0 ? g.ksp : g.ksq, kj2 = type == 0 ? g.ksq : g.ksp;
     DBSRG_RUN(c, "k_fill_s",
               k_fill_s<<<nb, 256, 0, c->stream>>>(ns, ks, nv, g.ksp, g.ksq, kj1, kj2, cd->lo1,
-                                                  cd->hi2, cd->rkd, tab, band));
+                                                  cd->hi2, cd->tlo1, cd->thi2, cd->rkd, tab,
+                                                  band));
   }
   v[idx] = tab;
   *out = tab;

@@ -235,3 +235,22 @@ def test_asymptotic_coefficients_at_other_spline_orders(ks, ksp, ksq):
     a.close()
     assert np.abs(m.acf).max() > 0 and relmax(acf, m.acf) <= PLAIN
     assert relmax(h, m.hch) <= PLAIN
+
+
+@pytest.mark.parametrize("ks,ksp,ksq,ns", [(3, 2, 3, 9), (4, 3, 4, 23), (9, 8, 9, 40), (11, 10, 11, 35)])
+def test_tables_at_other_orders(ks, ksp, ksq, ns):
+    """R^k and S^k tables whose elements' pairs share cells, meet at one and share
+    none.  Elements of disjoint pairs are products of two sums of up to ks
+    positive moments: relative to themselves some tens of roundings, 1e-12 each."""
+    t = np.concatenate([np.zeros(ks - 1), np.linspace(0.0, 1.0, ns - ks + 2) ** 2 * 9.0,
+                        np.full(ks - 1, 9.0)])
+    a, g = Assembler(t, ks, ksp, ksq), O.Grid(t, ks, ksp, ksq)
+    for k in (0, 3):
+        for fam, typs, ref in ((RK, range(4), g.mrk), (SK, range(2), g.msk)):
+            for typ in typs:
+                x, r = a.get_table(fam, typ, k), ref(typ, k)
+                assert relmax(x, r) <= TIGHT
+                far = np.abs(np.subtract.outer(np.arange(ns), np.arange(ns))) >= 2 * ks - 1
+                x, r = x[far], r[far]
+                assert np.all(np.abs(x - r) <= 1e-12 * np.abs(r)), (fam, typ, k)
+    a.close()
