@@ -351,11 +351,16 @@ __global__ void k_sum_parts(size_t n, int nz, const double *P, double *A) {
 // exchange contraction, convol case 3 with 's','s' storage
 // (dbsr_lib_dbs.f90:2344-2356) and cases 3/4 with 'n','n' storage
 // (:2370-2378, :2418-2426; convol_sk :2632-2640, :2690-2698), written as a
-// gather: one thread owns output a(x,y) of NB segments and sums the table
-// entries that the reference scatters into it.
-constexpr int XNB = 4;
+// gather: one thread owns output a(x,y) of XNB segments and sums the table
+// entries that the reference scatters into it.  Bound by the loads in flight of
+// short lists, by the FP64 pipe of long ones.  ns 101, 15 segments: 105 us (floor of
+// the FP64 pipe 80); 144 us with four segments a thread and branches around the
+// terms that the grid's ends cut off, 139 with four and 103 with one segment.  ns 120, 40
+// channels: 4.4 ms a list with two or four, 5.2 with one, which reads the table
+// twice as often.
+constexpr int XNB = 2, XNT = 128, XUN = 3;
 
-__global__ void __launch_bounds__(256) k_exchange(int ns, int ks, int mode, int nsg,
+__global__ void __launch_bounds__(XNT) k_exchange(int ns, int ks, int mode, int nsg,
                                                  const double *__restrict__ rkb,
                                                  const double *__restrict__ D,
                                                  double *__restrict__ A) {
@@ -376,62 +381,48 @@ __global__ void __launch_bounds__(256) k_exchange(int ns, int ks, int mode, int 
   auto DV = [&](int b, int i, int j) -> double {
     return __ldg(&Db[(size_t)b * nn + (size_t)(i - 1) + (size_t)ns * (size_t)(j - 1)]);
   };
+  // one term: density element (i, j), table element (ti, tj, ip, jp); the loads of
+  // a term that does not exist are predicated away, not branched around, so that
+  // those of several terms are in flight together
+  auto term = [&](bool ok, int i, int j, int ti, int tj, int ip, int jp, int kb) {
+    const double c = ok ? TB(ti, tj, ip, jp, kb) : 0.0;
+#pragma unroll
+    for (int b = 0; b < XNB; b++) {
+      const double d = ok && b < nb ? DV(b, i, j) : 0.0;
+      acc[b] = fma(c, d, acc[b]);
+    }
+  };
   if (mode == 0) {  // R table, 's','s', case 3: four symmetric terms
     for (int jp = 1; jp <= ks; jp++) {
+      const bool y1 = y - jp + 1 >= 1, y2 = jp > 1 && y + jp - 1 <= ns;
+#pragma unroll XUN
       for (int ip = 1; ip <= ks; ip++) {
+        const bool x1 = x + ip - 1 <= ns, x2 = ip > 1 && x - ip + 1 >= 1;
         // T1: a(i,jj) += c*d(ii,j), i=x, jj=y -> j=y-jp+1, ii=x+ip-1
-        if (y - jp + 1 >= 1 && x + ip - 1 <= ns) {
-          double c = TB(x, y - jp + 1, ip, jp, ks);
-#pragma unroll
-          for (int b = 0; b < XNB; b++)
-            if (b < nb) acc[b] = fma(c, DV(b, x + ip - 1, y - jp + 1), acc[b]);
-        }
+        term(y1 && x1, x + ip - 1, y - jp + 1, x, y - jp + 1, ip, jp, ks);
         // T2 (ip>1): a(ii,jj) += c*d(i,j): ii=x -> i=x-ip+1, jj=y -> j=y-jp+1
-        if (ip > 1 && x - ip + 1 >= 1 && y - jp + 1 >= 1) {
-          double c = TB(x - ip + 1, y - jp + 1, ip, jp, ks);
-#pragma unroll
-          for (int b = 0; b < XNB; b++)
-            if (b < nb) acc[b] = fma(c, DV(b, x - ip + 1, y - jp + 1), acc[b]);
-        }
+        term(y1 && x2, x - ip + 1, y - jp + 1, x - ip + 1, y - jp + 1, ip, jp, ks);
         // T3 (jp>1): a(i,j) += c*d(ii,jj): i=x, j=y
-        if (jp > 1 && x + ip - 1 <= ns && y + jp - 1 <= ns) {
-          double c = TB(x, y, ip, jp, ks);
-#pragma unroll
-          for (int b = 0; b < XNB; b++)
-            if (b < nb) acc[b] = fma(c, DV(b, x + ip - 1, y + jp - 1), acc[b]);
-        }
+        term(y2 && x1, x + ip - 1, y + jp - 1, x, y, ip, jp, ks);
         // T4 (ip>1,jp>1): a(ii,j) += c*d(i,jj): ii=x -> i=x-ip+1, j=y
-        if (ip > 1 && jp > 1 && x - ip + 1 >= 1 && y + jp - 1 <= ns) {
-          double c = TB(x - ip + 1, y, ip, jp, ks);
-#pragma unroll
-          for (int b = 0; b < XNB; b++)
-            if (b < nb) acc[b] = fma(c, DV(b, x - ip + 1, y + jp - 1), acc[b]);
-        }
+        term(y2 && x2, x - ip + 1, y + jp - 1, x - ip + 1, y, ip, jp, ks);
       }
     }
   } else {  // S table 'n','n' (kb = 2ks-1)
     const int kb = 2 * ks - 1;
     for (int jp = 1; jp <= kb; jp++) {
+      // case 3: a(i,jj) += c*d(ii,j), i=x, jj=y -> j=y-jp+ks, ii=x+ip-ks;
+      // case 4: a(ii,j) += c*d(i,jj), ii=x -> i=x-ip+ks, j=y, jj=y+jp-ks
+      const int j = mode == 1 ? y - jp + ks : y, jj = mode == 1 ? y : y + jp - ks;
+      if (j < max(1, 1 + ks - jp) || j > min(ns, ns + ks - jp)) continue;
+#pragma unroll 4 * XUN
       for (int ip = 1; ip <= kb; ip++) {
-        if (mode == 1) {
-          // case 3: a(i,jj) += c*d(ii,j), i=x, jj=y -> j=y-jp+ks, ii=x+ip-ks
-          int j = y - jp + ks, ii = x + ip - ks;
-          if (j < max(1, 1 + ks - jp) || j > min(ns, ns + ks - jp)) continue;
-          if (x < max(1, 1 + ks - ip) || x > min(ns, ns + ks - ip)) continue;
-          double c = TB(x, j, ip, jp, kb);
-#pragma unroll
-          for (int b = 0; b < XNB; b++)
-            if (b < nb) acc[b] = fma(c, DV(b, ii, j), acc[b]);
-        } else {
-          // case 4: a(ii,j) += c*d(i,jj), ii=x -> i=x-ip+ks, j=y, jj=y+jp-ks
-          int i = x - ip + ks, jj = y + jp - ks;
-          if (y < max(1, 1 + ks - jp) || y > min(ns, ns + ks - jp)) continue;
-          if (i < max(1, 1 + ks - ip) || i > min(ns, ns + ks - ip)) continue;
-          double c = TB(i, y, ip, jp, kb);
-#pragma unroll
-          for (int b = 0; b < XNB; b++)
-            if (b < nb) acc[b] = fma(c, DV(b, i, jj), acc[b]);
-        }
+        const int i = mode == 1 ? x : x - ip + ks, ii = mode == 1 ? x + ip - ks : x;
+        const bool ok = i >= max(1, 1 + ks - ip) && i <= min(ns, ns + ks - ip);
+        if (mode == 1)
+          term(ok, ii, j, i, j, ip, jp, kb);
+        else
+          term(ok, i, jj, i, j, ip, jp, kb);
       }
     }
   }
@@ -1163,9 +1154,9 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
         if ((rc2 = band_contract(c, P.kb, icv, tabs[a], nm, Xa, Ya))) return rc2;
       } else {
         int mode = P.tabfam == 0 ? 0 : (icv == 3 ? 1 : 2);
-        dim3 gx((unsigned)(((size_t)ns * ns + 255) / 256), (unsigned)((nm + XNB - 1) / XNB));
+        dim3 gx((unsigned)(((size_t)ns * ns + XNT - 1) / XNT), (unsigned)((nm + XNB - 1) / XNB));
         DBSRG_RUN(c, "k_exchange",
-                  k_exchange<<<gx, 256, 0, st>>>(ns, ks, mode, nm, tabs[a], Xa, Ya));
+                  k_exchange<<<gx, XNT, 0, st>>>(ns, ks, mode, nm, tabs[a], Xa, Ya));
       }
     }
     int mode = P.sym_d == 'x' ? 0 : 1;
@@ -1267,8 +1258,8 @@ int band_contract(dbsrg_ctx *c, int kb, int icase, const double *rkb, int nsg, c
 // products (dbsr_lib_dbs.f90:2344-2470)
 int exchange_contract(dbsrg_ctx *c, const double *rkb, int nsg, const double *X, double *Y) {
   const int ns = c->g.ns, ks = c->g.ks;
-  dim3 gx((unsigned)(((size_t)ns * ns + 255) / 256), (unsigned)((nsg + XNB - 1) / XNB));
-  DBSRG_RUN(c, "k_exchange", k_exchange<<<gx, 256, 0, c->stream>>>(ns, ks, 0, nsg, rkb, X, Y));
+  dim3 gx((unsigned)(((size_t)ns * ns + XNT - 1) / XNT), (unsigned)((nsg + XNB - 1) / XNB));
+  DBSRG_RUN(c, "k_exchange", k_exchange<<<gx, XNT, 0, c->stream>>>(ns, ks, 0, nsg, rkb, X, Y));
   return DBSRG_OK;
 }
 
