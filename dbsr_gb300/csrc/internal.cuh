@@ -227,6 +227,7 @@ struct dbsrg_ctx {
   // error word of the tensor-core kernels (bounded waits), read whenever the
   // context waits for its stream
   int *kerr = nullptr;
+  int *hkerr = nullptr;  // its pinned copy (drain)
   // pinned staging for host lists
   void *pinned = nullptr;
   size_t pinned_bytes = 0;
