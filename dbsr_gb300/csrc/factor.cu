@@ -80,52 +80,46 @@ __global__ void k_bound_rows(int ns, int nb, const int *b2o, const double *pq, d
 }
 
 // ---------------------------------------------------------------------------
-// far-field vectors of one electron: Ulo(x,a) = sum_iv sum_xc mlo(pair;iv) p_a(xc)
-// (and Uhi with mhi), x the output function, xc the contracted one, and their
-// float-float copies where asked for.  Both electrons' vectors (R^k: those of
-// the P and Q pairs, which every type of the k shares) in one launch
-// (blockIdx.y).  A thread sums up to ks cells of ks functions, nine loads in
-// flight: bound by the latency of those loads.  ns 283, 20 orbitals: 19 us a k,
-// against 4 x 26 us (and 8 conversions of 6 us) with a launch per type that
-// loaded one value at a time.
+// far-field vectors of one electron: Ulo(x,a) = sum_xc tlo(x,xc) p_a(xc) (and Uhi
+// with thi), x the output function, xc the contracted one, t the moments of the
+// pair summed over its cells (k_moment_sums), and their float-float copies where
+// asked for.  Both electrons' vectors (R^k: those of the P and Q pairs, which
+// every type of the k shares) in one launch (blockIdx.y).  A thread takes the up
+// to 2 ks - 1 functions xc, nine loads in flight.  ns 283, 20 orbitals: 8 us a k,
+// 15.5 summing the cells of every pair for each orbital.
 struct FarSide {
-  PairSpec e;
-  int out_first, ko, kc, ccomp;
-  const double *mlo, *mhi;
+  int sym, out_first, ccomp;  // sym: t[min + ns |xc - x|], else t[first + ns (second - first + ks-1)]
+  const double *tlo, *thi;
   double *Ulo, *Uhi;
   float2 *Flo, *Fhi;
 };
 
-__global__ void k_far_vectors(int ns, int nv, int kk, int nb, const int *b2o, const double *pq,
+__global__ void k_far_vectors(int ns, int ks, int nb, const int *b2o, const double *pq,
                               const FarSide s0, const FarSide s1) {
   const FarSide &sd = blockIdx.y ? s1 : s0;
-  const PairSpec e = sd.e;
-  const int out_first = sd.out_first, ko = sd.ko, kc = sd.kc, ccomp = sd.ccomp;
-  const double *mlo = sd.mlo, *mhi = sd.mhi;
+  const int sym = sd.sym, out_first = sd.out_first, ccomp = sd.ccomp;
+  const double *tlo = sd.tlo, *thi = sd.thi;
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= ns * nb) return;
-  int x = q % ns + 1, a = q / ns;
-  const double *p = pq + (size_t)ns * (ccomp - 1) + (size_t)2 * ns * (b2o ? b2o[a] - 1 : a) - 1;
+  const int x = q % ns, a = q / ns;  // 0-based
+  const double *p = pq + (size_t)ns * (ccomp - 1) + (size_t)2 * ns * (b2o ? b2o[a] - 1 : a);
   double slo = 0.0, shi = 0.0;
-  for (int iv = max(1, x - ko + 1); iv <= min(nv, x); iv++) {
-    const int ho = x - iv + 1;
-    for (int u0 = 0; u0 < kc; u0 += 9) {
-      double pv[9], lv[9], hv[9];
+  for (int d0 = 1 - ks; d0 < ks; d0 += 9) {
+    double pv[9], lv[9], hv[9];
 #pragma unroll
-      for (int u = 0; u < 9; u++) {
-        const int hc = u0 + u + 1, xc = iv + u0 + u;
-        const bool ok = hc <= kc && xc <= ns;
-        const size_t o = (size_t)(out_first ? pidx(e, ho, hc) : pidx(e, hc, ho)) +
-                         (size_t)kk * (iv - 1);
-        pv[u] = ok ? p[xc] : 0.0;
-        lv[u] = ok ? mlo[o] : 0.0;
-        hv[u] = ok && mhi ? mhi[o] : 0.0;
-      }
+    for (int u = 0; u < 9; u++) {
+      const int d = d0 + u, xc = x + d;
+      const bool ok = d < ks && xc >= 0 && xc < ns;
+      const int o = sym ? min(x, xc) + ns * abs(d)
+                        : (out_first ? x + ns * (d + ks - 1) : xc + ns * (ks - 1 - d));
+      pv[u] = ok ? p[xc] : 0.0;
+      lv[u] = ok ? tlo[o] : 0.0;
+      hv[u] = ok && thi ? thi[o] : 0.0;
+    }
 #pragma unroll
-      for (int u = 0; u < 9; u++) {
-        slo = fma(lv[u], pv[u], slo);
-        shi = fma(hv[u], pv[u], shi);
-      }
+    for (int u = 0; u < 9; u++) {
+      slo = fma(lv[u], pv[u], slo);
+      shi = fma(hv[u], pv[u], shi);
     }
   }
   sd.Ulo[q] = slo;
@@ -894,19 +888,21 @@ int ensure_fscratch(dbsrg_ctx *c, size_t bytes) {
 // the four R^k vectors of one k over nb orbitals (b2o null: all of them)
 static int r_far_vectors(dbsrg_ctx *c, int k, int nb, const int *b2o, double *W, float2 *Wf) {
   const DeviceGrid &g = c->g;
-  const int ns = g.ns, kk = g.ks * g.ks;
+  const int ns = g.ns;
   const size_t m = (size_t)ns * nb;
   const CellData *pp, *qq;
   int rc;
-  if ((rc = get_celldata(c, 0, 0, k, &pp)) || (rc = get_celldata(c, 0, 1, k, &qq))) return rc;
+  if ((rc = get_celldata(c, 0, 0, k, &pp)) || (rc = get_celldata(c, 0, 1, k, &qq)) ||
+      (rc = moment_sums(c, 0, 0, k)))
+    return rc;
   auto side = [&](int comp, const CellData &cd) {
-    const int o = comp == 1 ? 0 : 2, ord = comp == 1 ? g.ksp : g.ksq;
-    return FarSide{{ord, ord, 1}, 1, ord, ord, comp, cd.lo1, cd.hi1, W + o * m, W + (o + 1) * m,
+    const int o = comp == 1 ? 0 : 2;
+    return FarSide{1, 1, comp, cd.tlo1, cd.thi1, W + o * m, W + (o + 1) * m,
                    Wf ? Wf + o * m : nullptr, Wf ? Wf + (o + 1) * m : nullptr};
   };
   const dim3 gv((unsigned)((m + 63) / 64), 2);
   DBSRG_RUN(c, "k_far_vectors",
-            k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.nv, kk, nb, b2o, c->pq, side(1, *pp),
+            k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.ks, nb, b2o, c->pq, side(1, *pp),
                                                     side(2, *qq)));
   return DBSRG_OK;
 }
@@ -951,7 +947,7 @@ static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const
     return DBSRG_OK;
   }
   const DeviceGrid &g = c->g;
-  const int ns = g.ns, nb = c->nbound, kk = g.ks * g.ks;
+  const int ns = g.ns, nb = c->nbound;
   const size_t m = (size_t)ns * nb;
   const dim3 gv((unsigned)((m + 63) / 64), 2);
   const TableBases tb = table_bases(g, family, type);
@@ -974,25 +970,21 @@ static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const
     f.first = a;
   } else {
     const CellData *cd;
-    if ((rc = get_celldata(c, family, type, k, &cd))) return rc;
+    if ((rc = get_celldata(c, family, type, k, &cd)) || (rc = moment_sums(c, family, type, k)))
+      return rc;
     double *base = (double *)cache_alloc(c, 3 * m * sizeof(double));
     if (!base) return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
     f.U = base;
     f.V = base + m;
     f.Vf = (float2 *)(base + 2 * m);
-    auto ord = [&](int b) { return b == 1 ? g.ksp : g.ksq; };
-    // electron 1: case 3 output = first function, contracted = second
-    int o1f = cs == 3 ? 1 : 0;
-    int ko1 = ord(cs == 3 ? tb.a1 : tb.a2), kc1 = ord(cs == 3 ? tb.a2 : tb.a1);
-    int cc1 = cs == 3 ? tb.a2 : tb.a1;
-    // electron 2: case 3 output = second function, contracted = first
-    int o2f = cs == 3 ? 0 : 1;
-    int ko2 = ord(cs == 3 ? tb.b2 : tb.b1), kc2 = ord(cs == 3 ? tb.b1 : tb.b2);
-    int cc2 = cs == 3 ? tb.b1 : tb.b2;
-    const FarSide s1{tb.e1, o1f, ko1, kc1, cc1, cd->lo1, nullptr, f.U, nullptr, nullptr, nullptr};
-    const FarSide s2{tb.e2, o2f, ko2, kc2, cc2, cd->hi2, nullptr, f.V, nullptr, f.Vf, nullptr};
+    // electron 1: case 3 output = first function, contracted = second; electron 2:
+    // output = second, contracted = first; case 4 the other way
+    const int o1f = cs == 3 ? 1 : 0, o2f = 1 - o1f;
+    const int cc1 = cs == 3 ? tb.a2 : tb.a1, cc2 = cs == 3 ? tb.b1 : tb.b2;
+    const FarSide s1{0, o1f, cc1, cd->tlo1, nullptr, f.U, nullptr, nullptr, nullptr};
+    const FarSide s2{0, o2f, cc2, cd->thi2, nullptr, f.V, nullptr, f.Vf, nullptr};
     DBSRG_RUN(c, "k_far_vectors",
-              k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.nv, kk, nb, c->b2o, c->pq, s1, s2));
+              k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.ks, nb, c->b2o, c->pq, s1, s2));
   }
   v[idx] = f;
   *out = &v.at(idx);

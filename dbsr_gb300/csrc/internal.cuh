@@ -381,6 +381,7 @@ int far_vectors_all(dbsrg_ctx *c, int k, double *W);
 int get_rtable(dbsrg_ctx *c, int type, int k, const double **out);
 int get_stable(dbsrg_ctx *c, int type, int k, const double **out);
 int get_quad(dbsrg_ctx *c, int k, bool bound, const double **out);
+int moment_sums(dbsrg_ctx *c, int family, int type, int k);  // CellData's sums, once built
 int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out);
 // the cell data of every R^k type of one k in two launches, and the band tables
 // of types 0, 1 and 2 in one (type 3's exchange reads type 2's)

@@ -761,7 +761,7 @@ int ensure_r_cells(dbsrg_ctx *c, int k) {
 }
 
 // the sums of table (family, type, k)'s moments, R^k those of all types of the k
-static int moment_sums(dbsrg_ctx *c, int family, int type, int k) {
+int moment_sums(dbsrg_ctx *c, int family, int type, int k) {
   const DeviceGrid &g = c->g;
   TotalSet ts{};
   int n;
