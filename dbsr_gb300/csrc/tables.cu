@@ -800,6 +800,7 @@ int moment_sums(dbsrg_ctx *c, int family, int type, int k) {
     set(0, tb.e1, cd.lo1, cd.tlo1);
     set(1, tb.e2, cd.hi2, cd.thi2);
   }
+  if (c->stream != c->bstream[0] && c->stream != c->bstream[1]) c->stream_built = true;
   const int m = g.ns * (family == 0 ? g.ks : 2 * g.ks - 1);
   DBSRG_RUN(c, "k_moment_sums", k_moment_sums<<<dim3((m + 127) / 128, n), 128, 0, c->stream>>>(
                                     g.ns, g.ks, g.nv, ts));
