@@ -54,7 +54,7 @@ __global__ void k_rk_vsum(size_t per, int nup, const int *upair, KdTypes kd, dou
 // positions.  One thread per (entry, type, role, row) with 17-term sums and a
 // launch per run of entries took 355 ms of the evaluation's 367.7 (44 453
 // launches, and the terms of every entry written and read back); with this
-// kernel the evaluation takes 15.2 ms, 12 of them the pair potentials.
+// kernel the evaluation takes 5.3 ms, 2.7 of them the pair potentials.
 constexpr int MC = 128;
 constexpr int UE = 4;
 __global__ void __launch_bounds__(2 * MC) k_rk_pot(int ns, int ks, int nup, size_t per,

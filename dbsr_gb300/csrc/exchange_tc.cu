@@ -993,9 +993,11 @@ static void xfused_work(const XQuad *hxq, int nxq, int ns, int lower, int nbk, d
 // the same time whatever a record's strips cost (S^k: products on one side of the
 // diagonal only).  Strips in turn -- block b takes strips b, b + nblk, .., cut
 // into y segments where there are few -- left the busiest SM with up to 1.6 times
-// the mean: ns 283, 26 segments a list 73 -> 67 us, ns 351 106 -> 93, ns 400,
-// 80 channels 494 -> 429 us.  (Changing the blocks' places from round to round
-// instead loads an A operand for every strip: 87 us at ns 283.)
+// the mean: ns 283, 26 segments a list 73 -> 62 us, ns 351 106 -> 87, ns 400,
+// 80 channels 494 -> 383 us.  (Changing the blocks' places from round to round
+// instead loads an A operand for every strip: 87 us at ns 283.)  The products are
+// all that counts of the costs: a tile's own at 2/3 of a product's 65, 92 and
+// 425 us, at 1/6 63, 87 and 389, at 1/12 62, 87 and 383.
 constexpr int TILE_COST = 1, PROD_COST = 12;  // reading and writing a tile, one product
 
 // fills p.start; the number of blocks

@@ -28,7 +28,9 @@
 //                + sum_{pair2} rkd(pair1,pair2;iv) rho_ab(pair2)   (iv = jv)
 // Suf/Pre the suffix/prefix sums over cells of the moment-weighted density of
 // the pair, and rho_ab the pair density in the reference's storage (the
-// symmetric 's' storage sums both orders, p1(f)p2(s)+p1(s)p2(f)).
+// symmetric 's' storage sums both orders, p1(f)p2(s)+p1(s)p2(f)).  Within the
+// cells that an output belongs to, both terms are summed into one small matrix
+// before any orbital is taken (k_pair_direct).
 //
 // The per-segment work is then a sum of a few dozen potential rows per
 // output element, fused into the scatter for the direct cases.  All of this

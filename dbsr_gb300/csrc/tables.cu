@@ -716,8 +716,9 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
 // launch; every type takes two of each) and the diagonal cells of types 0, 1
 // and 2 (one launch; type 3 reads type 2's with the electrons exchanged).  A
 // list takes all types of its k, so nothing is built that it does not read.
-// ns 283: moments 4 x 18 -> 18 us a k, diagonal cells 4 x 40 -> 95 us, band
-// tables (ensure_r_band_tables) 4 x 39 -> 87 us against a launch per type.
+// ns 283, against a launch per type of the kernels of the day: moments 4 x 18 -> 18 us
+// a k (10 now), diagonal cells 4 x 40 -> 95 (50 in the mean of R^k and S^k now), band tables
+// (ensure_r_band_tables) 4 x 39 -> 87 (44 now).
 int ensure_r_cells(dbsrg_ctx *c, int k) {
   const DeviceGrid &g = c->g;
   const int nv = g.nv, kk = g.ks * g.ks;
