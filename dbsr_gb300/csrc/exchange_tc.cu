@@ -149,14 +149,18 @@ struct ZArgs {
 // exponents.  The sums read the pair potentials of every entry, and an entry
 // costs a load latency: the four warps of a block share the 17 band diagonals
 // and the two fields, so that each has few enough values an entry to load those
-// of ZEB entries together.  Long lists are bound by the L2 reads of the
-// potentials, short ones by the chain of their entries.  One warp per block,
-// one entry at a time: 72 us a launch at ns 283 and 26 segments, 177 us at
-// ns 400 and 160.
-constexpr int ZROWS = 32, ZW = 4, ZEB = 4;
+// of EB entries together.  Short lists are bound by the chain of their entries
+// and take four at once, long ones by the L2 reads of the potentials, where
+// more warps with fewer registers each serve better: two.  One warp per block,
+// one entry at a time: 72 us a launch at ns 283 and 26 segments; four warps, EB 4
+// and 2: 35 and 37 us there, 15.0 and 15.8 at ns 200, 182 and 169 at ns 400 with 80
+// channels, 381 and 349 with 120.  Two warps a block: 41, 18, 169 and 337.
+constexpr int ZROWS = 32, ZW = 4;
+// blocks an SM from which a launch is long: 6 at ns 283, 30 to 50 at ns 400
+constexpr int ZLONG = 16;
 constexpr int ZND = 5;  // most band diagonals of a warp
 // ONE: at most 32 bound orbitals (one chunk)
-template <bool ONE>
+template <bool ONE, int EB>
 __global__ void __launch_bounds__(ZROWS * ZW) k_zdigits(const ZArgs z) {
   // [mode][nb][ZROWS] float-float: per row one column; sized by the bound
   // orbitals (and the modes) in use, which sets how many blocks share an SM
@@ -208,7 +212,7 @@ __global__ void __launch_bounds__(ZROWS * ZW) k_zdigits(const ZArgs z) {
       }
       e += N;
     };
-    while (e + ZEB <= si.end) batch(std::integral_constant<int, ZEB>());
+    while (e + EB <= si.end) batch(std::integral_constant<int, EB>());
     while (e < si.end) batch(std::integral_constant<int, 1>());
     double *yb = z.Yb + ((size_t)a * z.nm + slot) * kper + (size_t)ns * d0 + y;
 #pragma unroll
@@ -1116,8 +1120,6 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
   z.ez = ez;
   z.Yb = Yb;
   const size_t zsm = (size_t)(x.lower ? 2 : 1) * nb * ZROWS * sizeof(float2);
-  const void *zk = nbk == 1 ? (const void *)k_zdigits<true> : (const void *)k_zdigits<false>;
-  if ((rc = raise_smem_limit(c, zk, zsm))) return rc;
   // executed work: per PQ type, row and entry one multiply-add per field
   // (Z, and Zl for R^k) and per band diagonal (17), float-float; the entry's
   // band potential values (17 float-float pairs a row) read, the digits and
@@ -1128,10 +1130,18 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
                     2.0 * TS * (double)x.na * (1 + x.lower) * x.nm * nbk * NR * TILE;
   // every row of the operand, zeros past ns
   const dim3 gz((unsigned)(NR * 32 / ZROWS), (unsigned)x.nm, (unsigned)x.na);
+  auto zdigits = [&](auto k) -> int {
+    const int zrc = raise_smem_limit(c, (const void *)k, zsm);
+    if (zrc) return zrc;
+    DBSRG_RUN_W(c, "k_zdigits", zb, zf, k<<<gz, ZROWS * ZW, zsm, st>>>(z));
+    return DBSRG_OK;
+  };
+  const bool zlong = (double)gz.x * gz.y * gz.z > (double)ZLONG * c->nsm;
   if (nbk == 1)
-    DBSRG_RUN_W(c, "k_zdigits", zb, zf, k_zdigits<true><<<gz, ZROWS * ZW, zsm, st>>>(z));
+    rc = zlong ? zdigits(k_zdigits<true, 2>) : zdigits(k_zdigits<true, 4>);
   else
-    DBSRG_RUN_W(c, "k_zdigits", zb, zf, k_zdigits<false><<<gz, ZROWS * ZW, zsm, st>>>(z));
+    rc = zlong ? zdigits(k_zdigits<false, 2>) : zdigits(k_zdigits<false, 4>);
+  if (rc) return rc;
   XArgs p{};
   p.ns = ns;
   p.NR = NR;

@@ -231,3 +231,17 @@ def test_pair_potentials_on_small_grids(precision, tol, ks, ksp, ksq, ns):
     ref, racf = oracle(w, lists)
     check(h, ref, tol)
     assert relmax(acf, racf) <= 1e-12
+
+
+def test_long_exchange_lists_in_entry_pairs():
+    """A launch of enough segments that the Z digits take two entries at once
+    (blocks of 32 rows, segments and types beyond sixteen an SM), segments with odd
+    and even numbers of entries; every block against the oracle."""
+    kappas = [-1, 1, -2, 2, -3, 3, -4, 4, -5, 5] * 5
+    w = synth._build("long", 611, 60, 20.0, 8.0, synth.TARGET_ORBITALS[:4], kappas, 1,
+                     8 * 1275, 0.5, breit=False)
+    L = max((L for L in w.lists if (L.icase, L.itype) == (2, 4)), key=lambda L: len(set(L.k1)))
+    assert 2 * 4 * len(set(L.k1)) > 16 * 152
+    h, _ = run(w, SPLIT_BF16, [L])
+    ref, _ = oracle(w, [L])
+    check(h, ref, 1e-10)
