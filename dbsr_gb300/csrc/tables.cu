@@ -735,14 +735,15 @@ int ensure_r_cells(dbsrg_ctx *c, int k) {
   double *const mo[4] = {r.mom, r.mom + m, r.mom + 2 * m, r.mom + 3 * m};
   if ((rc = compute_moment_set(c, 4, wh, kp, mo))) return rc;
   TriSet ts{};
-  for (int t = 0; t < 3; t++) {
+  for (int i = 0; i < 3; i++) {
+    const int t = 2 - i;  // the largest first: the blocks that end the launch are short
     const TableBases tb = table_bases(g, 0, t);
     const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
     if (!r.diag[t] && !(r.diag[t] = (double *)cache_alloc(c, 2 * f * sizeof(double))))
       return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
-    ts.type[t] = t;
-    ts.rkd[t] = r.diag[t];
-    ts.rkf[t] = (float2 *)(r.diag[t] + f);
+    ts.type[i] = t;
+    ts.rkd[i] = r.diag[t];
+    ts.rkf[i] = (float2 *)(r.diag[t] + f);
   }
   if ((rc = compute_diag_set(c, 3, ts, k))) return rc;
   for (int t = 0; t < 4; t++) {
