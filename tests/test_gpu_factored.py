@@ -196,10 +196,10 @@ def test_direct_lists_by_segment_and_by_pairs(precision, tol, ns, nch, norb, rou
 @pytest.mark.parametrize("ns,nch,norb,per_slot", [(60, 1, 3, 20), (61, 2, 20, 7), (130, 3, 33, 9),
                                                   (257, 2, 6, 5)])
 def test_exchange_strips_and_entry_batches(ns, nch, norb, per_slot):
-    """Exchange lists whose strips are split into y segments (one channel: few
-    strips; ns above two 128-row tiles), segments with fewer entries than a
-    load batch, whole batches and a remainder, more than one orbital chunk;
-    odd and even ns; every block against the oracle."""
+    """Exchange lists whose tiles are fewer than the blocks, or cut strips into
+    ranges (one channel: few strips; ns above two 128-row tiles), segments with
+    fewer entries than a load batch, whole batches and a remainder, more than one
+    orbital chunk; odd and even ns; every block against the oracle."""
     orbs = [(n + 1 + i // 30, k) for i, (n, k) in enumerate(synth.TARGET_ORBITALS * 2)][:norb]
     w = synth._build("strips", 500 + ns, ns, 20.0, 8.0, orbs, [-1, 2, 1][:nch], 1,
                      per_slot * nch * (nch + 1), 1.0, breit=True)
