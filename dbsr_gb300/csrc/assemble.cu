@@ -1417,12 +1417,15 @@ int assemble_windows(dbsrg_ctx *c, int nlists, const dbsrg_list *lists, int nwin
 // potential and digit operand the lists read, and every contraction and
 // scatter are captured from the contraction stream (the table streams join
 // through the events of prepare_list).  A replay repeats all of that from
-// the orbitals in the context's orbital buffer.
+// the orbitals in the context's orbital buffer.  Products of the orbitals that
+// other calls cached beside the graph's own (lists it does not hold, another
+// precision form, the orthogonality) are dropped when a replay brings new ones.
 struct GraphState {
   std::vector<ListPlan> plans;
   std::vector<void *> mem;
   cudaGraphExec_t exec = nullptr;
   long long launches = 0;
+  std::set<const void *> built;  // the orbital products that a replay rebuilds
 };
 
 void graph_drop(dbsrg_ctx *c) {
@@ -1526,6 +1529,7 @@ int graph_capture(dbsrg_ctx *c, int nlists, const dbsrg_list *lists) {
     return fail(rc);
   }
   g->launches = c->launches - l0;
+  g->built = orbital_products(c);
   c->launches = l0;
   restore();
   c->graph = g;
@@ -1536,6 +1540,7 @@ int graph_launch(dbsrg_ctx *c, const double *pq) {
   GraphState *g = c->graph;
   if (!g) return set_err(c, DBSRG_ESTATE, "no captured assembly");
   if (pq) {
+    drop_orbital_products(c, g->built);
     int rc = copy_in(c, c->pq, pq, sizeof(double) * 2 * (size_t)c->g.ns * c->nbf);
     if (rc) return rc;
   }

@@ -252,8 +252,6 @@ void free_tables(dbsrg_ctx *c) {
     cache_free(c, p);
   for (double *p : c->stab)
     cache_free(c, p);
-  for (auto *v : {&c->quad, &c->quadb})
-    for (double *p : *v) cache_free(c, p);
   for (double *p : c->rbtab)
     cache_free(c, p);
   for (double *p : c->sbtab)
@@ -269,8 +267,6 @@ void free_tables(dbsrg_ctx *c) {
   free_orbital_products(c);
   c->rtab.clear();
   c->stab.clear();
-  c->quad.clear();
-  c->quadb.clear();
   c->rcell.clear();
   c->rshare.clear();
   c->scell.clear();
@@ -536,15 +532,11 @@ int dbsrg_set_orbitals(dbsrg_ctx *c, int nbf, const double *pq, const int *ipbs)
   if (!c || nbf < 1 || !pq || !ipbs) return set_err(c, DBSRG_EINVAL, "bad orbital arguments");
   cudaSetDevice(c->device);
   SETTLE(c);
-  graph_drop(c);
+  free_orbital_products(c);
   if (c->pq) cudaFree(c->pq);
   if (c->ipbs) cudaFree(c->ipbs);
   c->pq = nullptr;
   c->ipbs = nullptr;
-  for (auto *v : {&c->quad, &c->quadb}) {
-    for (double *p : *v) cache_free(c, p);
-    v->clear();
-  }
   size_t n = (size_t)2 * c->g.ns * nbf;
   DBSRG_TRY(c, cudaMalloc((void **)&c->pq, n * sizeof(double)));
   DBSRG_TRY(c, cudaMalloc((void **)&c->ipbs, nbf * sizeof(int)));
@@ -559,7 +551,6 @@ int dbsrg_set_orbitals(dbsrg_ctx *c, int nbf, const double *pq, const int *ipbs)
   rc = copy_in(c, c->ipbs, c->h_ipbs.data(), nbf * sizeof(int));
   if (rc) return rc;
   // dense numbering of the bound orbitals (ipbs = 0) for the factored path
-  free_orbital_products(c);
   if (c->bmap) cudaFree(c->bmap);
   if (c->b2o) cudaFree(c->b2o);
   c->bmap = nullptr;

@@ -1273,29 +1273,74 @@ static int get_pairpot_band(dbsrg_ctx *c, int family, int type, int k, int cs,
   return DBSRG_OK;
 }
 
+std::set<const void *> orbital_products(const dbsrg_ctx *c) {
+  std::set<const void *> v;
+  for (const auto &kv : c->rfarw) v.insert({kv.second.W, kv.second.D});
+  for (const auto &kv : c->sfar) v.insert({kv.second.U, kv.second.Ud});
+  for (const auto &kv : c->ppot) v.insert(kv.second);
+  for (const auto *q : {&c->quad, &c->quadb}) v.insert(q->begin(), q->end());
+  v.insert({c->brows, c->vch});
+  v.erase(nullptr);
+  return v;
+}
+
+void drop_orbital_products(dbsrg_ctx *c, const std::set<const void *> &keep) {
+  const std::set<const void *> all = orbital_products(c);
+  if (std::includes(keep.begin(), keep.end(), all.begin(), all.end())) return;
+  cudaStreamSynchronize(c->stream);
+  auto kept = [&](const void *p) { return keep.count(p) != 0; };
+  for (auto it = c->rfarw.begin(); it != c->rfarw.end();) {
+    RFar &r = it->second;
+    const bool w = kept(r.W), d = w && kept(r.D);
+    // the types' views go with the vectors, their digits with the digits
+    for (auto f = c->rfar.begin(); f != c->rfar.end();) {
+      if (f->second.sh == &r && !d) f->second.Ud = nullptr, f->second.eu = nullptr;
+      f = f->second.sh == &r && !w ? c->rfar.erase(f) : std::next(f);
+    }
+    if (!d) {
+      cache_free(c, r.D);
+      r.D = nullptr;
+      r.e = nullptr;
+    }
+    if (!w) cache_free(c, r.W);
+    it = w ? std::next(it) : c->rfarw.erase(it);
+  }
+  for (auto it = c->sfar.begin(); it != c->sfar.end();) {
+    FarField &f = it->second;
+    const bool u = kept(f.U);
+    if (!u || !kept(f.Ud)) {
+      cache_free(c, f.Ud);
+      f.Ud = nullptr;
+      f.eu = nullptr;
+    }
+    if (!u) cache_free(c, f.U);
+    it = u ? std::next(it) : c->sfar.erase(it);
+  }
+  for (auto it = c->ppot.begin(); it != c->ppot.end();) {
+    const bool k = kept(it->second);
+    if (!k) cache_free(c, it->second);
+    it = k ? std::next(it) : c->ppot.erase(it);
+  }
+  for (auto *q : {&c->quad, &c->quadb})
+    for (double *&p : *q)
+      if (!kept(p)) {
+        cache_free(c, p);
+        p = nullptr;
+      }
+  if (!kept(c->brows)) {
+    cache_free(c, c->brows);
+    c->brows = nullptr;
+    c->browsf = nullptr;
+  }
+  if (!kept(c->vch)) {
+    cache_free(c, c->vch);
+    c->vch = nullptr;
+  }
+}
+
 void free_orbital_products(dbsrg_ctx *c) {
   graph_drop(c);
-  if (!c->rfarw.empty() || !c->sfar.empty() || !c->ppot.empty() || c->brows || c->vch)
-    cudaStreamSynchronize(c->stream);
-  for (auto &kv : c->rfarw) {
-    cache_free(c, kv.second.W);
-    cache_free(c, kv.second.D);
-  }
-  for (auto &kv : c->sfar) {
-    cache_free(c, kv.second.U);
-    cache_free(c, kv.second.Ud);
-  }
-  c->rfarw.clear();
-  c->rfar.clear();
-  c->sfar.clear();
-  for (auto &kv : c->ppot)
-    cache_free(c, kv.second);
-  c->ppot.clear();
-  cache_free(c, c->brows);
-  c->brows = nullptr;
-  c->browsf = nullptr;
-  cache_free(c, c->vch);
-  c->vch = nullptr;
+  drop_orbital_products(c, {});
 }
 
 int factored_contract(dbsrg_ctx *c, const FactorJob &j) {

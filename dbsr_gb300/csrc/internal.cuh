@@ -17,6 +17,7 @@
 #include <cstdint>
 #include <functional>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -355,8 +356,12 @@ int ensure_pscratch(dbsrg_ctx *c, int which, size_t bytes);
 // orbital set; *built set when they were made now
 int ensure_bound_rows(dbsrg_ctx *c, bool *built);
 int ensure_pinned(dbsrg_ctx *c, size_t bytes);
-// frees the far-field vectors, pair potentials and bound rows (they depend
-// on the orbitals and the tables)
+// what is cached of the orbitals (and the tables): far-field vectors and their
+// digits, pair potentials, asymptotic coefficients, bound rows, overlap vectors;
+// the buffers of all of them, those outside keep back to the pool (the entries
+// forgotten), and all of them with the captured graph
+std::set<const void *> orbital_products(const dbsrg_ctx *c);
+void drop_orbital_products(dbsrg_ctx *c, const std::set<const void *> &keep);
 void free_orbital_products(dbsrg_ctx *c);
 // the cached tables and orbital products back to the pool (capi.cu)
 void free_tables(dbsrg_ctx *c);

@@ -223,7 +223,8 @@ int dbsrg_assemble_streamed_host(dbsrg_ctx *ctx, int nlists,
  * the orbitals' count and ipbs unchanged; NULL: the orbitals held) into
  * the context: every table and orbital product is rebuilt and the matrix
  * assembled anew, equal to what dbsrg_set_orbitals and dbsrg_gen_matrix
- * would give.  A replay repeats the capture's precision, tuning and
+ * would give.  What other calls cached from the orbitals held before (lists
+ * outside the graph, orthogonality) is dropped then and rebuilt on use.  A replay repeats the capture's precision, tuning and
  * matrix parts.  The whole matrix must be allocated (no window).  The
  * graph is dropped by dbsrg_graph_release and by every call that frees
  * or replaces memory it names: dbsrg_set_orbitals, dbsrg_alloc_matrix*,

@@ -117,3 +117,46 @@ def test_graph_needs_the_whole_matrix():
     with pytest.raises(DbsrgError, match="ESTATE"):
         a.graph_capture(items(w))
     a.close()
+
+
+@pytest.mark.parametrize("captured_in", [FACTOR_FP64, SPLIT_BF16])
+@pytest.mark.parametrize("eager_in", [FACTOR_FP64, SPLIT_BF16])
+def test_replay_with_new_orbitals_leaves_no_product_of_the_old_ones(captured_in, eager_in):
+    """A graph of some lists only: what the other calls cached from the orbitals
+    held before a replay (overlap vectors, pair potentials, far-field vectors and
+    their digits, asymptotic coefficients) is not used after it.  The eager lists
+    and the orthogonality projection before and after a replay with new orbitals
+    equal those of a context that never held the old ones, and the graph still
+    replays."""
+    w = synth.structures_case()
+    m = synth.small(ns=50, nch=w.nch, mk=w.mk, n_entries=400, breit=True, seed=63, norb=4)
+    lists = items(w) + items(m)
+    captured = [it for it in lists if it[:2] == (2, 4) and it[2] == 1]
+    assert captured
+    assert {(0, 3), (2, 1), (2, 2), (2, 3), (2, 4), (3, 6), (3, 8)} <= {it[:2] for it in lists}
+    io = np.zeros((w.nbf, w.nch), dtype=np.int32, order="F")
+    io[: w.nbound, :] = 1
+
+    def others(a):
+        a.zero_matrix()
+        a.set_precision(eager_in)
+        for it in lists:
+            a.gen_matrix(*it)
+        a.orth_channels(io)
+        return (a.get_matrix(), a.get_acf()) + a.get_perturbers()
+
+    pq2 = perturbed(w.pq, 9)
+    fresh = make(w, captured_in, pq2, structures=True)
+    ref2 = others(fresh)
+    fresh.close()
+    a = make(w, captured_in, structures=True)
+    a.graph_capture(captured)
+    first = (a.get_matrix(), a.get_acf())
+    old = others(a)
+    assert not np.array_equal(old[0], ref2[0])
+    a.graph_launch(pq2)
+    assert same(others(a), ref2)
+    a.graph_launch(w.pq)
+    assert same((a.get_matrix(), a.get_acf()), first)
+    assert same(others(a), old)
+    a.close()
