@@ -441,18 +441,16 @@ __global__ void k_pair_cellsum(int ns, int kk, int nb, const PairCellArgs g) {
   }
 }
 
-// (2) exclusive suffix (sum over later cells) or prefix sums per pair, in place
-// (as float-float pairs in the split form): eight pairs a block, each with
-// sixteen runs of cells (blockIdx.y: twice the table, odd ones its second array,
-// prefix sums).  Bound by
-// the FP64 instructions, so the pairs are spread over many blocks: ns 300, 30
-// orbitals, split form 23 us with 32 pairs a block.
+// (2) exclusive suffix (sum over later cells) or prefix sums per pair, in place:
+// eight pairs a block, each with sixteen runs of cells (blockIdx.y: twice the
+// table, odd ones its second array, prefix sums).  Bound by the FP64
+// instructions, so the pairs are spread over many blocks: an R^k list's four
+// tables at ns 300, 30 orbitals 16.5 us.
 constexpr int PSW = 16, PSP = 8;
 struct PairScanArgs {
   int np[4], suffix0[4];
   double *S[4][2];
 };
-template <bool FF>
 __global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, const PairScanArgs g) {
   __shared__ double tot[PSW][PSP];
   const int lane = threadIdx.x % PSP, w = threadIdx.x / PSP, q = blockIdx.x * PSP + lane;
@@ -485,11 +483,7 @@ __global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, const PairScanA
     for (int u = 0; u < 8; u++) {
       const int i = i0 + u;
       if (i >= hi) break;
-      double *x = s + (size_t)(suf ? hi - 1 - (i - lo) : i) * np;
-      if constexpr (FF)
-        *reinterpret_cast<float2 *>(x) = ffa::split(acc);
-      else
-        *x = acc;
+      s[(size_t)(suf ? hi - 1 - (i - lo) : i) * np] = acc;
       acc += v[u];
     }
   }
@@ -505,7 +499,11 @@ __global__ void __launch_bounds__(PSP * PSW) k_pair_scan(int nv, const PairScanA
 //   Kd_ab = sum_x P1_a(x) H_b(x) + SA_ab sum_cv L1 + SB_ab sum_cv L2,
 //   H_b(x) = sum_y W(x,y) P2_b(y),
 // with SA/SB the scanned sums beyond the window (L1 = lo1, SA after the window;
-// case 2: L1 = hi2, SA before it and the sum over cv' after).  Per pair an
+// case 2: L1 = hi2, SA before it and the sum over cv' after).  Those two terms are
+// FP64 in both forms: their factors, sums of r^k and of r^-(k+1), need its
+// exponents (first cell of a grid to 1e-4, k = 11: 1e45 and less than 1e-45),
+// their products do not.  As float-float pairs they took 72 us a list at ns 283
+// and 96 at ns 400, 20 orbitals (81 and 109 in FP64), and gave NaN there.  Per pair an
 // output takes up to 17 + 2 multiply-adds; contracting every diagonal cell by
 // itself and adding the separable terms cell by cell takes up to 81 + 18.
 // A block forms PDX consecutive f (a full sector of the result) of one dl
@@ -523,8 +521,8 @@ struct PairDirTable {
   const double *rkd;  // element (po, pd; cell) at rpo po + rpd pd + rcell cell
   size_t rcell;
   int rpo, rpd;
-  const double *L1, *L2, *M1, *M2;
-  const typename Val<FF>::T *P1, *P2, *SA, *SB;
+  const double *L1, *L2, *M1, *M2, *SA, *SB;
+  const typename Val<FF>::T *P1, *P2;
   typename Val<FF>::T *K;
 };
 template <bool FF>
@@ -555,8 +553,7 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
   T *H = W + PDX * PDW * PDW;              // [PDX][PDW][bw]
   T *p2w = H + PDX * PDW * bw;             // [PDR][bw]
   T *p1w = p2w + PDR * bw;                 // [PDR][pstr]
-  __shared__ double c1[PDX][KM], c2[PDX][KM];
-  __shared__ T t1[PDX], t2[PDX];
+  __shared__ double c1[PDX][KM], c2[PDX][KM], t1[PDX], t2[PDX];
   __shared__ int los[PDX], his[PDX], pos[PDX][KM];
   const size_t per = g.per;
   const int ns = g.ns, nb = g.nb, kk = g.kk, pstr = pair_row_stride(nb);
@@ -593,8 +590,8 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
       if (!p.suf) c1[fl][k] = r1;
       r1 += l1[k];
     }
-    t1[fl] = V::of(s1);
-    t2[fl] = V::of(s2s);
+    t1[fl] = s1;
+    t2[fl] = s2s;
     los[fl] = lo;
     his[fl] = hi;
   }
@@ -663,6 +660,7 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
     if (f > ns) continue;
     const int lo = los[fl], hi = his[fl], b0 = zb + 2 * g;
     V s0, s1;
+    double far0 = 0.0, far1 = 0.0;
     if (lo <= hi) {
       const T *pa = p1w + (lo - rb) * pstr + a, *h = H + fl * PDW * bw + 2 * g;
       const int nt = hi - lo + ed.k1;
@@ -675,11 +673,11 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
       const size_t ra = (size_t)((p.suf ? hi : lo) - 1) * p.np, rl = (size_t)(lo - 1) * p.np;
       const int q0 = pair_number(nb, p.symab, p.symab ? min(a, b0) : a, b0);
       const int q1 = pair_number(nb, p.symab, a, min(b0 + 1, nb - 1));
-      s0.mac(t1[fl], p.SA[ra + q0]);
-      s1.mac(t1[fl], p.SA[ra + q1]);
+      far0 = t1[fl] * p.SA[ra + q0];
+      far1 = t1[fl] * p.SA[ra + q1];
       if (p.SB) {
-        s0.mac(t2[fl], p.SB[rl + q0]);
-        s1.mac(t2[fl], p.SB[rl + q1]);
+        far0 = fma(t2[fl], p.SB[rl + q0], far0);
+        far1 = fma(t2[fl], p.SB[rl + q1], far1);
       }
     }
     const size_t o = (size_t)(f - 1) + (size_t)ns * col;
@@ -687,8 +685,8 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
       p.K[((size_t)a * nb + b) * per + o] = v;
       if (p.symab && a < b) p.K[((size_t)b * nb + a) * per + o] = v;
     };
-    if (!p.symab || a <= b0) put(b0, s0.get());
-    if (b0 + 1 < nb) put(b0 + 1, s1.get());
+    if (!p.symab || a <= b0) put(b0, V::of(far0 + s0.value()));
+    if (b0 + 1 < nb) put(b0 + 1, V::of(far1 + s1.value()));
   }
 }
 
@@ -1140,8 +1138,8 @@ int get_pairpots_direct(dbsrg_ctx *c, int n, const PairPotKey *want, bool ff, co
       t.M2 = ca.M2[i];
       t.P1 = rows + (size_t)(w.jp1 - 1) * nb * ns;
       t.P2 = rows + (size_t)(w.jp2 - 1) * nb * ns;
-      t.SA = (const T *)ca.S1[i];
-      t.SB = (const T *)ca.S2[i];
+      t.SA = ca.S1[i];
+      t.SB = ca.S2[i];
       t.K = (T *)K[i];
       // executed work: an output's n = k - |dl| cells hold r = n + k - 1 functions
       // and a banded matrix of r^2 - n (n - 1) elements: as many multiply-adds per
@@ -1161,7 +1159,7 @@ int get_pairpots_direct(dbsrg_ctx *c, int n, const PairPotKey *want, bool ff, co
     DBSRG_RUN(c, "k_pair_cellsum",
               k_pair_cellsum<<<dim3(nv, m), 256, sm1, st>>>(ns, kk, nb, ca));
     DBSRG_RUN(c, "k_pair_scan",
-              k_pair_scan<F><<<dim3((unsigned)((npmax + PSP - 1) / PSP), 2 * m), PSP * PSW, 0,
+              k_pair_scan<<<dim3((unsigned)((npmax + PSP - 1) / PSP), 2 * m), PSP * PSW, 0,
                                st>>>(nv, sa));
     const dim3 gd((unsigned)((ns + PDX - 1) / PDX), (unsigned)(ncol * m),
                   (unsigned)((nb + PDB - 1) / PDB));

@@ -245,3 +245,42 @@ def test_long_exchange_lists_in_entry_pairs():
     h, _ = run(w, SPLIT_BF16, [L])
     ref, _ = oracle(w, [L])
     check(h, ref, 1e-10)
+
+
+@pytest.mark.parametrize("precision,tol", [(FACTOR_FP64, 1e-12), (SPLIT_BF16, 1e-10)])
+@pytest.mark.parametrize("norb,route", [(4, "k_scatter_dp"), (60, "k_seg_apply")])
+def test_direct_lists_at_high_multipoles_near_the_nucleus(precision, tol, norb, route):
+    """Direct lists at k = 10 and 11 (S^k up to mk + 1) on a grid whose first cell
+    ends at 1e-4, with functions there in every orbital: the moments r^-(k+1) of
+    its cells are beyond 3.4e38 and the r^k below 1e-38, their products ordinary
+    numbers.  By pairs and by segment, structures 6, 7, 16 and 17; every block
+    against the oracle."""
+    orbs = [(n + 1 + i // 30, k) for i, (n, k) in enumerate(synth.TARGET_ORBITALS * 2)][:norb]
+    w = synth._build("high", 821, 60, 20.0, 8.0, orbs, [-1, 2, 1], 1, 400, 1.0, breit=True)
+    w.t = np.concatenate([np.zeros(9), np.geomspace(1e-4, 20.0, 52), np.full(8, 20.0)])
+    rng = np.random.default_rng(822)
+    w.pq[:] = 0.0
+    w.pq[:59, 0, : w.nbound] = rng.uniform(-1, 1, (59, w.nbound))
+    w.pq[:60, 1, : w.nbound] = rng.uniform(-1, 1, (60, w.nbound))
+    w.mk = 10
+    lists = []
+    for L in w.lists:
+        if (L.icase, L.itype) == (2, 3):
+            lists.append(synth.CList(2, 3, 10, L.k1, L.k2, L.k3, L.k4, L.c))
+        elif L.icase == 3 and L.itype in (6, 16):
+            for it in (L.itype, L.itype + 1):
+                lists.append(synth.CList(3, it, 11 - L.kpol % 2, L.k1, L.k2, L.k3, L.k4, L.c))
+    assert {L.kpol for L in lists if L.icase == 3} == {10, 11}
+    a = Assembler(w.t, w.ks, w.ksp, w.ksq)
+    a.set_orbitals(w.pq, w.ipbs)
+    a.alloc_matrix(w.nch, w.icc, w.iicc, w.mk)
+    a.set_precision(precision)
+    a.timing(True)
+    for L in lists:
+        a.gen_matrix(L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
+    assert route in a.timing_report()
+    h = a.get_matrix()
+    a.close()
+    assert np.isfinite(h).all()
+    ref, _ = oracle(w, lists)
+    check(h, ref, tol)
