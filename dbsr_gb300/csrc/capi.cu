@@ -101,10 +101,15 @@ int raise_smem_limit(dbsrg_ctx *c, const void *fn, size_t bytes) {
   static std::mutex mu;
   static std::map<std::pair<int, const void *>, size_t> limit;
   std::lock_guard<std::mutex> lk(mu);
-  size_t &cur = limit[{c->device, fn}];
-  if (bytes <= cur || bytes <= 48 * 1024) return DBSRG_OK;
+  auto it = limit.find({c->device, fn});
+  if (it == limit.end()) {  // without a call: 48 KB together with the static arrays
+    cudaFuncAttributes at;
+    DBSRG_TRY(c, cudaFuncGetAttributes(&at, fn));
+    it = limit.emplace(std::make_pair(c->device, fn), 48 * 1024 - at.sharedSizeBytes).first;
+  }
+  if (bytes <= it->second) return DBSRG_OK;
   DBSRG_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  cur = bytes;
+  it->second = bytes;
   return DBSRG_OK;
 }
 

@@ -284,3 +284,26 @@ def test_direct_lists_at_high_multipoles_near_the_nucleus(precision, tol, norb, 
     assert np.isfinite(h).all()
     ref, _ = oracle(w, lists)
     check(h, ref, tol)
+
+
+def test_direct_pair_potentials_of_a_hundred_orbitals():
+    """Direct lists by pairs at 100 bound orbitals (as many segments as take that
+    route): the kernel's dynamic shared memory is just below 48 KB, its static
+    arrays take it above, so the limit has to be raised; every block against the
+    oracle."""
+    orbs = [(n + 1 + i // 30, k) for i, (n, k) in enumerate(synth.TARGET_ORBITALS * 4)][:100]
+    w = synth._build("hundred", 831, 60, 20.0, 8.0, orbs, [-1] * 20, 0, 8 * 210, 1.0, breit=False)
+    L = next(L for L in w.lists if (L.icase, L.itype, L.kpol) == (2, 3, 0))
+    assert len(set(L.k1)) > 192
+    ref, _ = oracle(w, [L])
+    for precision, tol in ((FACTOR_FP64, 1e-12), (SPLIT_BF16, 1e-10)):
+        a = Assembler(w.t, w.ks, w.ksp, w.ksq)
+        a.set_orbitals(w.pq, w.ipbs)
+        a.alloc_matrix(w.nch, w.icc, w.iicc, w.mk)
+        a.set_precision(precision)
+        a.timing(True)
+        a.gen_matrix(L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
+        assert "k_pair_direct" in a.timing_report()
+        h = a.get_matrix()
+        a.close()
+        check(h, ref, tol)
