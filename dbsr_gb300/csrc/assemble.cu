@@ -638,9 +638,9 @@ __global__ void k_update_hx(int ms, int ich, int jch, const double *d, double cc
 int get_vch(dbsrg_ctx *c, const double **out) {
   if (!c->vch) {
     const int ns = c->g.ns;
-    double *v = (double *)cache_alloc(c, sizeof(double) * 2 * (size_t)ns * c->nbf);
+    CacheBuffer buf(c, sizeof(double) * 2 * (size_t)ns * c->nbf);
+    double *v = (double *)buf.p;
     if (!v) return set_err(c, DBSRG_ENOMEM, "overlap vectors allocation failed");
-    c->vch = v;
     for (int b0 = 0; b0 < c->nbf; b0 += 65535) {  // grid y limit
       const dim3 gv((unsigned)((ns + 31) / 32), (unsigned)std::min(65535, c->nbf - b0), 2);
       DBSRG_RUN(c, "k_vch",
@@ -648,6 +648,8 @@ int get_vch(dbsrg_ctx *c, const double **out) {
                                                       c->pq + (size_t)2 * ns * b0,
                                                       v + (size_t)2 * ns * b0));
     }
+    buf.keep();
+    c->vch = v;
   }
   *out = c->vch;
   return DBSRG_OK;

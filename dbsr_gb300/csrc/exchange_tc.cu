@@ -1068,16 +1068,17 @@ int split_exchange(dbsrg_ctx *c, const SplitExchange &x) {
     const size_t dn = (size_t)nbk * TS * sl, en = (size_t)nbk * NR * EXP_PER_ROWTILE;
     void *d = f->sh ? f->sh->D : nullptr;
     if (!d) {
-      if (!(d = cache_alloc(c, nvec * (dn * sizeof(__nv_bfloat16) + en * sizeof(int)))))
-        return set_err(c, DBSRG_ENOMEM, "digit allocation failed");
+      CacheBuffer buf(c, nvec * (dn * sizeof(__nv_bfloat16) + en * sizeof(int)));
+      if (!(d = buf.p)) return set_err(c, DBSRG_ENOMEM, "digit allocation failed");
       int *e = (int *)((__nv_bfloat16 *)d + nvec * dn);
+      DBSRG_RUN(c, "k_udigits",
+                k_udigits<<<dim3((unsigned)(NR * 32 / 32), (unsigned)nbk, (unsigned)nvec), 32, 0,
+                            st>>>(ns, nb, NR, f->sh ? f->sh->W : f->U, (__nv_bfloat16 *)d, e));
+      buf.keep();
       if (f->sh) {
         f->sh->D = d;
         f->sh->e = e;
       }
-      DBSRG_RUN(c, "k_udigits",
-                k_udigits<<<dim3((unsigned)(NR * 32 / 32), (unsigned)nbk, (unsigned)nvec), 32, 0,
-                            st>>>(ns, nb, NR, f->sh ? f->sh->W : f->U, (__nv_bfloat16 *)d, e));
     }
     f->Ud = (__nv_bfloat16 *)d + (size_t)f->first * dn;
     f->eu = (f->sh ? f->sh->e : (int *)((__nv_bfloat16 *)d + nvec * dn)) + (size_t)f->first * en;

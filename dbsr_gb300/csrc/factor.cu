@@ -915,13 +915,12 @@ static int ensure_rfar(dbsrg_ctx *c, int k, RFar **out) {
   RFar &r = c->rfarw[k];
   if (!r.W) {
     const size_t m = (size_t)c->g.ns * c->nbound;
-    double *W = (double *)cache_alloc(c, 8 * m * sizeof(double));
+    CacheBuffer buf(c, 8 * m * sizeof(double));
+    double *W = (double *)buf.p;
     if (!W) return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
     const int rc = r_far_vectors(c, k, c->nbound, c->b2o, W, (float2 *)(W + 4 * m));
-    if (rc) {
-      cache_free(c, W);
-      return rc;
-    }
+    if (rc) return rc;
+    buf.keep();
     r.W = W;
     r.Wf = (float2 *)(W + 4 * m);
   }
@@ -972,7 +971,8 @@ static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const
     const CellData *cd;
     if ((rc = get_celldata(c, family, type, k, &cd)) || (rc = moment_sums(c, family, type, k)))
       return rc;
-    double *base = (double *)cache_alloc(c, 3 * m * sizeof(double));
+    CacheBuffer buf(c, 3 * m * sizeof(double));
+    double *base = (double *)buf.p;
     if (!base) return set_err(c, DBSRG_ENOMEM, "far-field allocation failed");
     f.U = base;
     f.V = base + m;
@@ -985,6 +985,7 @@ static int get_farfield(dbsrg_ctx *c, int family, int type, int k, int cs, const
     const FarSide s2{0, o2f, cc2, cd->thi2, nullptr, f.V, nullptr, f.Vf, nullptr};
     DBSRG_RUN(c, "k_far_vectors",
               k_far_vectors<<<gv, 64, 0, c->stream>>>(ns, g.ks, nb, c->b2o, c->pq, s1, s2));
+    buf.keep();
   }
   v[idx] = f;
   *out = &v.at(idx);
@@ -996,12 +997,16 @@ static int ensure_brows(dbsrg_ctx *c) {
   if (c->brows) return DBSRG_OK;
   const int ns = c->g.ns, nb = c->nbound;
   const size_t m = (size_t)ns * nb;
-  if (!(c->brows = (double *)cache_alloc(c, 4 * m * sizeof(double))))
-    return set_err(c, DBSRG_ENOMEM, "bound-orbital rows allocation failed");
-  c->browsf = (float2 *)(c->brows + 2 * m);
+  CacheBuffer buf(c, 4 * m * sizeof(double));
+  double *rows = (double *)buf.p;
+  if (!rows) return set_err(c, DBSRG_ENOMEM, "bound-orbital rows allocation failed");
+  float2 *rowsf = (float2 *)(rows + 2 * m);
   DBSRG_RUN(c, "k_bound_rows",
             k_bound_rows<<<dim3((unsigned)((m + 255) / 256), 2), 256, 0, c->stream>>>(
-                ns, nb, c->b2o, c->pq, c->brows, c->browsf));
+                ns, nb, c->b2o, c->pq, rows, rowsf));
+  buf.keep();
+  c->brows = rows;
+  c->browsf = rowsf;
   return DBSRG_OK;
 }
 

@@ -341,6 +341,17 @@ int ensure_lstate(dbsrg_ctx *c, int par, size_t bytes);
 // cache buffers through the pool (nullptr when the device is out of memory)
 void *cache_alloc(dbsrg_ctx *c, size_t bytes);
 void cache_free(dbsrg_ctx *c, void *p);
+// a cache buffer of a build, given back unless kept: what a cache holds is
+// entered there once its launches are made, so a build that fails leaves nothing
+// that the next call would take for built
+struct CacheBuffer {
+  dbsrg_ctx *c;
+  void *p;
+  CacheBuffer(dbsrg_ctx *ctx, size_t bytes) : c(ctx), p(cache_alloc(ctx, bytes)) {}
+  CacheBuffer(const CacheBuffer &) = delete;
+  ~CacheBuffer() { cache_free(c, p); }
+  void keep() { p = nullptr; }
+};
 void pool_trim(dbsrg_ctx *c);
 int copy_out(dbsrg_ctx *c, void *dst, const void *src, size_t n);
 // scratch arenas (device)

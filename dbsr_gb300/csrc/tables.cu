@@ -691,9 +691,9 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
   const TableBases tb = table_bases(g, family, type);
   const size_t f = (size_t)npairs(tb.e1) * npairs(tb.e2) * nv;
   const size_t ts1 = (size_t)g.ns * (2 * g.ks - 1);  // sums of one moment array
-  double *base = nullptr;
-  if (!(base = (double *)cache_alloc(c, (2 * m + 2 * f + 2 * ts1) * sizeof(double))))
-    return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
+  CacheBuffer buf(c, (2 * m + 2 * f + 2 * ts1) * sizeof(double));
+  double *base = (double *)buf.p;
+  if (!base) return set_err(c, DBSRG_ENOMEM, "cell data allocation failed");
   CellData cd;
   cd.lo1 = base;
   cd.hi2 = base + m;
@@ -701,12 +701,13 @@ int get_celldata(dbsrg_ctx *c, int family, int type, int k, const CellData **out
   cd.rkf = (float2 *)(cd.rkd + f);
   const int wh[2] = {2, type == 0 ? 2 : 3}, kp[2] = {k, -(k + 1)};
   double *const mo[2] = {cd.lo1, cd.hi2};
-  if ((rc = compute_moment_set(c, 2, wh, kp, mo))) return rc;
   TriSet ts{};
   ts.type[0] = type == 0 ? 4 : 5;
   ts.rkd[0] = cd.rkd;
   ts.rkf[0] = cd.rkf;
-  if ((rc = compute_diag_set(c, 1, ts, k))) return rc;
+  if ((rc = compute_moment_set(c, 2, wh, kp, mo)) || (rc = compute_diag_set(c, 1, ts, k)))
+    return rc;
+  buf.keep();
   v[idx] = cd;
   *out = &v[idx];
   return DBSRG_OK;
@@ -762,11 +763,14 @@ int ensure_r_cells(dbsrg_ctx *c, int k) {
   return DBSRG_OK;
 }
 
-// the sums of table (family, type, k)'s moments, R^k those of all types of the k
+// the sums of table (family, type, k)'s moments, R^k those of all types of the k;
+// entered in the cell data (which marks them as built) once they are launched
 int moment_sums(dbsrg_ctx *c, int family, int type, int k) {
   const DeviceGrid &g = c->g;
   TotalSet ts{};
   int n;
+  const size_t per = (size_t)g.ns * (family == 0 ? g.ks : 2 * g.ks - 1);
+  double *T;
   auto set = [&](int i, const PairSpec &e, const double *M, double *T) {
     ts.k1[i] = e.k1;
     ts.k2[i] = e.k2;
@@ -778,8 +782,27 @@ int moment_sums(dbsrg_ctx *c, int family, int type, int k) {
     CellData *cd = &c->rcell[(size_t)k * 4];
     if (cd[0].tlo1) return DBSRG_OK;
     n = 4;
-    const size_t per = (size_t)g.ns * g.ks;
-    double *T = c->rshare[k].mom + 4 * (size_t)g.ks * g.ks * g.nv;
+    T = c->rshare[k].mom + 4 * (size_t)g.ks * g.ks * g.nv;
+    for (int b = 0; b < 2; b++) {  // electron 1 of types 0 and 1: the P and Q pairs
+      const PairSpec e = table_bases(g, 0, b).e1;
+      set(2 * b, e, cd[b].lo1, T + 2 * b * per);
+      set(2 * b + 1, e, cd[b].hi1, T + (2 * b + 1) * per);
+    }
+  } else {
+    CellData &cd = c->scell[(size_t)k * 2 + type];
+    if (cd.tlo1) return DBSRG_OK;
+    n = 2;
+    const TableBases tb = table_bases(g, 1, type);
+    T = (double *)(cd.rkf + (size_t)npairs(tb.e1) * npairs(tb.e2) * g.nv);
+    set(0, tb.e1, cd.lo1, T);
+    set(1, tb.e2, cd.hi2, T + per);
+  }
+  if (c->stream != c->bstream[0] && c->stream != c->bstream[1]) c->stream_built = true;
+  DBSRG_RUN(c, "k_moment_sums",
+            k_moment_sums<<<dim3((unsigned)((per + 127) / 128), n), 128, 0, c->stream>>>(
+                g.ns, g.ks, g.nv, ts));
+  if (family == 0) {
+    CellData *cd = &c->rcell[(size_t)k * 4];
     for (int t = 0; t < 4; t++) {
       const bool pa = t == 0 || t == 2, pb = t == 0 || t == 3;
       cd[t].tlo1 = T + (pa ? 0 : 2 * per);
@@ -787,25 +810,11 @@ int moment_sums(dbsrg_ctx *c, int family, int type, int k) {
       cd[t].tlo2 = T + (pb ? 0 : 2 * per);
       cd[t].thi2 = cd[t].tlo2 + per;
     }
-    for (int b = 0; b < 2; b++) {  // electron 1 of types 0 and 1: the P and Q pairs
-      const PairSpec e = table_bases(g, 0, b).e1;
-      set(2 * b, e, cd[b].lo1, cd[b].tlo1);
-      set(2 * b + 1, e, cd[b].hi1, cd[b].thi1);
-    }
   } else {
     CellData &cd = c->scell[(size_t)k * 2 + type];
-    if (cd.tlo1) return DBSRG_OK;
-    n = 2;
-    const TableBases tb = table_bases(g, 1, type);
-    cd.tlo1 = (double *)(cd.rkf + (size_t)npairs(tb.e1) * npairs(tb.e2) * g.nv);
-    cd.thi2 = cd.tlo1 + (size_t)g.ns * (2 * g.ks - 1);
-    set(0, tb.e1, cd.lo1, cd.tlo1);
-    set(1, tb.e2, cd.hi2, cd.thi2);
+    cd.tlo1 = T;
+    cd.thi2 = T + per;
   }
-  if (c->stream != c->bstream[0] && c->stream != c->bstream[1]) c->stream_built = true;
-  const int m = g.ns * (family == 0 ? g.ks : 2 * g.ks - 1);
-  DBSRG_RUN(c, "k_moment_sums", k_moment_sums<<<dim3((m + 127) / 128, n), 128, 0, c->stream>>>(
-                                    g.ns, g.ks, g.nv, ts));
   return DBSRG_OK;
 }
 
@@ -882,16 +891,13 @@ static int get_table_any(dbsrg_ctx *c, int family, int type, int k, int band,
   const CellData *cd;
   int rc = get_celldata(c, family, type, k, &cd);
   if (rc) return rc;
-  double *tab = nullptr;
-  if (!(tab = (double *)cache_alloc(c, nt * sizeof(double))))
-    return set_err(c, DBSRG_ENOMEM, "table allocation failed");
+  CacheBuffer buf(c, nt * sizeof(double));
+  double *tab = (double *)buf.p;
+  if (!tab) return set_err(c, DBSRG_ENOMEM, "table allocation failed");
   if (family == 0) {
     if ((rc = fill_r(c, 1, &type, k, &tab, band))) return rc;
   } else {
-    if ((rc = moment_sums(c, 1, type, k))) {
-      cache_free(c, tab);
-      return rc;
-    }
+    if ((rc = moment_sums(c, 1, type, k))) return rc;
     const unsigned nb = (unsigned)((nt + 255) / 256);
     int kj1 = type == 0 ? g.ksp : g.ksq, kj2 = type == 0 ? g.ksq : g.ksp;
     DBSRG_RUN(c, "k_fill_s",
@@ -899,6 +905,7 @@ static int get_table_any(dbsrg_ctx *c, int family, int type, int k, int band,
                                                   cd->hi2, cd->tlo1, cd->thi2, cd->rkd, tab,
                                                   band));
   }
+  buf.keep();
   v[idx] = tab;
   *out = tab;
   return DBSRG_OK;
@@ -953,25 +960,19 @@ int get_quad(dbsrg_ctx *c, int k, bool bound, const double **out) {
   const size_t m = (size_t)g.ns * n, nq = (size_t)2 * n * n;
   int rc;
   const double *W;
-  double *q;
-  if (bound) {
-    if ((rc = get_rfar(c, k, &W))) return rc;
-    q = (double *)cache_alloc(c, nq * sizeof(double));
-  } else {
-    q = (double *)cache_alloc(c, (nq + 4 * m) * sizeof(double));
-  }
+  if (bound && (rc = get_rfar(c, k, &W))) return rc;
+  CacheBuffer buf(c, (nq + (bound ? 0 : 4 * m)) * sizeof(double));
+  double *q = (double *)buf.p;
   if (!q) return set_err(c, DBSRG_ENOMEM, "quad allocation failed");
   if (!bound) {
-    if ((rc = far_vectors_all(c, k, q + nq))) {
-      cache_free(c, q);
-      return rc;
-    }
+    if ((rc = far_vectors_all(c, k, q + nq))) return rc;
     W = q + nq;
   }
-  v[k] = q;
   DBSRG_RUN(c, "k_quad_dot",
             k_quad_dot<<<dim3((unsigned)(((size_t)n * n + 7) / 8), 2), 256, 0, c->stream>>>(
                 n, g.ns, c->pq, (size_t)2 * g.ns, bound ? c->b2o : nullptr, W, 2 * m, q));
+  buf.keep();
+  v[k] = q;
   *out = q;
   return DBSRG_OK;
 }

@@ -1,0 +1,71 @@
+"""Failure paths of the host code, with the library's objects linked to a CUDA
+runtime that needs no GPU (tests/fake): a launch that fails, memory that runs out."""
+import numpy as np
+import pytest
+
+from dbsr_gb300 import SPLIT_BF16, Assembler, _lib, synth
+from dbsr_gb300._lib import DbsrgError
+
+from fake import library
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return library(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture
+def fake(lib, monkeypatch):
+    monkeypatch.setattr(_lib, "_lib", lib)
+    lib.fake_limit(2**63)
+    lib.fake_fail(None)
+    lib.fake_clear_log()
+    return lib
+
+
+def context(w):
+    a = Assembler(w.t, w.ks, w.ksp, w.ksq, tuning=None)
+    a.set_orbitals(w.pq, w.ipbs)
+    a.alloc_matrix(w.nch, w.icc, w.iicc, w.mk)
+    a.set_precision(SPLIT_BF16)
+    return a
+
+
+def all_bound(w):
+    io = np.zeros((w.nbf, w.nch), dtype=np.int32, order="F")
+    io[: w.nbound, :] = 1
+    return io
+
+
+CALLS = {
+    "k_moment_sums R": lambda a, w: a.get_table(0, 2, 1),
+    "k_moment_sums S": lambda a, w: a.get_table(1, 1, 1),
+    "k_fill_r": lambda a, w: a.get_table(0, 2, 1),
+    "k_fill_s": lambda a, w: a.get_table(1, 1, 1),
+    "k_triang": lambda a, w: a.get_table(1, 0, 1),
+    "k_vch": lambda a, w: a.orth_channels(all_bound(w)),
+    "k_bound_rows": lambda a, w: a.backward([1], [1], [1], [2], [2], [1.0]),
+}
+
+
+@pytest.mark.parametrize("case", CALLS)
+def test_a_failed_launch_leaves_nothing_that_reads_as_built(fake, case):
+    """A build whose launch fails: the call reports it, what it was to fill is not
+    taken for filled by the next call, and its memory comes back."""
+    kernel, call = case.split()[0], CALLS[case]
+    w = synth.small(ns=40, nch=2, mk=1, n_entries=20, breit=False, seed=3)
+    a = context(w)
+    call(a, w)  # the scratch of such a call
+    a.release_tables()
+    used = fake.fake_used()
+    fake.fake_fail(kernel.encode())
+    with pytest.raises(DbsrgError, match="ECUDA"):
+        call(a, w)
+    fake.fake_fail(None)
+    fake.fake_clear_log()
+    call(a, w)
+    assert kernel in fake.fake_log().decode()
+    a.release_tables()
+    assert fake.fake_used() == used
+    a.close()
+    assert fake.fake_used() == 0
