@@ -1548,6 +1548,7 @@ int graph_launch(dbsrg_ctx *c, const double *pq) {
   }
   DBSRG_TRY(c, cudaGraphLaunch(g->exec, c->stream));
   c->launches += g->launches;
+  c->stream_built = true;
   if (c->async) {
     c->pending = true;
     return DBSRG_OK;

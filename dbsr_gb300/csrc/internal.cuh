@@ -182,7 +182,8 @@ struct dbsrg_ctx {
   // list after a state change, the timing mode), both table streams first
   // wait for it (sready).  A pair-potential build made on the contraction
   // stream itself sets stream_built, with the same effect at the next
-  // preparation, since it shares pscratch[0].  The bound-orbital rows
+  // preparation, since it shares pscratch[0]; so do moment sums built there and
+  // a graph replay, which rebuilds there all that its graph holds.  The bound-orbital rows
   // (shared by every k) are made on the contraction stream before the first
   // preparation that needs them.
   cudaStream_t bstream[2] = {nullptr, nullptr};

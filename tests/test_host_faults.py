@@ -69,3 +69,29 @@ def test_a_failed_launch_leaves_nothing_that_reads_as_built(fake, case):
     assert fake.fake_used() == used
     a.close()
     assert fake.fake_used() == 0
+
+
+def test_builds_after_a_queued_replay_wait_for_it(fake):
+    """Asynchronous mode: a replay rewrites the tables and orbital products of its
+    graph on the contraction stream, so what a later list builds from them on a
+    table stream is queued behind it."""
+    w = synth.structures_case()
+    a = context(w)
+    a.alloc_perturbers(w.npert, w.icb, w.ibb)
+    a.set_targets(w.ntarg, w.iptar, w.iitar, 1)
+    lists = {L.kpol: (L.icase, L.itype, L.kpol, L.k1, L.k2, L.k3, L.k4, L.c)
+             for L in w.lists if (L.icase, L.itype) == (2, 1)}
+    a.set_async(True)
+    a.graph_capture([lists[0]])
+    a.graph_launch(w.pq)
+    fake.fake_clear_log()
+    a.graph_launch(w.pq)
+    a.gen_matrix(*lists[2])
+    log = [x.split() for x in fake.fake_log().decode().splitlines()]
+    main = next(x[1] for x in log if x[0] == "graph")
+    log = log[[x[0] for x in log].index("graph") + 1:]
+    build = next(i for i, x in enumerate(log) if x[0] == "launch" and "k_pair" in x[2])
+    assert log[build][1] != main
+    after = {x[2] for x in log[:build] if x[:2] == ["record", main]}
+    assert any(x[0] == "wait" and x[1] == log[build][1] and x[2] in after for x in log[:build])
+    a.close()
