@@ -287,10 +287,7 @@ extern "C" int dbsrg_channel_basis(dbsrg_ctx *c, const double *sol, const int *n
   const double *D = sol;
   double *dD = nullptr, *dWt = nullptr;
   if (!is_device_ptr(sol)) {
-    if (cudaMalloc(&dD, blk * nch * 8)) {
-      cudaGetLastError();
-      return set_err(c, DBSRG_ENOMEM, "channel_basis: allocation failed");
-    }
+    if ((rc = device_alloc(c, (void **)&dD, blk * nch * 8))) return rc;
     if ((rc = copy_in(c, dD, sol, blk * nch * 8))) {
       cudaFree(dD);
       return rc;
@@ -305,10 +302,9 @@ extern "C" int dbsrg_channel_basis(dbsrg_ctx *c, const double *sol, const int *n
     if (out) return copy_out(c, out, c->hch, blk * c->iicc * 8);
     return DBSRG_OK;
   }
-  if (cudaMalloc(&dWt, blk * 8)) {
-    cudaGetLastError();
+  if ((rc = device_alloc(c, (void **)&dWt, blk * 8))) {
     if (dD) cudaFree(dD);
-    return set_err(c, DBSRG_ENOMEM, "channel_basis: allocation failed");
+    return rc;
   }
   const double one = 1.0, zero = 0.0;
   int bad = 0;

@@ -139,8 +139,10 @@ int grow_buffer(dbsrg_ctx *c, void **p, size_t *have, size_t bytes) {
   cudaError_t e = cudaMalloc(p, want);
   if (e != cudaSuccess) {
     cudaGetLastError();
+    pool_trim(c);
     e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
+      cudaGetLastError();
       *p = nullptr;
       return cuda_check(c, e, "scratch allocation");
     }
@@ -208,6 +210,35 @@ void pool_trim(dbsrg_ctx *c) {
   c->pool.clear();
   for (void *p : c->retired) cudaFree(p);
   c->retired.clear();
+}
+
+void scratch_release(dbsrg_ctx *c) {
+  pool_trim(c);
+  for (cudaStream_t s : {c->sstream, c->bstream[0], c->bstream[1], c->stream})
+    if (s) cudaStreamSynchronize(s);
+  auto release = [](void *&p, size_t &bytes) {
+    if (p) cudaFree(p);
+    p = nullptr;
+    bytes = 0;
+  };
+  release(c->scratch, c->scratch_bytes);
+  release(c->scratch2, c->scratch2_bytes);
+  release(c->tscratch, c->tscratch_bytes);
+  release(c->fscratch, c->fscratch_bytes);
+  release(c->tcscratch, c->tcscratch_bytes);
+  for (int i = 0; i < 2; i++) release(c->pscratch[i], c->pscratch_bytes[i]);
+  for (int i = 0; i < dbsrg_ctx::NLSTATE; i++) release(c->lstate[i], c->lstate_bytes[i]);
+}
+
+int device_alloc(dbsrg_ctx *c, void **p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return DBSRG_OK;
+  cudaGetLastError();
+  scratch_release(c);
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return DBSRG_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return cuda_check(c, e, "allocation");
 }
 
 int ensure_lstate(dbsrg_ctx *c, int par, size_t bytes) {
@@ -411,7 +442,7 @@ int dbsrg_release_tables(dbsrg_ctx *c) {
   SETTLE(c);
   DBSRG_TRY(c, cudaStreamSynchronize(c->stream));
   free_tables(c);
-  pool_trim(c);
+  scratch_release(c);
   return DBSRG_OK;
 }
 
@@ -615,12 +646,14 @@ int dbsrg_alloc_matrix_window(dbsrg_ctx *c, int nch, const int *icc, int iicc, i
   for (int v : c->h_icc)
     if (v < 0 || v > iicc) return set_err(c, DBSRG_ERANGE, "icc entry out of range");
   const size_t ms = c->g.ms;
-  DBSRG_TRY(c, cudaMalloc((void **)&c->icc, sizeof(int) * (size_t)nch * nch));
-  DBSRG_TRY(c, cudaMalloc((void **)&c->hmem, sizeof(double) * ms * ms * nwin));
+  int rc;
+  if ((rc = device_alloc(c, (void **)&c->icc, sizeof(int) * (size_t)nch * nch)) ||
+      (rc = device_alloc(c, (void **)&c->hmem, sizeof(double) * ms * ms * nwin)))
+    return rc;
   c->hch = c->hmem;
   c->hcap = nwin;
-  DBSRG_TRY(c, cudaMalloc((void **)&c->acf, sizeof(double) * (size_t)iicc * (mk + 1)));
-  int rc = copy_in(c, c->icc, c->h_icc.data(), sizeof(int) * (size_t)nch * nch);
+  if ((rc = device_alloc(c, (void **)&c->acf, sizeof(double) * (size_t)iicc * (mk + 1)))) return rc;
+  rc = copy_in(c, c->icc, c->h_icc.data(), sizeof(int) * (size_t)nch * nch);
   if (rc) return rc;
   c->nch = nch;
   c->iicc = iicc;

@@ -354,6 +354,11 @@ struct CacheBuffer {
   void keep() { p = nullptr; }
 };
 void pool_trim(dbsrg_ctx *c);
+// the pool and every scratch buffer back to the device, and device memory that may
+// take them where there is no other (between lists only: what a list under way
+// holds in the scratch is lost)
+void scratch_release(dbsrg_ctx *c);
+int device_alloc(dbsrg_ctx *c, void **p, size_t bytes);
 int copy_out(dbsrg_ctx *c, void *dst, const void *src, size_t n);
 // scratch arenas (device)
 // grows a scratch buffer to at least bytes; the old one is retired, not

@@ -158,10 +158,9 @@ extern "C" int dbsrg_record_matrix(dbsrg_ctx *c, const double *sol, const int *n
   // the solutions on the device, once, for the perturber rows
   const double *D = sol;
   if (!is_device_ptr(sol)) {
-    if (cudaMalloc(&dD, blk * nch * 8)) {
-      cudaGetLastError();
+    if ((rc = device_alloc(c, (void **)&dD, blk * nch * 8))) {
       cleanup();
-      return set_err(c, DBSRG_ENOMEM, "record_matrix: allocation failed");
+      return rc;
     }
     if ((rc = copy_in(c, dD, sol, blk * nch * 8))) {
       cleanup();

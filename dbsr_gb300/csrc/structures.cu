@@ -1068,7 +1068,7 @@ int dbsrg_alloc_perturbers(dbsrg_ctx *c, int npert, const int *icb, int iicb, co
   for (int v : b)
     if (v < 0 || v > iibb) return set_err(c, DBSRG_ERANGE, "ibb entry out of range");
   const size_t ms = c->g.ms;
-  DBSRG_TRY(c, cudaMalloc((void **)&c->hcp, sizeof(double) * ms * std::max(iicb, 1)));
+  if ((rc = device_alloc(c, (void **)&c->hcp, sizeof(double) * ms * std::max(iicb, 1)))) return rc;
   DBSRG_TRY(c, cudaMalloc((void **)&c->hp, sizeof(double) * std::max(iibb, 1)));
   c->npert = npert;
   c->iicb = iicb;
@@ -1152,7 +1152,7 @@ int dbsrg_set_dhl(dbsrg_ctx *c, int nkap, const int *kap_list, const double *hd,
   int rc;
   if ((rc = fetch(c, kl, kap_list, nkap)) || (rc = fetch(c, kb, kbs, c->nbf))) return rc;
   const size_t bytes = sizeof(double) * c->g.ms * c->g.ms * nkap;
-  DBSRG_TRY(c, cudaMalloc((void **)&c->hd, bytes));
+  if ((rc = device_alloc(c, (void **)&c->hd, bytes))) return rc;
   if ((rc = copy_in(c, c->hd, hd, bytes))) return rc;
   DBSRG_TRY(c, cudaStreamSynchronize(c->stream));
   c->nkap = nkap;

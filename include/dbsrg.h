@@ -224,14 +224,15 @@ int dbsrg_assemble_streamed_host(dbsrg_ctx *ctx, int nlists,
  * the context: every table and orbital product is rebuilt and the matrix
  * assembled anew, equal to what dbsrg_set_orbitals and dbsrg_gen_matrix
  * would give.  What other calls cached from the orbitals held before (lists
- * outside the graph, orthogonality) is dropped then and rebuilt on use.  A replay repeats the capture's precision, tuning and
- * matrix parts.  The whole matrix must be allocated (no window).  The
- * graph is dropped by dbsrg_graph_release and by every call that frees
- * or replaces memory it names: dbsrg_set_orbitals, dbsrg_alloc_matrix*,
- * dbsrg_alloc_perturbers, dbsrg_set_targets, dbsrg_set_dhl,
- * dbsrg_invalidate_tables, dbsrg_release_tables, dbsrg_destroy; after
- * that dbsrg_graph_launch returns DBSRG_ESTATE.  No counterpart in
- * DBSR_MAT3, which builds each matrix once. */
+ * outside the graph, orthogonality) is dropped then and rebuilt on use.
+ * A replay repeats the capture's precision, tuning and matrix parts.  The
+ * whole matrix must be allocated (no window).  The graph is dropped by
+ * dbsrg_graph_release and by every call that frees or replaces memory it
+ * names: dbsrg_set_orbitals, dbsrg_alloc_matrix*, dbsrg_alloc_perturbers,
+ * dbsrg_set_targets, dbsrg_set_dhl, dbsrg_invalidate_tables,
+ * dbsrg_release_tables, dbsrg_destroy; after that dbsrg_graph_launch
+ * returns DBSRG_ESTATE.  No counterpart in DBSR_MAT3, which builds each
+ * matrix once. */
 int dbsrg_graph_capture(dbsrg_ctx *ctx, int nlists, const dbsrg_list *lists);
 int dbsrg_graph_launch(dbsrg_ctx *ctx, const double *pq);
 int dbsrg_graph_release(dbsrg_ctx *ctx);
@@ -509,7 +510,8 @@ int dbsrg_get_diag_cells(dbsrg_ctx *ctx, int type, int k, double *out);
 int dbsrg_get_grid_array(dbsrg_ctx *ctx, const char *name, double *out);
 
 /* Free the cached R^k/S^k tables and everything derived from them (cell
- * data, far fields, pair potentials), returning the memory to the device
+ * data, far fields, pair potentials) and the context's scratch buffers,
+ * returning the memory to the device
  * (the reference keeps its tables for the whole run,
  * dbsr_lib_dbs.f90:1595-1624). */
 int dbsrg_release_tables(dbsrg_ctx *ctx);

@@ -95,3 +95,56 @@ def test_builds_after_a_queued_replay_wait_for_it(fake):
     after = {x[2] for x in log[:build] if x[:2] == ["record", main]}
     assert any(x[0] == "wait" and x[1] == log[build][1] and x[2] in after for x in log[:build])
     a.close()
+
+
+def blocks(nch, pairs):
+    """icc of the diagonal blocks (none) and of the given channel pairs."""
+    icc = np.zeros((nch, nch), dtype=np.int32, order="F")
+    for b, (i, j) in enumerate(pairs):
+        icc[i, j] = icc[j, i] = b + 1
+    return icc, len(pairs)
+
+
+def basis_context(ns, nch, pairs):
+    w = synth.small(ns=40, nch=2, mk=1, n_entries=20, breit=False, seed=3)
+    t = np.concatenate([np.zeros(8), np.linspace(0.0, 10.0, ns - 7), np.full(8, 10.0)])
+    a = Assembler(t, w.ks, w.ksp, w.ksq, tuning=None)
+    icc, iicc = blocks(nch, pairs)
+    a.alloc_matrix(nch, icc, iicc, 0)
+    a.set_precision(SPLIT_BF16)
+    sol = np.zeros((2 * ns, 2 * ns, nch), order="F")
+    return a, sol, np.full(nch, 2 * ns, dtype=np.int32)
+
+
+def test_channel_basis_takes_fewer_blocks_at_once_when_memory_is_short(fake):
+    """The workspace follows the free memory: with room for a few blocks beside the
+    channels' digits the call works through them a few at a time, and releasing the
+    tables gives back what it kept."""
+    pairs = [(i, j) for i in range(8) for j in range(i)]
+    a, sol, nsol = basis_context(40, 8, pairs)
+    a.channel_basis(sol, nsol)
+    whole = fake.fake_log().decode().count("k_sgemm")
+    a.release_tables()
+    used = fake.fake_used()
+    a.channel_basis(sol, nsol)
+    kept = fake.fake_used() - used
+    a.release_tables()
+    assert fake.fake_used() == used
+    fake.fake_limit(used + sol.nbytes + kept // 3)
+    fake.fake_clear_log()
+    a.channel_basis(sol, nsol)
+    assert fake.fake_log().decode().count("k_sgemm") > whole
+    # a matrix that needs the memory of the workspace kept takes it
+    fake.fake_limit(fake.fake_used() + 1000)
+    icc, iicc = blocks(8, pairs + [(0, 0)])
+    a.alloc_matrix(8, icc, iicc, 0)
+    a.close()
+
+
+def test_a_large_channel_basis_workspace_is_given_back(fake):
+    """A workspace beyond a gigabyte lives for the call only."""
+    a, sol, nsol = basis_context(420, 70, [(i, 0) for i in range(1, 33)])
+    used = fake.fake_used()
+    a.channel_basis(sol, nsol)
+    assert fake.fake_used() == used
+    a.close()
