@@ -86,7 +86,8 @@ __global__ void k_list_entries(int n, const int *ipt, const int *k1, const int *
 // between them, one run of entries per thread and the keys looked up in the list.
 constexpr int SEGKEYS = 4096;
 
-// dscal: [0] number of segments, [1] error (set here or by the entries)
+// dscal: [0] number of segments, [2] a pair without a block, [4] a channel out of
+// range ([1], [3]: k_list_entries)
 __global__ void __launch_bounds__(1024) k_list_segments(int n, const int *__restrict__ k1,
                                                         int nch, int iicc, const int *icc,
                                                         int *seg_start, SegInfo *info,
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(1024) k_list_segments(int n, const int *__rest
     si.partner = -1;
     si.owner = 1;
     if (si.ich < 1 || si.jch < 1 || si.ich > nch || si.jch > nch) {
-      atomicExch(dscal + 1, 1);
+      atomicExch(dscal + 4, 1);
     } else {
       const int b = icc[(si.ich - 1) + (size_t)nch * (si.jch - 1)];
       if (b < 1 || b > iicc)
@@ -780,8 +781,8 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
   P.lcd = (double *)take(dbytes);
   P.lpair = (int *)take(ibytes);  // factored path: bound-orbital pair of each entry
   int *seg_start = (int *)take(sizeof(int) * (size_t)(n + 2));
-  // [0] segments [1] error [2] block error [3] pair error, and behind them the
-  // segment table: read back together
+  // [0] segments [1] entry error [2] block error [3] pair error [4] channel error,
+  // and behind them the segment table: read back together
   constexpr size_t HDR = 64;
   int *dscal = (int *)take(HDR + sizeof(SegInfo) * (size_t)(n + 1));
   P.info = (SegInfo *)((char *)dscal + HDR);
@@ -791,12 +792,6 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
   P.dxq = (XQuad *)take(sizeof(XQuad) * 4 * (size_t)(n + 1));
   P.lcdf = (float2 *)take(sizeof(float2) * (size_t)n);
   P.factored = c->precision != DBSRG_PLAIN_FP64;
-  if (icase != 0 && P.factored) {
-    // the factored contraction works with ordered pairs of bound orbitals
-    if (c->nbound < 1) return set_err(c, DBSRG_ESTATE, "no bound orbitals (ipbs = 0)");
-    if (c->nbound > 128)
-      return set_err(c, DBSRG_EINVAL, "factored contraction: 1..128 bound orbitals (ipbs = 0)");
-  }
   if ((rc = ensure_pinned(c, HDR + sizeof(SegInfo) * 2048))) return rc;
   // lists resident and aligned on this device are read where they are (the
   // read-back below waits for that), others copied in
@@ -880,6 +875,32 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
     return DBSRG_OK;
   }
 
+  // ---- segments: count, errors and the table in one read-back into pinned
+  // memory (of as many segments as there are channel pairs, at most 2048; a
+  // longer table takes a second one)
+  DBSRG_RUN_S(c, ss, "k_list_segments",
+              k_list_segments<<<1, 1024, 0, ss>>>(n, P.lk1, c->nch, c->iicc, c->icc, seg_start,
+                                                  P.info, dscal));
+  const size_t nfirst = std::min<size_t>({(size_t)n, (size_t)c->nch * c->nch, (size_t)2048});
+  DBSRG_TRY(c, cudaMemcpyAsync(c->pinned, dscal, HDR + sizeof(SegInfo) * nfirst,
+                               cudaMemcpyDeviceToHost, ss));
+  DBSRG_TRY(c, cudaStreamSynchronize(ss));
+  int hs[5];
+  std::memcpy(hs, c->pinned, sizeof(hs));
+  if (hs[1] == 3) return set_err(c, DBSRG_EINVAL, "non-finite coefficient in list");
+  if (hs[1]) return set_err(c, DBSRG_ERANGE, "channel or orbital index out of range in list");
+  const int nseg = hs[0];
+  if (nseg < 1 || nseg > n) return set_err(c, DBSRG_ECUDA, "inconsistent segment count");
+  P.nseg = nseg;
+  std::vector<SegInfo> hinfo(nseg);
+  std::memcpy(hinfo.data(), (char *)c->pinned + HDR,
+              sizeof(SegInfo) * std::min<size_t>(nseg, nfirst));
+  if ((size_t)nseg > nfirst) {
+    DBSRG_TRY(c, cudaMemcpyAsync(hinfo.data() + nfirst, P.info + nfirst,
+                                 sizeof(SegInfo) * (nseg - nfirst), cudaMemcpyDeviceToHost, ss));
+    DBSRG_TRY(c, cudaStreamSynchronize(ss));
+  }
+
   // ---- the case: PQ types, storage and convol case
   if (icase == 2) {
     if (itype != 3 && itype != 4) return set_err(c, DBSRG_EINVAL, "R_data: unknown itype");
@@ -942,31 +963,12 @@ int plan_list(dbsrg_ctx *c, int icase, int itype, int kpol, int n, const int *ip
   P.per = (size_t)ns * P.ncol;
   P.split_x = P.factored && P.icv >= 3 && c->precision == DBSRG_SPLIT_BF16;
 
-  // ---- segments: count, errors and the table in one read-back into pinned
-  // memory (of as many segments as there are channel pairs, at most 2048; a
-  // longer table takes a second one)
-  DBSRG_RUN_S(c, ss, "k_list_segments",
-              k_list_segments<<<1, 1024, 0, ss>>>(n, P.lk1, c->nch, c->iicc, c->icc, seg_start,
-                                                  P.info, dscal));
-  const size_t nfirst = std::min<size_t>({(size_t)n, (size_t)c->nch * c->nch, (size_t)2048});
-  DBSRG_TRY(c, cudaMemcpyAsync(c->pinned, dscal, HDR + sizeof(SegInfo) * nfirst,
-                               cudaMemcpyDeviceToHost, ss));
-  DBSRG_TRY(c, cudaStreamSynchronize(ss));
-  int hs[4];
-  std::memcpy(hs, c->pinned, sizeof(hs));
-  if (hs[1] == 3) return set_err(c, DBSRG_EINVAL, "non-finite coefficient in list");
-  if (hs[1]) return set_err(c, DBSRG_ERANGE, "channel or orbital index out of range in list");
-  const int nseg = hs[0];
-  if (nseg < 1 || nseg > n) return set_err(c, DBSRG_ECUDA, "inconsistent segment count");
-  P.nseg = nseg;
-  std::vector<SegInfo> hinfo(nseg);
-  std::memcpy(hinfo.data(), (char *)c->pinned + HDR,
-              sizeof(SegInfo) * std::min<size_t>(nseg, nfirst));
-  if ((size_t)nseg > nfirst) {
-    DBSRG_TRY(c, cudaMemcpyAsync(hinfo.data() + nfirst, P.info + nfirst,
-                                 sizeof(SegInfo) * (nseg - nfirst), cudaMemcpyDeviceToHost, ss));
-    DBSRG_TRY(c, cudaStreamSynchronize(ss));
-  }
+  // the errors of the segments, which come after those of the entries and of the
+  // call's arguments
+  if (P.factored && c->nbound < 1) return set_err(c, DBSRG_ESTATE, "no bound orbitals (ipbs = 0)");
+  if (P.factored && c->nbound > 128)
+    return set_err(c, DBSRG_EINVAL, "factored contraction: 1..128 bound orbitals (ipbs = 0)");
+  if (hs[4]) return set_err(c, DBSRG_ERANGE, "channel or orbital index out of range in list");
   if (hs[2]) return set_err(c, DBSRG_ERANGE, "channel pair has no block in icc");
   if (hs[3]) return set_err(c, DBSRG_EINVAL, "factored contraction: K2/K3 must be bound orbitals");
   for (int s = 0; s < nseg; s++) {

@@ -69,3 +69,48 @@ def test_injected_wait_timeout_is_reported_and_the_context_recovers():
     a.set_wait_limit(2_000_000_000)
     assert np.array_equal(assemble(a, w), ref)
     a.close()
+
+
+@pytest.mark.parametrize("precision", [FACTOR_FP64, SPLIT_BF16])
+def test_a_list_with_two_faults_reports_the_first_checked(precision):
+    """Entries (coefficients, orbitals) are checked first, then the call's
+    arguments and the bound orbitals there are, then the channels."""
+    w = synth.small(ns=50, nch=3, mk=2, n_entries=200, breit=True, seed=103)
+    L = next(L for L in w.lists if (L.icase, L.itype) == (2, 3))
+    S = next(L for L in w.lists if (L.icase, L.itype) == (3, 6))
+
+    def refused(a, code, M, k1=None, k2=None, c=None, itype=None, kpol=None):
+        with pytest.raises(DbsrgError, match=code):
+            a.gen_matrix(M.icase, M.itype if itype is None else itype,
+                         M.kpol if kpol is None else kpol, M.k1 if k1 is None else k1,
+                         M.k2 if k2 is None else k2, M.k3, M.k4, M.c if c is None else c)
+
+    def last(x, v):
+        x = x.copy()
+        x[-1] = v
+        return x
+
+    a = fresh(w, precision)
+    ref = assemble(a, w)
+    for M in (L, S):
+        channel = last(M.k1, 77 * 2**15 + 78)
+        orbital = last(M.k2, 0)
+        refused(a, "ERANGE", M, k1=channel)
+        refused(a, "EINVAL", M, k1=channel, c=last(M.c, np.nan))
+        refused(a, "ERANGE", M, k2=orbital, itype=39)
+        refused(a, "EINVAL", M, k1=channel, itype=39)
+        refused(a, "ERANGE", M, k1=channel, kpol=w.mk + 2)
+    assert np.array_equal(a.get_matrix(), ref)
+    a.set_orbitals(w.pq, np.ones_like(w.ipbs))  # no bound orbitals
+    refused(a, "ESTATE", L, k1=last(L.k1, 77 * 2**15 + 78))
+    refused(a, "ERANGE", L, k2=last(L.k2, 0))
+    a.close()
+    pq = np.zeros((w.ns, 2, 129), order="F")
+    pq[:, :, : w.nbf] = w.pq
+    b = Assembler(w.t, w.ks, w.ksp, w.ksq)
+    b.set_orbitals(pq, np.zeros(129, np.int32))
+    b.alloc_matrix(w.nch, w.icc, w.iicc, w.mk)
+    b.set_precision(precision)
+    refused(b, "EINVAL", L, k1=last(L.k1, 77 * 2**15 + 78))
+    refused(b, "ERANGE", L, k2=last(L.k2, 0))
+    b.close()
