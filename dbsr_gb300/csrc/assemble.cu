@@ -1126,8 +1126,6 @@ int exec_list(dbsrg_ctx *c, const ListPlan &P, int w, bool prep = false) {
       job.nown = nown;
       job.own = ob;
       job.info = P.info;
-      job.k2 = P.lk2;
-      job.k3 = P.lk3;
       job.pairs = P.lpair;
       job.cd = P.lcd;
       job.cdf = P.lcdf;
@@ -1215,10 +1213,10 @@ int band_contract(dbsrg_ctx *c, int kb, int icase, const double *rkb, int nsg, c
   const unsigned nrt = (unsigned)((per + GBM - 1) / GBM);
   // split of the contracted band columns: four blocks an SM with one segment
   // tile (a block holds 8 warps, and the FP64 pipe wants 16 or more).  It
-  // depends on the table's shape only: a segment's sum has the same order
+  // depends on the table's shape (and the device) only: a segment's sum has the same order
   // whatever segments share the launch, so windows and chunks of a list give
   // the same bits.
-  const int want = std::min<int>(kb, (4 * 152 + (int)nrt - 1) / (int)nrt);
+  const int want = std::min<int>(kb, (4 * c->nsm + (int)nrt - 1) / (int)nrt);
   const int cper = (kb + want - 1) / want, nz = (kb + cper - 1) / cper;
   for (int s0 = 0; s0 < nsg;) {
     // segments per tile: the least padding, the wider tile where two pad the

@@ -822,9 +822,10 @@ static std::vector<int> host_windows(int iicc, int nwin, int nslot) {
 // the library: at most tune_windows windows, of at least 2 GB each.  A window
 // costs every list a round of launches (5 to 9 ms at 59 lists), what it hides
 // is the copy of the one before (2 GB: 10 ms on this link), so smaller ones
-// cost more than they hide.  24 channels of ns 351 (1.2 GB): 93 ms with 16
-// windows, 36 with one; 6 GB: 102 with 16, 65-70 with two to six; 16.6 GB: 155
-// with 16, 130 with 8; at 37 GB the 16 windows of the tuning stay.  Two
+// cost more than they hide.  With tune_windows 16, the tuned value for ns near 400
+// (8 where nothing is tuned): 24 channels of ns 351 (1.2 GB) 93 ms in 16 windows,
+// 36 in one; 6 GB 102 in 16, 65-70 in two to six; 16.6 GB 155 in 16, 130 in 8.
+// From 2 GB times tune_windows on (32 GB, or 16) this rule changes nothing.  Two
 // windows have to fit the allocation.
 static int default_window(const dbsrg_ctx *c, int iicc) {
   const int least = std::max(1, (iicc + c->tune_windows - 1) / c->tune_windows);

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(SCL * SCW) k_seg_scan(int nv, int nmp, unsigne
 // 3.9e-14).
 template <bool FF>
 struct ApplyArgs {
-  int ns, nv, ks, kk, nm, nmp, ncol, icv, sym;
+  int ns, nv, ks, kk, nm, nmp, ncol, sym;
   int nwin;   // window rows
   int ntype;  // table types summed into one output
   PairSpec eo[2], ed[2][2];  // per output (blockIdx.z) and type
@@ -455,7 +455,7 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
       p.nwin = std::max(p.nwin, eo.k1 + ed.k1 - 1);
       rmax = std::max(rmax, npairs(eo) * npairs(ed));
       nw = std::max(nw, sym ? (eo.k1 + 1) / 2 : eo.k1);
-          }
+    }
   ca.ns = p.ns = ns;
   ca.nv = p.nv = nv;
   ca.ks = p.ks = ks;
@@ -472,7 +472,6 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
   DBSRG_RUN(c, "k_seg_scan", k_seg_scan<<<dim3((unsigned)(nmp / SCL), (unsigned)nset), SCL * SCW, 0,
                                           st>>>(nv, nmp, sufmask, S));
   p.nm = nm;
-  p.icv = j.icv;
   p.ntype = ntype;
   p.rho = rho;
   p.S = S;

@@ -1176,8 +1176,10 @@ int get_pairpots_direct(dbsrg_ctx *c, int n, const PairPotKey *want, bool ff, co
   const std::integral_constant<int, DBSRG_MAXK> kmax;
   if (ks <= FAR)
     rc = ff ? potentials(std::true_type(), k9) : potentials(std::false_type(), k9);
+  else if (!ff)  // the energy functional; lists of the factored forms end at order 9
+    rc = potentials(std::false_type(), kmax);
   else
-    rc = ff ? potentials(std::true_type(), kmax) : potentials(std::false_type(), kmax);
+    rc = set_err(c, DBSRG_EINVAL, "factored contraction: spline order above 9");
   for (int i = 0; i < m; i++) {
     if (rc)
       cache_free(c, K[i]);

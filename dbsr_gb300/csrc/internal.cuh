@@ -481,7 +481,6 @@ struct FactorJob {
   int nown;          // owner segments of the chunk
   const int *own;    // member slot of each owner
   const SegInfo *info;
-  const int *k2, *k3;
   const int *pairs;  // ordered bound-orbital pair index of every entry
   const double *cd;
   const float2 *cdf;  // split form: the coefficients as float-float pairs
@@ -490,7 +489,7 @@ struct FactorJob {
   bool split;        // exchange on the tensor cores (split BF16), fused scatter
   int nxq;           // split exchange: (owner block, quadrant) records of the chunk
   const struct XQuad *xq;
-  const struct XQuad *hxq;  // host copy of the records (work accounting)
+  const struct XQuad *hxq;  // host copy of the records (tile ranges)
   bool prep;         // build (or find) the cached inputs only, launch no contraction
   long long nent;    // entries of the member segments (executed-work statements)
 };
