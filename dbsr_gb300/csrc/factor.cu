@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
     if (f > ns) continue;
     const int lo = los[fl], hi = his[fl], b0 = zb + 2 * g;
     V s0, s1;
-    double far0 = 0.0, far1 = 0.0;
+    Val<false> far0, far1;
     if (lo <= hi) {
       const T *pa = p1w + (lo - rb) * pstr + a, *h = H + fl * PDW * bw + 2 * g;
       const int nt = hi - lo + ed.k1;
@@ -673,11 +673,16 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
       const size_t ra = (size_t)((p.suf ? hi : lo) - 1) * p.np, rl = (size_t)(lo - 1) * p.np;
       const int q0 = pair_number(nb, p.symab, p.symab ? min(a, b0) : a, b0);
       const int q1 = pair_number(nb, p.symab, a, min(b0 + 1, nb - 1));
-      far0 = t1[fl] * p.SA[ra + q0];
-      far1 = t1[fl] * p.SA[ra + q1];
+      if constexpr (!FF) far0.v = s0.v, far1.v = s1.v;
+      far0.mac(t1[fl], p.SA[ra + q0]);
+      far1.mac(t1[fl], p.SA[ra + q1]);
       if (p.SB) {
-        far0 = fma(t2[fl], p.SB[rl + q0], far0);
-        far1 = fma(t2[fl], p.SB[rl + q1], far1);
+        far0.mac(t2[fl], p.SB[rl + q0]);
+        far1.mac(t2[fl], p.SB[rl + q1]);
+      }
+      if constexpr (FF) {
+        far0.v += s0.value();
+        far1.v += s1.value();
       }
     }
     const size_t o = (size_t)(f - 1) + (size_t)ns * col;
@@ -685,8 +690,8 @@ __global__ void __launch_bounds__(PDT) k_pair_direct(const PairDirArgs<FF> g) {
       p.K[((size_t)a * nb + b) * per + o] = v;
       if (p.symab && a < b) p.K[((size_t)b * nb + a) * per + o] = v;
     };
-    if (!p.symab || a <= b0) put(b0, V::of(far0 + s0.value()));
-    if (b0 + 1 < nb) put(b0 + 1, V::of(far1 + s1.value()));
+    if (!p.symab || a <= b0) put(b0, V::of(far0.v));
+    if (b0 + 1 < nb) put(b0 + 1, V::of(far1.v));
   }
 }
 
