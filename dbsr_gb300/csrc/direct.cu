@@ -504,14 +504,22 @@ int run(dbsrg_ctx *c, const FactorJob &j) {
 // them, counted 1.6 times since its blocks are few (0.7 T/s against the pair
 // potentials' 1.2 where both are long), the cell moments about 40 kd (FP64); a pair
 // potential about 4000 an output for its small matrix, 120 per second orbital and
-// 14 per pair; both ways one an entry and band element.  So pairs up to some 28
-// orbitals, segments above unless a list has many.  Assemblies by pairs and mostly
-// by segment: ns 80, 2 channels 1.41 and 1.63 ms; ns 200, 12 channels 4.56 and 4.92;
-// ns 222, 14 channels in FP64 10.4 and 10.9; ns 283, 32 channels 11.8 and 12.4;
-// ns 400, 80 channels 47.6 and 49.7 (before the tensor-core kernel's ranges).
+// 14 per pair; both ways one an entry and band element.  So pairs up to some 30
+// orbitals, segments above unless a list has many.  The direct lists of a matrix
+// (R^k k = 0..2 and S^k, 11 lists, ns 300, tables rebuilt), ms by pairs and by
+// segment:
+//   orbitals               20         28         36         48         64         88
+//   split, 16 segments  1.71 1.81  2.14 1.80  3.10 1.83  4.13 1.83  5.94 1.82  10.0 1.89
+//          49           1.79 2.28  2.20 2.27  3.22 2.26  4.22 2.29  6.05 2.28  10.0 2.32
+//          121          1.85 3.32  2.23 3.31  3.32 3.33  4.30 3.32  6.18 3.34  10.2 3.35
+//   FP64,  16 segments  2.23 2.28  2.95 2.32  4.18 2.33  5.94 2.30  9.03 2.34  15.5 2.35
+//          121          2.38 5.14  3.08 5.19  4.33 5.24  6.09 5.15  9.15 5.21  15.7 5.14
+// (ns 150 and 400 cross at the same counts, 10 to 100 entries a segment too).  The
+// rule takes segments from 31 orbitals with up to 32 segments, from some 50 with 49
+// and from 70 to 80 with 121, where they are never the slower way.
 // The lists of a one-channel matrix (the SCF potentials) hold one segment each
 // and come once per orbital, so the pair potentials of an iteration serve all
-// of them: 30 orbitals at ns 300 took 76 ms by segment, 66 ms by pairs.
+// of them: 30 orbitals at ns 300 take 29.3 ms by segment, 18.4 by pairs.
 bool direct_by_segment(const dbsrg_ctx *c, int family, int icv, int na, const int *types,
                        long long nseg, long long nent) {
   const DeviceGrid &g = c->g;
